@@ -17,7 +17,7 @@ import shutil
 import subprocess
 
 __all__ = ["FLOORS_PATH", "LIB_PATH", "SOURCES", "TORCH_BINDING_PATH", "build_floors_library",
-           "build_library", "build_torch_binding", "is_stale"]
+           "build_host_module", "build_library", "build_torch_binding", "host_module_path", "is_stale"]
 
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
@@ -135,6 +135,27 @@ def build_floors_library(force: bool = False) -> pathlib.Path:
     return FLOORS_PATH
 
 
+def _compile_against_torch(src: pathlib.Path, target: pathlib.Path, extra: list[str]) -> None:
+    """One host C++ compiler call against the installed torch; replaces ``target`` atomically."""
+    import torch
+    from torch.utils import cpp_extension
+
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        raise RuntimeError(f"no host C++ compiler found: cannot build {target.name}")
+    torch_lib = pathlib.Path(torch.__file__).parent / "lib"
+    tmp = target.with_suffix(f".so.tmp{os.getpid()}")
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", str(src),
+           *[f"-I{p}" for p in cpp_extension.include_paths("cuda")],
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-o", str(tmp), f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+           "-lc10_cuda", *extra, f"-Wl,-rpath,{torch_lib}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"building {target.name} failed:\n{res.stderr[-4000:]}")
+    os.replace(tmp, target)
+
+
 def build_torch_binding(force: bool = False) -> pathlib.Path:
     """Compile ``csrc/torch_binding.cpp`` against the installed torch into
     ``_lib/libmsda_b200_torch.so`` (links ``libmsda_b200.so`` next to it).  Needs a host C++
@@ -145,31 +166,47 @@ def build_torch_binding(force: bool = False) -> pathlib.Path:
             and TORCH_BINDING_PATH.stat().st_mtime > max(src.stat().st_mtime,
                                                          LIB_PATH.stat().st_mtime)):
         return TORCH_BINDING_PATH
-    import torch
-    from torch.utils import cpp_extension
-
-    cxx = shutil.which("g++") or shutil.which("c++")
-    if cxx is None:
-        raise RuntimeError("no host C++ compiler found: cannot build the torch binding")
-    torch_lib = pathlib.Path(torch.__file__).parent / "lib"
-    tmp = TORCH_BINDING_PATH.with_suffix(".so.tmp")
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", str(src),
-           *[f"-I{p}" for p in cpp_extension.include_paths("cuda")],
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-o", str(tmp), f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
-           "-lc10_cuda", f"-L{LIB_DIR}", "-lmsda_b200", "-Wl,-rpath,$ORIGIN",
-           f"-Wl,-rpath,{torch_lib}"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"building the torch binding failed:\n{res.stderr[-4000:]}")
-    os.replace(tmp, TORCH_BINDING_PATH)
+    _compile_against_torch(src, TORCH_BINDING_PATH,
+                           [f"-L{LIB_DIR}", "-lmsda_b200", "-Wl,-rpath,$ORIGIN"])
     return TORCH_BINDING_PATH
+
+
+def host_module_path() -> pathlib.Path:
+    """Where the native call path for the installed torch lies (its ABI is torch's: one file per
+    torch and Python version)."""
+    import sys
+
+    import torch
+
+    return LIB_DIR / f"msda_b200_host-{torch.__version__}-cp{sys.version_info[0]}{sys.version_info[1]}.so"
+
+
+def build_host_module(force: bool = False) -> pathlib.Path:
+    """Compile ``csrc/torch_host.cpp`` (the eager call path, a CPython extension) against the
+    installed torch.  It links nothing of this package: the loader binds the C ABI by address."""
+    import sysconfig
+
+    src = CSRC / "torch_host.cpp"
+    target = host_module_path()
+
+    def fresh() -> bool:
+        return target.exists() and target.stat().st_mtime > max(
+            src.stat().st_mtime, HEADERS[-1].stat().st_mtime)
+
+    if not force and fresh():
+        return target
+    with _build_lock():
+        if force or not fresh():
+            _compile_against_torch(src, target, [f"-I{sysconfig.get_paths()['include']}",
+                                                 "-ltorch_python"])
+    return target
 
 
 if __name__ == "__main__":
     import sys
 
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host_module(force="--force" in sys.argv))
     print(build_floors_library(force="--force" in sys.argv))
     if "--torch-binding" in sys.argv:
         print(build_torch_binding(force="--force" in sys.argv))

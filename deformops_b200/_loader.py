@@ -11,18 +11,23 @@ with :class:`KernelUnavailableError`.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
+import warnings
 
-from ._build import LIB_PATH, build_library, is_stale
+from ._build import (LIB_PATH, build_host_module, build_library, host_module_path, is_stale)
 from .core.errors import KernelBuildError, KernelUnavailableError
 
-__all__ = ["ABI_VERSION", "Shim", "library_path", "load_library", "loaded"]
+__all__ = ["ABI_VERSION", "Shim", "host_module", "library_path", "load_library", "loaded"]
 
 ABI_VERSION = 5
 
 _lock = threading.Lock()
 _shim: "Shim | None" = None
+_host = None
+_host_tried = False
 
 
 def _reset_lock_in_child() -> None:
@@ -129,3 +134,35 @@ def load_library(*, compile: "bool | None" = None) -> Shim:
         except OSError as exc:
             raise KernelUnavailableError(f"cannot load {path}: {exc}") from exc
         return _shim
+
+
+def host_module():
+    """The native eager call path (``csrc/torch_host.cpp``) bound to the loaded library, or
+    ``None`` where it cannot be had: the Python operators serve every call then, slower.
+
+    Built on first use like the library itself, unless ``DEFORMOPS_B200_COMPILE=0``.
+    """
+    global _host, _host_tried
+    if _host_tried:
+        return _host
+    shim = load_library()
+    with _lock:
+        if _host_tried:
+            return _host
+        try:
+            path = host_module_path()
+            if os.environ.get("DEFORMOPS_B200_COMPILE", "1") != "0":
+                path = build_host_module()
+            loader = importlib.machinery.ExtensionFileLoader("msda_b200_host", str(path))
+            spec = importlib.util.spec_from_file_location("msda_b200_host", path, loader=loader)
+            module = importlib.util.module_from_spec(spec)
+            loader.exec_module(module)
+            functions = (shim.forward, shim.backward, shim.forward_offsets, shim.backward_offsets,
+                         shim.scratch_bytes, shim.lib.msda_b200_last_error)
+            module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in functions))
+            _host = module
+        except Exception as exc:  # noqa: BLE001 - the Python operators remain
+            warnings.warn(f"deformops_b200: the native call path is not available ({exc}); "
+                          "calls go through the Python operators", RuntimeWarning, stacklevel=3)
+        _host_tried = True
+        return _host

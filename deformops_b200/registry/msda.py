@@ -20,7 +20,7 @@ import torch
 from torch import Tensor
 
 from .. import ops as _ops
-from .._loader import load_library
+from .._loader import host_module, load_library
 from ..core.errors import NoBackendError
 from ..core.runtime import Method, is_training_from, resolve_method, sm_version_for
 from ..core.sanitize import check_msda_call
@@ -192,6 +192,21 @@ class CudaBackend(MSDABackend):
                        softmax=Method(method) is Method.SOFTMAX)
 
 
+#: what the native path takes as ``method``; anything else is resolved (or refused) in Python
+_SOFTMAX_OF = {"linear": False, "softmax": True}
+
+
+def _native_path(value: Any):
+    """The native call path when this may be an ordinary eager call on a CUDA tensor, else None.
+
+    It takes the call over from the checks to the launch and answers None for everything that
+    is not ordinary after all (see ``csrc/torch_host.cpp``).  Under Dynamo or export the
+    operators below have to appear in the graph."""
+    if torch.compiler.is_compiling() or not isinstance(value, Tensor) or not value.is_cuda:
+        return None
+    return host_module()
+
+
 _CALL_OPTIONS = frozenset({"chunk_step", "num_points", "channels_per_thread", "threads_per_block",
                            "fp32acc"})
 
@@ -246,6 +261,14 @@ class _MSDA:
         rank, size, dtype or device; :class:`NoBackendError` when the kernels cannot take
         the call (the message says why).
         """
+        if not options and (backend is None or backend is Backend.CUDA):
+            native = _native_path(value)
+            use_softmax = bool(softmax) if method is None else _SOFTMAX_OF.get(method)
+            if native is not None and use_softmax is not None:
+                out = native.msda(value, spatial_shapes, level_start_index, sampling_locations,
+                                  attention_weights, use_softmax)
+                if out is not None:
+                    return out
         self._only_cuda(backend)
         context = self.context_of(value, spatial_shapes, level_start_index, sampling_locations,
                                   attention_weights, method=method, softmax=softmax, **options)
@@ -295,6 +318,13 @@ def msda_from_offsets(value: Tensor, spatial_shapes: Tensor, level_start_index: 
     and weights, and to two-coordinate reference points; boxes that require a gradient take
     the unfused route (locations in torch, then :data:`msda`).
     """
+    native = _native_path(value)
+    use_softmax = bool(softmax) if method is None else _SOFTMAX_OF.get(method)
+    if native is not None and use_softmax is not None:
+        out = native.msda_offsets(value, spatial_shapes, level_start_index, reference_points,
+                                  offsets, attention_weights, use_softmax)
+        if out is not None:
+            return out
     resolved = resolve_method(method, softmax=softmax)
     if reference_points.ndim != 4 or reference_points.shape[-1] not in (2, 4):
         raise ValueError("reference points must be (B, Q, L, 2) or (B, Q, L, 4); got "
