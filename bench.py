@@ -295,7 +295,7 @@ class AbiCall:
         self.dims = w.dims
         B, S, G, D, Q, L, K = w.dims
         self.code = DTYPE_CODES[w.value.dtype]
-        self.nscratch = shim.scratch_bytes(B, S, G, D, Q, L, K, self.code)
+        self.nscratch = shim.workspace_bytes(B, S, G, D, Q, L, K, self.code, 0)
         self.scratch = torch.empty(max(self.nscratch, 16), dtype=torch.uint8, device=device)
 
     def buffers(self, w, device):
@@ -319,7 +319,7 @@ class AbiCall:
             raise RuntimeError(self.shim.last_error())
 
     def backward(self, d):
-        # one call = header memset + prepare kernel + backward kernel + finalize kernel
+        # one call = memset of header and tables + count, scatter, walk and finish kernels
         B, S, G, D, Q, L, K = self.dims
         st = self.shim.backward(_p(d["value"]), _p(d["shapes"]), _p(d["starts"]),
                                 _p(d["sampling_locations"]), _p(d["attention_weights"]),
@@ -815,9 +815,9 @@ def main():
             "repeats": {"count": len(repeats_ms), "ms_per_step_median": ms_per_step,
                         "ms_per_step_min": rep_min / args.steps, "ms_per_step_max": rep_max / args.steps},
             "clocks": clock_summary,
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": 5 * args.steps,
             "kernels_ms": {"forward": fwd_ms, "backward_call": bwd_ms, **spread,
-                           "backward_call_launches": "header memset + prepare, backward and finalize kernels"},
+                           "backward_call_launches": "memset + sort_count, sort_scatter, sorted_walk and sorted_finish kernels"},
             "roofline": {"bound": "hbm", "kernel": "msda backward (whole call, grad_value clear included)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": peak_kind, "traffic": traffic,

@@ -46,6 +46,7 @@ class Shim:
     #: every symbol ``include/msda_b200.h`` declares
     SYMBOLS = ("msda_b200_abi_version", "msda_b200_last_error", "msda_b200_forward",
                "msda_b200_backward", "msda_b200_backward_scratch_bytes",
+               "msda_b200_backward_workspace_bytes",
                "msda_b200_forward_offsets", "msda_b200_backward_offsets",
                "msda_b200_backward_static_scratch", "msda_b200_launch_geometry")
 
@@ -69,6 +70,9 @@ class Shim:
         self.scratch_bytes = self.lib.msda_b200_backward_scratch_bytes
         self.scratch_bytes.restype = _i64
         self.scratch_bytes.argtypes = [_i64] * 7 + [_int]
+        self.workspace_bytes = self.lib.msda_b200_backward_workspace_bytes
+        self.workspace_bytes.restype = _i64
+        self.workspace_bytes.argtypes = [_i64] * 7 + [_int, _int]
         self.forward_offsets = self.lib.msda_b200_forward_offsets
         self.forward_offsets.restype = _int
         self.forward_offsets.argtypes = ([_vp] * 4 + [_int, _vp, _int, _vp, _vp] + [_i64] * 7
@@ -158,7 +162,7 @@ def host_module():
             module = importlib.util.module_from_spec(spec)
             loader.exec_module(module)
             functions = (shim.forward, shim.backward, shim.forward_offsets, shim.backward_offsets,
-                         shim.scratch_bytes, shim.lib.msda_b200_last_error)
+                         shim.workspace_bytes, shim.lib.msda_b200_last_error)
             module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in functions))
             _host = module
         except Exception as exc:  # noqa: BLE001 - the Python operators remain

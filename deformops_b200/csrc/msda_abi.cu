@@ -6,6 +6,7 @@
 
 #include "../../include/msda_b200.h"
 #include "msda_common.cuh"
+#include "msda_sorted.cuh"
 
 namespace {
 
@@ -24,6 +25,9 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 int element_size(int dtype) {
     return dtype == MSDA_B200_F64 ? 8 : dtype == MSDA_B200_F32 ? 4 : 2;
 }
+
+// what a sorted backward asks for at most when that holds several samples; more samples take turns
+constexpr int64_t kWorkspaceTarget = 256ll << 20;
 
 constexpr size_t kSmemBudget = 96 * 1024;   // per CTA, so that at least two CTAs share an SM
 
@@ -178,6 +182,22 @@ int64_t msda_b200_backward_scratch_bytes(int64_t B, int64_t S, int64_t G, int64_
     if (B <= 0 || S <= 0 || G <= 0 || D <= 0 || Q <= 0 || L <= 0 || K <= 0) return 0;
     return msda_b200::kScratchHeaderBytes +
            2 * B * (S * G * D + msda_b200::extra_elems_per_sample(Q, G, D, L, K));
+}
+
+int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q,
+                                           int64_t L, int64_t K, int dtype, int apply_softmax) {
+    const int64_t scratch = msda_b200_backward_scratch_bytes(B, S, G, D, Q, L, K, dtype);
+    if (scratch == 0) return 0;
+    msda_b200::Params p{};
+    p.B = B, p.S = S, p.Q = Q;
+    p.G = (int)G, p.D = (int)D, p.L = (int)L, p.K = (int)K;
+    if (!msda_b200::sorting_pays(p, dtype)) return scratch;
+    // all samples at once, or as many as the target holds (at least one)
+    int64_t samples = B;
+    while (samples > 1 && msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples) > kWorkspaceTarget)
+        samples = samples > 8 ? samples - samples / 8 : samples - 1;
+    const int64_t sorted = msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples);
+    return sorted > scratch ? sorted : scratch;
 }
 
 int msda_b200_launch_geometry(int64_t B, int64_t G, int64_t D, int64_t Q, int64_t L, int64_t K,
@@ -376,6 +396,21 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
     DeviceGuard guard(device);
     if (guard.err != cudaSuccess) return cuda_fail(guard.err, "backward: selecting the device");
     cudaError_t e;
+    if (use_scratch && msda_b200::sorting_pays(p, dtype)) {
+        const bool softmax = apply_softmax != 0;
+        const int64_t samples = msda_b200::sorted_samples_per_turn(p, softmax, scratch_bytes);
+        if (samples > 0) {
+            for (int64_t b = 0; b < B; b += samples) {
+                const int64_t n = samples < B - b ? samples : B - b;
+                const msda_b200::Params part = msda_b200::samples_of(p, b, n);
+                msda_b200::SortPlan sp;
+                msda_b200::plan_sorted(sp, part, softmax, n, scratch);
+                e = msda_b200::launch_backward_sorted(part, sp, dtype, softmax, s);
+                if (e != cudaSuccess) return cuda_fail(e, "backward: kernel launch (sorted)");
+            }
+            return MSDA_B200_OK;
+        }
+    }
     if (use_scratch) {
         e = msda_b200::launch_prepare_grad_value(p, dtype, apply_softmax != 0, s);
         if (e != cudaSuccess) return cuda_fail(e, "backward: clearing grad_value / scratch");

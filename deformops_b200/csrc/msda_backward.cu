@@ -313,28 +313,6 @@ __global__ void __launch_bounds__(256, MSDA_BWD_MIN_CTAS) backward_kernel(const 
 }
 
 // ---- scaled float16 image: preparation and finalisation ----------------------------------------
-// largest magnitude pattern among the eight 16-bit elements of a vector
-__device__ __forceinline__ unsigned max_magnitude_bits(const uint4 &v) {
-    const unsigned a = __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu);
-    const unsigned b = __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu);
-    const unsigned m = __vmaxu2(a, b);
-    return max(m & 0xffffu, m >> 16);
-}
-
-// largest magnitude pattern over vectors first, first + stride, ... of `p`: four loads in flight
-__device__ __forceinline__ unsigned scan_max_magnitude(const uint4 *__restrict__ p, int64_t n,
-                                                       int64_t first, int64_t stride) {
-    unsigned m = 0;
-    int64_t v = first;
-    for (; v + 3 * stride < n; v += 4 * stride) {
-        const uint4 a = p[v], b = p[v + stride], c = p[v + 2 * stride], d = p[v + 3 * stride];
-        m = max(max(m, max(max_magnitude_bits(a), max_magnitude_bits(b))),
-                max(max_magnitude_bits(c), max_magnitude_bits(d)));
-    }
-    for (; v < n; v += stride) m = max(m, max_magnitude_bits(p[v]));
-    return m;
-}
-
 // Clears the float16 image the backward kernel adds into and records the largest |grad_out|
 // (and, without softmax, |attn|) element in the scratch header.  The header cells were set to
 // zero on the stream before this kernel.

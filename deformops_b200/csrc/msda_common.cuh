@@ -339,6 +339,28 @@ __device__ __forceinline__ int grad_scale_exponent(const unsigned *header, int64
     return e < -100 ? -100 : (e > 100 ? 100 : e);
 }
 
+// largest magnitude pattern among the eight 16-bit elements of a vector
+__device__ __forceinline__ unsigned max_magnitude_bits(const uint4 &v) {
+    const unsigned a = __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu);
+    const unsigned b = __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu);
+    const unsigned m = __vmaxu2(a, b);
+    return max(m & 0xffffu, m >> 16);
+}
+
+// largest magnitude pattern over vectors first, first + stride, ... of `p`: four loads in flight
+__device__ __forceinline__ unsigned scan_max_magnitude(const uint4 *__restrict__ p, int64_t n,
+                                                       int64_t first, int64_t stride) {
+    unsigned m = 0;
+    int64_t v = first;
+    for (; v + 3 * stride < n; v += 4 * stride) {
+        const uint4 a = p[v], b = p[v + stride], c = p[v + 2 * stride], d = p[v + 3 * stride];
+        m = max(max(m, max(max_magnitude_bits(a), max_magnitude_bits(b))),
+                max(max_magnitude_bits(c), max_magnitude_bits(d)));
+    }
+    for (; v < n; v += stride) m = max(m, max_magnitude_bits(p[v]));
+    return m;
+}
+
 // ---------------------------------------------------------------------------------
 // Level table -> shared memory (read from device memory: no host synchronisation)
 // ---------------------------------------------------------------------------------
@@ -438,11 +460,30 @@ __device__ __forceinline__ PointGeom locate(float x, float y, int H, int W, int 
     return g;
 }
 
+// Location of a predicted offset, in the float32 arithmetic of the torch expressions of the
+// layers it replaces: `ref + offset / (W, H)` and `ref.xy + offset / K * ref.wh * 0.5`.
+__device__ __forceinline__ float2 location_from_offset(const Params &p, float2 off, int64_t bq, int l,
+                                                       float Wf, float Hf) {
+    if (p.ref_coords == 2) {
+        const float2 r = __ldg(reinterpret_cast<const float2 *>(p.ref) + bq * p.L + l);
+        return make_float2(r.x + off.x / Wf, r.y + off.y / Hf);
+    }
+    const float4 r = __ldg(reinterpret_cast<const float4 *>(p.ref) + bq * p.L + l);
+    const float Kf = (float)p.K;
+    return make_float2(r.x + off.x / Kf * r.z * 0.5f, r.y + off.y / Kf * r.w * 0.5f);
+}
+// Derivative of the pixel coordinate with respect to that offset.
+__device__ __forceinline__ float2 offset_derivative(const Params &p, int64_t bq, int l, float Wf, float Hf) {
+    if (p.ref_coords == 2) return make_float2(1.f, 1.f);
+    const float4 r = __ldg(reinterpret_cast<const float4 *>(p.ref) + bq * p.L + l);
+    const float Kf = (float)p.K;
+    // d(location)/d(offset) = wh * 0.5 / K, evaluated as the forward expression at offset 1
+    return make_float2(Wf * (1.f / Kf * r.z * 0.5f), Hf * (1.f / Kf * r.w * 0.5f));
+}
+
 // Sample location of element `e` = (pair, point) of level `l`, and in `dpix` the derivative of
 // the pixel coordinate with respect to what the caller differentiates: the location itself
-// (W, H), or the predicted offset when the call carries reference points.  The offset
-// arithmetic follows the torch expressions of the layers it replaces, in float32:
-// `ref + offset / (W, H)` and `ref.xy + offset / K * ref.wh * 0.5`.
+// (W, H), or the predicted offset when the call carries reference points.
 template <typename T>
 __device__ __forceinline__ float2 sample_location(const Params &p, int64_t e, int64_t pair, int l,
                                                   float Wf, float Hf, float2 &dpix) {
@@ -460,17 +501,10 @@ __device__ __forceinline__ float2 sample_location(const Params &p, int64_t e, in
     } else {
         off = ld_stream_f2(loc2 + e);
     }
-    const int64_t bq = pair / p.G;
-    if (p.ref_coords == 2) {
-        const float2 r = __ldg(reinterpret_cast<const float2 *>(p.ref) + bq * p.L + l);
-        dpix = make_float2(1.f, 1.f);
-        return make_float2(r.x + off.x / Wf, r.y + off.y / Hf);
-    }
-    const float4 r = __ldg(reinterpret_cast<const float4 *>(p.ref) + bq * p.L + l);
-    const float Kf = (float)p.K;
-    // d(location)/d(offset) = wh * 0.5 / K, evaluated as the forward expression at offset 1
-    dpix = make_float2(Wf * (1.f / Kf * r.z * 0.5f), Hf * (1.f / Kf * r.w * 0.5f));
-    return make_float2(r.x + off.x / Kf * r.z * 0.5f, r.y + off.y / Kf * r.w * 0.5f);
+    // (a 64-bit division costs as much as the rest of the point)
+    const int64_t bq = pair <= 0x7fffffffll ? (int64_t)((unsigned)pair / (unsigned)p.G) : pair / p.G;
+    dpix = offset_derivative(p, bq, l, Wf, Hf);
+    return location_from_offset(p, off, bq, l, Wf, Hf);
 }
 
 // softmax statistics of one pair's P logits: (max, 1 / sum of exp(logit - max))

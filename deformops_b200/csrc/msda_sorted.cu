@@ -1,0 +1,1223 @@
+// Backward on sorted points (16-bit values, dense sampling): grad_value as a product on the
+// tensor cores instead of one reduction per bilinear corner.
+//
+// What bounds the direct backward (msda_backward.cu) is each SM's path to L2: four 64-byte
+// reductions per sample point, 16 bytes of payload a clock.  Where a level receives several
+// points per pixel those reductions hit the same few rows over and over.  Here the points of a
+// (sample, head) plane are first sorted by the cell they fall in - a counting sort, two passes
+// over the locations - and a warp then walks the sorted points with the pixels of its cell held
+// on the tensor cores:
+//
+//   cell        one pixel row r0 and kCols = 7 adjacent pixel columns c0 of the top left corner;
+//               all four corners of its points lie in a window of 2 rows x 8 columns = the 16
+//               rows of an m16n8k16 tile
+//   scatter     acc[16 pixels][D] += W[16 pixels][16 points] * grad_out[16 points][D], W holding
+//               the points' corner weights (zero elsewhere), float32 accumulation
+//   dots        dot[16 pixels][8 points] = value[16 pixels][D] * grad_out[8 points][D]^T, of which
+//               a point's four corners are picked out
+//
+// Cells are numbered down a column strip, so the window's lower row is the next cell's upper
+// row: an accumulated pixel row leaves the warp once per strip, as one 16-byte reduction per
+// eight channels, instead of once per corner and point (at 21 504 queries and 12 points per query
+// 33 million rows of reductions become about 1 million).
+//
+// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 435 us
+// against 512 us, of which counting 51, writing records 105, the walk 247, the last pass 22;
+// grad_value 1.7e-3 off the float32 result against 2.2e-3.
+//
+// Accumulation is float32 inside a warp's run of points; the few sums that meet in memory (two
+// strips share a column, two runs share a row) meet in float16, scaled as in the direct backward
+// (msda_common.cuh), in grad_value itself, which the last kernel rewrites in its own type.
+#include "msda_sorted.cuh"
+
+namespace msda_b200 {
+
+namespace {
+
+constexpr int kSortThreads = 512;
+constexpr int kSortPoints = 8;         // points per thread of the sort kernels,
+constexpr int kSortBatch = 4;          // loaded this many at a time
+constexpr int kSharedCells = 8192;     // most cells of a plane that are counted in shared memory
+constexpr int kSortCtaPoints = kSortThreads * kSortPoints;
+
+constexpr int kNextItem = 2;           // header cell: runs of the walk handed out so far
+
+// ---- cells ---------------------------------------------------------------------------------------
+struct CellTable {
+    int first[kMaxLevels + 1];   // first cell of the level; [L]: number of cells
+    int rows[kMaxLevels];        // cells per strip: H + 1 (r0 = -1 .. H - 1); 0: not sorted
+};
+
+// A table whose levels overlap can ask for more cells than there is room for (levels that tile
+// `value` cannot): the levels that do not fit are not sorted, direct_point() serves them.
+__device__ inline void plan_cells(CellTable &c, const LevelTable &t, int L, int bound) {
+    int n = 0;
+    for (int l = 0; l < L; ++l) {
+        const long long cells =
+            t.H[l] > 0 ? (t.H[l] + 1ll) * ((t.W[l] + kCols) / kCols) : 0;   // ceil((W + 1) / kCols)
+        const bool fits = n + cells <= bound;
+        c.first[l] = n;
+        c.rows[l] = fits ? t.H[l] + 1 : 0;
+        if (fits) n += (int)cells;
+    }
+    c.first[L] = n;
+}
+
+// A sort CTA takes the points of a stretch of queries of one (sample, head) plane.  A thread
+// keeps to one point index and steps over queries, so all that depends on the level is in
+// registers, and a warp's loads run over consecutive points.  Heads vary fastest over CTAs (those
+// that read one stretch of locations run side by side), samples slowest: the records being
+// written at a time are one or two samples' and stay in L2 until their sectors are complete.
+struct SortLane {
+    int plane, b, g;
+    int pt, l;              // point of the query and its level
+    int H, W, cell0, rows;  // of the level
+    int ql, nq, step;       // first query of the thread (chunk-relative), queries of the chunk, stride
+    int64_t q0;             // first query of the chunk
+    bool active;
+};
+__device__ __forceinline__ SortLane sort_lane(const Params &p, const SortPlan &sp, const LevelTable &lt,
+                                              const CellTable &ct, unsigned cta) {
+    SortLane s;
+    const unsigned per_sample = (unsigned)sp.chunks * (unsigned)p.G;
+    s.b = (int)(cta / per_sample);
+    const int chunk = (int)((cta - (unsigned)s.b * per_sample) / (unsigned)p.G);
+    s.g = (int)(cta - (unsigned)s.b * per_sample) - chunk * p.G;
+    s.plane = s.b * p.G + s.g;
+    const int P = p.L * p.K;
+    s.step = kSortThreads / P;
+    s.ql = (int)threadIdx.x / P;
+    s.pt = (int)threadIdx.x - s.ql * P;
+    s.l = s.pt / p.K;
+    s.active = s.ql < s.step;
+    s.H = lt.H[s.l];
+    s.W = lt.W[s.l];
+    s.cell0 = ct.first[s.l];
+    s.rows = ct.rows[s.l];
+    s.q0 = (int64_t)chunk * sp.chunk_queries;
+    s.nq = (int)min((int64_t)sp.chunk_queries, p.Q - s.q0);
+    return s;
+}
+
+// Where a point of the thread's level falls; false if it is skipped.  The same float32
+// arithmetic as locate().
+struct PointCell {
+    int cell, col;
+    float fr, fc;
+};
+__device__ __forceinline__ bool find_cell(const SortLane &s, float2 xy, PointCell &o) {
+    const float Wf = (float)s.W, Hf = (float)s.H;
+    const float px = fmaf(xy.x, Wf, -0.5f), py = fmaf(xy.y, Hf, -0.5f);
+    if (!(py >= -1.f && px >= -1.f && py < Hf && px < Wf && s.H > 0)) return false;
+    const float r0f = floorf(py), c0f = floorf(px);
+    o.fr = py - r0f;
+    o.fc = px - c0f;
+    const unsigned c1 = (unsigned)((int)c0f + 1), strip = c1 / kCols;
+    o.col = (int)(c1 - strip * kCols);
+    o.cell = s.cell0 + (int)strip * s.rows + (int)r0f + 1;
+    return true;
+}
+
+// Sample location of the thread's point of query `q` of the chunk: sample_location() without its
+// 64-bit divisions.  `base` is the element index of the same point of the chunk's first query.
+template <typename T, bool REF>
+__device__ __forceinline__ float2 point_xy(const Params &p, const SortLane &s, int64_t base, int q) {
+    const int64_t e = base + (int64_t)(q * (p.G * p.L * p.K));
+    if constexpr (REF) {
+        const float2 off = p.offsets16 ? VecTraits<T>::unpack2(__ldg(reinterpret_cast<const uint32_t *>(p.loc) + e))
+                                       : __ldg(reinterpret_cast<const float2 *>(p.loc) + e);
+        return location_from_offset(p, off, (int64_t)s.b * p.Q + s.q0 + q, s.l, (float)s.W, (float)s.H);
+    } else {
+        return __ldg(reinterpret_cast<const float2 *>(p.loc) + e);
+    }
+}
+
+// Adds the counts the CTA made in shared memory to the plane's.
+__device__ __forceinline__ void merge_counts(const unsigned *hist, unsigned *plane, int cells) {
+    for (int c = threadIdx.x; c < cells; c += kSortThreads)
+        if (hist[c] != 0) atomicAdd(plane + c, hist[c]);
+}
+
+// Takes the CTA's counts per cell to `begin`, where the cell's points begin in the CTA's order,
+// and leaves in their place the difference to where they begin in the plane's.  Returns how
+// many points there are.
+__device__ __forceinline__ unsigned scan_cells(unsigned *counts, unsigned short *begin, unsigned *cursor,
+                                               unsigned *warp_sums, int cells) {
+    constexpr int kEach = 8;      // adjacent cells a thread takes (the arrays are padded to this)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned base = 0;
+    for (int c0 = 0; c0 < cells; c0 += kSortThreads * kEach) {
+        const int at = c0 + threadIdx.x * kEach;
+        unsigned n[kEach], place[kEach], sum = 0;
+#pragma unroll
+        for (int i = 0; i < kEach; i += 4) {
+            const uint4 v = at < cells ? *reinterpret_cast<const uint4 *>(counts + at + i) : make_uint4(0u, 0u, 0u, 0u);
+            n[i] = v.x, n[i + 1] = v.y, n[i + 2] = v.z, n[i + 3] = v.w;
+        }
+        // (the round trips to L2 overlap, and the scan with them)
+#pragma unroll
+        for (int i = 0; i < kEach; ++i) {
+            if (at + i >= cells) n[i] = 0u;
+            place[i] = n[i] != 0 ? atomicAdd(cursor + at + i, n[i]) : 0u;
+            sum += n[i];
+        }
+        unsigned incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) warp_sums[warp] = incl;
+        __syncthreads();
+        unsigned before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < kSortThreads / 32; ++w) {
+            const unsigned s = warp_sums[w];
+            before += w < warp ? s : 0u;
+            total += s;
+        }
+        unsigned first = base + before + incl - sum;
+        if (at < cells) {
+            unsigned b[kEach];
+#pragma unroll
+            for (int i = 0; i < kEach; ++i) {
+                b[i] = first;
+                place[i] -= first;
+                first += n[i];
+            }
+#pragma unroll
+            for (int i = 0; i < kEach; i += 4)
+                *reinterpret_cast<uint4 *>(counts + at + i) = make_uint4(place[i], place[i + 1], place[i + 2], place[i + 3]);
+            *reinterpret_cast<uint4 *>(begin + at) = make_uint4(b[0] | b[1] << 16, b[2] | b[3] << 16,
+                                                                b[4] | b[5] << 16, b[6] | b[7] << 16);
+        }
+        base += total;
+        __syncthreads();
+    }
+    return base;
+}
+
+// f(i, value) for the P 16-bit values of a pair, four at a time where that is aligned
+template <typename T, typename F>
+__device__ __forceinline__ void for_values(const T *x, int P, F f) {
+    using VT = VecTraits<T>;
+    if ((P & 3) == 0) {
+#pragma unroll 4
+        for (int i = 0; i < P; i += 4) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(x + i));
+            const float2 a = VT::unpack2(v.x), b = VT::unpack2(v.y);
+            f(i, a.x), f(i + 1, a.y), f(i + 2, b.x), f(i + 3, b.y);
+        }
+    } else {
+        for (int i = 0; i < P; ++i) f(i, VT::to_float(x[i]));
+    }
+}
+
+// What has to be known or done before anything is accumulated: largest magnitudes for the scale,
+// zeros in grad_value, softmax statistics (max, 1 / sum) of every pair.  The share of one of
+// `ctas` CTAs.
+template <typename T, bool SOFTMAX>
+__device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &sp, int cta, int ctas) {
+    constexpr bool WITH_ATTN = !SOFTMAX;
+    unsigned *header = sp.header;
+    __shared__ unsigned cta_max[2];
+    if (threadIdx.x < 2) cta_max[threadIdx.x] = 0u;
+    __syncthreads();
+    const int64_t stride = (int64_t)ctas * blockDim.x;
+    const int64_t first = (int64_t)cta * blockDim.x + threadIdx.x;
+    const int64_t go_vecs = p.B * p.Q * (p.G * p.D / 8);
+    unsigned mg = scan_max_magnitude(reinterpret_cast<const uint4 *>(p.grad_out), go_vecs, first, stride);
+    unsigned ma = 0;
+    if constexpr (WITH_ATTN) {
+        // (a later sample's weights need not begin on a 16-byte boundary: whole vectors in the
+        // middle, single elements at both ends)
+        const unsigned short *at = reinterpret_cast<const unsigned short *>(p.attn);
+        const int64_t n = p.B * p.Q * p.G * p.L * p.K;
+        const int64_t head = min((int64_t)((16u - (unsigned)(reinterpret_cast<uintptr_t>(at) & 15u)) & 15u) / 2, n);
+        const int64_t body = (n - head) / 8;
+        ma = scan_max_magnitude(reinterpret_cast<const uint4 *>(at + head), body, first, stride);
+        for (int64_t i = first; i < head; i += stride) ma = max(ma, at[i] & 0x7fffu);
+        for (int64_t i = head + body * 8 + first; i < n; i += stride) ma = max(ma, at[i] & 0x7fffu);
+    }
+    if constexpr (SOFTMAX) {
+        const int P = p.L * p.K;
+        for (int64_t i = first; i < p.B * p.Q * p.G; i += stride) {
+            const T *x = reinterpret_cast<const T *>(p.attn) + i * P;
+            float m = -INFINITY, sum = 0.f;
+            for_values(x, P, [&](int, float v) { m = fmaxf(m, v); });
+            for_values(x, P, [&](int, float v) { sum += expf(v - m); });
+            sp.stats[i] = make_float2(m, 1.f / sum);
+        }
+    }
+    uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
+    const int64_t vecs = p.B * p.S * (p.G * p.D / 8);
+    for (int64_t v = first; v < vecs; v += stride) gv[v] = make_uint4(0u, 0u, 0u, 0u);
+    mg = __reduce_max_sync(0xffffffffu, mg);
+    if constexpr (WITH_ATTN) ma = __reduce_max_sync(0xffffffffu, ma);
+    if ((threadIdx.x & 31) == 0) {
+        if (mg != 0) atomicMax(&cta_max[0], mg);
+        if (WITH_ATTN && ma != 0) atomicMax(&cta_max[1], ma);
+    }
+    __syncthreads();
+    if (threadIdx.x < (WITH_ATTN ? 2 : 1) && cta_max[threadIdx.x] != 0)
+        atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
+}
+
+// Exclusive prefix sum of a plane's cell counts by one CTA, in chunks of its size: `counts`
+// becomes the cursor the scatter kernel hands places out from, `offsets` the cells' first places
+// (offsets[cells]: the plane's points), `item_cell` the cell in which each run of
+// sp.item_points places begins.
+__device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item_cell, int cells,
+                                  int item_points) {
+    __shared__ unsigned warp_sums[kSortThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned base = 0;
+    for (int c0 = 0; c0 < cells; c0 += kSortThreads * 4) {
+        const int at = c0 + threadIdx.x * 4;
+        unsigned n[4], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            n[i] = at + i < cells ? __ldcg(counts + at + i) : 0u;
+            sum += n[i];
+        }
+        unsigned incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) warp_sums[warp] = incl;
+        __syncthreads();
+        unsigned before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < kSortThreads / 32; ++w) {
+            const unsigned s = warp_sums[w];
+            before += w < warp ? s : 0u;
+            total += s;
+        }
+        unsigned at_place = base + before + incl - sum;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (at + i < cells) {
+                counts[at + i] = at_place;
+                offsets[at + i] = at_place;
+                for (unsigned m = (at_place + item_points - 1) / item_points;
+                     m * (unsigned)item_points < at_place + n[i]; ++m)
+                    item_cell[m] = at + i;
+                at_place += n[i];
+            }
+        }
+        base += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) offsets[cells] = base;
+}
+
+// Bound by latency: a CTA's life is a dozen round trips to memory, so more CTAs per SM count for
+// more than registers (2 / 3 / 4 per SM: 64 / 55 / 50 us at the headline shape; reading its
+// operands alone takes 28 us).
+// ---- pass 1: count the points of every cell -------------------------------------------------------
+template <typename T, bool SOFTMAX, bool REF>
+__global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __grid_constant__ Params p,
+    const __grid_constant__ SortPlan sp) {
+    // the first CTAs look for the magnitudes and clear grad_value, beside those that count
+    if (blockIdx.x < (unsigned)sp.prepare_ctas) {
+        prepare_share<T, SOFTMAX>(p, sp, (int)blockIdx.x, sp.prepare_ctas);
+        return;
+    }
+    extern __shared__ unsigned hist[];
+    __shared__ LevelTable lt;
+    __shared__ CellTable ct;
+    __shared__ bool last;
+    load_level_table(lt, p);
+    __syncthreads();
+    if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
+    __syncthreads();
+    const int cells = ct.first[p.L];
+    const bool in_shared = cells <= sp.shared_cells;
+    if (in_shared)
+        for (int i = threadIdx.x; i < cells; i += kSortThreads) hist[i] = 0u;
+    const SortLane c = sort_lane(p, sp, lt, ct, blockIdx.x - sp.prepare_ctas);
+    unsigned *counts = sp.counts + (int64_t)c.plane * sp.cell_stride;
+    const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
+    __syncthreads();
+    if (c.active && c.rows > 0) {
+        const int64_t base = pair0 * (p.L * p.K) + c.pt;
+        for (int r0 = 0; r0 < kSortPoints; r0 += kSortBatch) {
+            float2 xy[kSortBatch];
+#pragma unroll
+            for (int r = 0; r < kSortBatch; ++r) {
+                const int q = c.ql + (r0 + r) * c.step;
+                xy[r] = q < c.nq ? point_xy<T, REF>(p, c, base, q) : make_float2(-1e9f, -1e9f);
+            }
+            PointCell at;
+#pragma unroll
+            for (int r = 0; r < kSortBatch; ++r) {
+                if (!find_cell(c, xy[r], at)) continue;
+                if (in_shared)
+                    atomicAdd(hist + at.cell, 1u);
+                else
+                    atomicAdd(counts + at.cell, 1u);
+            }
+        }
+    }
+    __syncthreads();
+    if (in_shared) merge_counts(hist, counts, cells);
+    // the plane's last CTA turns its counts into places
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(sp.tickets + c.plane, 1u) == (unsigned)(sp.chunks - 1);
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        scan_plane(counts, sp.offsets + (int64_t)c.plane * sp.cell_stride,
+                   sp.item_cell + (int64_t)c.plane * sp.items, cells, sp.item_points);
+    }
+}
+
+// Gradients of one point, wherever they were formed.  The weight's goes out in float32: the last
+// kernel rounds it, after the softmax Jacobian where there is one (and scattered two-byte
+// stores take half as long again as four-byte ones: 2.3 cycles of an SM each against 1.5).
+template <typename T>
+__device__ __forceinline__ void store_point_gradients(const Params &p, const SortPlan &sp, int64_t e,
+                                                      float2 grad_loc, float grad_weight) {
+    if (p.ref != nullptr && p.offsets16)
+        reinterpret_cast<uint32_t *>(p.grad_loc)[e] = VecTraits<T>::pack2(grad_loc);
+    else
+        reinterpret_cast<float2 *>(p.grad_loc)[e] = grad_loc;
+    sp.grad_prob[e] = grad_weight;
+}
+
+// One point without sorting, one thread: what the walk does for points the sort leaves out.
+template <typename T>
+__device__ __noinline__ void direct_point(const Params &p, const SortPlan &sp, const LevelTable &lt,
+                                          int64_t pair, int pt, float a, float scale) {
+    using VT = VecTraits<T>;
+    const int l = pt / p.K;
+    const int64_t e = pair * (p.L * p.K) + pt;
+    float2 dpix;
+    const float2 xy = sample_location<T>(p, e, pair, l, (float)lt.W[l], (float)lt.H[l], dpix);
+    const PointGeom geo = locate(xy.x, xy.y, lt.H[l], lt.W[l], lt.start[l], p.G * p.D);
+    const int64_t bq = pair / p.G;
+    const int64_t sample = ((bq / p.Q) * p.S * p.G + (pair - bq * p.G)) * p.D;
+    const T *value = reinterpret_cast<const T *>(p.value) + sample;
+    const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + pair * p.D;
+    __half *image = reinterpret_cast<__half *>(p.grad_value) + sample;
+    const int off[4] = {geo.off00, geo.off00 + p.G * p.D, geo.off00 + geo.rowstride,
+                        geo.off00 + geo.rowstride + p.G * p.D};
+    const float w[4] = {(1.f - geo.fr) * (1.f - geo.fc), (1.f - geo.fr) * geo.fc,
+                        geo.fr * (1.f - geo.fc), geo.fr * geo.fc};
+    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int ch = 0; ch < p.D; ch += 8) {
+        float2 go[4], f[4];
+        VT::unpack(ldg16(grad_out + ch), go);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool inside = geo.flags & (1u << c);
+            VT::unpack(ldg16_if(value + off[c] + ch, inside), f);
+            const float s = a * w[c] * scale;
+            float2 gv[4], d2 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                ffma2(d2, f[i], go[i]);
+                gv[i] = fmul2(go[i], make_float2(s, s));
+            }
+            dot[c] += d2.x + d2.y;
+            red_if<__half>(image + off[c] + ch, gv, inside);
+        }
+    }
+    const float gx = (1.f - geo.fr) * (dot[1] - dot[0]) + geo.fr * (dot[3] - dot[2]);
+    const float gy = (1.f - geo.fc) * (dot[2] - dot[0]) + geo.fc * (dot[3] - dot[1]);
+    const float ga = w[0] * dot[0] + w[1] * dot[1] + w[2] * dot[2] + w[3] * dot[3];
+    store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
+}
+
+// An inf or NaN in grad_out has to reach its own corners only: a tile product would spread
+// it to the zero entries beside them (0 * inf), so such a call takes direct_point() throughout.
+template <typename T>
+__device__ __forceinline__ bool unsortable_call(const unsigned *header) {
+    return header[0] >= (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u);
+}
+
+// ---- pass 2: write the points' records in order of their cells ------------------------------------
+// A record: fractions of the pixel coordinate (column, row), weight, and where the point came
+// from: query << 12 | point << 3 | column of the cell.  The CTA orders its records by cell before
+// they leave: a warp's stores then fall on a few stretches of memory instead of 32 places (with
+// the locations kept from being evaluated twice: 105 us at the headline shape against 126).
+template <typename T, bool SOFTMAX, bool REF>
+__global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __grid_constant__ Params p,
+    const __grid_constant__ SortPlan sp) {
+    using VT = VecTraits<T>;
+    extern __shared__ uint4 smem[];
+    __shared__ LevelTable lt;
+    __shared__ CellTable ct;
+    __shared__ unsigned warp_sums[kSortThreads / 32];
+    // the CTA's records, by thread; in order of their cells: which record, which cell; and per
+    // cell: its count, then what takes a place in the CTA's order to one in the plane's, and its
+    // first place in the CTA's
+    uint4 *local = smem;
+    unsigned *shift = reinterpret_cast<unsigned *>(local + kSortCtaPoints);
+    unsigned short *order = reinterpret_cast<unsigned short *>(shift + sp.shared_cells);
+    unsigned short *cell_of = order + kSortCtaPoints;
+    unsigned short *begin = cell_of + kSortCtaPoints;
+    load_level_table(lt, p);
+    __syncthreads();
+    if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
+    __syncthreads();
+    const int cells = ct.first[p.L];
+    const bool in_shared = cells <= sp.shared_cells;
+    if (in_shared)
+        for (int i = threadIdx.x; i < cells; i += kSortThreads) shift[i] = 0u;
+    const SortLane c = sort_lane(p, sp, lt, ct, blockIdx.x);
+    unsigned *cursor = sp.counts + (int64_t)c.plane * sp.cell_stride;
+    uint4 *records = sp.records + (int64_t)c.plane * sp.plane_points;
+    const T *attn = reinterpret_cast<const T *>(p.attn);
+    const int P = p.L * p.K;
+    const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
+    const int64_t base = pair0 * P + c.pt;
+    const bool sorted = c.rows > 0 && !unsortable_call<T>(sp.header);
+    const int nq = c.active ? c.nq : 0;
+    __syncthreads();
+    unsigned at[kSortPoints];     // cell << 16 | rank among the CTA's points of the cell; ~0: not sorted
+    unsigned left_out = 0;        // points direct_point() has to take
+#pragma unroll
+    for (int r0 = 0; r0 < kSortPoints; r0 += kSortBatch) {
+        float2 xy[kSortBatch], stats[SOFTMAX ? kSortBatch : 1];
+        T weight[kSortBatch];
+#pragma unroll
+        for (int r = 0; r < kSortBatch; ++r) {
+            const int q = c.ql + (r0 + r) * c.step;
+            if (q < nq) {
+                xy[r] = point_xy<T, REF>(p, c, base, q);
+                if constexpr (SOFTMAX) stats[r] = __ldg(sp.stats + pair0 + (int64_t)(q * p.G));
+                weight[r] = attn[base + (int64_t)(q * (p.G * P))];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kSortBatch; ++r) {
+            at[r0 + r] = ~0u;
+            const int q = c.ql + (r0 + r) * c.step;
+            if (q >= nq) continue;
+            PointCell pc;
+            if (!find_cell(c, xy[r], pc)) {
+                // a skipped point: exact zeros
+                store_point_gradients<T>(p, sp, base + (int64_t)(q * (p.G * P)), make_float2(0.f, 0.f), 0.f);
+            } else if (!sorted) {
+                left_out |= 1u << (r0 + r);
+            } else {
+                float a = VT::to_float(weight[r]);
+                if constexpr (SOFTMAX) a = expf(a - stats[r].x) * stats[r].y;
+                const uint4 record =
+                    make_uint4(__float_as_uint(pc.fc), __float_as_uint(pc.fr), __float_as_uint(a),
+                               ((unsigned)(c.q0 + q) << 12) | ((unsigned)c.pt << 3) | (unsigned)pc.col);
+                if (in_shared) {
+                    local[(r0 + r) * kSortThreads + threadIdx.x] = record;
+                    at[r0 + r] = ((unsigned)pc.cell << 16) | atomicAdd(shift + pc.cell, 1u);
+                } else {
+                    const unsigned place = atomicAdd(cursor + pc.cell, 1u);
+                    if (place < (unsigned)sp.plane_points) records[place] = record;
+                }
+            }
+        }
+    }
+    if (in_shared) {
+        __syncthreads();
+        const unsigned points = scan_cells(shift, begin, cursor, warp_sums, cells);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortPoints; ++r) {
+            if (at[r] == ~0u) continue;
+            const unsigned i = begin[at[r] >> 16] + (at[r] & 0xffffu);
+            order[i] = (unsigned short)(r * kSortThreads + threadIdx.x);
+            cell_of[i] = (unsigned short)(at[r] >> 16);
+        }
+        __syncthreads();
+        // neighbours in the CTA's order are neighbours in the plane's for as long as a cell lasts
+#pragma unroll 4
+        for (unsigned i = threadIdx.x; i < points; i += kSortThreads) {
+            const unsigned place = i + shift[cell_of[i]];
+            if (place < (unsigned)sp.plane_points) records[place] = local[order[i]];
+        }
+    }
+    if (left_out != 0) {
+        const float scale = ldexpf(1.f, grad_scale_exponent<T>(sp.header, p.Q, p.K, SOFTMAX));
+        for (int r = 0; r < kSortPoints; ++r) {
+            if (!(left_out >> r & 1u)) continue;
+            const int q = c.ql + r * c.step;
+            const int64_t pair = pair0 + (int64_t)q * p.G;
+            float a = VT::to_float(attn[pair * P + c.pt]);
+            if constexpr (SOFTMAX) a = expf(a - sp.stats[pair].x) * sp.stats[pair].y;
+            direct_point<T>(p, sp, lt, pair, c.pt, a, scale);
+        }
+    }
+}
+
+// ---- the walk over sorted points ------------------------------------------------------------------
+template <typename T> struct Mma;
+template <> struct Mma<__nv_bfloat16> {
+    __device__ static __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                     "{%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+};
+template <> struct Mma<__half> {
+    __device__ static __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                     "{%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// transposes an 8x8 matrix of 16-bit elements held one row of pairs per four lanes
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+__device__ __forceinline__ uint4 lds16(uint32_t addr) {
+    uint4 r;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "r"(addr)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ uint2 lds8(uint32_t addr) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr) : "memory");
+    return r;
+}
+__device__ __forceinline__ float lds4(uint32_t addr) {
+    float r;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(addr) : "memory");
+    return r;
+}
+
+constexpr int kStep = 32;          // points a warp takes at a time, one per lane
+constexpr int kWalkWarps = 4;      // warps per CTA, each on its own run
+
+// byte offset of 16-byte chunk `chunk` of row `row` of a step's grad_out rows (2*D bytes each):
+// chunks permuted so that the row-wise reads (8 lanes: two to four rows) touch every bank once.
+// Rows 8 apart have the same permutation.
+template <int D>
+__device__ __forceinline__ uint32_t row_offset(int row, int chunk) {
+    if constexpr (D == 32) return row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
+    if constexpr (D == 64) return row * 128 + ((chunk ^ ((row & 1) << 2) ^ ((row >> 1) & 3)) << 4);
+    return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4);
+}
+
+// What a lane holds of one row of a D-channel matrix whose k index runs over channels: register
+// 2*s + h is the k = 2*(lane%4) + {0,1} + 8*h pair of k-step s.  The channels are dealt to k in
+// the order a 16-byte load per lane delivers them (lane c of four: channels 8c .. 8c+7 of every
+// 32; D = 16: 4c .. 4c+3).  Both operands of the dot products use it, so it does not matter
+// there, and in the transposed registers it leaves each lane with adjacent channels.
+template <int D>
+__device__ __forceinline__ void row_from_shared(uint32_t (&w)[D / 8], uint32_t base,
+                                                const uint32_t (&at)[D == 64 ? 2 : 1]) {
+    if constexpr (D == 16) {
+        const uint2 v = lds8(base + at[0]);
+        w[0] = v.x, w[1] = v.y;
+    } else {
+#pragma unroll
+        for (int h = 0; h < D / 32; ++h) {
+            const uint4 v = lds16(base + at[h]);
+            w[4 * h] = v.x, w[4 * h + 1] = v.y, w[4 * h + 2] = v.z, w[4 * h + 3] = v.w;
+        }
+    }
+}
+template <typename T, int D>
+__device__ __forceinline__ void row_from_global(uint32_t (&w)[D / 8], const T *row, int c, bool inside) {
+    if constexpr (D == 16) {
+        uint2 v = make_uint2(0u, 0u);
+        if (inside) v = __ldg(reinterpret_cast<const uint2 *>(row) + c);
+        w[0] = v.x, w[1] = v.y;
+    } else {
+#pragma unroll
+        for (int h = 0; h < D / 32; ++h) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (inside) v = ldg16(reinterpret_cast<const uint4 *>(row) + h * 4 + c);
+            w[4 * h] = v.x, w[4 * h + 1] = v.y, w[4 * h + 2] = v.z, w[4 * h + 3] = v.w;
+        }
+    }
+}
+
+// Adds one accumulated pixel row (8 pixels x D channels; this lane: pixel lane/4, the channels
+// of its loads) into the float16 image.
+template <int D>
+__device__ __forceinline__ void flush_row(float (&acc)[D / 8][4], int half, float scale, __half *pixel,
+                                          bool inside, int c) {
+    uint32_t v[D / 8];
+#pragma unroll
+    for (int t = 0; t < D / 8; ++t)
+        v[t] = VecTraits<__half>::pack2(make_float2(acc[t][2 * half] * scale, acc[t][2 * half + 1] * scale));
+    if (!inside) return;
+    if constexpr (D == 16) {
+        asm volatile("red.relaxed.gpu.global.add.noftz.v2.f16x2 [%0], {%1, %2};" ::"l"(pixel + 4 * c), "r"(v[0]),
+                     "r"(v[1]));
+    } else {
+#pragma unroll
+        for (int h = 0; h < D / 32; ++h)
+            asm volatile("red.relaxed.gpu.global.add.noftz.v4.f16x2 [%0], {%1, %2, %3, %4};" ::"l"(
+                             pixel + 32 * h + 8 * c),
+                         "r"(v[4 * h]), "r"(v[4 * h + 1]), "r"(v[4 * h + 2]), "r"(v[4 * h + 3]));
+    }
+}
+
+// What bounds the walk is the SM's load/store pipe, about five of its cycles a point (ncu, the
+// headline shape: 64 % busy while the SM works, issue slots 50 %, tensor cores 24 %): the two
+// stores per point to addresses of their own take 45 us of 247, the grad_out rows 27, the rest
+// goes through shared memory.  Hence the weights' way over the tensor cores below.  More warps do
+// not help - 12, 16, 20, 24 per SM: 252, 246, 261, 312 us - nor does having grad_out rows in
+// registers instead of shared memory (300 us), or the next cell's value row early (257 us).
+// (CTAs per SM the registers are held to: more than these spill)
+constexpr int walk_ctas(int D) { return D == 64 ? 3 : 4; }
+__host__ __device__ constexpr int walk_warp_bytes(int D) { return 2 * kStep * D * 2 + kStep * 16 + kStep / 8 * 512; }
+
+template <typename T, int D, bool REF>
+__global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
+    sorted_walk_kernel(const __grid_constant__ Params p, const __grid_constant__ SortPlan sp, bool softmax) {
+    using VT = VecTraits<T>;
+    constexpr int NT = D / 8;       // channel tiles of eight
+    constexpr int KS = D / 16;      // k-steps of the dot products
+    constexpr bool kSplit = std::is_same<T, __nv_bfloat16>::value;   // weights as two bf16 terms
+    extern __shared__ uint4 smem[];
+    __shared__ LevelTable lt;
+    __shared__ CellTable ct;
+    load_level_table(lt, p);
+    __syncthreads();
+    if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
+    __syncthreads();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = lane >> 2, c = lane & 3;
+    if (unsortable_call<T>(sp.header)) return;
+    const int cells = ct.first[p.L];
+    const int GD = p.G * D, GP = p.G * p.L * p.K;
+    // float16 weights are kept near 1 whatever their largest magnitude
+    float weight_scale = 1.f;
+    if constexpr (!kSplit) {
+        const float ma = softmax ? 1.f : magnitude_from_bits<T>(sp.header[1]);
+        if (ma > 0.f && ma < INFINITY) weight_scale = ldexpf(1.f, -ilogbf(ma));
+    }
+    const float flush_scale =
+        ldexpf(1.f, grad_scale_exponent<T>(sp.header, p.Q, p.K, softmax)) / weight_scale;
+
+    // shared memory of the warp: grad_out rows of two steps, the step's weights, and the dot
+    // products of the window's 16 pixels with its points, in blocks of eight points
+    constexpr int kRows = kStep * D * 2;   // bytes
+    constexpr int kWarpBytes = walk_warp_bytes(D);
+    uint4 *mine = smem + warp * (kWarpBytes / 16);
+    const uint32_t s_rows = (uint32_t)__cvta_generic_to_shared(mine);
+    const uint32_t s_weights = s_rows + 2 * kRows;
+    const uint32_t s_dots = s_weights + kStep * 16;
+    // (rows that a short step leaves out are multiplied by zero: they have to be finite)
+    for (int i = lane; i < 2 * kRows / 16; i += 32) mine[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    uint32_t at_row[D == 64 ? 2 : 1];      // this lane's part of row j
+    if constexpr (D == 16)
+        at_row[0] = row_offset<D>(j, c >> 1) + (c & 1) * 8;
+    else
+#pragma unroll
+        for (int h = 0; h < D / 32; ++h) at_row[h] = row_offset<D>(j, h * 4 + c);
+    // the lane's share of the copies: row r0 of every kRowsPerTurn, one 16-byte chunk.  Rows of
+    // D = 64's odd turns are four on, where the permutation differs in one bit
+    constexpr int kRowsPerTurn = 32 / NT;
+    const int r0 = lane / NT;
+    const uint32_t at_copy = row_offset<D>(r0, lane % NT);
+    // the identity as the A operand of an m16n8k16 product (upper left and lower right corner)
+    const uint32_t one = VT::pack2(make_float2(j == 2 * c ? 1.f : 0.f, j == 2 * c + 1 ? 1.f : 0.f));
+
+    // ---- runs of places, handed out as the warps come for them
+    for (;;) {
+    unsigned item = 0;
+    if (lane == 0) item = atomicAdd(sp.header + kNextItem, 1u);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= (unsigned)(p.B * p.G) * (unsigned)sp.items) break;
+    const int plane = (int)(item / (unsigned)sp.items);
+    const int run = (int)(item - (unsigned)plane * (unsigned)sp.items);
+    const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
+    const int total = (int)__ldg(offsets + cells);
+    int cell = __ldg(sp.item_cell + (int64_t)plane * sp.items + run);
+    int pos = run * sp.item_points;
+    const int stop = min(pos + sp.item_points, total);
+    if (pos >= stop) continue;
+
+    const int b = plane / p.G, g = plane - b * p.G;
+    const T *value = reinterpret_cast<const T *>(p.value) + ((int64_t)b * p.S * p.G + g) * D;
+    const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + ((int64_t)b * p.Q * p.G + g) * D;
+    __half *image = reinterpret_cast<__half *>(p.grad_value) + ((int64_t)b * p.S * p.G + g) * D;
+    const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
+    // element of the per-point outputs that point 0 of query 0 of this plane has
+    const int64_t plane_point = ((int64_t)b * p.Q * p.G + g) * (p.L * p.K);
+
+    auto fetch_record = [&](int place) { return __ldg(records + min(place + lane, total - 1)); };
+    const T *chunk_of_row = grad_out + lane % NT * 8;
+    auto fetch_rows = [&](const uint4 &rec, int n, uint32_t buffer) {
+        const unsigned mine = rec.w >> 12;
+#pragma unroll
+        for (int i = 0; i < kStep / kRowsPerTurn; ++i) {
+            const unsigned q = __shfl_sync(0xffffffffu, mine, i * kRowsPerTurn + r0);
+            const uint32_t to = buffer + i * kRowsPerTurn * D * 2 + (D == 64 && (i & 1) ? at_copy ^ 32u : at_copy);
+            if (i * kRowsPerTurn + r0 < n) cp_async16(to, chunk_of_row + (size_t)(q * (unsigned)GD));
+        }
+        cp_async_commit();
+    };
+
+    // ---- where the run begins
+    int level = 0, strip_end = 0, row = 0, H = 0, W = 0, col0 = 0, start = 0;
+    auto enter_strip = [&]() {
+        while (level + 1 < p.L && cell >= ct.first[level + 1]) ++level;
+        const int rows = ct.rows[level];
+        const int strip = (cell - ct.first[level]) / rows;
+        strip_end = ct.first[level] + (strip + 1) * rows;
+        row = cell - (strip_end - rows) - 1;
+        H = lt.H[level], W = lt.W[level], start = lt.start[level];
+        col0 = strip * kCols - 1;
+    };
+    enter_strip();
+    int window = cell;      // the lanes hold the ends of cells window .. window + 31
+    int ends = (int)__ldg(offsets + min(window + 1 + lane, cells));
+    // the first cell at or after `window` that ends beyond `place` (which is below total)
+    auto cell_at = [&](int place, int &end) {
+        unsigned more;
+        while ((more = __ballot_sync(0xffffffffu, ends > place)) == 0) {
+            window += 32;
+            ends = (int)__ldg(offsets + min(window + 1 + lane, cells));
+        }
+        const int k = __ffs(more) - 1;
+        end = __shfl_sync(0xffffffffu, ends, k);
+        return window + k;
+    };
+
+    uint32_t vtop[NT], vbot[NT];     // the window's value rows, this lane's pixel
+    auto load_row = [&](uint32_t (&w)[NT], int r) {
+        const int x = col0 + j;
+        row_from_global<T, D>(w, value + (int64_t)(start + r * W + x) * GD, c,
+                              (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W);
+    };
+    load_row(vtop, row);
+    load_row(vbot, row + 1);
+    float acc[NT][4];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+    auto flush = [&](int half, int r) {
+        const int x = col0 + j;
+        flush_row<D>(acc, half, flush_scale, image + (int64_t)(start + r * W + x) * GD,
+                     (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W, c);
+    };
+
+    // ---- first steps
+    int cell_end;
+    cell_at(pos, cell_end);
+    int n = min(min(kStep, cell_end - pos), stop - pos);
+    uint4 rec = fetch_record(pos), rec_next = fetch_record(pos + n);
+    uint32_t buffer = s_rows;
+    fetch_rows(rec, n, buffer);
+
+    for (;;) {
+        // ---- what comes next, and its rows on their way
+        const int pos_next = pos + n;
+        const bool more = pos_next < stop;
+        int cell_next = cell, n_next = 0;
+        if (more) {
+            if (pos_next >= cell_end) cell_next = cell_at(pos_next, cell_end);
+            n_next = min(min(kStep, cell_end - pos_next), stop - pos_next);
+        }
+        const uint4 rec_after = fetch_record(pos_next + n_next);
+        const uint32_t other = buffer ^ s_rows ^ (s_rows + kRows);
+        fetch_rows(rec_next, n_next, other);
+
+        // ---- one lane per point: its four weights
+        const float fc = __uint_as_float(rec.x), fr = __uint_as_float(rec.y), a = __uint_as_float(rec.z);
+        {
+            const float w = lane < n ? a * weight_scale : 0.f;
+            const float top = w * (1.f - fr), bot = w * fr;
+            const float2 tw = make_float2(top * (1.f - fc), top * fc), bw = make_float2(bot * (1.f - fc), bot * fc);
+            uint4 s;
+            s.x = VT::pack2(tw);
+            s.y = VT::pack2(bw);
+            if constexpr (kSplit) {
+                // what the first term leaves; three low bits of it hold the column in the cell
+                const float2 th = VT::unpack2(s.x), bh = VT::unpack2(s.y);
+                s.z = VT::pack2(make_float2(tw.x - th.x, tw.y - th.y));
+                s.w = (VT::pack2(make_float2(bw.x - bh.x, bw.y - bh.y)) & ~7u) | (rec.w & 7u);
+            } else {
+                s.z = 0u;
+                s.w = rec.w & 7u;
+            }
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_weights + lane * 16), "r"(s.x),
+                         "r"(s.y), "r"(s.z), "r"(s.w)
+                         : "memory");
+        }
+        cp_async_wait<1>();
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && n <= 16) break;
+            uint32_t go[2][NT];
+            uint32_t hi[4], lo[4];     // weights of pixels x points: the A operand
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int block = h * 2 + e;
+                row_from_shared<D>(go[e], buffer + block * 8 * D * 2, at_row);
+                // dot products of the window's pixels with eight points
+                float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int s = 0; s < KS; ++s) {
+                    const uint32_t av[4] = {vtop[2 * s], vbot[2 * s], vtop[2 * s + 1], vbot[2 * s + 1]};
+                    Mma<T>::run(dot, av, go[e][2 * s], go[e][2 * s + 1]);
+                }
+                const uint32_t to = s_dots + block * 512 + lane * 8;   // pixel j: 32 bytes, points 2c and 2c+1
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(dot[0]), "f"(dot[1]) : "memory");
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 256), "f"(dot[2]), "f"(dot[3]) : "memory");
+                // The weights with the pixels as k, the points as n: this lane has point j and
+                // pixel columns 2c, 2c + 1 of either row.  The point's words hold its columns col
+                // and col + 1; they go where 2c - col is -1, 0 or 1 (shift 0, 16, 32).
+                const uint4 w = lds16(s_weights + (block * 8 + j) * 16);
+                const uint32_t shift = 16u + 32u * c - 16u * (w.w & 7u);
+                uint32_t pick = __funnelshift_rc(0x32101044u, 0x44444432u, shift);
+                if (shift > 32u) pick = 0x4444u;
+                // a product with the identity turns that into pixels x points, which is what the
+                // accumulation below takes: the tensor cores have time for it, the shared memory
+                // that four words per lane and point would pass through has not
+                float t[4] = {0.f, 0.f, 0.f, 0.f};
+                const uint32_t unit[4] = {one, 0u, 0u, one};
+                Mma<T>::run(t, unit, __byte_perm(w.x, 0u, pick), __byte_perm(w.y, 0u, pick));
+                hi[2 * e] = VT::pack2(make_float2(t[0], t[1]));
+                hi[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+                if constexpr (kSplit) {
+                    t[0] = t[1] = t[2] = t[3] = 0.f;
+                    Mma<T>::run(t, unit, __byte_perm(w.z, 0u, pick), __byte_perm(w.w & ~7u, 0u, pick));
+                    lo[2 * e] = VT::pack2(make_float2(t[0], t[1]));
+                    lo[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const uint32_t b0 = transpose8x8(go[0][t]), b1 = transpose8x8(go[1][t]);
+                Mma<T>::run(acc[t], hi, b0, b1);
+                if constexpr (kSplit) Mma<T>::run(acc[t], lo, b0, b1);
+            }
+        }
+        __syncwarp();
+        // ---- gradients of the points: one lane each
+        if (lane < n) {
+            const uint32_t at = s_dots + (lane >> 3) * 512 + (rec.w & 7u) * 32 + (lane & 7) * 4;
+            const float d00 = lds4(at), d01 = lds4(at + 32), d10 = lds4(at + 256), d11 = lds4(at + 288);
+            const float wr0 = 1.f - fr, wc0 = 1.f - fc;
+            const float gx = wr0 * (d01 - d00) + fr * (d11 - d10);
+            const float gy = wc0 * (d10 - d00) + fc * (d11 - d01);
+            const float ga = wr0 * wc0 * d00 + wr0 * fc * d01 + fr * wc0 * d10 + fr * fc * d11;
+            const unsigned q = rec.w >> 12;
+            const int64_t e = plane_point + (size_t)(q * (unsigned)GP + ((rec.w >> 3) & 511u));
+            float2 dpix = make_float2((float)W, (float)H);
+            if constexpr (REF) {
+                dpix = offset_derivative(p, (int64_t)b * p.Q + q, level, dpix.x, dpix.y);
+                store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
+            } else {
+                reinterpret_cast<float2 *>(p.grad_loc)[e] = make_float2(a * dpix.x * gx, a * dpix.y * gy);
+                sp.grad_prob[e] = ga;
+            }
+        }
+        __syncwarp();
+        if (!more) break;
+        pos = pos_next;
+        n = n_next;
+        buffer = other;
+        rec = rec_next;
+        rec_next = rec_after;
+        if (cell_next == cell) continue;
+        // ---- into the next cell
+        if (cell_next == cell + 1 && cell_next < strip_end) {
+            // one row down: the upper row is complete, the lower one becomes the upper
+            flush(0, row);
+            ++row;
+            cell = cell_next;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                acc[t][0] = acc[t][2], acc[t][1] = acc[t][3];
+                acc[t][2] = acc[t][3] = 0.f;
+                vtop[t] = vbot[t];
+            }
+            load_row(vbot, row + 1);
+        } else {
+            flush(0, row);
+            flush(1, row + 1);
+            if (cell_next < strip_end) {
+                row += cell_next - cell;
+                cell = cell_next;
+            } else {
+                cell = cell_next;
+                enter_strip();
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+            load_row(vtop, row);
+            load_row(vbot, row + 1);
+        }
+    }
+    flush(0, row);
+    flush(1, row + 1);
+    cp_async_wait<0>();
+    }
+}
+
+// ---- last pass: grad_value from the scaled float16 image, in place; softmax Jacobian --------------
+template <typename T, bool SOFTMAX>
+__global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_constant__ Params p,
+    const __grid_constant__ SortPlan sp) {
+    using VT = VecTraits<T>;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int P = p.L * p.K;
+    T *grad_attn = reinterpret_cast<T *>(p.grad_attn);
+    if constexpr (SOFTMAX) {
+        // gradient of the logits, p_i (g_i - sum_j p_j g_j): one thread per (query, head) pair,
+        // whose P values are adjacent
+        const T *attn = reinterpret_cast<const T *>(p.attn);
+        const int64_t pairs = p.B * p.Q * p.G;
+        for (int64_t pair = first; pair < pairs; pair += stride) {
+            const float *g = sp.grad_prob + pair * P;
+            const float2 st = sp.stats[pair];
+            float inner = 0.f;
+            if ((P & 3) == 0) {
+#pragma unroll 4
+                for (int i = 0; i < P; i += 4) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(attn + pair * P + i));
+                    const float2 x0 = VT::unpack2(v.x), x1 = VT::unpack2(v.y);
+                    const float4 gv = *reinterpret_cast<const float4 *>(g + i);
+                    inner += expf(x0.x - st.x) * gv.x + expf(x0.y - st.x) * gv.y + expf(x1.x - st.x) * gv.z +
+                             expf(x1.y - st.x) * gv.w;
+                }
+                inner *= st.y;
+#pragma unroll 4
+                for (int i = 0; i < P; i += 4) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(attn + pair * P + i));
+                    const float2 x0 = VT::unpack2(v.x), x1 = VT::unpack2(v.y);
+                    const float4 gv = *reinterpret_cast<const float4 *>(g + i);
+                    const float2 a = make_float2(expf(x0.x - st.x) * st.y * (gv.x - inner),
+                                                 expf(x0.y - st.x) * st.y * (gv.y - inner));
+                    const float2 b = make_float2(expf(x1.x - st.x) * st.y * (gv.z - inner),
+                                                 expf(x1.y - st.x) * st.y * (gv.w - inner));
+                    *reinterpret_cast<uint2 *>(grad_attn + pair * P + i) = make_uint2(VT::pack2(a), VT::pack2(b));
+                }
+            } else {
+                for (int i = 0; i < P; ++i) inner += expf(VT::to_float(attn[pair * P + i]) - st.x) * g[i];
+                inner *= st.y;
+                for (int i = 0; i < P; ++i)
+                    grad_attn[pair * P + i] =
+                        VT::from_float(expf(VT::to_float(attn[pair * P + i]) - st.x) * st.y * (g[i] - inner));
+            }
+        }
+    } else {
+        // four values a thread (the first element of a pass is 16-byte aligned only if the
+        // samples before it are; grad_prob always is)
+        const int64_t points = p.B * p.Q * p.G * P;
+        const bool whole = (reinterpret_cast<uintptr_t>(grad_attn) & 7u) == 0;
+        const int64_t body = whole ? points / 4 : 0;
+        for (int64_t i = first; i < body; i += stride) {
+            const float4 g = __ldcs(reinterpret_cast<const float4 *>(sp.grad_prob) + i);
+            const uint2 v = make_uint2(VT::pack2(make_float2(g.x, g.y)), VT::pack2(make_float2(g.z, g.w)));
+            __stcs(reinterpret_cast<uint2 *>(grad_attn) + i, v);
+        }
+        for (int64_t i = body * 4 + first; i < points; i += stride) grad_attn[i] = VT::from_float(sp.grad_prob[i]);
+    }
+    const float inv = ldexpf(1.f, -grad_scale_exponent<T>(sp.header, p.Q, p.K, SOFTMAX));
+    uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
+    const int64_t total = p.B * p.S * (p.G * p.D / 8);
+    constexpr int kTurn = 4;
+    for (int64_t v0 = first; v0 < total; v0 += kTurn * stride) {
+        uint4 raw[kTurn];
+#pragma unroll
+        for (int u = 0; u < kTurn; ++u)
+            raw[u] = v0 + u * stride < total ? gv[v0 + u * stride] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < kTurn; ++u) {
+            if (v0 + u * stride >= total) break;
+            if ((raw[u].x | raw[u].y | raw[u].z | raw[u].w) == 0u) continue;   // zero in either type
+            float2 f[4];
+            VecTraits<__half>::unpack(raw[u], f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) f[i] = fmul2(f[i], make_float2(inv, inv));
+            gv[v0 + u * stride] = VT::pack(f);
+        }
+    }
+}
+
+template <typename T, int D, bool REF>
+cudaError_t launch_walk(const Params &p, const SortPlan &sp, bool softmax, cudaStream_t stream) {
+    constexpr size_t smem = (size_t)kWalkWarps * walk_warp_bytes(D);
+    auto walk = sorted_walk_kernel<T, D, REF>;
+    // as many CTAs as the GPU holds at once; the warps fetch their runs (asked once: every GPU
+    // this is built for has the same limits)
+    static const int resident = [walk] {
+        int device = 0, sms = 0, per_sm = 0;
+        cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (cudaGetDevice(&device) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk, kWalkWarps * 32, smem) != cudaSuccess)
+            return 0;
+        return sms * per_sm;
+    }();
+    if (resident <= 0) return cudaErrorInvalidConfiguration;
+    const int64_t ctas = (p.B * p.G * (int64_t)sp.items + kWalkWarps - 1) / kWalkWarps;
+    walk<<<(unsigned)std::min<int64_t>(ctas, resident), kWalkWarps * 32, smem, stream>>>(p, sp, softmax);
+    return cudaGetLastError();
+}
+
+template <typename T, int D, bool SOFTMAX>
+cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_t stream) {
+    const unsigned planes = (unsigned)(p.B * p.G);
+    const size_t hist = (size_t)sp.shared_cells * sizeof(unsigned);
+    const size_t scatter_smem = (size_t)kSortCtaPoints * 20 + (size_t)sp.shared_cells * 6;
+    cudaError_t e = cudaMemsetAsync(sp.header, 0, sp.cleared_bytes, stream);
+    if (e != cudaSuccess) return e;
+    auto count = p.ref != nullptr ? sort_count_kernel<T, SOFTMAX, true> : sort_count_kernel<T, SOFTMAX, false>;
+    auto scatter = p.ref != nullptr ? sort_scatter_kernel<T, SOFTMAX, true> : sort_scatter_kernel<T, SOFTMAX, false>;
+    count<<<planes * (unsigned)sp.chunks + sp.prepare_ctas, kSortThreads, hist, stream>>>(p, sp);
+    e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
+    if (e != cudaSuccess) return e;
+    scatter<<<planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream>>>(p, sp);
+    e = p.ref != nullptr ? launch_walk<T, D, true>(p, sp, SOFTMAX, stream)
+                         : launch_walk<T, D, false>(p, sp, SOFTMAX, stream);
+    if (e != cudaSuccess) return e;
+    const int64_t vecs = p.B * p.S * (p.G * D / 8);
+    const int64_t blocks = (vecs + 1023) / 1024;
+    sorted_finish_kernel<T, SOFTMAX><<<(unsigned)std::min<int64_t>(blocks, 148 * 4), 256, 0, stream>>>(p, sp);
+    return cudaGetLastError();
+}
+
+template <typename T, bool SOFTMAX>
+cudaError_t launch_sorted_head(const Params &p, const SortPlan &sp, cudaStream_t stream) {
+    switch (p.D) {
+        case 16: return launch_sorted_typed<T, 16, SOFTMAX>(p, sp, stream);
+        case 32: return launch_sorted_typed<T, 32, SOFTMAX>(p, sp, stream);
+        case 64: return launch_sorted_typed<T, 64, SOFTMAX>(p, sp, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+int64_t round_up(int64_t n, int64_t to) { return (n + to - 1) / to * to; }
+
+}  // namespace
+
+// Where sorting wins (B200, backward call, us, direct -> sorted; bf16, 8 heads, 4 points):
+//   points per value position   12: everything below; 7, random positions: 116 -> 126; 4: 116 ->
+//                               158 (cells of a few points leave the tile products half empty)
+//   points in the call          0.5 M 60 -> 63, 1.0 M 86 -> 73 .. 89 -> 85, 2 M 147 -> 133, 4 M
+//                               265 -> 231, 8 M 512 -> 435, 33 M 1973 -> 1654
+//   channels per head           16: 430 -> 380, 32: 512 -> 435, 64 (half the heads): 441 -> 304
+//   offsets instead of          the arithmetic of the locations is done once more: 16 channels
+//   locations                   228 -> 251, 32: 157 -> 159 at 2 M points, 285 -> 275 at 4 M, 551
+//                               -> 503 at 8 M; 64 (1.8 M points): 241 -> 202
+bool sorting_pays(const Params &p, int dtype) {
+    const int64_t P = (int64_t)p.L * p.K, points = p.B * p.G * p.Q * P;
+    if (dtype != 1 && dtype != 2) return false;
+    if (p.D != 16 && p.D != 32 && p.D != 64) return false;
+    // (fields of a record; 32-bit offsets inside a sample; cells in 16 bits beside a rank)
+    if (P > 512 || p.Q > (1 << 20) || p.Q * P * p.G >= (1ll << 31) || p.Q * p.G * p.D >= (1ll << 31) ||
+        p.S >= (1ll << 29))
+        return false;
+    if (p.Q * P < 8 * p.S) return false;
+    if (p.ref != nullptr && p.D < 64) return p.D == 32 && points >= 3000000;
+    return points >= 1000000;
+}
+
+// With room for some samples only, they take turns; a turn of few points costs more in launches
+// and partly filled waves than sorting saves (four turns of 2 M points: 546 us against 512).
+int64_t sorted_samples_per_turn(const Params &p, bool softmax, int64_t bytes) {
+    int64_t n = p.B;
+    while (n > 0 && sorted_workspace_bytes(p, softmax, n) > bytes) n = n > 8 ? n - n / 8 : n - 1;
+    if (n == 0 || n == p.B) return n;
+    const int64_t turns = (p.B + n - 1) / n;
+    n = (p.B + turns - 1) / turns;                       // turns of about the same size
+    return n * p.G * p.Q * p.L * p.K >= 4000000 ? n : 0;
+}
+
+Params samples_of(const Params &p, int64_t b, int64_t n) {
+    // (16-bit values; offsets may be of that type too)
+    const int64_t GD = (int64_t)p.G * p.D, pairs = p.Q * p.G, points = pairs * p.L * p.K;
+    const int64_t point_bytes = p.ref != nullptr && p.offsets16 ? 4 : 8;
+    auto at = [b](const void *base, int64_t bytes) {
+        return const_cast<char *>(static_cast<const char *>(base)) + b * bytes;
+    };
+    Params r = p;
+    r.B = n;
+    r.value = at(p.value, p.S * GD * 2);
+    r.loc = reinterpret_cast<const float *>(at(p.loc, points * point_bytes));
+    r.attn = at(p.attn, points * 2);
+    r.grad_out = at(p.grad_out, p.Q * GD * 2);
+    r.grad_value = at(p.grad_value, p.S * GD * 2);
+    r.grad_loc = reinterpret_cast<float *>(at(p.grad_loc, points * point_bytes));
+    r.grad_attn = at(p.grad_attn, points * 2);
+    if (p.ref != nullptr) r.ref = p.ref + b * p.Q * p.L * p.ref_coords;
+    return r;
+}
+
+int64_t sorted_workspace_bytes(const Params &p, bool softmax, int64_t samples) {
+    SortPlan sp;
+    return plan_sorted(sp, p, softmax, samples, nullptr);
+}
+
+int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples, void *workspace) {
+    const int64_t P = (int64_t)p.L * p.K;
+    const int64_t planes = samples * p.G;
+    sp.plane_points = p.Q * P;
+    sp.chunk_queries = (int)(kSortThreads / P * kSortPoints);
+    sp.chunks = (int)((p.Q + sp.chunk_queries - 1) / sp.chunk_queries);
+    // a strip is at most 7 pixels short of its width and a level one row high: H + 1 <= 2 H and
+    // ceil((W + 1) / 7) <= W leave at most two cells per pixel
+    sp.prepare_ctas = (int)std::min<int64_t>(148 * 2, 1 + samples * (p.S + p.Q) * p.G * p.D / (8 * kSortThreads * 4));
+    sp.cell_bound = (int)(2 * p.S + 2 * p.L);
+    // a pyramid of ordinary proportions has a cell per five to six pixels
+    sp.shared_cells = (int)std::min<int64_t>(kSharedCells, std::min<int64_t>(sp.cell_bound, round_up(p.S / 5 + 256, 8)));
+    sp.cell_stride = round_up(sp.cell_bound + 1, 32);
+    // Runs of a few hundred points (128 / 256 / 512: 290 / 254 / 276 us of walk at the headline
+    // shape: shorter ones flush too often, longer ones end too unevenly), shorter where that would
+    // leave the GPU's warps without one, longer where a pixel collects thousands of points: every
+    // run adds to it once, in float16
+    const int64_t even = planes * sp.plane_points / (148 * 16 * 4);
+    const int64_t density = sp.plane_points / std::max<int64_t>(p.S, 1);
+    sp.item_points = (int)(std::min<int64_t>(256, std::max<int64_t>(128, even / 32 * 32)) *
+                           std::min<int64_t>(16, 1 + density / 128));
+    sp.items = (int)((sp.plane_points + sp.item_points - 1) / sp.item_points);
+    char *at = static_cast<char *>(workspace);
+    int64_t used = 0;
+    auto take = [&](int64_t bytes) {
+        char *r = at + used;
+        used += round_up(bytes, 256);
+        return r;
+    };
+    sp.header = reinterpret_cast<unsigned *>(take(kScratchHeaderBytes));
+    sp.tickets = reinterpret_cast<unsigned *>(take(planes * 4));
+    sp.counts = reinterpret_cast<unsigned *>(take(planes * sp.cell_stride * 4));
+    sp.cleared_bytes = (size_t)used;
+    sp.offsets = reinterpret_cast<unsigned *>(take(planes * sp.cell_stride * 4));
+    sp.item_cell = reinterpret_cast<int *>(take(planes * sp.items * 4));
+    sp.records = reinterpret_cast<uint4 *>(take(planes * sp.plane_points * 16));
+    sp.grad_prob = reinterpret_cast<float *>(take(planes * sp.plane_points * 4));
+    sp.stats = softmax ? reinterpret_cast<float2 *>(take(planes * p.Q * 8)) : nullptr;
+    return used;
+}
+
+cudaError_t launch_backward_sorted(const Params &p, const SortPlan &sp, int dtype, bool softmax,
+                                   cudaStream_t stream) {
+    if (dtype == 1)
+        return softmax ? launch_sorted_head<__half, true>(p, sp, stream)
+                       : launch_sorted_head<__half, false>(p, sp, stream);
+    return softmax ? launch_sorted_head<__nv_bfloat16, true>(p, sp, stream)
+                   : launch_sorted_head<__nv_bfloat16, false>(p, sp, stream);
+}
+
+}  // namespace msda_b200

@@ -109,8 +109,7 @@ extern "C" int msda_b200_backward_static_scratch(
     // same code path as the caller-scratch entry point from here on; it clears the header and
     // the image this call accumulates into before adding anything
     return msda_b200_backward(value, spatial_shapes, level_start_index, loc, attn, grad_out,
-                              grad_value, grad_loc, grad_attn, scratch,
-                              scratch ? kStaticScratchFloats * (int64_t)sizeof(float) : 0,
+                              grad_value, grad_loc, grad_attn, scratch, scratch ? need : 0,
                               scratch_adds, B, S, G, D, Q, L, K, dtype, apply_softmax,
                               /*zero_grad_value=*/1, device, stream);
 }

@@ -46,7 +46,7 @@ struct Abi {
     decltype(&msda_b200_backward) backward = nullptr;
     decltype(&msda_b200_forward_offsets) forward_offsets = nullptr;
     decltype(&msda_b200_backward_offsets) backward_offsets = nullptr;
-    decltype(&msda_b200_backward_scratch_bytes) scratch_bytes = nullptr;
+    decltype(&msda_b200_backward_workspace_bytes) workspace_bytes = nullptr;
     decltype(&msda_b200_last_error) last_error = nullptr;
 } abi;
 
@@ -137,7 +137,7 @@ variable_list run_backward(const Call &c, const Tensor &grad_in) {
     Tensor grad_value = empty(c.value.sizes(), c.value.scalar_type(), device);
     Tensor grad_points = empty(c.points.sizes(), c.points.scalar_type(), device);
     Tensor grad_attn = empty(c.attn.sizes(), c.attn.scalar_type(), device);
-    const int64_t nbytes = abi.scratch_bytes(c.B, c.S, c.G, c.D, c.Q, c.L, c.K, dtype);
+    const int64_t nbytes = abi.workspace_bytes(c.B, c.S, c.G, c.D, c.Q, c.L, c.K, dtype, c.softmax);
     Tensor scratch;
     if (nbytes > 0) scratch = empty({nbytes}, at::kByte, device);
     void *scratch_ptr = nbytes > 0 ? scratch.mutable_data_ptr() : nullptr;
@@ -347,7 +347,7 @@ PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     abi.backward = reinterpret_cast<decltype(abi.backward)>(p[1]);
     abi.forward_offsets = reinterpret_cast<decltype(abi.forward_offsets)>(p[2]);
     abi.backward_offsets = reinterpret_cast<decltype(abi.backward_offsets)>(p[3]);
-    abi.scratch_bytes = reinterpret_cast<decltype(abi.scratch_bytes)>(p[4]);
+    abi.workspace_bytes = reinterpret_cast<decltype(abi.workspace_bytes)>(p[4]);
     abi.last_error = reinterpret_cast<decltype(abi.last_error)>(p[5]);
     abi.forward = reinterpret_cast<decltype(abi.forward)>(p[0]);
     Py_RETURN_NONE;

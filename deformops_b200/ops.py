@@ -184,7 +184,8 @@ def _make_backward(softmax: bool) -> Callable[..., tuple[Tensor, Tensor, Tensor]
         stream = torch.cuda.current_stream(value.device).cuda_stream
         # scratch of a 16-bit backward (one float16 image of grad_value plus a header); comes
         # from torch's caching allocator, so steady-state calls reuse one block per stream
-        nbytes = shim.scratch_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype]) if Q > 0 else 0
+        nbytes = (shim.workspace_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype], int(softmax))
+                  if Q > 0 else 0)
         scratch = (torch.empty(nbytes, dtype=torch.uint8, device=value.device)
                    if nbytes else None)
         st = shim.backward(_ptr(value), _ptr(spatial_shapes), _ptr(level_start_index), _ptr(loc),
@@ -341,7 +342,8 @@ def _offsets_backward_cuda(value, spatial_shapes, level_start_index, reference_p
     value, reference_points, offsets, attn, grad_output = map(
         _aligned, (value, reference_points, offsets, attn, grad_output))
     stream = torch.cuda.current_stream(value.device).cuda_stream
-    nbytes = shim.scratch_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype]) if Q > 0 else 0
+    nbytes = (shim.workspace_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype], int(softmax))
+              if Q > 0 else 0)
     scratch = (torch.empty(nbytes, dtype=torch.uint8, device=value.device)
                if nbytes else None)
     st = shim.backward_offsets(

@@ -1,0 +1,154 @@
+"""The sorted backward (``csrc/msda_sorted.cu``), which takes dense 16-bit calls of a million
+points and more, against the float64 oracle where it can go wrong: strips and rows at the edges of
+levels, ragged chunks of queries, every head size it has, several turns over the samples, level
+tables it cannot sort, non-finite gradients."""
+
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+import torch
+
+from oracle import msda_oracle as orc
+from tests._abi import _p, abi_backward, dev, dims, to_np
+from tests._golden import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(seed, B, Q, G, D, K, levels, spread=0.3):
+    g = torch.Generator().manual_seed(seed)
+    shapes = torch.tensor(levels, dtype=torch.int64)
+    sizes = shapes[:, 0] * shapes[:, 1]
+    starts = torch.cumsum(sizes, 0) - sizes
+    L, S = len(levels), int(sizes.sum())
+    value = torch.randn(B, S, G, D, generator=g)
+    loc = torch.rand(B, Q, G, L, K, 2, generator=g) * (1 + spread) - spread / 2
+    logits = torch.randn(B, Q, G, L * K, generator=g)
+    grad_out = torch.randn(B, Q, G * D, generator=g)
+    return value, shapes, starts, loc, logits, grad_out
+
+
+def _workspace_backward(value, shapes, starts, loc, attn, grad_out, softmax, nbytes=None):
+    """``msda_b200_backward`` with the scratch it is fastest with (or ``nbytes`` of it)."""
+    from deformops_b200._loader import load_library
+    from deformops_b200.ops import DTYPE_CODES
+
+    shim = load_library()
+    B, S, G, D, Q, L, K = dims(value, loc)
+    code = DTYPE_CODES[value.dtype]
+    if nbytes is None:
+        nbytes = shim.workspace_bytes(B, S, G, D, Q, L, K, code, int(softmax))
+        assert nbytes > shim.scratch_bytes(B, S, G, D, Q, L, K, code), "the call would not be sorted"
+    grads = [torch.full_like(t, float("nan")) for t in (value, loc, attn)]
+    scratch = torch.full((nbytes,), 0xFF, dtype=torch.uint8, device=value.device)
+    st = shim.backward(_p(value), _p(shapes), _p(starts), _p(loc), _p(attn), _p(grad_out),
+                       *[_p(t) for t in grads], _p(scratch), nbytes, 0, B, S, G, D, Q, L, K, code,
+                       int(softmax), 1, value.device.index,
+                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0, shim.last_error()
+    return grads
+
+
+def _check(got, ins, grad_out, softmax, shapes, loc, value_bar=1e-2):
+    truth = orc.backward(*[t.cpu() for t in ins], grad_out.cpu(), softmax=softmax)
+    wh = shapes.flip(-1).double().cpu()[None, None, None, :, None, :]
+    pix = loc.double().cpu() * wh - 0.5
+    keep = ((pix - pix.round()).abs() >= 1e-3).all(-1, keepdim=True).numpy()
+    assert rel_err(to_np(got[0]), truth[0]) <= value_bar
+    assert rel_err(to_np(got[1]) * keep, truth[1].reshape(got[1].shape) * keep) <= 1e-4
+    assert rel_err(to_np(got[2]), truth[2].reshape(got[2].shape)) <= 1e-2
+
+
+@pytest.mark.parametrize("dtype,softmax,D,K,levels,B,Q,G", [
+    # widths that end with, one short of and one beyond a strip (W + 1 = 14, 7, 8, 22); heights 1, 2
+    (torch.bfloat16, False, 32, 4, [(13, 13), (1, 6), (2, 7), (5, 21)], 1, 8209, 8),
+    (torch.float16, True, 32, 5, [(11, 20), (6, 10)], 2, 6500, 8),
+    (torch.bfloat16, True, 64, 3, [(9, 30), (5, 15), (3, 8)], 1, 40111, 3),
+    (torch.float16, False, 64, 8, [(16, 14)], 1, 32769, 4),
+    (torch.bfloat16, False, 16, 1, [(20, 20), (10, 10), (5, 5), (3, 3), (2, 2)], 3, 8333, 9),
+    (torch.float16, True, 16, 64, [(12, 33), (6, 17)], 1, 2051, 4),
+    # more cells than a CTA counts in shared memory: narrow levels
+    (torch.bfloat16, False, 32, 4, [(3000, 2)], 1, 13000, 20),
+])
+def test_sorted_backward_matches_the_oracle(dtype, softmax, D, K, levels, B, Q, G):
+    value, shapes, starts, loc, logits, grad_out = _inputs(K * D + Q, B, Q, G, D, K, levels)
+    attn = logits if softmax else logits.softmax(-1)
+    v, a, go = dev(value, dtype), dev(attn, dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, softmax)
+    _check(got, (v, sh, st, l, a), go, softmax, shapes, l)
+
+
+def test_samples_take_turns_when_the_scratch_holds_only_some():
+    """Three samples of 4.1 M points, scratch for one and for two: the same gradients, from
+    sample bases that are not 16-byte aligned in the weights (Q * G * P odd multiples of 2)."""
+    from deformops_b200._loader import load_library
+
+    B, Q, G, D, K, levels = 3, 45763, 5, 16, 6, [(24, 20), (7, 5), (4, 3)]
+    value, shapes, starts, loc, logits, grad_out = _inputs(3, B, Q, G, D, K, levels)
+    dtype = torch.bfloat16
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    full = load_library().workspace_bytes(B, v.shape[1], G, D, Q, len(levels), K, 2, 0)
+    for nbytes in (full * 45 // 100, full * 9 // 10):
+        got = _workspace_backward(v, sh, st, l, a, go, False, nbytes)
+        _check(got, (v, sh, st, l, a), go, False, shapes, l)
+
+
+@pytest.mark.parametrize("coords,offset_dtype", [(2, torch.bfloat16), (4, torch.float32)])
+def test_sorted_backward_from_offsets(coords, offset_dtype):
+    """Reference points and offsets in place of locations (three million points)."""
+    from deformops_b200.registry import locations_from_offsets, msda, msda_from_offsets
+
+    B, Q, G, D, K, levels = 1, 24000, 8, 32, 8, [(15, 22), (8, 11)]
+    value, shapes, starts, loc, logits, grad_out = _inputs(5, B, Q, G, D, K, levels)
+    dtype = torch.bfloat16
+    g = torch.Generator().manual_seed(6)
+    ref = torch.rand(B, Q, len(levels), coords, generator=g)
+    off = dev(torch.randn(loc.shape, generator=g) * 2, offset_dtype)
+    v, a, go = dev(value, dtype), dev(logits, dtype), dev(grad_out, dtype)
+    r, sh, st = dev(ref, torch.float32), dev(shapes), dev(starts)
+    fused = [t.clone().requires_grad_(True) for t in (v, off, a)]
+    out = msda_from_offsets(fused[0], sh, st, r, fused[1], fused[2], method="softmax")
+    got = torch.autograd.grad(out, fused, go)
+    plain = [t.clone().requires_grad_(True) for t in (v, off, a)]
+    ref_out = msda(plain[0], sh, st, locations_from_offsets(r, plain[1].float(), sh), plain[2],
+                   method="softmax")
+    want = torch.autograd.grad(ref_out, plain, go)
+    assert torch.equal(out, ref_out)
+    for x, y in zip(got, want):                     # (either is rounded to bfloat16)
+        assert x.dtype == y.dtype and rel_err(to_np(x), to_np(y)) <= 1e-2
+
+
+def test_levels_that_overlap_are_served_unsorted():
+    """Sixteen levels on the same rows ask for more cells than a plane has room for.  (The points
+    left out add up in float16, thousands to an element here.)"""
+    B, Q, G, D, K, levels = 1, 4200, 2, 16, 8, [(60, 1)] * 16
+    value, shapes, starts, loc, logits, grad_out = _inputs(7, B, Q, G, D, K, levels)
+    value, starts = value[:, :60].contiguous(), torch.zeros_like(starts)
+    dtype = torch.float16
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, False)
+    _check(got, (v, sh, st, l, a), go, False, shapes, l, value_bar=5e-2)
+
+
+def test_non_finite_gradients_stay_in_their_corners():
+    B, Q, G, D, K, levels = 1, 17000, 8, 32, 4, [(18, 16), (9, 8)]
+    value, shapes, starts, loc, logits, grad_out = _inputs(9, B, Q, G, D, K, levels)
+    dtype = torch.bfloat16
+    grad_out[0, 11, 40] = float("inf")
+    grad_out[0, 12, 200] = float("nan")
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, False)
+    direct = abi_backward(v, sh, st, l, a, go)
+    assert torch.equal(torch.isfinite(got[0]), torch.isfinite(direct[0]))
+    for x, y in zip(got, direct):
+        assert not (torch.isfinite(y) & ~torch.isfinite(x)).any()
+    assert 0 < int((~torch.isfinite(got[0])).sum()) <= 2 * 2 * K * 4
+    fine = torch.isfinite(got[0])
+    assert rel_err(to_np(got[0][fine]), to_np(direct[0][fine])) <= 2e-2
+    assert rel_err(to_np(got[1])[0, 100:], to_np(direct[1])[0, 100:]) <= 1e-5
