@@ -24,7 +24,7 @@ CSRC = PKG / "csrc"
 LIB_DIR = PKG / "_lib"
 LIB_PATH = LIB_DIR / "libmsda_b200.so"
 SOURCES = ["msda_forward.cu", "msda_backward.cu", "msda_abi.cu", "msda_static_scratch.cu",
-           "msda_f64.cu", "msda_sorted.cu"]
+           "msda_f64.cu", "msda_sorted.cu", "msda_linear.cu"]
 HEADERS = [CSRC / "msda_common.cuh", CSRC / "msda_sorted.cuh", PKG.parent / "include" / "msda_b200.h"]
 #: bench-only microbenchmarks of the hardware floors (csrc/floors/bench_floors.cu); never
 #: loaded by the package itself

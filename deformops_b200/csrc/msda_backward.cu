@@ -145,7 +145,8 @@ __global__ void __launch_bounds__(256, MSDA_BWD_MIN_CTAS) backward_kernel(const 
         const int64_t pair0 = group * ppw;
         const int nlive = (int)min((int64_t)ppw, total_pairs - pair0);
         if constexpr (SOFTMAX) {
-            if (lane < nlive) s_stats[lane] = softmax_stats(attn + (pair0 + lane) * P, P);
+            const float2 st = slot_softmax_stats(attn + (pair0 + slot) * P, P, lph, sub, slot < nlive);
+            if (sub == 0) s_stats[slot] = st;
             __syncwarp();
         }
         const bool live = slot < nlive;

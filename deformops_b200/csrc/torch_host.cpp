@@ -16,7 +16,9 @@
 // copy of the library that deformops_b200/_loader.py loaded.
 #include <Python.h>
 
+#include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/record_function.h>
@@ -30,6 +32,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <atomic>
 #include <cstdlib>
@@ -48,6 +51,8 @@ struct Abi {
     decltype(&msda_b200_backward_offsets) backward_offsets = nullptr;
     decltype(&msda_b200_backward_workspace_bytes) workspace_bytes = nullptr;
     decltype(&msda_b200_last_error) last_error = nullptr;
+    decltype(&msda_b200_column_sums) column_sums = nullptr;
+    decltype(&msda_b200_column_sums_scratch_bytes) column_sums_scratch_bytes = nullptr;
 } abi;
 
 std::atomic<int64_t> g_kernels{0}, g_memsets{0};
@@ -200,6 +205,60 @@ struct MsdaFunction : torch::autograd::Function<MsdaFunction<SOFTMAX>> {
     }
 };
 
+// ---- projections with a bias gradient of our own ------------------------------------------------
+Tensor column_sums(const Tensor &x) {
+    const at::Device device = x.device();
+    const c10::cuda::CUDAGuard on_device(device);
+    Tensor out = empty({x.size(1)}, x.scalar_type(), device);
+    Tensor scratch = empty({abi.column_sums_scratch_bytes(x.size(0), x.size(1))}, at::kByte, device);
+    check_status(abi.column_sums(x.const_data_ptr(), out.mutable_data_ptr(), scratch.mutable_data_ptr(),
+                                 x.size(0), x.size(1), dtype_code(x.scalar_type()),
+                                 c10::cuda::getCurrentCUDAStream(device.index()).stream()),
+                 "msda_b200_column_sums");
+    g_kernels.fetch_add(2, std::memory_order_relaxed);
+    return out;
+}
+
+Tensor bias_gradient(const Tensor &g) {
+    // a graph of the gradients needs an operator that has a derivative itself
+    return at::GradMode::is_enabled() && g.requires_grad() ? g.sum(0) : column_sums(g.contiguous());
+}
+
+// y = x W^T + b for each of one or two (W, b); the gradients of x meet in one tensor
+struct LinearFunction : torch::autograd::Function<LinearFunction> {
+    static variable_list forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &w0,
+                                 const Tensor &b0, const std::optional<Tensor> &w1,
+                                 const std::optional<Tensor> &b1) {
+        ctx->save_for_backward({x, w0, w1.value_or(Tensor())});
+        ctx->set_materialize_grads(false);
+        at::AutoDispatchBelowADInplaceOrView below;
+        variable_list out = {at::linear(x, w0, b0)};
+        if (w1) out.push_back(at::linear(x, *w1, *b1));
+        return out;
+    }
+    static variable_list backward(torch::autograd::AutogradContext *ctx, const variable_list &grads) {
+        const variable_list saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0];
+        const Tensor rows = x.reshape({-1, x.size(-1)});
+        variable_list out(5);
+        for (size_t i = 0; i < grads.size(); ++i) {
+            if (!grads[i].defined()) continue;
+            const Tensor &w = saved[1 + i];
+            const Tensor g = grads[i].reshape({-1, grads[i].size(-1)});
+            if (ctx->needs_input_grad(0)) {
+                if (!out[0].defined())
+                    out[0] = at::mm(g, w);
+                else
+                    out[0] = at::GradMode::is_enabled() ? at::addmm(out[0], g, w) : out[0].addmm_(g, w);
+            }
+            if (ctx->needs_input_grad(1 + 2 * i)) out[1 + 2 * i] = at::mm(g.t(), rows);
+            if (ctx->needs_input_grad(2 + 2 * i)) out[2 + 2 * i] = bias_gradient(g);
+        }
+        if (out[0].defined()) out[0] = out[0].view(x.sizes());
+        return out;
+    }
+};
+
 // ---- acceptance ------------------------------------------------------------------------------
 bool plain_thread_state() {
     if (at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
@@ -332,12 +391,58 @@ PyObject *py_msda_offsets(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
+// Below this many rows torch's own reduction is as quick and its call shorter.
+constexpr int64_t kLinearRows = 2048;
+
+bool linear_acceptable(const Tensor &x, const Tensor &w, const Tensor &b) {
+    return w.dim() == 2 && b.dim() == 1 && w.size(1) == x.size(-1) && b.size(0) == w.size(0) &&
+           w.scalar_type() == x.scalar_type() && b.scalar_type() == x.scalar_type();
+}
+
+// linear(x, weight, bias) -> Tensor | None;
+// linear_pair(x, weight, bias, weight, bias) -> (Tensor, Tensor) | None
+template <int N>
+PyObject *py_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(nargs == 1 + 2 * N, "wrong number of arguments");
+    if (abi.forward == nullptr || !all_plain(args, nargs) || !plain_thread_state() ||
+        !at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) ||
+        c10::impl::tls_is_dispatch_key_excluded(c10::DispatchKey::AutogradCUDA))
+        Py_RETURN_NONE;
+    const Tensor &x = THPVariable_Unpack(args[0]);
+    const at::Device device = x.device();
+    bool grad = false;
+    for (Py_ssize_t i = 0; i < nargs; ++i) {
+        const Tensor &t = THPVariable_Unpack(args[i]);
+        if (!plain_tensor(t, device)) Py_RETURN_NONE;
+        grad = grad || t.requires_grad();
+    }
+    if (!grad || dtype_code(x.scalar_type()) < 0 || x.dim() < 2 || !x.is_contiguous() || x.size(-1) == 0 ||
+        x.numel() / x.size(-1) < kLinearRows || !supported_device(device))
+        Py_RETURN_NONE;
+    for (int i = 0; i < N; ++i)
+        if (!linear_acceptable(x, THPVariable_Unpack(args[1 + 2 * i]), THPVariable_Unpack(args[2 + 2 * i])))
+            Py_RETURN_NONE;
+    variable_list out;
+    {
+        pybind11::gil_scoped_release no_gil;
+        std::optional<Tensor> w1, b1;
+        if constexpr (N == 2) w1 = THPVariable_Unpack(args[3]), b1 = THPVariable_Unpack(args[4]);
+        out = LinearFunction::apply(x, THPVariable_Unpack(args[1]), THPVariable_Unpack(args[2]), w1, b1);
+    }
+    if constexpr (N == 1) return THPVariable_Wrap(std::move(out[0]));
+    THPObjectPtr a(THPVariable_Wrap(std::move(out[0]))), b(THPVariable_Wrap(std::move(out[N - 1])));
+    if (!a || !b) return nullptr;
+    return PyTuple_Pack(2, a.get(), b.get());
+    END_HANDLE_TH_ERRORS
+}
+
 // bind(addresses of the ABI functions in the order of struct Abi)
 PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
-    TORCH_CHECK(nargs == 6, "bind takes six addresses");
-    void *p[6];
-    for (int i = 0; i < 6; ++i) {
+    TORCH_CHECK(nargs == 8, "bind takes eight addresses");
+    void *p[8];
+    for (int i = 0; i < 8; ++i) {
         p[i] = PyLong_AsVoidPtr(args[i]);
         if (p[i] == nullptr) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
@@ -349,6 +454,8 @@ PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     abi.backward_offsets = reinterpret_cast<decltype(abi.backward_offsets)>(p[3]);
     abi.workspace_bytes = reinterpret_cast<decltype(abi.workspace_bytes)>(p[4]);
     abi.last_error = reinterpret_cast<decltype(abi.last_error)>(p[5]);
+    abi.column_sums = reinterpret_cast<decltype(abi.column_sums)>(p[6]);
+    abi.column_sums_scratch_bytes = reinterpret_cast<decltype(abi.column_sums_scratch_bytes)>(p[7]);
     abi.forward = reinterpret_cast<decltype(abi.forward)>(p[0]);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
@@ -366,6 +473,8 @@ PyCFunction as_method(F f) {
 PyMethodDef methods[] = {
     {"msda", as_method(py_msda), METH_FASTCALL, nullptr},
     {"msda_offsets", as_method(py_msda_offsets), METH_FASTCALL, nullptr},
+    {"linear", as_method(py_linear<1>), METH_FASTCALL, nullptr},
+    {"linear_pair", as_method(py_linear<2>), METH_FASTCALL, nullptr},
     {"bind", as_method(py_bind), METH_FASTCALL, nullptr},
     {"launches", py_launches, METH_NOARGS, "kernels and memsets issued through this module"},
     {nullptr, nullptr, 0, nullptr}};

@@ -27,6 +27,7 @@ from typing import Any
 import torch
 from torch import Tensor, nn
 
+from ..core.linear import project, project_pair
 from ..core.runtime import Method
 from ..registry.msda import (Backend, MSDABackend, locations_from_offsets, msda,
                              msda_from_offsets)
@@ -88,12 +89,13 @@ class Mask2FormerPixelDecoderEncoderMultiscaleDeformableAttention(_HF_M2F):
         shapes = torch.tensor([list(s) for s in spatial_shapes_list], dtype=torch.int64,
                               device=hidden_states.device)
 
-        value = self.value_proj(encoder_hidden_states)
+        value = project(self.value_proj, encoder_hidden_states)
         if attention_mask is not None:
             value = value.masked_fill(attention_mask[..., None], 0.0)
         value = value.view(B, S, G, self.d_model // G)
-        offsets = self.sampling_offsets(hidden_states).view(B, Q, G, L, K, 2)
-        logits = self.attention_weights(hidden_states).view(B, Q, G, L * K)
+        offsets, logits = project_pair(self.sampling_offsets, self.attention_weights, hidden_states)
+        offsets = offsets.view(B, Q, G, L, K, 2)
+        logits = logits.view(B, Q, G, L * K)
 
         if reference_points.shape[-1] not in (2, 4):
             raise ValueError("Last dim of reference_points must be 2 or 4, but got "
@@ -112,7 +114,7 @@ class Mask2FormerPixelDecoderEncoderMultiscaleDeformableAttention(_HF_M2F):
             out = msda_from_offsets(value, shapes, level_start_index, reference_points, offsets,
                                     logits, method=Method.SOFTMAX)
         weights = torch.softmax(logits, -1).view(B, Q, G, L, K) if output_attentions else None
-        return self.output_proj(out), weights
+        return project(self.output_proj, out), weights
 
 
 def patch(model: nn.Module, *, backend: "Backend | MSDABackend | None" = None) -> nn.Module:

@@ -26,6 +26,7 @@ from typing import Any
 import torch
 from torch import Tensor, nn
 
+from ..core.linear import project, project_pair
 from ..core.runtime import Method
 from ..registry.msda import Backend, MSDABackend, msda, msda_from_offsets
 
@@ -107,8 +108,8 @@ class MultiScaleDeformAttn2d(nn.Module):
     def sampling_locations(self, q: Tensor, p: Tensor, spatial_shapes: Tensor) -> Tensor:
         """``(B, Q, G, L, K, 2)`` normalised sample locations predicted from the queries."""
         B, Q, _ = q.shape
-        offset = self.proj_offset(q).view(B, Q, self.num_heads, self.num_levels,
-                                          self.num_points, 2)
+        offset = project(self.proj_offset, q).view(B, Q, self.num_heads, self.num_levels,
+                                                   self.num_points, 2)
         ref = p[:, :, None, :, None, :]
         if p.shape[-1] == 2:
             wh = spatial_shapes.flip(-1).to(offset.dtype)             # (L, 2) as (width, height)
@@ -122,29 +123,31 @@ class MultiScaleDeformAttn2d(nn.Module):
         """``q (B,Q,dim)``, ``p (B,Q,L,2|4)``, ``v (B,N,dim_value)`` -> ``(B,Q,dim_output)``."""
         B, Q, _ = q.shape
         N = v.shape[1]
-        value = self.proj_value(v)
+        value = project(self.proj_value, v)
         if padding_mask is not None:
             value = value.masked_fill(padding_mask[..., None], 0.0)
         value = value.view(B, N, self.num_heads, self.dim // self.num_heads)
-        weights = self.proj_weights(q).view(B, Q, self.num_heads,
-                                            self.num_levels * self.num_points)
-
-        if isinstance(self.backend, MSDABackend):
-            locations = self.sampling_locations(q, p, spatial_shapes)
-            out = self.backend.forward(value, spatial_shapes, level_start_index, locations,
-                                       weights, self.chunk_step, self.method)
-        elif self.fuse_locations:
+        fused = self.fuse_locations and not isinstance(self.backend, MSDABackend)
+        if fused:
             # the kernels add the offsets to the reference points themselves; no location
             # tensor is built
             msda._only_cuda(self.backend)
-            offset = self.proj_offset(q).view(B, Q, self.num_heads, self.num_levels,
-                                              self.num_points, 2)
+            offset, weights = project_pair(self.proj_offset, self.proj_weights, q)
+            offset = offset.view(B, Q, self.num_heads, self.num_levels, self.num_points, 2)
+        else:
+            locations = self.sampling_locations(q, p, spatial_shapes)
+            weights = project(self.proj_weights, q)
+        weights = weights.view(B, Q, self.num_heads, self.num_levels * self.num_points)
+
+        if isinstance(self.backend, MSDABackend):
+            out = self.backend.forward(value, spatial_shapes, level_start_index, locations,
+                                       weights, self.chunk_step, self.method)
+        elif fused:
             out = msda_from_offsets(value, spatial_shapes, level_start_index, p, offset, weights,
                                     method=self.method)
         else:
-            locations = self.sampling_locations(q, p, spatial_shapes)
             options: dict[str, Any] = {"method": self.method, "backend": self.backend}
             if self.backend is not None:
                 options["chunk_step"] = self.chunk_step
             out = msda(value, spatial_shapes, level_start_index, locations, weights, **options)
-        return self.proj_output(out)
+        return project(self.proj_output, out)

@@ -138,6 +138,16 @@ int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int6
                                            int64_t L, int64_t K, int dtype, int apply_softmax);
 
 /*
+ * out[c] = sum over r of x[r][c], for a contiguous (rows, cols) matrix: the bias gradient of a
+ * layer's projection.  float32 accumulation, the same result on every run; x and out in `dtype`
+ * (float32, float16, bfloat16).  `scratch` holds msda_b200_column_sums_scratch_bytes(...) bytes.
+ * Launches two kernels on `stream`, whose device has to be current.
+ */
+int msda_b200_column_sums(const void *x, void *out, void *scratch, int64_t rows, int64_t cols,
+                          int dtype, void *stream);
+int64_t msda_b200_column_sums_scratch_bytes(int64_t rows, int64_t cols);
+
+/*
  * Forward / backward with the caller's location arithmetic fused in.  Instead of a location
  * tensor the call takes what a deformable-attention layer predicts and where it anchors it:
  *   offsets           (B, Q, G, L, K, 2)  float32 or `dtype` (offsets_dtype says which)
