@@ -467,22 +467,17 @@ template <typename T, bool SOFTMAX, bool SCALED>
 cudaError_t launch_kernel(const Params &p, cudaStream_t stream) {
     const size_t smem = backward_smem_bytes(p, SOFTMAX);
     auto kernel = backward_kernel<T, SOFTMAX, SCALED>;
-    if (smem > 48 * 1024) {  // opt in to large dynamic shared memory only when needed
+    if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     // Two adjacent passes per CTA once that still leaves every SM several waves of CTAs
     // (the per-CTA prologue is paid half as often; worth about 0.2 % at the headline shape).
+    static Residency residency;
     Params q = p;
-    int device = 0, sms = 0, per_sm = 0;
-    q.passes = 1;
-    if (cudaGetDevice(&device) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p.threads, smem) ==
-            cudaSuccess &&
-        sms > 0 && per_sm > 0 && p.grid >= 8u * (unsigned)(sms * per_sm))
-        q.passes = 2;
+    const unsigned resident = residency.ctas(kernel, p.threads, smem);
+    q.passes = resident > 0 && p.grid >= 8u * resident ? 2 : 1;
     const int64_t per_cta = (int64_t)(p.threads / 32) * q.passes;   // groups one CTA covers
     const int64_t ctas = (p.num_groups + per_cta - 1) / per_cta;
     if (ctas > 0x7fffffffll) return cudaErrorInvalidConfiguration;   // > 10^11 pairs

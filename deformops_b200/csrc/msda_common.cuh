@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace msda_b200 {
 
 constexpr int kMaxLevels = 16;           // level table kept in shared memory
@@ -248,14 +250,14 @@ __device__ __forceinline__ void grid_launch_dependents() {
 // rate, went from 0.052 to 0.065 ms with it, the headline shape from 0.530 to 0.525 ms), so it
 // is used only for calls whose kernels run long enough to hide that.
 inline bool worth_dependent_launch(const Params &p) {
-    return p.B * p.Q * p.G * (int64_t)(p.L * p.K) >= ((int64_t)1 << 21);
+    return p.B * p.Q * p.G * (int64_t)(p.L * p.K) >= ((int64_t)1 << 20);
 }
 
-template <typename Kernel>
+template <typename Kernel, typename... More>
 inline cudaError_t launch_after_predecessor(Kernel kernel, unsigned grid, unsigned threads, size_t smem,
-                                            cudaStream_t stream, const Params &p) {
+                                            cudaStream_t stream, const Params &p, const More &...more) {
     if (!worth_dependent_launch(p)) {
-        kernel<<<grid, threads, smem, stream>>>(p);
+        kernel<<<grid, threads, smem, stream>>>(p, more...);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
@@ -268,8 +270,36 @@ inline cudaError_t launch_after_predecessor(Kernel kernel, unsigned grid, unsign
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
+    return cudaLaunchKernelEx(&cfg, kernel, p, more...);
 }
+
+// Shared memory a kernel may ask for without opting in, beside the level table and the like that
+// these kernels hold statically.
+constexpr size_t kPlainSmem = 46 * 1024;
+
+// CTAs of a kernel the GPU holds at once for a block size and a shared memory size.  The runtime is
+// asked once per combination (a query costs the host about as much as a launch); every GPU
+// this is built for answers alike.
+class Residency {
+  public:
+    template <typename Kernel>
+    unsigned ctas(Kernel kernel, int threads, size_t smem) {
+        const uint64_t key = (uint64_t)smem << 12 | (uint64_t)threads;
+        const uint64_t known = last_.load(std::memory_order_relaxed);
+        if (known >> 24 == key) return (unsigned)(known & 0xffffffu);
+        int device = 0, sms = 0, per_sm = 0;
+        if (cudaGetDevice(&device) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+            return 0;
+        const unsigned resident = (unsigned)sms * (unsigned)per_sm;
+        last_.store(key << 24 | resident, std::memory_order_relaxed);
+        return resident;
+    }
+
+  private:
+    std::atomic<uint64_t> last_{0};
+};
 
 __device__ __forceinline__ uint4 ld_stream16(const void *p) {
     uint4 r;

@@ -26,17 +26,21 @@
 #ifndef MSDA_FWD_MIN_CTAS
 #define MSDA_FWD_MIN_CTAS 4
 #endif
+// the same for calls that do not fill the GPU: their time is one warp's chain of round trips
+#ifndef MSDA_FWD_SMALL_UNROLL
+#define MSDA_FWD_SMALL_UNROLL 4
+#endif
 
 namespace msda_b200 {
 
 namespace {
 
-template <typename T, bool SOFTMAX>
-__global__ void __launch_bounds__(256, MSDA_FWD_MIN_CTAS) forward_kernel(const Params p) {
+template <typename T, bool SOFTMAX, bool SMALL>
+__global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_kernel(const Params p) {
     using VT = VecTraits<T>;
     constexpr int V = VT::kVec;
     constexpr int NV2 = V / 2;
-    constexpr int kUnroll = MSDA_FWD_UNROLL;
+    constexpr int kUnroll = SMALL ? MSDA_FWD_SMALL_UNROLL : MSDA_FWD_UNROLL;
     extern __shared__ uint4 smem[];
     __shared__ LevelTable lt;
 
@@ -159,11 +163,11 @@ __global__ void __launch_bounds__(256, MSDA_FWD_MIN_CTAS) forward_kernel(const P
     }
 }
 
-template <typename T, bool SOFTMAX>
-cudaError_t launch_typed(const Params &p, cudaStream_t stream) {
+template <typename T, bool SOFTMAX, bool SMALL>
+cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     const size_t smem = forward_smem_bytes(p, SOFTMAX);
-    auto kernel = forward_kernel<T, SOFTMAX>;
-    if (smem > 48 * 1024) {  // opt in to large dynamic shared memory only when needed
+    auto kernel = forward_kernel<T, SOFTMAX, SMALL>;
+    if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -172,21 +176,31 @@ cudaError_t launch_typed(const Params &p, cudaStream_t stream) {
     // groups with the grid stride.  Measured on B200 at the headline shape: 0.175 ms against
     // 0.193 ms for one CTA per eight groups (the level table is loaded once per CTA instead of
     // eighteen times, and the resident CTAs sweep the queries as one compact front).
+    static Residency residency;
     Params q = p;
-    int device = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&device) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p.threads, smem) ==
-            cudaSuccess &&
-        sms > 0 && per_sm > 0) {
+    unsigned resident = residency.ctas(kernel, p.threads, smem);
 #ifdef MSDA_FWD_CTAS_PER_SM
-        per_sm = MSDA_FWD_CTAS_PER_SM;
+    resident = 148 * MSDA_FWD_CTAS_PER_SM;
 #endif
-        const unsigned resident = (unsigned)sms * (unsigned)per_sm;
-        if (q.grid > resident) q.grid = resident;
-    }
+    if (resident > 0 && q.grid > resident) q.grid = resident;
     kernel<<<q.grid, q.threads, smem, stream>>>(q);
     return cudaGetLastError();
+}
+
+template <typename T, bool SOFTMAX>
+cudaError_t launch_typed(const Params &p, cudaStream_t stream) {
+    // Up to four groups per SM the call lasts as long as one warp's chain of loads: more points in
+    // flight per warp, and as few warps per CTA as still reach every SM.  Measured on B200, a
+    // decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in flight 6.1, 6 6.6;
+    // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
+    constexpr int kSms = 148;
+    if (p.num_groups > 4 * kSms) return launch_as<T, SOFTMAX, false>(p, stream);
+    Params q = p;
+    int warps = 1;
+    while (warps < p.threads / 32 && warps * kSms < p.num_groups) warps *= 2;
+    q.threads = warps * 32;
+    q.grid = (unsigned)((p.num_groups + warps - 1) / warps);
+    return launch_as<T, SOFTMAX, true>(q, stream);
 }
 
 }  // namespace
