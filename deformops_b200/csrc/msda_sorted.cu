@@ -320,6 +320,7 @@ __device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item
 template <typename T, bool SOFTMAX, bool REF>
 __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __grid_constant__ Params p,
     const __grid_constant__ SortPlan sp) {
+    grid_launch_dependents();
     // the first CTAs look for the magnitudes and clear grad_value, beside those that count
     if (blockIdx.x < (unsigned)sp.prepare_ctas) {
         prepare_share<T, SOFTMAX>(p, sp, (int)blockIdx.x, sp.prepare_ctas);
@@ -469,6 +470,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     if (in_shared)
         for (int i = threadIdx.x; i < cells; i += kSortThreads) shift[i] = 0u;
     const SortLane c = sort_lane(p, sp, lt, ct, blockIdx.x);
+    grid_launch_dependents();
+    grid_dependency_wait();     // everything above reads the caller's tables only
     unsigned *cursor = sp.counts + (int64_t)c.plane * sp.cell_stride;
     uint4 *records = sp.records + (int64_t)c.plane * sp.plane_points;
     const T *attn = reinterpret_cast<const T *>(p.attn);
@@ -699,6 +702,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
     if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
     __syncthreads();
 
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = lane >> 2, c = lane & 3;
     if (unsortable_call<T>(sp.header)) return;
@@ -977,6 +982,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
 template <typename T, bool SOFTMAX>
 __global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_constant__ Params p,
     const __grid_constant__ SortPlan sp) {
+    grid_dependency_wait();
     using VT = VecTraits<T>;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1072,8 +1078,8 @@ cudaError_t launch_walk(const Params &p, const SortPlan &sp, bool softmax, cudaS
     }();
     if (resident <= 0) return cudaErrorInvalidConfiguration;
     const int64_t ctas = (p.B * p.G * (int64_t)sp.items + kWalkWarps - 1) / kWalkWarps;
-    walk<<<(unsigned)std::min<int64_t>(ctas, resident), kWalkWarps * 32, smem, stream>>>(p, sp, softmax);
-    return cudaGetLastError();
+    return launch_after_predecessor(walk, (unsigned)std::min<int64_t>(ctas, resident), kWalkWarps * 32, smem, stream,
+                                    p, sp, softmax);
 }
 
 template <typename T, int D, bool SOFTMAX>
@@ -1088,14 +1094,15 @@ cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_
     count<<<planes * (unsigned)sp.chunks + sp.prepare_ctas, kSortThreads, hist, stream>>>(p, sp);
     e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
     if (e != cudaSuccess) return e;
-    scatter<<<planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream>>>(p, sp);
+    e = launch_after_predecessor(scatter, planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream, p, sp);
+    if (e != cudaSuccess) return e;
     e = p.ref != nullptr ? launch_walk<T, D, true>(p, sp, SOFTMAX, stream)
                          : launch_walk<T, D, false>(p, sp, SOFTMAX, stream);
     if (e != cudaSuccess) return e;
     const int64_t vecs = p.B * p.S * (p.G * D / 8);
     const int64_t blocks = (vecs + 1023) / 1024;
-    sorted_finish_kernel<T, SOFTMAX><<<(unsigned)std::min<int64_t>(blocks, 148 * 4), 256, 0, stream>>>(p, sp);
-    return cudaGetLastError();
+    return launch_after_predecessor(sorted_finish_kernel<T, SOFTMAX>, (unsigned)std::min<int64_t>(blocks, 148 * 4),
+                                    256, 0, stream, p, sp);
 }
 
 template <typename T, bool SOFTMAX>
