@@ -191,7 +191,8 @@ int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int6
     msda_b200::Params p{};
     p.B = B, p.S = S, p.Q = Q;
     p.G = (int)G, p.D = (int)D, p.L = (int)L, p.K = (int)K;
-    if (!msda_b200::sorting_pays(p, dtype)) return scratch;
+    if (!msda_b200::sorting_pays(p, dtype))
+        return msda_b200::fused_backward_pays(p) ? (scratch + 15) / 16 * 16 + msda_b200::kFusedBytes : scratch;
     // all samples at once, or as many as the target holds (at least one)
     int64_t samples = B;
     while (samples > 1 && msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples) > kWorkspaceTarget)
@@ -409,6 +410,15 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
                 if (e != cudaSuccess) return cuda_fail(e, "backward: kernel launch (sorted)");
             }
             return MSDA_B200_OK;
+        }
+    }
+    if (use_scratch && msda_b200::fused_backward_pays(p)) {
+        const int64_t usual =
+            (msda_b200_backward_scratch_bytes(B, S, G, D, Q, L, K, dtype) + 15) / 16 * 16;
+        if (scratch_bytes >= usual + msda_b200::kFusedBytes) {
+            p.fused_magnitudes = static_cast<char *>(scratch) + usual;
+            e = msda_b200::launch_backward_fused(p, dtype, apply_softmax != 0, s);
+            return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "backward: kernel launch (cooperative)");
         }
     }
     if (use_scratch) {

@@ -26,6 +26,9 @@
 // that receives more than 256 additions per element gets extra replicas of itself there.
 // prepare_kernel clears what is added into and finds the magnitudes the scale is derived from,
 // finalize_kernel sums the replicas, unscales and writes grad_value in its own type.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <type_traits>
 
 #include "msda_common.cuh"
@@ -74,9 +77,179 @@ namespace msda_b200 {
 
 namespace {
 
-// SCALED: grad_value contributions go, times 2^e, into the float16 image of the scratch
-template <typename T, bool SOFTMAX, bool SCALED>
-__global__ void __launch_bounds__(256, MSDA_BWD_MIN_CTAS) backward_kernel(const Params p) {
+// ---- scaled float16 image: preparation and finalisation ----------------------------------------
+// Clears the float16 image the backward adds into and leaves the largest |grad_out| (and, without
+// softmax, |attn|) element that the CTA's threads found in cta_max[0] / [1].
+template <bool WITH_ATTN>
+__device__ __forceinline__ void prepare_image(const Params &p, unsigned (&cta_max)[2]) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint4 *image = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(p.scratch) + kScratchHeaderBytes);
+    const int64_t image_vecs = p.B * p.S * (p.G * p.D / 8);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    // (the extras are cleared in full: at most K*Q*G*D*L / 64 elements per sample)
+    const int64_t clear_vecs = image_vecs + p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
+    unsigned mg = 0, ma = 0;
+    const int64_t go_vecs = p.B * p.Q * (p.G * p.D / 8);
+    const uint4 *go = reinterpret_cast<const uint4 *>(p.grad_out);
+    mg = scan_max_magnitude(go, go_vecs, first, stride);
+    if constexpr (WITH_ATTN) {
+        // (B*Q*G*L*K 16-bit elements; the tail that does not fill a vector is read singly)
+        const int64_t n = p.B * p.Q * p.G * p.L * p.K;
+        const uint4 *at = reinterpret_cast<const uint4 *>(p.attn);
+        ma = scan_max_magnitude(at, n / 8, first, stride);
+        const unsigned short *tail = reinterpret_cast<const unsigned short *>(p.attn);
+        for (int64_t i = (n / 8) * 8 + first; i < n; i += stride) ma = max(ma, tail[i] & 0x7fffu);
+    }
+    // the clearing stores come after the scan's loads were issued: they need no answer, and the
+    // loads' round trips to DRAM are the longest thing this kernel waits for
+    for (int64_t v = first; v < clear_vecs; v += stride) image[v] = zero;
+    // one atomic per CTA and cell: the warps' maxima meet in shared memory first (every warp
+    // finishes at about the same time, and same-address atomics are served one after another)
+    if (threadIdx.x < 2) cta_max[threadIdx.x] = 0u;
+    __syncthreads();
+    mg = __reduce_max_sync(0xffffffffu, mg);
+    if constexpr (WITH_ATTN) ma = __reduce_max_sync(0xffffffffu, ma);
+    if ((threadIdx.x & 31) == 0) {
+        if (mg != 0) atomicMax(&cta_max[0], mg);
+        if (WITH_ATTN && ma != 0) atomicMax(&cta_max[1], ma);
+    }
+    __syncthreads();
+}
+
+// ... as a kernel of its own, which records the magnitudes in the scratch header.  The header
+// cells were set to zero on the stream before this kernel.
+template <bool WITH_ATTN>
+__global__ void __launch_bounds__(256, MSDA_PREP_MIN_CTAS) prepare_kernel(const Params p) {
+    grid_launch_dependents();   // the backward kernel may load its tables meanwhile
+    __shared__ unsigned cta_max[2];
+    prepare_image<WITH_ATTN>(p, cta_max);
+    unsigned *header = reinterpret_cast<unsigned *>(p.scratch);
+    if (threadIdx.x < (WITH_ATTN ? 2 : 1) && cta_max[threadIdx.x] != 0)
+        atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
+}
+
+// grad_value = (image + the replicas of the position's level) * 2^-e, rounded to T.
+// Positions of levels that have replicas form a small range of every sample (the coarse levels:
+// 1 024 of 21 504 positions at the headline shape); everything outside it takes the short path.
+// `lt` has its replicas planned; `extra_range` is the CTA's.
+__device__ __forceinline__ void find_extra_range(const LevelTable &lt, int L, int (&extra_range)[2]) {
+    int lo = 0x7fffffff, hi = 0;
+    for (int l = 0; l < L; ++l)
+        if (lt.rep[l] > 1) {
+            lo = min(lo, lt.start[l]);
+            hi = max(hi, lt.start[l] + lt.H[l] * lt.W[l]);
+        }
+    extra_range[0] = lo;
+    extra_range[1] = hi;
+}
+
+template <typename T>
+__device__ __forceinline__ void finalize_image(const Params &p, const LevelTable &lt,
+                                               const int (&extra_range)[2], int exponent) {
+    using VT = VecTraits<T>;
+    const int extra_lo = extra_range[0], extra_hi = extra_range[1];
+    const bool any_extra = extra_lo < extra_hi;
+    const int GD = p.G * p.D;
+    const int vec_per_row = GD / 8;
+    const int S = (int)p.S;
+    const int64_t extra_sample = extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K);
+    const float inv = ldexpf(1.f, -exponent);
+    const float2 inv2 = make_float2(inv, inv);
+    const uint4 *image = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(p.scratch) +
+                                                         kScratchHeaderBytes);
+    const __half *extras = reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)GD;
+    uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
+    const int64_t total = p.B * p.S * (int64_t)vec_per_row;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // where the thread's current vector lies - sample b, position s of the sample, vector col of
+    // the position's row - kept up to date by additions: one division per thread, none per vector
+    // (first and stride are below 2^31: the grid is capped at a few thousand CTAs of 256 threads)
+    const unsigned first_row = (unsigned)first / (unsigned)vec_per_row;
+    int col = (int)((unsigned)first - first_row * (unsigned)vec_per_row);
+    int64_t b = first_row / (unsigned)S;
+    int s = (int)(first_row - (unsigned)b * (unsigned)S);
+    const unsigned step_rows_all = (unsigned)stride / (unsigned)vec_per_row;
+    const int step_cols = (int)((unsigned)stride - step_rows_all * (unsigned)vec_per_row);
+    const int step_samples = (int)(step_rows_all / (unsigned)S);          // whole samples per stride
+    const int step_rows = (int)(step_rows_all - (unsigned)step_samples * (unsigned)S);
+    constexpr int kTurn = MSDA_FIN_VECS;
+    for (int64_t v0 = first; v0 < total; v0 += kTurn * stride) {
+        // several vectors per turn, their image loads issued together
+        uint4 raw[kTurn];
+#pragma unroll
+        for (int u = 0; u < kTurn; ++u)
+            raw[u] = v0 + u * stride < total ? ld_stream16(image + v0 + u * stride)
+                                             : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < kTurn; ++u) {
+            const int64_t v = v0 + u * stride;
+            if (v >= total) break;
+            float2 f[4];
+            VecTraits<__half>::unpack(raw[u], f);
+            if (any_extra) {
+                if (s >= extra_lo && s < extra_hi) {
+                    const __half *sample_extras = extras + b * extra_sample + col * 8;
+                    // every level whose range holds this position (one, for a well-formed table)
+                    for (int l = 0; l < p.L; ++l) {
+                        const int at = s - lt.start[l];
+                        if (lt.rep[l] <= 1 || at < 0 || at >= lt.H[l] * lt.W[l]) continue;
+                        const __half *src = sample_extras + lt.rep_base[l] + (int64_t)at * GD;
+                        for (int r = 1; r < lt.rep[l]; ++r) {
+                            float2 x[4];
+                            VecTraits<__half>::unpack(
+                                ld_stream16(src + (int64_t)(r - 1) * lt.level_elems[l]), x);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                f[i].x += x[i].x;
+                                f[i].y += x[i].y;
+                            }
+                        }
+                    }
+                }
+                // on to the vector one stride further
+                col += step_cols;
+                s += step_rows;
+                b += step_samples;
+                if (col >= vec_per_row) {
+                    col -= vec_per_row;
+                    ++s;
+                }
+                if (s >= S) {
+                    s -= S;
+                    ++b;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) f[i] = fmul2(f[i], inv2);
+            gv[v] = VT::pack(f);
+        }
+    }
+}
+
+template <typename T, bool SOFTMAX>
+__global__ void __launch_bounds__(256, MSDA_FIN_MIN_CTAS) finalize_kernel(const Params p) {
+    __shared__ LevelTable lt;
+    __shared__ int extra_range[2];
+    load_level_table(lt, p);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        plan_replicas(lt, p);
+        find_extra_range(lt, p.L, extra_range);
+    }
+    __syncthreads();
+    grid_dependency_wait();     // the image is complete once the backward kernel has finished
+    finalize_image<T>(p, lt, extra_range,
+                      grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch), p.Q, p.K, SOFTMAX));
+}
+
+// SCALED: grad_value contributions go, times 2^e, into the float16 image of the scratch.
+// FUSED: the sweeps before and after are part of the same cooperative launch, between grid
+// barriers.  A small call is bound by the host's launches (a header memset and three kernels took it
+// 16 us, one cooperative launch 6), not by the GPU.
+template <typename T, bool SOFTMAX, bool SCALED, bool FUSED>
+__global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_kernel(const Params p) {
     using VT = VecTraits<T>;
     constexpr int V = VT::kVec;
     constexpr int NV2 = V / 2;
@@ -112,10 +285,32 @@ __global__ void __launch_bounds__(256, MSDA_BWD_MIN_CTAS) backward_kernel(const 
     // written by the kernel before this one
     grid_dependency_wait();
     grid_launch_dependents();
+    __shared__ unsigned magnitudes[2];
+    const unsigned *header = reinterpret_cast<const unsigned *>(p.scratch);
+    if constexpr (FUSED) {
+        // every CTA leaves what it found in a place of its own: nothing has to be zero beforehand
+        prepare_image<!SOFTMAX>(p, magnitudes);
+        uint2 *found = reinterpret_cast<uint2 *>(p.fused_magnitudes);
+        if (threadIdx.x == 0) found[blockIdx.x] = make_uint2(magnitudes[0], magnitudes[1]);
+        cooperative_groups::this_grid().sync();
+        unsigned mg = 0, ma = 0;
+        for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+            const uint2 m = __ldcg(found + i);
+            mg = max(mg, m.x);
+            ma = max(ma, m.y);
+        }
+        mg = __reduce_max_sync(0xffffffffu, mg);
+        ma = __reduce_max_sync(0xffffffffu, ma);
+        if (lane == 0) {
+            atomicMax(&magnitudes[0], mg);
+            atomicMax(&magnitudes[1], ma);
+        }
+        __syncthreads();
+        header = magnitudes;
+    }
     float scale = 1.f;
     if constexpr (SCALED) {
-        scale = ldexpf(1.f, grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch),
-                                                   p.Q, K, SOFTMAX));
+        scale = ldexpf(1.f, grad_scale_exponent<T>(header, p.Q, K, SOFTMAX));
         if (threadIdx.x == 0) plan_replicas(lt, p);
         __syncthreads();
     }
@@ -311,162 +506,18 @@ __global__ void __launch_bounds__(256, MSDA_BWD_MIN_CTAS) backward_kernel(const 
         }
         __syncwarp();
     }
-}
-
-// ---- scaled float16 image: preparation and finalisation ----------------------------------------
-// Clears the float16 image the backward kernel adds into and records the largest |grad_out|
-// (and, without softmax, |attn|) element in the scratch header.  The header cells were set to
-// zero on the stream before this kernel.
-template <bool WITH_ATTN>
-__global__ void __launch_bounds__(256, MSDA_PREP_MIN_CTAS) prepare_kernel(const Params p) {
-    grid_launch_dependents();   // the backward kernel may load its tables meanwhile
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned *header = reinterpret_cast<unsigned *>(p.scratch);
-    uint4 *image = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(p.scratch) + kScratchHeaderBytes);
-    const int64_t image_vecs = p.B * p.S * (p.G * p.D / 8);
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    // (the extras are cleared in full: at most K*Q*G*D*L / 64 elements per sample)
-    const int64_t clear_vecs = image_vecs + p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
-    unsigned mg = 0, ma = 0;
-    const int64_t go_vecs = p.B * p.Q * (p.G * p.D / 8);
-    const uint4 *go = reinterpret_cast<const uint4 *>(p.grad_out);
-    mg = scan_max_magnitude(go, go_vecs, first, stride);
-    if constexpr (WITH_ATTN) {
-        // (B*Q*G*L*K 16-bit elements; the tail that does not fill a vector is read singly)
-        const int64_t n = p.B * p.Q * p.G * p.L * p.K;
-        const uint4 *at = reinterpret_cast<const uint4 *>(p.attn);
-        ma = scan_max_magnitude(at, n / 8, first, stride);
-        const unsigned short *tail = reinterpret_cast<const unsigned short *>(p.attn);
-        for (int64_t i = (n / 8) * 8 + first; i < n; i += stride) ma = max(ma, tail[i] & 0x7fffu);
-    }
-    // the clearing stores come after the scan's loads were issued: they need no answer, and the
-    // loads' round trips to DRAM are the longest thing this kernel waits for
-    for (int64_t v = first; v < clear_vecs; v += stride) image[v] = zero;
-    // one atomic per CTA and cell: the warps' maxima meet in shared memory first (every warp
-    // finishes at about the same time, and same-address atomics are served one after another)
-    __shared__ unsigned cta_max[2];
-    if (threadIdx.x < 2) cta_max[threadIdx.x] = 0u;
-    __syncthreads();
-    mg = __reduce_max_sync(0xffffffffu, mg);
-    if constexpr (WITH_ATTN) ma = __reduce_max_sync(0xffffffffu, ma);
-    if ((threadIdx.x & 31) == 0) {
-        if (mg != 0) atomicMax(&cta_max[0], mg);
-        if (WITH_ATTN && ma != 0) atomicMax(&cta_max[1], ma);
-    }
-    __syncthreads();
-    if (threadIdx.x < (WITH_ATTN ? 2 : 1) && cta_max[threadIdx.x] != 0)
-        atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
-}
-
-// grad_value = (image + the replicas of the position's level) * 2^-e, rounded to T.
-// Positions of levels that have replicas form a small range of every sample (the coarse levels:
-// 1 024 of 21 504 positions at the headline shape); everything outside it takes the short path.
-template <typename T, bool SOFTMAX>
-__global__ void __launch_bounds__(256, MSDA_FIN_MIN_CTAS) finalize_kernel(const Params p) {
-    using VT = VecTraits<T>;
-    __shared__ LevelTable lt;
-    __shared__ int extra_range[2];
-    load_level_table(lt, p);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        plan_replicas(lt, p);
-        int lo = 0x7fffffff, hi = 0;
-        for (int l = 0; l < p.L; ++l)
-            if (lt.rep[l] > 1) {
-                lo = min(lo, lt.start[l]);
-                hi = max(hi, lt.start[l] + lt.H[l] * lt.W[l]);
-            }
-        extra_range[0] = lo;
-        extra_range[1] = hi;
-    }
-    __syncthreads();
-    grid_dependency_wait();     // the image is complete once the backward kernel has finished
-    const int extra_lo = extra_range[0], extra_hi = extra_range[1];
-    const bool any_extra = extra_lo < extra_hi;
-    const int GD = p.G * p.D;
-    const int vec_per_row = GD / 8;
-    const int S = (int)p.S;
-    const int64_t extra_sample = extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K);
-    const float inv = ldexpf(1.f, -grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch),
-                                                          p.Q, p.K, SOFTMAX));
-    const float2 inv2 = make_float2(inv, inv);
-    const uint4 *image = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(p.scratch) +
-                                                         kScratchHeaderBytes);
-    const __half *extras = reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)GD;
-    uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
-    const int64_t total = p.B * p.S * (int64_t)vec_per_row;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    // where the thread's current vector lies - sample b, position s of the sample, vector col of
-    // the position's row - kept up to date by additions: one division per thread, none per vector
-    // (first and stride are below 2^31: the grid is capped at a few thousand CTAs of 256 threads)
-    const unsigned first_row = (unsigned)first / (unsigned)vec_per_row;
-    int col = (int)((unsigned)first - first_row * (unsigned)vec_per_row);
-    int64_t b = first_row / (unsigned)S;
-    int s = (int)(first_row - (unsigned)b * (unsigned)S);
-    const unsigned step_rows_all = (unsigned)stride / (unsigned)vec_per_row;
-    const int step_cols = (int)((unsigned)stride - step_rows_all * (unsigned)vec_per_row);
-    const int step_samples = (int)(step_rows_all / (unsigned)S);          // whole samples per stride
-    const int step_rows = (int)(step_rows_all - (unsigned)step_samples * (unsigned)S);
-    constexpr int kTurn = MSDA_FIN_VECS;
-    for (int64_t v0 = first; v0 < total; v0 += kTurn * stride) {
-        // several vectors per turn, their image loads issued together
-        uint4 raw[kTurn];
-#pragma unroll
-        for (int u = 0; u < kTurn; ++u)
-            raw[u] = v0 + u * stride < total ? ld_stream16(image + v0 + u * stride)
-                                             : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int u = 0; u < kTurn; ++u) {
-            const int64_t v = v0 + u * stride;
-            if (v >= total) break;
-            float2 f[4];
-            VecTraits<__half>::unpack(raw[u], f);
-            if (any_extra) {
-                if (s >= extra_lo && s < extra_hi) {
-                    const __half *sample_extras = extras + b * extra_sample + col * 8;
-                    // every level whose range holds this position (one, for a well-formed table)
-                    for (int l = 0; l < p.L; ++l) {
-                        const int at = s - lt.start[l];
-                        if (lt.rep[l] <= 1 || at < 0 || at >= lt.H[l] * lt.W[l]) continue;
-                        const __half *src = sample_extras + lt.rep_base[l] + (int64_t)at * GD;
-                        for (int r = 1; r < lt.rep[l]; ++r) {
-                            float2 x[4];
-                            VecTraits<__half>::unpack(
-                                ld_stream16(src + (int64_t)(r - 1) * lt.level_elems[l]), x);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                f[i].x += x[i].x;
-                                f[i].y += x[i].y;
-                            }
-                        }
-                    }
-                }
-                // on to the vector one stride further
-                col += step_cols;
-                s += step_rows;
-                b += step_samples;
-                if (col >= vec_per_row) {
-                    col -= vec_per_row;
-                    ++s;
-                }
-                if (s >= S) {
-                    s -= S;
-                    ++b;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f[i] = fmul2(f[i], inv2);
-            gv[v] = VT::pack(f);
-        }
+    if constexpr (FUSED) {
+        __shared__ int extra_range[2];
+        if (threadIdx.x == 0) find_extra_range(lt, p.L, extra_range);
+        cooperative_groups::this_grid().sync();
+        finalize_image<T>(p, lt, extra_range, grad_scale_exponent<T>(magnitudes, p.Q, K, SOFTMAX));
     }
 }
 
 template <typename T, bool SOFTMAX, bool SCALED>
 cudaError_t launch_kernel(const Params &p, cudaStream_t stream) {
     const size_t smem = backward_smem_bytes(p, SOFTMAX);
-    auto kernel = backward_kernel<T, SOFTMAX, SCALED>;
+    auto kernel = backward_kernel<T, SOFTMAX, SCALED, false>;
     if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -485,6 +536,39 @@ cudaError_t launch_kernel(const Params &p, cudaStream_t stream) {
     if constexpr (SCALED) return launch_after_predecessor(kernel, q.grid, q.threads, smem, stream, q);
     kernel<<<q.grid, q.threads, smem, stream>>>(q);
     return cudaGetLastError();
+}
+
+// The whole scaled backward in one cooperative launch: at most as many CTAs as the GPU holds, each
+// walking adjacent sets of groups.
+template <typename T, bool SOFTMAX>
+cudaError_t launch_fused(const Params &p, cudaStream_t stream) {
+    const size_t smem = backward_smem_bytes(p, SOFTMAX);
+    auto kernel = backward_kernel<T, SOFTMAX, true, true>;
+    if (smem > kPlainSmem) {
+        cudaError_t e =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    static Residency residency;
+    const int64_t resident = std::min<int64_t>(residency.ctas(kernel, p.threads, smem), kFusedCtas);
+    if (resident <= 0) return cudaErrorInvalidConfiguration;
+    Params q = p;
+    const int nwarps = p.threads / 32;
+    const int64_t sets = (p.num_groups + nwarps - 1) / nwarps;
+    const int64_t sweep = p.B * p.S * (p.G * p.D / 8) / (p.threads * 4);   // CTAs the image can use
+    q.grid = (unsigned)std::max<int64_t>(1, std::min(resident, std::max(sets, sweep)));
+    q.passes = (int)((sets + q.grid - 1) / q.grid);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.grid, 1, 1);
+    cfg.blockDim = dim3(q.threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, q);
 }
 
 template <typename T, bool SOFTMAX>
@@ -523,6 +607,11 @@ cudaError_t launch_backward(const Params &p, int dtype, bool softmax, cudaStream
                            : launch_typed<__nv_bfloat16, false>(p, stream);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_backward_fused(const Params &p, int dtype, bool softmax, cudaStream_t stream) {
+    if (dtype == 1) return softmax ? launch_fused<__half, true>(p, stream) : launch_fused<__half, false>(p, stream);
+    return softmax ? launch_fused<__nv_bfloat16, true>(p, stream) : launch_fused<__nv_bfloat16, false>(p, stream);
 }
 
 cudaError_t launch_prepare_grad_value(const Params &p, int dtype, bool softmax, cudaStream_t stream) {

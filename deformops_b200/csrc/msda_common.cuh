@@ -63,6 +63,7 @@ struct Params {
     int point_chunk;        // descriptors per pair held in shared memory at a time
     int64_t num_groups;     // ceil(B*Q*G / pairs per warp)
     unsigned grid;
+    void *fused_magnitudes;  // one-launch backward: 8 bytes per CTA
     int passes;             // backward: adjacent sets of groups one CTA walks (0 or 1: one)
     // Fused location arithmetic.  When `ref` is set, `loc` / `grad_loc` hold the predicted
     // offsets (B,Q,G,L,K,2) and their gradient, and a point samples at
@@ -565,6 +566,17 @@ __host__ __device__ inline int backward_stage_floats(int pairs_per_warp, int P, 
 // launchers implemented in msda_forward.cu / msda_backward.cu; dtype: 0 f32, 1 f16, 2 bf16
 cudaError_t launch_forward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 cudaError_t launch_backward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
+// The scaled backward in one cooperative launch, for calls that are bound by the host: what its
+// scratch needs beyond the usual is 8 bytes for each of at most kFusedCtas CTAs.
+// (Host time of forward + backward of a decoder layer, B200: 78 us with separate launches, 73 so.
+// On the GPU it takes as long with 154 000 points (47 us against 49), longer with 516 000: 62
+// against 58, where the GPU is what bounds the call.)
+constexpr int kFusedCtas = 1024;
+constexpr int64_t kFusedBytes = 8 * kFusedCtas;
+inline bool fused_backward_pays(const Params &p) {
+    return p.B * p.Q * p.G * (int64_t)(p.L * p.K) <= ((int64_t)1 << 18);
+}
+cudaError_t launch_backward_fused(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 cudaError_t launch_prepare_grad_value(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 cudaError_t launch_finalize_grad_value(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 // float64 kernels (msda_f64.cu): loc / grad_loc point at doubles

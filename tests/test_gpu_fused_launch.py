@@ -1,0 +1,32 @@
+"""The 16-bit backward in one cooperative launch (small calls whose scratch has room for it), against
+the float64 oracle: a single CTA, replicas of a coarse level, several sets of groups per CTA."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import msda_oracle as orc
+from tests._abi import dev, to_np
+from tests._golden import rel_err
+from tests.test_gpu_sorted import _inputs, _workspace_backward
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("softmax,D,K,levels,B,Q,G", [
+    (False, 32, 1, [(3, 2)], 1, 1, 1),
+    (True, 32, 4, [(9, 7), (2, 2)], 2, 700, 8),
+    (False, 8, 2, [(20, 17), (5, 4)], 3, 5400, 4),
+    (True, 64, 3, [(13, 9)], 1, 4000, 20),
+])
+def test_one_launch_backward_matches_the_oracle(dtype, softmax, D, K, levels, B, Q, G):
+    value, shapes, starts, loc, logits, grad_out = _inputs(Q, B, Q, G, D, K, levels)
+    v, go = dev(value, dtype), dev(grad_out, dtype)
+    a = dev(logits if softmax else logits.softmax(-1), dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, softmax)
+    truth = orc.backward(*[t.cpu() for t in (v, sh, st, l, a)], go.cpu(), softmax=softmax)
+    assert rel_err(to_np(got[0]), truth[0]) <= 1e-2
+    assert rel_err(to_np(got[2]), truth[2].reshape(got[2].shape)) <= 1e-2

@@ -40,7 +40,7 @@ def _workspace_backward(value, shapes, starts, loc, attn, grad_out, softmax, nby
     code = DTYPE_CODES[value.dtype]
     if nbytes is None:
         nbytes = shim.workspace_bytes(B, S, G, D, Q, L, K, code, int(softmax))
-        assert nbytes > shim.scratch_bytes(B, S, G, D, Q, L, K, code), "the call would not be sorted"
+        assert nbytes > shim.scratch_bytes(B, S, G, D, Q, L, K, code), "the scratch is the plain one"
     grads = [torch.full_like(t, float("nan")) for t in (value, loc, attn)]
     scratch = torch.full((nbytes,), 0xFF, dtype=torch.uint8, device=value.device)
     st = shim.backward(_p(value), _p(shapes), _p(starts), _p(loc), _p(attn), _p(grad_out),
