@@ -313,13 +313,13 @@ __device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item
     if (threadIdx.x == 0) offsets[cells] = base;
 }
 
+// ---- pass 1: count the points of every cell -------------------------------------------------------
 // Bound by latency: a CTA's life is a dozen round trips to memory, so more CTAs per SM count for
 // more than registers (2 / 3 / 4 per SM: 64 / 55 / 50 us at the headline shape; reading its
 // operands alone takes 28 us).
-// ---- pass 1: count the points of every cell -------------------------------------------------------
 template <typename T, bool SOFTMAX, bool REF>
 __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __grid_constant__ Params p,
-    const __grid_constant__ SortPlan sp) {
+                                                                     const __grid_constant__ SortPlan sp) {
     grid_launch_dependents();
     // the first CTAs look for the magnitudes and clear grad_value, beside those that count
     if (blockIdx.x < (unsigned)sp.prepare_ctas) {
@@ -447,7 +447,7 @@ __device__ __forceinline__ bool unsortable_call(const unsigned *header) {
 // the locations kept from being evaluated twice: 105 us at the headline shape against 126).
 template <typename T, bool SOFTMAX, bool REF>
 __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __grid_constant__ Params p,
-    const __grid_constant__ SortPlan sp) {
+                                                                       const __grid_constant__ SortPlan sp) {
     using VT = VecTraits<T>;
     extern __shared__ uint4 smem[];
     __shared__ LevelTable lt;
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
             const int q = c.ql + (r0 + r) * c.step;
             if (q < nq) {
                 xy[r] = point_xy<T, REF>(p, c, base, q);
-                if constexpr (SOFTMAX) stats[r] = __ldg(sp.stats + pair0 + (int64_t)(q * p.G));
+                if constexpr (SOFTMAX) stats[r] = sp.stats[pair0 + (int64_t)(q * p.G)];
                 weight[r] = attn[base + (int64_t)(q * (p.G * P))];
             }
         }
@@ -703,6 +703,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
     __syncthreads();
 
     grid_launch_dependents();
+    // (what the kernels before wrote is read with plain loads: an invariant load may be moved
+    // above the wait)
     grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = lane >> 2, c = lane & 3;
@@ -745,243 +747,243 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
 
     // ---- runs of places, handed out as the warps come for them
     for (;;) {
-    unsigned item = 0;
-    if (lane == 0) item = atomicAdd(sp.header + kNextItem, 1u);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= (unsigned)(p.B * p.G) * (unsigned)sp.items) break;
-    const int plane = (int)(item / (unsigned)sp.items);
-    const int run = (int)(item - (unsigned)plane * (unsigned)sp.items);
-    const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
-    const int total = (int)__ldg(offsets + cells);
-    int cell = __ldg(sp.item_cell + (int64_t)plane * sp.items + run);
-    int pos = run * sp.item_points;
-    const int stop = min(pos + sp.item_points, total);
-    if (pos >= stop) continue;
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(sp.header + kNextItem, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= (unsigned)(p.B * p.G) * (unsigned)sp.items) break;
+        const int plane = (int)(item / (unsigned)sp.items);
+        const int run = (int)(item - (unsigned)plane * (unsigned)sp.items);
+        const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
+        const int total = (int)offsets[cells];
+        int cell = sp.item_cell[(int64_t)plane * sp.items + run];
+        int pos = run * sp.item_points;
+        const int stop = min(pos + sp.item_points, total);
+        if (pos >= stop) continue;
 
-    const int b = plane / p.G, g = plane - b * p.G;
-    const T *value = reinterpret_cast<const T *>(p.value) + ((int64_t)b * p.S * p.G + g) * D;
-    const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + ((int64_t)b * p.Q * p.G + g) * D;
-    __half *image = reinterpret_cast<__half *>(p.grad_value) + ((int64_t)b * p.S * p.G + g) * D;
-    const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
-    // element of the per-point outputs that point 0 of query 0 of this plane has
-    const int64_t plane_point = ((int64_t)b * p.Q * p.G + g) * (p.L * p.K);
+        const int b = plane / p.G, g = plane - b * p.G;
+        const T *value = reinterpret_cast<const T *>(p.value) + ((int64_t)b * p.S * p.G + g) * D;
+        const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + ((int64_t)b * p.Q * p.G + g) * D;
+        __half *image = reinterpret_cast<__half *>(p.grad_value) + ((int64_t)b * p.S * p.G + g) * D;
+        const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
+        // element of the per-point outputs that point 0 of query 0 of this plane has
+        const int64_t plane_point = ((int64_t)b * p.Q * p.G + g) * (p.L * p.K);
 
-    auto fetch_record = [&](int place) { return __ldg(records + min(place + lane, total - 1)); };
-    const T *chunk_of_row = grad_out + lane % NT * 8;
-    auto fetch_rows = [&](const uint4 &rec, int n, uint32_t buffer) {
-        const unsigned mine = rec.w >> 12;
+        auto fetch_record = [&](int place) { return __ldcg(records + min(place + lane, total - 1)); };
+        const T *chunk_of_row = grad_out + lane % NT * 8;
+        auto fetch_rows = [&](const uint4 &rec, int n, uint32_t buffer) {
+            const unsigned mine = rec.w >> 12;
 #pragma unroll
-        for (int i = 0; i < kStep / kRowsPerTurn; ++i) {
-            const unsigned q = __shfl_sync(0xffffffffu, mine, i * kRowsPerTurn + r0);
-            const uint32_t to = buffer + i * kRowsPerTurn * D * 2 + (D == 64 && (i & 1) ? at_copy ^ 32u : at_copy);
-            if (i * kRowsPerTurn + r0 < n) cp_async16(to, chunk_of_row + (size_t)(q * (unsigned)GD));
-        }
-        cp_async_commit();
-    };
-
-    // ---- where the run begins
-    int level = 0, strip_end = 0, row = 0, H = 0, W = 0, col0 = 0, start = 0;
-    auto enter_strip = [&]() {
-        while (level + 1 < p.L && cell >= ct.first[level + 1]) ++level;
-        const int rows = ct.rows[level];
-        const int strip = (cell - ct.first[level]) / rows;
-        strip_end = ct.first[level] + (strip + 1) * rows;
-        row = cell - (strip_end - rows) - 1;
-        H = lt.H[level], W = lt.W[level], start = lt.start[level];
-        col0 = strip * kCols - 1;
-    };
-    enter_strip();
-    int window = cell;      // the lanes hold the ends of cells window .. window + 31
-    int ends = (int)__ldg(offsets + min(window + 1 + lane, cells));
-    // the first cell at or after `window` that ends beyond `place` (which is below total)
-    auto cell_at = [&](int place, int &end) {
-        unsigned more;
-        while ((more = __ballot_sync(0xffffffffu, ends > place)) == 0) {
-            window += 32;
-            ends = (int)__ldg(offsets + min(window + 1 + lane, cells));
-        }
-        const int k = __ffs(more) - 1;
-        end = __shfl_sync(0xffffffffu, ends, k);
-        return window + k;
-    };
-
-    uint32_t vtop[NT], vbot[NT];     // the window's value rows, this lane's pixel
-    auto load_row = [&](uint32_t (&w)[NT], int r) {
-        const int x = col0 + j;
-        row_from_global<T, D>(w, value + (int64_t)(start + r * W + x) * GD, c,
-                              (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W);
-    };
-    load_row(vtop, row);
-    load_row(vbot, row + 1);
-    float acc[NT][4];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-    auto flush = [&](int half, int r) {
-        const int x = col0 + j;
-        flush_row<D>(acc, half, flush_scale, image + (int64_t)(start + r * W + x) * GD,
-                     (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W, c);
-    };
-
-    // ---- first steps
-    int cell_end;
-    cell_at(pos, cell_end);
-    int n = min(min(kStep, cell_end - pos), stop - pos);
-    uint4 rec = fetch_record(pos), rec_next = fetch_record(pos + n);
-    uint32_t buffer = s_rows;
-    fetch_rows(rec, n, buffer);
-
-    for (;;) {
-        // ---- what comes next, and its rows on their way
-        const int pos_next = pos + n;
-        const bool more = pos_next < stop;
-        int cell_next = cell, n_next = 0;
-        if (more) {
-            if (pos_next >= cell_end) cell_next = cell_at(pos_next, cell_end);
-            n_next = min(min(kStep, cell_end - pos_next), stop - pos_next);
-        }
-        const uint4 rec_after = fetch_record(pos_next + n_next);
-        const uint32_t other = buffer ^ s_rows ^ (s_rows + kRows);
-        fetch_rows(rec_next, n_next, other);
-
-        // ---- one lane per point: its four weights
-        const float fc = __uint_as_float(rec.x), fr = __uint_as_float(rec.y), a = __uint_as_float(rec.z);
-        {
-            const float w = lane < n ? a * weight_scale : 0.f;
-            const float top = w * (1.f - fr), bot = w * fr;
-            const float2 tw = make_float2(top * (1.f - fc), top * fc), bw = make_float2(bot * (1.f - fc), bot * fc);
-            uint4 s;
-            s.x = VT::pack2(tw);
-            s.y = VT::pack2(bw);
-            if constexpr (kSplit) {
-                // what the first term leaves; three low bits of it hold the column in the cell
-                const float2 th = VT::unpack2(s.x), bh = VT::unpack2(s.y);
-                s.z = VT::pack2(make_float2(tw.x - th.x, tw.y - th.y));
-                s.w = (VT::pack2(make_float2(bw.x - bh.x, bw.y - bh.y)) & ~7u) | (rec.w & 7u);
-            } else {
-                s.z = 0u;
-                s.w = rec.w & 7u;
+            for (int i = 0; i < kStep / kRowsPerTurn; ++i) {
+                const unsigned q = __shfl_sync(0xffffffffu, mine, i * kRowsPerTurn + r0);
+                const uint32_t to = buffer + i * kRowsPerTurn * D * 2 + (D == 64 && (i & 1) ? at_copy ^ 32u : at_copy);
+                if (i * kRowsPerTurn + r0 < n) cp_async16(to, chunk_of_row + (size_t)(q * (unsigned)GD));
             }
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_weights + lane * 16), "r"(s.x),
-                         "r"(s.y), "r"(s.z), "r"(s.w)
-                         : "memory");
-        }
-        cp_async_wait<1>();
-        __syncwarp();
+            cp_async_commit();
+        };
+
+        // ---- where the run begins
+        int level = 0, strip_end = 0, row = 0, H = 0, W = 0, col0 = 0, start = 0;
+        auto enter_strip = [&]() {
+            while (level + 1 < p.L && cell >= ct.first[level + 1]) ++level;
+            const int rows = ct.rows[level];
+            const int strip = (cell - ct.first[level]) / rows;
+            strip_end = ct.first[level] + (strip + 1) * rows;
+            row = cell - (strip_end - rows) - 1;
+            H = lt.H[level], W = lt.W[level], start = lt.start[level];
+            col0 = strip * kCols - 1;
+        };
+        enter_strip();
+        int window = cell;      // the lanes hold the ends of cells window .. window + 31
+        int ends = (int)offsets[min(window + 1 + lane, cells)];
+        // the first cell at or after `window` that ends beyond `place` (which is below total)
+        auto cell_at = [&](int place, int &end) {
+            unsigned more;
+            while ((more = __ballot_sync(0xffffffffu, ends > place)) == 0) {
+                window += 32;
+                ends = (int)offsets[min(window + 1 + lane, cells)];
+            }
+            const int k = __ffs(more) - 1;
+            end = __shfl_sync(0xffffffffu, ends, k);
+            return window + k;
+        };
+
+        uint32_t vtop[NT], vbot[NT];     // the window's value rows, this lane's pixel
+        auto load_row = [&](uint32_t (&w)[NT], int r) {
+            const int x = col0 + j;
+            row_from_global<T, D>(w, value + (int64_t)(start + r * W + x) * GD, c,
+                                  (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W);
+        };
+        load_row(vtop, row);
+        load_row(vbot, row + 1);
+        float acc[NT][4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && n <= 16) break;
-            uint32_t go[2][NT];
-            uint32_t hi[4], lo[4];     // weights of pixels x points: the A operand
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int block = h * 2 + e;
-                row_from_shared<D>(go[e], buffer + block * 8 * D * 2, at_row);
-                // dot products of the window's pixels with eight points
-                float dot[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int s = 0; s < KS; ++s) {
-                    const uint32_t av[4] = {vtop[2 * s], vbot[2 * s], vtop[2 * s + 1], vbot[2 * s + 1]};
-                    Mma<T>::run(dot, av, go[e][2 * s], go[e][2 * s + 1]);
-                }
-                const uint32_t to = s_dots + block * 512 + lane * 8;   // pixel j: 32 bytes, points 2c and 2c+1
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(dot[0]), "f"(dot[1]) : "memory");
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 256), "f"(dot[2]), "f"(dot[3]) : "memory");
-                // The weights with the pixels as k, the points as n: this lane has point j and
-                // pixel columns 2c, 2c + 1 of either row.  The point's words hold its columns col
-                // and col + 1; they go where 2c - col is -1, 0 or 1 (shift 0, 16, 32).
-                const uint4 w = lds16(s_weights + (block * 8 + j) * 16);
-                const uint32_t shift = 16u + 32u * c - 16u * (w.w & 7u);
-                uint32_t pick = __funnelshift_rc(0x32101044u, 0x44444432u, shift);
-                if (shift > 32u) pick = 0x4444u;
-                // a product with the identity turns that into pixels x points, which is what the
-                // accumulation below takes: the tensor cores have time for it, the shared memory
-                // that four words per lane and point would pass through has not
-                float t[4] = {0.f, 0.f, 0.f, 0.f};
-                const uint32_t unit[4] = {one, 0u, 0u, one};
-                Mma<T>::run(t, unit, __byte_perm(w.x, 0u, pick), __byte_perm(w.y, 0u, pick));
-                hi[2 * e] = VT::pack2(make_float2(t[0], t[1]));
-                hi[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+        for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+        auto flush = [&](int half, int r) {
+            const int x = col0 + j;
+            flush_row<D>(acc, half, flush_scale, image + (int64_t)(start + r * W + x) * GD,
+                         (unsigned)r < (unsigned)H && (unsigned)x < (unsigned)W, c);
+        };
+
+        // ---- first steps
+        int cell_end;
+        cell_at(pos, cell_end);
+        int n = min(min(kStep, cell_end - pos), stop - pos);
+        uint4 rec = fetch_record(pos), rec_next = fetch_record(pos + n);
+        uint32_t buffer = s_rows;
+        fetch_rows(rec, n, buffer);
+
+        for (;;) {
+            // ---- what comes next, and its rows on their way
+            const int pos_next = pos + n;
+            const bool more = pos_next < stop;
+            int cell_next = cell, n_next = 0;
+            if (more) {
+                if (pos_next >= cell_end) cell_next = cell_at(pos_next, cell_end);
+                n_next = min(min(kStep, cell_end - pos_next), stop - pos_next);
+            }
+            const uint4 rec_after = fetch_record(pos_next + n_next);
+            const uint32_t other = buffer ^ s_rows ^ (s_rows + kRows);
+            fetch_rows(rec_next, n_next, other);
+
+            // ---- one lane per point: its four weights
+            const float fc = __uint_as_float(rec.x), fr = __uint_as_float(rec.y), a = __uint_as_float(rec.z);
+            {
+                const float w = lane < n ? a * weight_scale : 0.f;
+                const float top = w * (1.f - fr), bot = w * fr;
+                const float2 tw = make_float2(top * (1.f - fc), top * fc), bw = make_float2(bot * (1.f - fc), bot * fc);
+                uint4 s;
+                s.x = VT::pack2(tw);
+                s.y = VT::pack2(bw);
                 if constexpr (kSplit) {
-                    t[0] = t[1] = t[2] = t[3] = 0.f;
-                    Mma<T>::run(t, unit, __byte_perm(w.z, 0u, pick), __byte_perm(w.w & ~7u, 0u, pick));
-                    lo[2 * e] = VT::pack2(make_float2(t[0], t[1]));
-                    lo[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+                    // what the first term leaves; three low bits of it hold the column in the cell
+                    const float2 th = VT::unpack2(s.x), bh = VT::unpack2(s.y);
+                    s.z = VT::pack2(make_float2(tw.x - th.x, tw.y - th.y));
+                    s.w = (VT::pack2(make_float2(bw.x - bh.x, bw.y - bh.y)) & ~7u) | (rec.w & 7u);
+                } else {
+                    s.z = 0u;
+                    s.w = rec.w & 7u;
+                }
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_weights + lane * 16), "r"(s.x),
+                             "r"(s.y), "r"(s.z), "r"(s.w)
+                             : "memory");
+            }
+            cp_async_wait<1>();
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h == 1 && n <= 16) break;
+                uint32_t go[2][NT];
+                uint32_t hi[4], lo[4];     // weights of pixels x points: the A operand
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int block = h * 2 + e;
+                    row_from_shared<D>(go[e], buffer + block * 8 * D * 2, at_row);
+                    // dot products of the window's pixels with eight points
+                    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int s = 0; s < KS; ++s) {
+                        const uint32_t av[4] = {vtop[2 * s], vbot[2 * s], vtop[2 * s + 1], vbot[2 * s + 1]};
+                        Mma<T>::run(dot, av, go[e][2 * s], go[e][2 * s + 1]);
+                    }
+                    const uint32_t to = s_dots + block * 512 + lane * 8;   // pixel j: 32 bytes, points 2c and 2c+1
+                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(dot[0]), "f"(dot[1]) : "memory");
+                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 256), "f"(dot[2]), "f"(dot[3]) : "memory");
+                    // The weights with the pixels as k, the points as n: this lane has point j and
+                    // pixel columns 2c, 2c + 1 of either row.  The point's words hold its columns col
+                    // and col + 1; they go where 2c - col is -1, 0 or 1 (shift 0, 16, 32).
+                    const uint4 w = lds16(s_weights + (block * 8 + j) * 16);
+                    const uint32_t shift = 16u + 32u * c - 16u * (w.w & 7u);
+                    uint32_t pick = __funnelshift_rc(0x32101044u, 0x44444432u, shift);
+                    if (shift > 32u) pick = 0x4444u;
+                    // a product with the identity turns that into pixels x points, which is what the
+                    // accumulation below takes: the tensor cores have time for it, the shared memory
+                    // that four words per lane and point would pass through has not
+                    float t[4] = {0.f, 0.f, 0.f, 0.f};
+                    const uint32_t unit[4] = {one, 0u, 0u, one};
+                    Mma<T>::run(t, unit, __byte_perm(w.x, 0u, pick), __byte_perm(w.y, 0u, pick));
+                    hi[2 * e] = VT::pack2(make_float2(t[0], t[1]));
+                    hi[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+                    if constexpr (kSplit) {
+                        t[0] = t[1] = t[2] = t[3] = 0.f;
+                        Mma<T>::run(t, unit, __byte_perm(w.z, 0u, pick), __byte_perm(w.w & ~7u, 0u, pick));
+                        lo[2 * e] = VT::pack2(make_float2(t[0], t[1]));
+                        lo[2 * e + 1] = VT::pack2(make_float2(t[2], t[3]));
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const uint32_t b0 = transpose8x8(go[0][t]), b1 = transpose8x8(go[1][t]);
+                    Mma<T>::run(acc[t], hi, b0, b1);
+                    if constexpr (kSplit) Mma<T>::run(acc[t], lo, b0, b1);
                 }
             }
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                const uint32_t b0 = transpose8x8(go[0][t]), b1 = transpose8x8(go[1][t]);
-                Mma<T>::run(acc[t], hi, b0, b1);
-                if constexpr (kSplit) Mma<T>::run(acc[t], lo, b0, b1);
+            __syncwarp();
+            // ---- gradients of the points: one lane each
+            if (lane < n) {
+                const uint32_t at = s_dots + (lane >> 3) * 512 + (rec.w & 7u) * 32 + (lane & 7) * 4;
+                const float d00 = lds4(at), d01 = lds4(at + 32), d10 = lds4(at + 256), d11 = lds4(at + 288);
+                const float wr0 = 1.f - fr, wc0 = 1.f - fc;
+                const float gx = wr0 * (d01 - d00) + fr * (d11 - d10);
+                const float gy = wc0 * (d10 - d00) + fc * (d11 - d01);
+                const float ga = wr0 * wc0 * d00 + wr0 * fc * d01 + fr * wc0 * d10 + fr * fc * d11;
+                const unsigned q = rec.w >> 12;
+                const int64_t e = plane_point + (size_t)(q * (unsigned)GP + ((rec.w >> 3) & 511u));
+                float2 dpix = make_float2((float)W, (float)H);
+                if constexpr (REF) {
+                    dpix = offset_derivative(p, (int64_t)b * p.Q + q, level, dpix.x, dpix.y);
+                    store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
+                } else {
+                    reinterpret_cast<float2 *>(p.grad_loc)[e] = make_float2(a * dpix.x * gx, a * dpix.y * gy);
+                    sp.grad_prob[e] = ga;
+                }
             }
-        }
-        __syncwarp();
-        // ---- gradients of the points: one lane each
-        if (lane < n) {
-            const uint32_t at = s_dots + (lane >> 3) * 512 + (rec.w & 7u) * 32 + (lane & 7) * 4;
-            const float d00 = lds4(at), d01 = lds4(at + 32), d10 = lds4(at + 256), d11 = lds4(at + 288);
-            const float wr0 = 1.f - fr, wc0 = 1.f - fc;
-            const float gx = wr0 * (d01 - d00) + fr * (d11 - d10);
-            const float gy = wc0 * (d10 - d00) + fc * (d11 - d01);
-            const float ga = wr0 * wc0 * d00 + wr0 * fc * d01 + fr * wc0 * d10 + fr * fc * d11;
-            const unsigned q = rec.w >> 12;
-            const int64_t e = plane_point + (size_t)(q * (unsigned)GP + ((rec.w >> 3) & 511u));
-            float2 dpix = make_float2((float)W, (float)H);
-            if constexpr (REF) {
-                dpix = offset_derivative(p, (int64_t)b * p.Q + q, level, dpix.x, dpix.y);
-                store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
-            } else {
-                reinterpret_cast<float2 *>(p.grad_loc)[e] = make_float2(a * dpix.x * gx, a * dpix.y * gy);
-                sp.grad_prob[e] = ga;
-            }
-        }
-        __syncwarp();
-        if (!more) break;
-        pos = pos_next;
-        n = n_next;
-        buffer = other;
-        rec = rec_next;
-        rec_next = rec_after;
-        if (cell_next == cell) continue;
-        // ---- into the next cell
-        if (cell_next == cell + 1 && cell_next < strip_end) {
-            // one row down: the upper row is complete, the lower one becomes the upper
-            flush(0, row);
-            ++row;
-            cell = cell_next;
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                acc[t][0] = acc[t][2], acc[t][1] = acc[t][3];
-                acc[t][2] = acc[t][3] = 0.f;
-                vtop[t] = vbot[t];
-            }
-            load_row(vbot, row + 1);
-        } else {
-            flush(0, row);
-            flush(1, row + 1);
-            if (cell_next < strip_end) {
-                row += cell_next - cell;
+            __syncwarp();
+            if (!more) break;
+            pos = pos_next;
+            n = n_next;
+            buffer = other;
+            rec = rec_next;
+            rec_next = rec_after;
+            if (cell_next == cell) continue;
+            // ---- into the next cell
+            if (cell_next == cell + 1 && cell_next < strip_end) {
+                // one row down: the upper row is complete, the lower one becomes the upper
+                flush(0, row);
+                ++row;
                 cell = cell_next;
-            } else {
-                cell = cell_next;
-                enter_strip();
-            }
 #pragma unroll
-            for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-            load_row(vtop, row);
-            load_row(vbot, row + 1);
+                for (int t = 0; t < NT; ++t) {
+                    acc[t][0] = acc[t][2], acc[t][1] = acc[t][3];
+                    acc[t][2] = acc[t][3] = 0.f;
+                    vtop[t] = vbot[t];
+                }
+                load_row(vbot, row + 1);
+            } else {
+                flush(0, row);
+                flush(1, row + 1);
+                if (cell_next < strip_end) {
+                    row += cell_next - cell;
+                    cell = cell_next;
+                } else {
+                    cell = cell_next;
+                    enter_strip();
+                }
+#pragma unroll
+                for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+                load_row(vtop, row);
+                load_row(vbot, row + 1);
+            }
         }
-    }
-    flush(0, row);
-    flush(1, row + 1);
-    cp_async_wait<0>();
+        flush(0, row);
+        flush(1, row + 1);
+        cp_async_wait<0>();
     }
 }
 
 // ---- last pass: grad_value from the scaled float16 image, in place; softmax Jacobian --------------
 template <typename T, bool SOFTMAX>
 __global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_constant__ Params p,
-    const __grid_constant__ SortPlan sp) {
+                                                              const __grid_constant__ SortPlan sp) {
     grid_dependency_wait();
     using VT = VecTraits<T>;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
