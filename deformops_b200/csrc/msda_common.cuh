@@ -512,6 +512,28 @@ __device__ __forceinline__ float2 offset_derivative(const Params &p, int64_t bq,
     return make_float2(Wf * (1.f / Kf * r.z * 0.5f), Hf * (1.f / Kf * r.w * 0.5f));
 }
 
+// A predicted offset, stored in float32 or the 16-bit value type.
+template <typename T>
+__device__ __forceinline__ float2 load_offset(const Params &p, int64_t e) {
+    const float2 *loc2 = reinterpret_cast<const float2 *>(p.loc);
+    if constexpr (sizeof(T) == 2) {
+        if (p.offsets16) return VecTraits<T>::unpack2(__ldg(reinterpret_cast<const uint32_t *>(p.loc) + e));
+    }
+    return ld_stream_f2(loc2 + e);
+}
+
+// The forward's location: REF says at compile time whether there are reference points.
+template <typename T, bool REF>
+__device__ __forceinline__ float2 forward_location(const Params &p, int64_t e, int64_t pair, int l,
+                                                   float Wf, float Hf) {
+    if constexpr (REF) {
+        const int64_t bq = pair <= 0x7fffffffll ? (int64_t)((unsigned)pair / (unsigned)p.G) : pair / p.G;
+        return location_from_offset(p, load_offset<T>(p, e), bq, l, Wf, Hf);
+    } else {
+        return ld_stream_f2(reinterpret_cast<const float2 *>(p.loc) + e);
+    }
+}
+
 // Sample location of element `e` = (pair, point) of level `l`, and in `dpix` the derivative of
 // the pixel coordinate with respect to what the caller differentiates: the location itself
 // (W, H), or the predicted offset when the call carries reference points.
@@ -523,15 +545,7 @@ __device__ __forceinline__ float2 sample_location(const Params &p, int64_t e, in
         dpix = make_float2(Wf, Hf);
         return ld_stream_f2(loc2 + e);
     }
-    float2 off;
-    if constexpr (sizeof(T) == 2) {
-        if (p.offsets16)
-            off = VecTraits<T>::unpack2(__ldg(reinterpret_cast<const uint32_t *>(p.loc) + e));
-        else
-            off = ld_stream_f2(loc2 + e);
-    } else {
-        off = ld_stream_f2(loc2 + e);
-    }
+    const float2 off = load_offset<T>(p, e);
     // (a 64-bit division costs as much as the rest of the point)
     const int64_t bq = pair <= 0x7fffffffll ? (int64_t)((unsigned)pair / (unsigned)p.G) : pair / p.G;
     dpix = offset_derivative(p, bq, l, Wf, Hf);

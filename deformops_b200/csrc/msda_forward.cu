@@ -35,7 +35,7 @@ namespace msda_b200 {
 
 namespace {
 
-template <typename T, bool SOFTMAX, bool SMALL>
+template <typename T, bool SOFTMAX, bool REF, bool SMALL>
 __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_kernel(const Params p) {
     using VT = VecTraits<T>;
     constexpr int V = VT::kVec;
@@ -98,9 +98,8 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
                 if (sl < nlive) {
                     const int64_t e = (pair0 + sl) * P + pt;
                     const int l = (int)(((float)pt + 0.5f) * inv_K);  // pt / K
-                    float2 dpix;
-                    const float2 xy = sample_location<T>(p, e, pair0 + sl, l, (float)lt.W[l],
-                                                         (float)lt.H[l], dpix);
+                    const float2 xy = forward_location<T, REF>(p, e, pair0 + sl, l, (float)lt.W[l],
+                                                               (float)lt.H[l]);
                     float a = VT::to_float(attn[e]);
                     if constexpr (SOFTMAX) {
                         const float2 st = stats[sl];
@@ -163,10 +162,10 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
     }
 }
 
-template <typename T, bool SOFTMAX, bool SMALL>
+template <typename T, bool SOFTMAX, bool REF, bool SMALL>
 cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     const size_t smem = forward_smem_bytes(p, SOFTMAX);
-    auto kernel = forward_kernel<T, SOFTMAX, SMALL>;
+    auto kernel = forward_kernel<T, SOFTMAX, REF, SMALL>;
     if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -187,20 +186,25 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <typename T, bool SOFTMAX>
-cudaError_t launch_typed(const Params &p, cudaStream_t stream) {
+template <typename T, bool SOFTMAX, bool REF>
+cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
     // Up to four groups per SM the call lasts as long as one warp's chain of loads: more points in
     // flight per warp, and as few warps per CTA as still reach every SM.  Measured on B200, a
     // decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in flight 6.1, 6 6.6;
     // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
     constexpr int kSms = 148;
-    if (p.num_groups > 4 * kSms) return launch_as<T, SOFTMAX, false>(p, stream);
+    if (p.num_groups > 4 * kSms) return launch_as<T, SOFTMAX, REF, false>(p, stream);
     Params q = p;
     int warps = 1;
     while (warps < p.threads / 32 && warps * kSms < p.num_groups) warps *= 2;
     q.threads = warps * 32;
     q.grid = (unsigned)((p.num_groups + warps - 1) / warps);
-    return launch_as<T, SOFTMAX, true>(q, stream);
+    return launch_as<T, SOFTMAX, REF, true>(q, stream);
+}
+
+template <typename T, bool SOFTMAX>
+cudaError_t launch_typed(const Params &p, cudaStream_t stream) {
+    return p.ref != nullptr ? launch_sized<T, SOFTMAX, true>(p, stream) : launch_sized<T, SOFTMAX, false>(p, stream);
 }
 
 }  // namespace
