@@ -523,12 +523,11 @@ __device__ __forceinline__ float2 load_offset(const Params &p, int64_t e) {
 }
 
 // The forward's location: REF says at compile time whether there are reference points.
-template <typename T, bool REF>
-__device__ __forceinline__ float2 forward_location(const Params &p, int64_t e, int64_t pair, int l,
+template <typename T, bool REF, typename Index>
+__device__ __forceinline__ float2 forward_location(const Params &p, int64_t e, Index pair, int l,
                                                    float Wf, float Hf) {
     if constexpr (REF) {
-        const int64_t bq = pair <= 0x7fffffffll ? (int64_t)((unsigned)pair / (unsigned)p.G) : pair / p.G;
-        return location_from_offset(p, load_offset<T>(p, e), bq, l, Wf, Hf);
+        return location_from_offset(p, load_offset<T>(p, e), (int64_t)(pair / (Index)p.G), l, Wf, Hf);
     } else {
         return ld_stream_f2(reinterpret_cast<const float2 *>(p.loc) + e);
     }

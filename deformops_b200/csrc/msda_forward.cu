@@ -35,7 +35,9 @@ namespace msda_b200 {
 
 namespace {
 
-template <typename T, bool SOFTMAX, bool REF, bool SMALL>
+// Index: what a (query, head) pair is numbered in.  Two 64-bit divisions per group were 2 % of the
+// kernel; calls of 2^31 pairs and more keep them.
+template <typename T, bool SOFTMAX, bool REF, bool SMALL, typename Index>
 __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_kernel(const Params p) {
     using VT = VecTraits<T>;
     constexpr int V = VT::kVec;
@@ -80,9 +82,9 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
         }
         const bool live = slot < nlive;
         const int64_t my_pair = pair0 + (live ? slot : 0);
-        const int64_t bq = my_pair / G;
-        const int g = (int)(my_pair - bq * G);
-        const int64_t b = bq / p.Q;
+        const Index bq = (Index)my_pair / (Index)G;
+        const int g = (int)((Index)my_pair - bq * (Index)G);
+        const int64_t b = (int64_t)(bq / (Index)p.Q);
         const T *vb = value + (b * p.S * G + g) * (int64_t)D;
 
         float2 acc[NV2];
@@ -98,8 +100,8 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
                 if (sl < nlive) {
                     const int64_t e = (pair0 + sl) * P + pt;
                     const int l = (int)(((float)pt + 0.5f) * inv_K);  // pt / K
-                    const float2 xy = forward_location<T, REF>(p, e, pair0 + sl, l, (float)lt.W[l],
-                                                               (float)lt.H[l]);
+                    const float2 xy = forward_location<T, REF, Index>(p, e, (Index)(pair0 + sl), l,
+                                                                      (float)lt.W[l], (float)lt.H[l]);
                     float a = VT::to_float(attn[e]);
                     if constexpr (SOFTMAX) {
                         const float2 st = stats[sl];
@@ -162,10 +164,10 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
     }
 }
 
-template <typename T, bool SOFTMAX, bool REF, bool SMALL>
+template <typename T, bool SOFTMAX, bool REF, bool SMALL, typename Index>
 cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     const size_t smem = forward_smem_bytes(p, SOFTMAX);
-    auto kernel = forward_kernel<T, SOFTMAX, REF, SMALL>;
+    auto kernel = forward_kernel<T, SOFTMAX, REF, SMALL, Index>;
     if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -193,13 +195,15 @@ cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
     // decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in flight 6.1, 6 6.6;
     // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
     constexpr int kSms = 148;
-    if (p.num_groups > 4 * kSms) return launch_as<T, SOFTMAX, REF, false>(p, stream);
+    if (p.num_groups > 4 * kSms)
+        return p.B * p.Q * p.G < (int64_t)1 << 31 ? launch_as<T, SOFTMAX, REF, false, unsigned>(p, stream)
+                                                  : launch_as<T, SOFTMAX, REF, false, int64_t>(p, stream);
     Params q = p;
     int warps = 1;
     while (warps < p.threads / 32 && warps * kSms < p.num_groups) warps *= 2;
     q.threads = warps * 32;
     q.grid = (unsigned)((p.num_groups + warps - 1) / warps);
-    return launch_as<T, SOFTMAX, REF, true>(q, stream);
+    return launch_as<T, SOFTMAX, REF, true, unsigned>(q, stream);
 }
 
 template <typename T, bool SOFTMAX>
