@@ -41,6 +41,7 @@ constexpr int kSharedCells = 8192;     // most cells of a plane that are counted
 constexpr int kSortCtaPoints = kSortThreads * kSortPoints;
 
 constexpr int kNextItem = 2;           // header cell: runs of the walk handed out so far
+constexpr unsigned kNonFinite = 0x7fffu;   // magnitude bits of a NaN in either type
 
 // ---- cells ---------------------------------------------------------------------------------------
 struct CellTable {
@@ -216,9 +217,11 @@ __device__ __forceinline__ void for_values(const T *x, int P, F f) {
 // What has to be known or done before anything is accumulated: largest magnitudes for the scale,
 // zeros in grad_value, softmax statistics (max, 1 / sum) of every pair.  The share of one of
 // `ctas` CTAs.
+// Header cell 1 is the largest |attn| element's; of a softmax, whose probabilities are at most 1, it
+// says whether a pair's are numbers at all (a NaN or +inf logit, or nothing but -inf, makes every
+// one of them NaN).
 template <typename T, bool SOFTMAX>
 __device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &sp, int cta, int ctas) {
-    constexpr bool WITH_ATTN = !SOFTMAX;
     unsigned *header = sp.header;
     __shared__ unsigned cta_max[2];
     if (threadIdx.x < 2) cta_max[threadIdx.x] = 0u;
@@ -228,7 +231,7 @@ __device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &s
     const int64_t go_vecs = p.B * p.Q * (p.G * p.D / 8);
     unsigned mg = scan_max_magnitude(reinterpret_cast<const uint4 *>(p.grad_out), go_vecs, first, stride);
     unsigned ma = 0;
-    if constexpr (WITH_ATTN) {
+    if constexpr (!SOFTMAX) {
         // (a later sample's weights need not begin on a 16-byte boundary: whole vectors in the
         // middle, single elements at both ends)
         const unsigned short *at = reinterpret_cast<const unsigned short *>(p.attn);
@@ -247,20 +250,20 @@ __device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &s
             for_values(x, P, [&](int, float v) { m = fmaxf(m, v); });
             for_values(x, P, [&](int, float v) { sum += expf(v - m); });
             sp.stats[i] = make_float2(m, 1.f / sum);
+            if (!(sum < INFINITY)) ma = kNonFinite;
         }
     }
     uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
     const int64_t vecs = p.B * p.S * (p.G * p.D / 8);
     for (int64_t v = first; v < vecs; v += stride) gv[v] = make_uint4(0u, 0u, 0u, 0u);
     mg = __reduce_max_sync(0xffffffffu, mg);
-    if constexpr (WITH_ATTN) ma = __reduce_max_sync(0xffffffffu, ma);
+    ma = __reduce_max_sync(0xffffffffu, ma);
     if ((threadIdx.x & 31) == 0) {
         if (mg != 0) atomicMax(&cta_max[0], mg);
-        if (WITH_ATTN && ma != 0) atomicMax(&cta_max[1], ma);
+        if (ma != 0) atomicMax(&cta_max[1], ma);
     }
     __syncthreads();
-    if (threadIdx.x < (WITH_ATTN ? 2 : 1) && cta_max[threadIdx.x] != 0)
-        atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
+    if (threadIdx.x < 2 && cta_max[threadIdx.x] != 0) atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
 }
 
 // Exclusive prefix sum of a plane's cell counts by one CTA, in chunks of its size: `counts`
@@ -433,11 +436,12 @@ __device__ __noinline__ void direct_point(const Params &p, const SortPlan &sp, c
     store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
 }
 
-// An inf or NaN in grad_out has to reach its own corners only: a tile product would spread
-// it to the zero entries beside them (0 * inf), so such a call takes direct_point() throughout.
+// An inf or NaN in grad_out or in a weight has to reach its own point's corners only: a tile
+// product would spread it to the zero entries beside them (0 * inf), so such a call takes
+// direct_point() throughout.
 template <typename T>
 __device__ __forceinline__ bool unsortable_call(const unsigned *header) {
-    return header[0] >= (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u);
+    return max(header[0], header[1]) >= (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u);
 }
 
 // ---- pass 2: write the points' records in order of their cells ------------------------------------

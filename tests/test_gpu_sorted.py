@@ -152,3 +152,28 @@ def test_non_finite_gradients_stay_in_their_corners():
     fine = torch.isfinite(got[0])
     assert rel_err(to_np(got[0][fine]), to_np(direct[0][fine])) <= 2e-2
     assert rel_err(to_np(got[1])[0, 100:], to_np(direct[1])[0, 100:]) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype,softmax,bad", [
+    (torch.bfloat16, False, float("inf")), (torch.float16, False, float("nan")),
+    (torch.bfloat16, True, float("nan")), (torch.float16, True, float("inf")),
+    (torch.bfloat16, True, float("-inf")),                      # an ordinary mask: all finite
+])
+def test_non_finite_weights_stay_in_their_corners(dtype, softmax, bad):
+    """The same elements are non-finite as on the direct path (a weight's own four corners, or its
+    pair's where the softmax spreads it), and the others have the same values."""
+    B, Q, G, D, K, levels = 1, 17000, 8, 32, 4, [(18, 16), (9, 8)]
+    value, shapes, starts, loc, logits, grad_out = _inputs(10, B, Q, G, D, K, levels)
+    loc[0, 11, 3] = loc[0, 11, 3].clamp(0.1, 0.9)               # (not a skipped point)
+    attn = logits if softmax else logits.softmax(-1)
+    attn[0, 11, 3, 5] = bad
+    v, a, go = dev(value, dtype), dev(attn, dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, softmax)
+    direct = abi_backward(v, sh, st, l, a, go, softmax=softmax)
+    for x, y, bar in zip(got, direct, (2e-2, 1e-4, 2e-2)):
+        fine = torch.isfinite(y)
+        assert torch.equal(torch.isfinite(x), fine)
+        assert rel_err(to_np(x[fine]), to_np(y[fine])) <= bar
+    spoilt = int((~torch.isfinite(got[0])).sum())
+    assert spoilt == 0 if bad == float("-inf") else 0 < spoilt <= len(levels) * K * 4 * D
