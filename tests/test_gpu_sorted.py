@@ -164,9 +164,9 @@ def test_non_finite_weights_stay_in_their_corners(dtype, softmax, bad):
     pair's where the softmax spreads it), and the others have the same values."""
     B, Q, G, D, K, levels = 1, 17000, 8, 32, 4, [(18, 16), (9, 8)]
     value, shapes, starts, loc, logits, grad_out = _inputs(10, B, Q, G, D, K, levels)
-    loc[0, 11, 3] = loc[0, 11, 3].clamp(0.1, 0.9)               # (not a skipped point)
+    loc[0, 11, 3, 0, 1] = torch.tensor([3.8 / 16, 8.1 / 18])     # its 2 x 8 window is inside the level
     attn = logits if softmax else logits.softmax(-1)
-    attn[0, 11, 3, 5] = bad
+    attn[0, 11, 3, 1] = bad
     v, a, go = dev(value, dtype), dev(attn, dtype), dev(grad_out, dtype)
     l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
     got = _workspace_backward(v, sh, st, l, a, go, softmax)
