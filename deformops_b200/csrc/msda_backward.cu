@@ -57,9 +57,6 @@
 #ifndef MSDA_FIN_CTAS_PER_SM
 #define MSDA_FIN_CTAS_PER_SM 4
 #endif
-#ifndef MSDA_FIN_VECS
-#define MSDA_FIN_VECS 4
-#endif
 #ifndef MSDA_FIN_MIN_CTAS
 #define MSDA_FIN_MIN_CTAS 4
 #endif
@@ -129,103 +126,14 @@ __global__ void __launch_bounds__(256, MSDA_PREP_MIN_CTAS) prepare_kernel(const 
         atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
 }
 
-// grad_value = (image + the replicas of the position's level) * 2^-e, rounded to T.
-// Positions of levels that have replicas form a small range of every sample (the coarse levels:
-// 1 024 of 21 504 positions at the headline shape); everything outside it takes the short path.
-// `lt` has its replicas planned; `extra_range` is the CTA's.
-__device__ __forceinline__ void find_extra_range(const LevelTable &lt, int L, int (&extra_range)[2]) {
-    int lo = 0x7fffffff, hi = 0;
-    for (int l = 0; l < L; ++l)
-        if (lt.rep[l] > 1) {
-            lo = min(lo, lt.start[l]);
-            hi = max(hi, lt.start[l] + lt.H[l] * lt.W[l]);
-        }
-    extra_range[0] = lo;
-    extra_range[1] = hi;
-}
-
+// grad_value from the image and the extras of the scratch
 template <typename T>
-__device__ __forceinline__ void finalize_image(const Params &p, const LevelTable &lt,
-                                               const int (&extra_range)[2], int exponent) {
-    using VT = VecTraits<T>;
-    const int extra_lo = extra_range[0], extra_hi = extra_range[1];
-    const bool any_extra = extra_lo < extra_hi;
-    const int GD = p.G * p.D;
-    const int vec_per_row = GD / 8;
-    const int S = (int)p.S;
-    const int64_t extra_sample = extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K);
-    const float inv = ldexpf(1.f, -exponent);
-    const float2 inv2 = make_float2(inv, inv);
+__device__ __forceinline__ void finalize_scratch(const Params &p, const LevelTable &lt,
+                                                 const int (&extra_range)[2], int exponent) {
     const uint4 *image = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(p.scratch) +
                                                          kScratchHeaderBytes);
-    const __half *extras = reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)GD;
-    uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
-    const int64_t total = p.B * p.S * (int64_t)vec_per_row;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    // where the thread's current vector lies - sample b, position s of the sample, vector col of
-    // the position's row - kept up to date by additions: one division per thread, none per vector
-    // (first and stride are below 2^31: the grid is capped at a few thousand CTAs of 256 threads)
-    const unsigned first_row = (unsigned)first / (unsigned)vec_per_row;
-    int col = (int)((unsigned)first - first_row * (unsigned)vec_per_row);
-    int64_t b = first_row / (unsigned)S;
-    int s = (int)(first_row - (unsigned)b * (unsigned)S);
-    const unsigned step_rows_all = (unsigned)stride / (unsigned)vec_per_row;
-    const int step_cols = (int)((unsigned)stride - step_rows_all * (unsigned)vec_per_row);
-    const int step_samples = (int)(step_rows_all / (unsigned)S);          // whole samples per stride
-    const int step_rows = (int)(step_rows_all - (unsigned)step_samples * (unsigned)S);
-    constexpr int kTurn = MSDA_FIN_VECS;
-    for (int64_t v0 = first; v0 < total; v0 += kTurn * stride) {
-        // several vectors per turn, their image loads issued together
-        uint4 raw[kTurn];
-#pragma unroll
-        for (int u = 0; u < kTurn; ++u)
-            raw[u] = v0 + u * stride < total ? ld_stream16(image + v0 + u * stride)
-                                             : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int u = 0; u < kTurn; ++u) {
-            const int64_t v = v0 + u * stride;
-            if (v >= total) break;
-            float2 f[4];
-            VecTraits<__half>::unpack(raw[u], f);
-            if (any_extra) {
-                if (s >= extra_lo && s < extra_hi) {
-                    const __half *sample_extras = extras + b * extra_sample + col * 8;
-                    // every level whose range holds this position (one, for a well-formed table)
-                    for (int l = 0; l < p.L; ++l) {
-                        const int at = s - lt.start[l];
-                        if (lt.rep[l] <= 1 || at < 0 || at >= lt.H[l] * lt.W[l]) continue;
-                        const __half *src = sample_extras + lt.rep_base[l] + (int64_t)at * GD;
-                        for (int r = 1; r < lt.rep[l]; ++r) {
-                            float2 x[4];
-                            VecTraits<__half>::unpack(
-                                ld_stream16(src + (int64_t)(r - 1) * lt.level_elems[l]), x);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                f[i].x += x[i].x;
-                                f[i].y += x[i].y;
-                            }
-                        }
-                    }
-                }
-                // on to the vector one stride further
-                col += step_cols;
-                s += step_rows;
-                b += step_samples;
-                if (col >= vec_per_row) {
-                    col -= vec_per_row;
-                    ++s;
-                }
-                if (s >= S) {
-                    s -= S;
-                    ++b;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f[i] = fmul2(f[i], inv2);
-            gv[v] = VT::pack(f);
-        }
-    }
+    finalize_image<T>(p, lt, extra_range, exponent, image,
+                      reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)(p.G * p.D));
 }
 
 template <typename T, bool SOFTMAX>
@@ -240,8 +148,8 @@ __global__ void __launch_bounds__(256, MSDA_FIN_MIN_CTAS) finalize_kernel(const 
     }
     __syncthreads();
     grid_dependency_wait();     // the image is complete once the backward kernel has finished
-    finalize_image<T>(p, lt, extra_range,
-                      grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch), p.Q, p.K, SOFTMAX));
+    finalize_scratch<T>(p, lt, extra_range,
+                        grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch), p.Q, p.K, SOFTMAX));
 }
 
 // SCALED: grad_value contributions go, times 2^e, into the float16 image of the scratch.
@@ -510,7 +418,7 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_k
         __shared__ int extra_range[2];
         if (threadIdx.x == 0) find_extra_range(lt, p.L, extra_range);
         cooperative_groups::this_grid().sync();
-        finalize_image<T>(p, lt, extra_range, grad_scale_exponent<T>(magnitudes, p.Q, K, SOFTMAX));
+        finalize_scratch<T>(p, lt, extra_range, grad_scale_exponent<T>(magnitudes, p.Q, K, SOFTMAX));
     }
 }
 

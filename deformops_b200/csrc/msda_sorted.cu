@@ -39,27 +39,34 @@ constexpr int kSortPoints = 8;         // points per thread of the sort kernels,
 constexpr int kSortBatch = 4;          // loaded this many at a time
 constexpr int kSharedCells = 8192;     // most cells of a plane that are counted in shared memory
 constexpr int kSortCtaPoints = kSortThreads * kSortPoints;
+constexpr int kWalkWarps = 4;          // warps per CTA of the walk, each on its own run
 
-constexpr int kNextItem = 2;           // header cell: runs of the walk handed out so far
+// header cells beside the two magnitudes
+constexpr int kNextItem = 2;           // runs of the walk handed out so far
+constexpr int kNoCells = 3;            // not zero: the levels' cells do not fit
 constexpr unsigned kNonFinite = 0x7fffu;   // magnitude bits of a NaN in either type
 
 // ---- cells ---------------------------------------------------------------------------------------
 struct CellTable {
     int first[kMaxLevels + 1];   // first cell of the level; [L]: number of cells
-    int rows[kMaxLevels];        // cells per strip: H + 1 (r0 = -1 .. H - 1); 0: not sorted
+    int rows[kMaxLevels];        // cells per strip: H + 1 (r0 = -1 .. H - 1)
+    bool fits;                   // the cells of all levels fit the room there is
 };
 
 // A table whose levels overlap can ask for more cells than there is room for (levels that tile
-// `value` cannot): the levels that do not fit are not sorted, direct_point() serves them.
+// `value` cannot): such a call is not sorted.
 __device__ inline void plan_cells(CellTable &c, const LevelTable &t, int L, int bound) {
     int n = 0;
+    c.fits = true;
     for (int l = 0; l < L; ++l) {
         const long long cells =
             t.H[l] > 0 ? (t.H[l] + 1ll) * ((t.W[l] + kCols) / kCols) : 0;   // ceil((W + 1) / kCols)
-        const bool fits = n + cells <= bound;
         c.first[l] = n;
-        c.rows[l] = fits ? t.H[l] + 1 : 0;
-        if (fits) n += (int)cells;
+        c.rows[l] = t.H[l] + 1;
+        if (n + cells <= bound)
+            n += (int)cells;
+        else
+            c.fits = false;
     }
     c.first[L] = n;
 }
@@ -337,6 +344,10 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __gri
     __syncthreads();
     if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
     __syncthreads();
+    if (!ct.fits) {
+        if (threadIdx.x == 0) sp.header[kNoCells] = 1u;   // (every CTA says the same)
+        return;
+    }
     const int cells = ct.first[p.L];
     const bool in_shared = cells <= sp.shared_cells;
     if (in_shared)
@@ -345,7 +356,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __gri
     unsigned *counts = sp.counts + (int64_t)c.plane * sp.cell_stride;
     const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
     __syncthreads();
-    if (c.active && c.rows > 0) {
+    if (c.active) {
         const int64_t base = pair0 * (p.L * p.K) + c.pt;
         for (int r0 = 0; r0 < kSortPoints; r0 += kSortBatch) {
             float2 xy[kSortBatch];
@@ -392,56 +403,135 @@ __device__ __forceinline__ void store_point_gradients(const Params &p, const Sor
     sp.grad_prob[e] = grad_weight;
 }
 
-// One point without sorting, one thread: what the walk does for points the sort leaves out.
+// What cannot be sorted: an inf or NaN in grad_out or in a weight has to reach its own point's
+// corners only, and a tile product would spread it to the zero entries beside them (0 * inf); and
+// tables without room for their cells.  A float16 step whose loss scale overflowed is such a call.
+// Its points take the walk kernel's place in the order they have, accumulate_unsorted(), with
+// the replicas of coarse levels that the direct backward gives them where the records would be.
 template <typename T>
-__device__ __noinline__ void direct_point(const Params &p, const SortPlan &sp, const LevelTable &lt,
-                                          int64_t pair, int pt, float a, float scale) {
-    using VT = VecTraits<T>;
-    const int l = pt / p.K;
-    const int64_t e = pair * (p.L * p.K) + pt;
-    float2 dpix;
-    const float2 xy = sample_location<T>(p, e, pair, l, (float)lt.W[l], (float)lt.H[l], dpix);
-    const PointGeom geo = locate(xy.x, xy.y, lt.H[l], lt.W[l], lt.start[l], p.G * p.D);
-    const int64_t bq = pair / p.G;
-    const int64_t sample = ((bq / p.Q) * p.S * p.G + (pair - bq * p.G)) * p.D;
-    const T *value = reinterpret_cast<const T *>(p.value) + sample;
-    const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + pair * p.D;
-    __half *image = reinterpret_cast<__half *>(p.grad_value) + sample;
-    const int off[4] = {geo.off00, geo.off00 + p.G * p.D, geo.off00 + geo.rowstride,
-                        geo.off00 + geo.rowstride + p.G * p.D};
-    const float w[4] = {(1.f - geo.fr) * (1.f - geo.fc), (1.f - geo.fr) * geo.fc,
-                        geo.fr * (1.f - geo.fc), geo.fr * geo.fc};
-    float dot[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int ch = 0; ch < p.D; ch += 8) {
-        float2 go[4], f[4];
-        VT::unpack(ldg16(grad_out + ch), go);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const bool inside = geo.flags & (1u << c);
-            VT::unpack(ldg16_if(value + off[c] + ch, inside), f);
-            const float s = a * w[c] * scale;
-            float2 gv[4], d2 = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ffma2(d2, f[i], go[i]);
-                gv[i] = fmul2(go[i], make_float2(s, s));
-            }
-            dot[c] += d2.x + d2.y;
-            red_if<__half>(image + off[c] + ch, gv, inside);
-        }
-    }
-    const float gx = (1.f - geo.fr) * (dot[1] - dot[0]) + geo.fr * (dot[3] - dot[2]);
-    const float gy = (1.f - geo.fc) * (dot[2] - dot[0]) + geo.fc * (dot[3] - dot[1]);
-    const float ga = w[0] * dot[0] + w[1] * dot[1] + w[2] * dot[2] + w[3] * dot[3];
-    store_point_gradients<T>(p, sp, e, make_float2(a * dpix.x * gx, a * dpix.y * gy), ga);
+__device__ __forceinline__ bool unsorted_call(const unsigned *header) {
+    return max(header[0], header[1]) >= (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u) ||
+           header[kNoCells] != 0u;
+}
+// (at most L * K*Q*G*D / 64 float16 a sample, D / 32 <= 2 bytes a point where a record is 16)
+__device__ __forceinline__ __half *unsorted_extras(const SortPlan &sp) {
+    return reinterpret_cast<__half *>(sp.records);
 }
 
-// An inf or NaN in grad_out or in a weight has to reach its own point's corners only: a tile
-// product would spread it to the zero entries beside them (0 * inf), so such a call takes
-// direct_point() throughout.
-template <typename T>
-__device__ __forceinline__ bool unsortable_call(const unsigned *header) {
-    return max(header[0], header[1]) >= (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u);
+// The points of a call without the sort.  A warp takes 32 adjacent points, each lane locates one;
+// then the D / 8 lanes of a slot gather and add a point's corners at a time, as in the direct
+// backward, the point's numbers coming and its gradients going by shuffles.  Such a call takes
+// 690 us at the headline shape (direct backward 515; one thread per point took 1540): half the
+// direct kernel's warps per SM, and twice its shuffles, four points in flight as quick as two.
+// Launching the direct kernels instead would cost every other call their empty launches.
+template <typename T, int D>
+__device__ __noinline__ void accumulate_unsorted(const Params &p, const SortPlan &sp, LevelTable &lt,
+                                                 bool softmax) {
+    using VT = VecTraits<T>;
+    constexpr int LPH = D / 8, kSlots = 32 / LPH;
+    if (threadIdx.x == 0) plan_replicas(lt, p);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, slot = lane / LPH, ch = lane % LPH * 8;
+    const unsigned P = (unsigned)(p.L * p.K), G = (unsigned)p.G;
+    const int GD = p.G * D;
+    const float scale = ldexpf(1.f, grad_scale_exponent<T>(sp.header, p.Q, p.K, softmax));
+    const unsigned points = (unsigned)p.Q * G * P, turns = (points + 31u) / 32u;   // of a sample
+    const int64_t extra_sample = extra_elems_per_sample(p.Q, p.G, D, p.L, p.K);
+    const T *attn = reinterpret_cast<const T *>(p.attn);
+    for (int64_t turn = (int64_t)blockIdx.x * kWalkWarps + (threadIdx.x >> 5); turn < p.B * turns;
+         turn += (int64_t)gridDim.x * kWalkWarps) {
+        const int64_t b = turn / turns;
+        const unsigned at = (unsigned)(turn - b * turns) * 32u + lane;
+        // ---- one lane per point
+        unsigned flags = 0, off = 0, red_off = 0, pair = 0;
+        float a = 0.f, fr = 0.f, fc = 0.f;
+        float2 dpix = make_float2(0.f, 0.f);
+        const int64_t e = b * points + at;
+        if (at < points) {
+            pair = at / P;
+            const unsigned pt = at - pair * P, q = pair / G;
+            const int l = (int)pt / p.K, head = (int)(pair - q * G) * D;
+            const int64_t whole_pair = b * (p.Q * p.G) + pair;
+            const float2 xy = sample_location<T>(p, e, whole_pair, l, (float)lt.W[l], (float)lt.H[l], dpix);
+            const PointGeom geo = locate(xy.x, xy.y, lt.H[l], lt.W[l], lt.start[l], GD);
+            flags = geo.flags | ((unsigned)l << kLevelShift);
+            fr = geo.fr, fc = geo.fc;
+            off = red_off = (unsigned)(geo.off00 + head);
+            if (lt.rep[l] > 1) {
+                const unsigned r = (q + pt) % (unsigned)lt.rep[l];
+                if (r > 0) {
+                    red_off = lt.rep_base[l] + (r - 1) * lt.level_elems[l] +
+                              (unsigned)((geo.r0 * lt.W[l] + geo.c0) * GD + head);
+                    flags |= kUseExtra;
+                }
+            }
+            if (flags & kInside) {
+                a = VT::to_float(attn[e]);
+                if (softmax) {
+                    const float2 st = sp.stats[whole_pair];
+                    a = expf(a - st.x) * st.y;
+                }
+            }
+        }
+        // ---- one slot per point
+        const T *value = reinterpret_cast<const T *>(p.value) + b * p.S * GD + ch;
+        const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + b * p.Q * GD + ch;
+        __half *image = reinterpret_cast<__half *>(p.grad_value) + b * p.S * GD + ch;
+        __half *extras = unsorted_extras(sp) + b * extra_sample + ch;
+        float gx = 0.f, gy = 0.f, ga = 0.f;      // of the lane's own point
+#pragma unroll 2
+        for (int i = 0; i < LPH; ++i) {
+            const int from = i * kSlots + slot;
+            const unsigned f = __shfl_sync(0xffffffffu, flags, from);
+            const unsigned o00 = __shfl_sync(0xffffffffu, off, from), q00 = __shfl_sync(0xffffffffu, red_off, from);
+            const float r = __shfl_sync(0xffffffffu, fr, from), c = __shfl_sync(0xffffffffu, fc, from);
+            const float s0 = __shfl_sync(0xffffffffu, a, from) * scale;
+            const unsigned row = __shfl_sync(0xffffffffu, pair, from);
+            const unsigned down = (unsigned)lt.rowstride[f >> kLevelShift];
+            const unsigned step[4] = {0u, (unsigned)GD, down, down + (unsigned)GD};
+            const float w[4] = {(1.f - r) * (1.f - c), (1.f - r) * c, r * (1.f - c), r * c};
+            float2 go[4];
+            VT::unpack(ldg16(grad_out + (size_t)row * D), go);
+            uint4 raw[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) raw[k] = ldg16_if(value + (int)(o00 + step[k]), f & (1u << k));
+            __half *to = f & kUseExtra ? extras : image;
+            float dot[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float2 v[4], gv[4], d2 = make_float2(0.f, 0.f);
+                VT::unpack(raw[k], v);
+                const float s = s0 * w[k];
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    ffma2(d2, v[n], go[n]);
+                    gv[n] = fmul2(go[n], make_float2(s, s));
+                }
+                dot[k] = d2.x + d2.y;
+                red_if<__half>(to + (q00 + step[k]), gv, f & (1u << k));
+            }
+            float x = (1.f - r) * (dot[1] - dot[0]) + r * (dot[3] - dot[2]);
+            float y = (1.f - c) * (dot[2] - dot[0]) + c * (dot[3] - dot[1]);
+            float g = w[0] * dot[0] + w[1] * dot[1] + w[2] * dot[2] + w[3] * dot[3];
+#pragma unroll
+            for (int o = LPH >> 1; o > 0; o >>= 1) {
+                x += __shfl_xor_sync(0xffffffffu, x, o);
+                y += __shfl_xor_sync(0xffffffffu, y, o);
+                g += __shfl_xor_sync(0xffffffffu, g, o);
+            }
+            const int mine = lane % kSlots * LPH;      // a lane of the slot that had this lane's point
+            x = __shfl_sync(0xffffffffu, x, mine);
+            y = __shfl_sync(0xffffffffu, y, mine);
+            g = __shfl_sync(0xffffffffu, g, mine);
+            if (lane / kSlots == i) gx = x, gy = y, ga = g;
+        }
+        if (at < points) {
+            const bool inside = flags & kInside;       // a skipped point: exact zeros
+            store_point_gradients<T>(p, sp, e,
+                                     inside ? make_float2(a * dpix.x * gx, a * dpix.y * gy) : make_float2(0.f, 0.f),
+                                     inside ? ga : 0.f);
+        }
+    }
 }
 
 // ---- pass 2: write the points' records in order of their cells ------------------------------------
@@ -482,11 +572,17 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     const int P = p.L * p.K;
     const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
     const int64_t base = pair0 * P + c.pt;
-    const bool sorted = c.rows > 0 && !unsortable_call<T>(sp.header);
     const int nq = c.active ? c.nq : 0;
+    if (unsorted_call<T>(sp.header)) {
+        uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
+        const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
+        for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs;
+             i += (int64_t)gridDim.x * kSortThreads)
+            extras[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
     __syncthreads();
-    unsigned at[kSortPoints];     // cell << 16 | rank among the CTA's points of the cell; ~0: not sorted
-    unsigned left_out = 0;        // points direct_point() has to take
+    unsigned at[kSortPoints];     // cell << 16 | rank among the CTA's points of the cell; ~0: skipped
 #pragma unroll
     for (int r0 = 0; r0 < kSortPoints; r0 += kSortBatch) {
         float2 xy[kSortBatch], stats[SOFTMAX ? kSortBatch : 1];
@@ -509,8 +605,6 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
             if (!find_cell(c, xy[r], pc)) {
                 // a skipped point: exact zeros
                 store_point_gradients<T>(p, sp, base + (int64_t)(q * (p.G * P)), make_float2(0.f, 0.f), 0.f);
-            } else if (!sorted) {
-                left_out |= 1u << (r0 + r);
             } else {
                 float a = VT::to_float(weight[r]);
                 if constexpr (SOFTMAX) a = expf(a - stats[r].x) * stats[r].y;
@@ -544,17 +638,6 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
         for (unsigned i = threadIdx.x; i < points; i += kSortThreads) {
             const unsigned place = i + shift[cell_of[i]];
             if (place < (unsigned)sp.plane_points) records[place] = local[order[i]];
-        }
-    }
-    if (left_out != 0) {
-        const float scale = ldexpf(1.f, grad_scale_exponent<T>(sp.header, p.Q, p.K, SOFTMAX));
-        for (int r = 0; r < kSortPoints; ++r) {
-            if (!(left_out >> r & 1u)) continue;
-            const int q = c.ql + r * c.step;
-            const int64_t pair = pair0 + (int64_t)q * p.G;
-            float a = VT::to_float(attn[pair * P + c.pt]);
-            if constexpr (SOFTMAX) a = expf(a - sp.stats[pair].x) * sp.stats[pair].y;
-            direct_point<T>(p, sp, lt, pair, c.pt, a, scale);
         }
     }
 }
@@ -612,7 +695,6 @@ __device__ __forceinline__ float lds4(uint32_t addr) {
 }
 
 constexpr int kStep = 32;          // points a warp takes at a time, one per lane
-constexpr int kWalkWarps = 4;      // warps per CTA, each on its own run
 
 // byte offset of 16-byte chunk `chunk` of row `row` of a step's grad_out rows (2*D bytes each):
 // chunks permuted so that the row-wise reads (8 lanes: two to four rows) touch every bank once.
@@ -712,7 +794,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
     grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = lane >> 2, c = lane & 3;
-    if (unsortable_call<T>(sp.header)) return;
+    if (unsorted_call<T>(sp.header)) {
+        accumulate_unsorted<T, D>(p, sp, lt, softmax);
+        return;
+    }
     const int cells = ct.first[p.L];
     const int GD = p.G * D, GP = p.G * p.L * p.K;
     // float16 weights are kept near 1 whatever their largest magnitude
@@ -1045,7 +1130,22 @@ __global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_cons
         }
         for (int64_t i = body * 4 + first; i < points; i += stride) grad_attn[i] = VT::from_float(sp.grad_prob[i]);
     }
-    const float inv = ldexpf(1.f, -grad_scale_exponent<T>(sp.header, p.Q, p.K, SOFTMAX));
+    const int exponent = grad_scale_exponent<T>(sp.header, p.Q, p.K, SOFTMAX);
+    if (unsorted_call<T>(sp.header)) {
+        __shared__ LevelTable lt;
+        __shared__ int extra_range[2];
+        load_level_table(lt, p);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            plan_replicas(lt, p);
+            find_extra_range(lt, p.L, extra_range);
+        }
+        __syncthreads();
+        finalize_image<T>(p, lt, extra_range, exponent, reinterpret_cast<const uint4 *>(p.grad_value),
+                          unsorted_extras(sp));
+        return;
+    }
+    const float inv = ldexpf(1.f, -exponent);
     uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
     const int64_t total = p.B * p.S * (p.G * p.D / 8);
     constexpr int kTurn = 4;
