@@ -1234,6 +1234,15 @@ int64_t round_up(int64_t n, int64_t to) { return (n + to - 1) / to * to; }
 //   offsets instead of          the arithmetic of the locations is done once more: 16 channels
 //   locations                   228 -> 251, 32: 157 -> 159 at 2 M points, 285 -> 275 at 4 M, 551
 //                               -> 503 at 8 M; 64 (1.8 M points): 241 -> 202
+//   positions                   the scatter kernel has two CTAs per SM up to 26 000, then one: at 42 000
+//                               510 -> 454, at 51 450 329 -> 298.  From about 55 000 a plane has more
+//                               than kSharedCells cells (one per 6.8 positions) and its records leave
+//                               unordered: 12 points per position, 58 968 positions, 16 channels 327 ->
+//                               345, 32: 370 -> 376, 64: 331 -> 251; 73 500: 747 -> 962, 880 -> 1027,
+//                               796 -> 665; 24 points, 73 500: 816 -> 769, 923 -> 814, 712 -> 529; 16
+//                               points on four levels: 490 -> 618, 600 -> 665, 509 -> 455; 40 on five,
+//                               where the few cells of the last one are counted by all: 1117 -> 1693,
+//                               1558 -> 1760, 1177 -> 1427
 bool sorting_pays(const Params &p, int dtype) {
     const int64_t P = (int64_t)p.L * p.K, points = p.B * p.G * p.Q * P;
     if (dtype != 1 && dtype != 2) return false;
@@ -1243,6 +1252,9 @@ bool sorting_pays(const Params &p, int dtype) {
         p.S >= (1ll << 29))
         return false;
     if (p.Q * P < 8 * p.S) return false;
+    if (p.S > 55000 &&
+        (p.ref != nullptr || p.L > 4 || p.D == 16 || (p.D == 32 && p.Q * P < 24 * p.S)))
+        return false;
     if (p.ref != nullptr && p.D < 64) return p.D == 32 && points >= 3000000;
     return points >= 1000000;
 }

@@ -265,6 +265,21 @@ def test_host_only_entry_points():
     assert "2^31" in shim.last_error()
 
 
+@pytest.mark.parametrize("S, L, K, G, D, sorts", [
+    (51450, 3, 4, 8, 32, True), (42000, 3, 4, 8, 16, True),         # cells counted in shared memory
+    (58968, 3, 4, 8, 32, False), (73500, 3, 4, 8, 16, False),       # too many: only where it still pays
+    (73500, 3, 8, 8, 32, True), (73500, 3, 8, 8, 16, False), (73500, 3, 4, 4, 64, True),
+    (74609, 5, 8, 4, 64, False),
+])
+def test_large_pyramids_are_sorted_only_where_that_is_faster(S, L, K, G, D, sorts):
+    from deformops_b200._loader import load_library
+
+    shim = load_library()
+    shape = (1, S, G, D, S, L, K, 2)
+    assert (shim.workspace_bytes(*shape, 0) > shim.scratch_bytes(*shape)) == sorts
+
+
+
 def test_error_message_is_thread_local():
     import threading
 
