@@ -416,9 +416,9 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
         const int64_t usual =
             (msda_b200_backward_scratch_bytes(B, S, G, D, Q, L, K, dtype) + 15) / 16 * 16;
         if (scratch_bytes >= usual + msda_b200::kFusedBytes) {
-            p.fused_magnitudes = static_cast<char *>(scratch) + usual;
+            p.fused_header = reinterpret_cast<unsigned *>(static_cast<char *>(scratch) + usual);
             e = msda_b200::launch_backward_fused(p, dtype, apply_softmax != 0, s);
-            return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "backward: kernel launch (cooperative)");
+            return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "backward: kernel launch (small call)");
         }
     }
     if (use_scratch) {

@@ -26,8 +26,6 @@
 // that receives more than 256 additions per element gets extra replicas of itself there.
 // prepare_kernel clears what is added into and finds the magnitudes the scale is derived from,
 // finalize_kernel sums the replicas, unscales and writes grad_value in its own type.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <type_traits>
 
@@ -76,11 +74,13 @@ namespace {
 
 // ---- scaled float16 image: preparation and finalisation ----------------------------------------
 // Clears the float16 image the backward adds into and leaves the largest |grad_out| (and, without
-// softmax, |attn|) element that the CTA's threads found in cta_max[0] / [1].
+// softmax, |attn|) element that the CTA's threads found in cta_max[0] / [1].  The part of one of
+// `shares` CTAs.
 template <bool WITH_ATTN>
-__device__ __forceinline__ void prepare_image(const Params &p, unsigned (&cta_max)[2]) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void prepare_image(const Params &p, unsigned (&cta_max)[2], int share,
+                                              int shares) {
+    const int64_t stride = (int64_t)shares * blockDim.x;
+    const int64_t first = (int64_t)share * blockDim.x + threadIdx.x;
     uint4 *image = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(p.scratch) + kScratchHeaderBytes);
     const int64_t image_vecs = p.B * p.S * (p.G * p.D / 8);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -120,7 +120,7 @@ template <bool WITH_ATTN>
 __global__ void __launch_bounds__(256, MSDA_PREP_MIN_CTAS) prepare_kernel(const Params p) {
     grid_launch_dependents();   // the backward kernel may load its tables meanwhile
     __shared__ unsigned cta_max[2];
-    prepare_image<WITH_ATTN>(p, cta_max);
+    prepare_image<WITH_ATTN>(p, cta_max, (int)blockIdx.x, (int)gridDim.x);
     unsigned *header = reinterpret_cast<unsigned *>(p.scratch);
     if (threadIdx.x < (WITH_ATTN ? 2 : 1) && cta_max[threadIdx.x] != 0)
         atomicMax(header + threadIdx.x, cta_max[threadIdx.x]);
@@ -129,11 +129,12 @@ __global__ void __launch_bounds__(256, MSDA_PREP_MIN_CTAS) prepare_kernel(const 
 // grad_value from the image and the extras of the scratch
 template <typename T>
 __device__ __forceinline__ void finalize_scratch(const Params &p, const LevelTable &lt,
-                                                 const int (&extra_range)[2], int exponent) {
+                                                 const int (&extra_range)[2], int exponent, int share,
+                                                 int shares) {
     const uint4 *image = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(p.scratch) +
                                                          kScratchHeaderBytes);
     finalize_image<T>(p, lt, extra_range, exponent, image,
-                      reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)(p.G * p.D));
+                      reinterpret_cast<const __half *>(image) + p.B * p.S * (int64_t)(p.G * p.D), share, shares);
 }
 
 template <typename T, bool SOFTMAX>
@@ -149,13 +150,55 @@ __global__ void __launch_bounds__(256, MSDA_FIN_MIN_CTAS) finalize_kernel(const 
     __syncthreads();
     grid_dependency_wait();     // the image is complete once the backward kernel has finished
     finalize_scratch<T>(p, lt, extra_range,
-                        grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch), p.Q, p.K, SOFTMAX));
+                        grad_scale_exponent<T>(reinterpret_cast<const unsigned *>(p.scratch), p.Q, p.K, SOFTMAX),
+                        (int)blockIdx.x, (int)gridDim.x);
+}
+
+// ---- the scaled backward in one launch ------------------------------------------------------------
+// A small call is bound by the host's launches, not by the GPU, so its two sweeps are part of the
+// backward kernel.  The phases - clear and find the magnitudes, add, convert - are handed out in
+// pieces by counters, and a CTA goes on to the next phase when the pieces of the last are done,
+// not when other CTAs arrive: a piece that was handed out is in the hands of a CTA that
+// runs and does not wait before it is done.  So however few CTAs the GPU has room for beside other
+// streams' kernels, they finish the call, and those that come late find nothing left.  (A
+// cooperative launch with grid barriers was as quick, 72.6 us of a decoder layer's forward + backward
+// against 72.9, but waited for room for all its CTAs: beside a one-thread kernel of 1 ms on another
+// stream a backward of 64 us took 1050; this one takes 69.)
+
+// The next piece of what `cell` counts, for the whole CTA; `slot` is shared.
+__device__ __forceinline__ unsigned next_piece(unsigned *cell, unsigned &slot) {
+    __syncthreads();               // (the piece before it is done, and `slot` read)
+    if (threadIdx.x == 0) slot = atomicAdd(cell, 1u);
+    __syncthreads();
+    return slot;
+}
+// Waits, the whole CTA, until `cell` counts `pieces` done; false if that takes longer than anything
+// that happens can (the other pieces run while this waits, see above), some seconds.
+__device__ __forceinline__ bool pieces_done(unsigned *header, FusedCell cell, unsigned pieces, unsigned &slot) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bool done = false;
+        for (unsigned turn = 0; turn < (1u << 22) && !done; ++turn) {
+            unsigned n;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(header + cell) : "memory");
+            done = n >= pieces;
+            if (!done) __nanosleep(100);
+        }
+        if (!done) atomicExch(header + kFusedGaveUp, 1u);
+        slot = done;
+    }
+    __syncthreads();
+    return slot != 0u;
+}
+// Counts a piece of the whole CTA as done: its writes are visible to whoever reads the count.
+__device__ __forceinline__ void count_done(unsigned *cell) {
+    __syncthreads();
+    __threadfence();
+    if (threadIdx.x == 0) atomicAdd(cell, 1u);
 }
 
 // SCALED: grad_value contributions go, times 2^e, into the float16 image of the scratch.
-// FUSED: the sweeps before and after are part of the same cooperative launch, between grid
-// barriers.  A small call is bound by the host's launches (a header memset and three kernels took it
-// 16 us, one cooperative launch 6), not by the GPU.
+// FUSED: the sweeps before and after are part of the same launch.
 template <typename T, bool SOFTMAX, bool SCALED, bool FUSED>
 __global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_kernel(const Params p) {
     using VT = VecTraits<T>;
@@ -193,26 +236,19 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_k
     // written by the kernel before this one
     grid_dependency_wait();
     grid_launch_dependents();
-    __shared__ unsigned magnitudes[2];
+    __shared__ unsigned magnitudes[2], slot_of_cta;
     const unsigned *header = reinterpret_cast<const unsigned *>(p.scratch);
     if constexpr (FUSED) {
-        // every CTA leaves what it found in a place of its own: nothing has to be zero beforehand
-        prepare_image<!SOFTMAX>(p, magnitudes);
-        uint2 *found = reinterpret_cast<uint2 *>(p.fused_magnitudes);
-        if (threadIdx.x == 0) found[blockIdx.x] = make_uint2(magnitudes[0], magnitudes[1]);
-        cooperative_groups::this_grid().sync();
-        unsigned mg = 0, ma = 0;
-        for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
-            const uint2 m = __ldcg(found + i);
-            mg = max(mg, m.x);
-            ma = max(ma, m.y);
+        const unsigned sweeps = (unsigned)p.passes;
+        for (unsigned i; (i = next_piece(p.fused_header + kFusedSweep, slot_of_cta)) < sweeps;) {
+            prepare_image<!SOFTMAX>(p, magnitudes, (int)i, (int)sweeps);
+            if (threadIdx.x < 2 && magnitudes[threadIdx.x] != 0)
+                atomicMax(p.fused_header + (threadIdx.x == 0 ? kFusedGradOut : kFusedAttn), magnitudes[threadIdx.x]);
+            count_done(p.fused_header + kFusedSwept);
         }
-        mg = __reduce_max_sync(0xffffffffu, mg);
-        ma = __reduce_max_sync(0xffffffffu, ma);
-        if (lane == 0) {
-            atomicMax(&magnitudes[0], mg);
-            atomicMax(&magnitudes[1], ma);
-        }
+        if (!pieces_done(p.fused_header, kFusedSwept, sweeps, slot_of_cta)) return;
+        if (threadIdx.x < 2)
+            magnitudes[threadIdx.x] = __ldcg(p.fused_header + (threadIdx.x == 0 ? kFusedGradOut : kFusedAttn));
         __syncthreads();
         header = magnitudes;
     }
@@ -241,9 +277,15 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_k
     // grid-stride loop here cost registers the kernel does not have: 0.617 ms per call with it
     // against 0.583 ms in this form.  The register allocation at 64 registers is sensitive to
     // the shape of this loop: check `-Xptxas -v` for spills after touching it.)
+    // (FUSED: a warp takes the next group.)
     const int passes = p.passes > 1 ? p.passes : 1;
-    for (int pass = 0; pass < passes; ++pass) {
-        const int64_t group = ((int64_t)blockIdx.x * passes + pass) * nwarps + warp;
+    for (int pass = 0; FUSED || pass < passes; ++pass) {
+        int64_t group = ((int64_t)blockIdx.x * passes + pass) * nwarps + warp;
+        if constexpr (FUSED) {
+            unsigned next = 0;
+            if (lane == 0) next = atomicAdd(p.fused_header + kFusedGroup, 1u);
+            group = __shfl_sync(0xffffffffu, next, 0);
+        }
         if (group >= p.num_groups) break;
         const int64_t pair0 = group * ppw;
         const int nlive = (int)min((int64_t)ppw, total_pairs - pair0);
@@ -413,12 +455,19 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : MSDA_BWD_MIN_CTAS) backward_k
             ga_out[idx] = VT::from_float(ga);
         }
         __syncwarp();
+        if constexpr (FUSED) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) atomicAdd(p.fused_header + kFusedGroups, 1u);
+        }
     }
     if constexpr (FUSED) {
         __shared__ int extra_range[2];
+        if (!pieces_done(p.fused_header, kFusedGroups, (unsigned)p.num_groups, slot_of_cta)) return;
         if (threadIdx.x == 0) find_extra_range(lt, p.L, extra_range);
-        cooperative_groups::this_grid().sync();
-        finalize_scratch<T>(p, lt, extra_range, grad_scale_exponent<T>(magnitudes, p.Q, K, SOFTMAX));
+        for (unsigned i; (i = next_piece(p.fused_header + kFusedLast, slot_of_cta)) < (unsigned)p.passes;)
+            finalize_scratch<T>(p, lt, extra_range, grad_scale_exponent<T>(magnitudes, p.Q, K, SOFTMAX), (int)i,
+                                p.passes);
     }
 }
 
@@ -446,8 +495,7 @@ cudaError_t launch_kernel(const Params &p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// The whole scaled backward in one cooperative launch: at most as many CTAs as the GPU holds, each
-// walking adjacent sets of groups.
+// The whole scaled backward in one launch.  `passes` is the number of shares of each sweep.
 template <typename T, bool SOFTMAX>
 cudaError_t launch_fused(const Params &p, cudaStream_t stream) {
     const size_t smem = backward_smem_bytes(p, SOFTMAX);
@@ -457,26 +505,17 @@ cudaError_t launch_fused(const Params &p, cudaStream_t stream) {
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    static Residency residency;
-    const int64_t resident = std::min<int64_t>(residency.ctas(kernel, p.threads, smem), kFusedCtas);
-    if (resident <= 0) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaMemsetAsync(p.fused_header, 0, kFusedBytes, stream);
+    if (e != cudaSuccess) return e;
+    constexpr int64_t kCtas = 148 * 2;      // what the GPU holds; fewer finish it as well
     Params q = p;
     const int nwarps = p.threads / 32;
     const int64_t sets = (p.num_groups + nwarps - 1) / nwarps;
     const int64_t sweep = p.B * p.S * (p.G * p.D / 8) / (p.threads * 4);   // CTAs the image can use
-    q.grid = (unsigned)std::max<int64_t>(1, std::min(resident, std::max(sets, sweep)));
-    q.passes = (int)((sets + q.grid - 1) / q.grid);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(q.grid, 1, 1);
-    cfg.blockDim = dim3(q.threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, q);
+    q.passes = (int)std::max<int64_t>(1, std::min(kCtas, sweep));
+    q.grid = (unsigned)std::min(kCtas, std::max<int64_t>(sets, q.passes));
+    kernel<<<q.grid, q.threads, smem, stream>>>(q);
+    return cudaGetLastError();
 }
 
 template <typename T, bool SOFTMAX>

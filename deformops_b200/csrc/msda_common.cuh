@@ -63,7 +63,7 @@ struct Params {
     int point_chunk;        // descriptors per pair held in shared memory at a time
     int64_t num_groups;     // ceil(B*Q*G / pairs per warp)
     unsigned grid;
-    void *fused_magnitudes;  // one-launch backward: 8 bytes per CTA
+    unsigned *fused_header;  // one-launch backward: FusedCell cells, zero at the start
     int passes;             // backward: adjacent sets of groups one CTA walks (0 or 1: one)
     // Fused location arithmetic.  When `ref` is set, `loc` / `grad_loc` hold the predicted
     // offsets (B,Q,G,L,K,2) and their gradient, and a point samples at
@@ -279,8 +279,8 @@ inline cudaError_t launch_after_predecessor(Kernel kernel, unsigned grid, unsign
 constexpr size_t kPlainSmem = 46 * 1024;
 
 // CTAs of a kernel the GPU holds at once for a block size and a shared memory size.  The runtime is
-// asked once per combination (a query costs the host about as much as a launch); every GPU
-// this is built for answers alike.
+// asked once per combination (a query costs the host about as much as a launch).  Every GPU this
+// is built for answers alike; where fewer SMs can be had, grids sized by it run in more waves.
 class Residency {
   public:
     template <typename Kernel>
@@ -587,6 +587,7 @@ __host__ __device__ inline int backward_stage_floats(int pairs_per_warp, int P, 
 // Positions of levels that have replicas form a small range of every sample (the coarse levels:
 // 1 024 of 21 504 positions at the headline shape); everything outside it takes the short path.
 // `lt` has its replicas planned; `extra_range` is the CTA's.  `image` may be grad_value itself.
+// The part of one of `shares` CTAs.
 __device__ __forceinline__ void find_extra_range(const LevelTable &lt, int L, int (&extra_range)[2]) {
     int lo = 0x7fffffff, hi = 0;
     for (int l = 0; l < L; ++l)
@@ -601,7 +602,8 @@ __device__ __forceinline__ void find_extra_range(const LevelTable &lt, int L, in
 template <typename T>
 __device__ __forceinline__ void finalize_image(const Params &p, const LevelTable &lt,
                                                const int (&extra_range)[2], int exponent,
-                                               const uint4 *image, const __half *extras) {
+                                               const uint4 *image, const __half *extras, int share,
+                                               int shares) {
     using VT = VecTraits<T>;
     const int extra_lo = extra_range[0], extra_hi = extra_range[1];
     const bool any_extra = extra_lo < extra_hi;
@@ -613,8 +615,8 @@ __device__ __forceinline__ void finalize_image(const Params &p, const LevelTable
     const float2 inv2 = make_float2(inv, inv);
     uint4 *gv = reinterpret_cast<uint4 *>(p.grad_value);
     const int64_t total = p.B * p.S * (int64_t)vec_per_row;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)shares * blockDim.x;
+    const int64_t first = (int64_t)share * blockDim.x + threadIdx.x;
     // where the thread's current vector lies - sample b, position s of the sample, vector col of
     // the position's row - kept up to date by additions: one division per thread, none per vector
     // (first and stride are below 2^31: the grid is capped at a few thousand CTAs of 256 threads)
@@ -683,13 +685,18 @@ __device__ __forceinline__ void finalize_image(const Params &p, const LevelTable
 // launchers implemented in msda_forward.cu / msda_backward.cu; dtype: 0 f32, 1 f16, 2 bf16
 cudaError_t launch_forward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 cudaError_t launch_backward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
-// The scaled backward in one cooperative launch, for calls that are bound by the host: what its
-// scratch needs beyond the usual is 8 bytes for each of at most kFusedCtas CTAs.
-// (Host time of forward + backward of a decoder layer, B200: 78 us with separate launches, 73 so.
-// On the GPU it takes as long with 154 000 points (47 us against 49), longer with 516 000: 62
-// against 58, where the GPU is what bounds the call.)
-constexpr int kFusedCtas = 1024;
-constexpr int64_t kFusedBytes = 8 * kFusedCtas;
+// The scaled backward in one launch, for calls that are bound by the host: what its scratch needs
+// beyond the usual is a header of its own.  (Forward + backward of a decoder layer, host bound, B200:
+// 79.7 us with the three launches, 72.9 so.  On the GPU 51.2 us against 53.2 with 154 000 points, 77.9
+// against 75.8 with 262 000.)
+enum FusedCell : unsigned {                // a line of memory each
+    kFusedGradOut = 0, kFusedAttn = 32,    // largest magnitudes
+    kFusedSweep = 64, kFusedSwept = 96,    // shares of the first sweep: handed out, done
+    kFusedGroup = 128, kFusedGroups = 160, // groups of pairs: handed out, done
+    kFusedLast = 192,                      // shares of the last sweep handed out
+    kFusedGaveUp = 224,                    // not zero: a wait ran into its limit
+};
+constexpr int64_t kFusedBytes = 1024;
 inline bool fused_backward_pays(const Params &p) {
     return p.B * p.Q * p.G * (int64_t)(p.L * p.K) <= ((int64_t)1 << 18);
 }

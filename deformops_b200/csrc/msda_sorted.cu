@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_cons
         }
         __syncthreads();
         finalize_image<T>(p, lt, extra_range, exponent, reinterpret_cast<const uint4 *>(p.grad_value),
-                          unsorted_extras(sp));
+                          unsorted_extras(sp), (int)blockIdx.x, (int)gridDim.x);
         return;
     }
     const float inv = ldexpf(1.f, -exponent);

@@ -1,4 +1,4 @@
-"""The 16-bit backward in one cooperative launch (small calls whose scratch has room for it), against
+"""The 16-bit backward in one launch (small calls whose scratch has room for it), against
 the float64 oracle: a single CTA, replicas of a coarse level, several sets of groups per CTA."""
 
 from __future__ import annotations
@@ -30,3 +30,24 @@ def test_one_launch_backward_matches_the_oracle(dtype, softmax, D, K, levels, B,
     truth = orc.backward(*[t.cpu() for t in (v, sh, st, l, a)], go.cpu(), softmax=softmax)
     assert rel_err(to_np(got[0]), truth[0]) <= 1e-2
     assert rel_err(to_np(got[2]), truth[2].reshape(got[2].shape)) <= 1e-2
+
+
+def test_one_launch_backward_runs_beside_another_streams_kernel():
+    """It takes the room that there is: a kernel that stays on one SM does not hold it up."""
+    dtype = torch.float16
+    value, shapes, starts, loc, logits, grad_out = _inputs(1, 4, 300, 8, 32, 4, [(50, 67), (25, 34)])
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    want = _workspace_backward(v, sh, st, l, a, go, False)        # (the kernel is loaded, the scratch cached)
+    torch.cuda.synchronize()
+    side, main = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(400_000_000)                            # one thread, about 0.2 s
+        left = side.record_event()
+    with torch.cuda.stream(main):
+        got = _workspace_backward(v, sh, st, l, a, go, False)
+    main.synchronize()
+    assert not left.query(), "the call waited for the other stream"
+    side.synchronize()
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    assert rel_err(to_np(got[0]), to_np(want[0])) <= 1e-2
