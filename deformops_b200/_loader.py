@@ -44,7 +44,7 @@ class Shim:
     """Typed handles on the exported functions of the library."""
 
     #: every symbol ``include/msda_b200.h`` declares
-    SYMBOLS = ("msda_b200_abi_version", "msda_b200_last_error", "msda_b200_forward",
+    SYMBOLS = ("msda_b200_abi_version", "msda_b200_last_error", "msda_b200_launches", "msda_b200_forward",
                "msda_b200_backward", "msda_b200_backward_scratch_bytes",
                "msda_b200_backward_workspace_bytes", "msda_b200_column_sums",
                "msda_b200_column_sums_scratch_bytes",
@@ -61,6 +61,8 @@ class Shim:
         self.lib.msda_b200_abi_version.argtypes = []
         self.lib.msda_b200_last_error.restype = ctypes.c_char_p
         self.lib.msda_b200_last_error.argtypes = []
+        self.lib.msda_b200_launches.restype = None
+        self.lib.msda_b200_launches.argtypes = [ctypes.POINTER(_i64), ctypes.POINTER(_i64)]
         self.forward = self.lib.msda_b200_forward
         self.forward.restype = _int
         self.forward.argtypes = [_vp] * 6 + [_i64] * 7 + [_int, _int, _int, _vp]
@@ -102,6 +104,12 @@ class Shim:
         if got != ABI_VERSION:
             raise KernelUnavailableError(
                 f"{path} has ABI version {got}, this package needs {ABI_VERSION}: rebuild it")
+
+    def launches(self) -> "tuple[int, int]":
+        """Kernels and memsets the library has enqueued since it was loaded."""
+        kernels, memsets = _i64(), _i64()
+        self.lib.msda_b200_launches(ctypes.byref(kernels), ctypes.byref(memsets))
+        return kernels.value, memsets.value
 
     def last_error(self) -> str:
         return self.lib.msda_b200_last_error().decode("utf-8", "replace")

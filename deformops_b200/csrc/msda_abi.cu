@@ -1,6 +1,7 @@
 // C ABI of the library (declared in include/msda_b200.h): argument checks, launch
 // geometry and error reporting.  Takes over the role of the reference's host entry
 // sources/deformops/backends/cuda/include/msda_launch.cuh:63-275 without any torch type.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -11,6 +12,7 @@
 namespace {
 
 thread_local char g_error[512] = "";
+std::atomic<int64_t> g_kernels{0}, g_memsets{0};
 
 int fail(int status, const char *fmt, ...) {
     va_list ap;
@@ -168,6 +170,11 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
 
 namespace msda_b200 {
 int set_last_error(int status, const char *message) { return fail(status, "%s", message); }
+
+void count_launches(int kernels, int memsets) {
+    g_kernels.fetch_add(kernels, std::memory_order_relaxed);
+    g_memsets.fetch_add(memsets, std::memory_order_relaxed);
+}
 }  // namespace msda_b200
 
 extern "C" {
@@ -175,6 +182,11 @@ extern "C" {
 int msda_b200_abi_version(void) { return MSDA_B200_ABI_VERSION; }
 
 const char *msda_b200_last_error(void) { return g_error; }
+
+void msda_b200_launches(int64_t *kernels, int64_t *memsets) {
+    *kernels = g_kernels.load(std::memory_order_relaxed);
+    *memsets = g_memsets.load(std::memory_order_relaxed);
+}
 
 int64_t msda_b200_backward_scratch_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q,
                                          int64_t L, int64_t K, int dtype) {
@@ -294,7 +306,9 @@ int forward_impl(const void *value, const int64_t *spatial_shapes, const int64_t
         const cudaError_t e =
             cudaMemsetAsync(out, 0, (size_t)(B * Q * G * D) * element_size(dtype),
                             static_cast<cudaStream_t>(stream));
-        return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "forward: clearing the output");
+        if (e != cudaSuccess) return cuda_fail(e, "forward: clearing the output");
+        msda_b200::count_launches(0, 1);
+        return MSDA_B200_OK;
     }
     if (!value || !spatial_shapes || !level_start_index || !loc || !attn || !out)
         return fail(MSDA_B200_INVALID_ARGUMENT, "forward: null pointer argument");
@@ -318,6 +332,7 @@ int forward_impl(const void *value, const int64_t *spatial_shapes, const int64_t
             : msda_b200::launch_forward(p, dtype, apply_softmax != 0,
                                         static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "forward: kernel launch");
+    msda_b200::count_launches(1, 0);
     return MSDA_B200_OK;
 }
 
@@ -346,7 +361,9 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
             pts.ref != nullptr && pts.offsets16 ? 2 : (dtype == MSDA_B200_F64 ? 8 : 4);
         cudaError_t e = cudaMemsetAsync(pts.grad, 0, points * 2 * loc_elem, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(grad_attn, 0, points * element_size(dtype), s);
-        return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "backward: clearing the gradients");
+        if (e != cudaSuccess) return cuda_fail(e, "backward: clearing the gradients");
+        msda_b200::count_launches(0, 2);
+        return MSDA_B200_OK;
     }
     const bool use_scratch = scratch != nullptr &&
                              (dtype == MSDA_B200_F16 || dtype == MSDA_B200_BF16) && S > 0 && Q > 0;
@@ -408,6 +425,7 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
                 msda_b200::plan_sorted(sp, part, softmax, n, scratch);
                 e = msda_b200::launch_backward_sorted(part, sp, dtype, softmax, s);
                 if (e != cudaSuccess) return cuda_fail(e, "backward: kernel launch (sorted)");
+                msda_b200::count_launches(4, 1);
             }
             return MSDA_B200_OK;
         }
@@ -418,15 +436,19 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
         if (scratch_bytes >= usual + msda_b200::kFusedBytes) {
             p.fused_header = reinterpret_cast<unsigned *>(static_cast<char *>(scratch) + usual);
             e = msda_b200::launch_backward_fused(p, dtype, apply_softmax != 0, s);
-            return e == cudaSuccess ? MSDA_B200_OK : cuda_fail(e, "backward: kernel launch (small call)");
+            if (e != cudaSuccess) return cuda_fail(e, "backward: kernel launch (small call)");
+            msda_b200::count_launches(1, 1);
+            return MSDA_B200_OK;
         }
     }
     if (use_scratch) {
         e = msda_b200::launch_prepare_grad_value(p, dtype, apply_softmax != 0, s);
         if (e != cudaSuccess) return cuda_fail(e, "backward: clearing grad_value / scratch");
+        msda_b200::count_launches(1, 1);
     } else if (zero_grad_value && S > 0) {
         e = cudaMemsetAsync(grad_value, 0, (size_t)(B * S * G * D) * element_size(dtype), s);
         if (e != cudaSuccess) return cuda_fail(e, "backward: clearing grad_value");
+        msda_b200::count_launches(0, 1);
     }
     if (Q == 0) return MSDA_B200_OK;
     if (dtype == MSDA_B200_F64)
@@ -434,9 +456,11 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
     else
         e = msda_b200::launch_backward(p, dtype, apply_softmax != 0, s);
     if (e != cudaSuccess) return cuda_fail(e, "backward: kernel launch");
+    msda_b200::count_launches(1, 0);
     if (use_scratch) {
         e = msda_b200::launch_finalize_grad_value(p, dtype, apply_softmax != 0, s);
         if (e != cudaSuccess) return cuda_fail(e, "backward: converting the scratch image");
+        msda_b200::count_launches(1, 0);
     }
     return MSDA_B200_OK;
 }

@@ -711,5 +711,7 @@ size_t backward_smem_bytes(const Params &p, bool softmax);
 // records `message` as the calling thread's last error (what msda_b200_last_error returns)
 // and hands `status` back; defined in msda_abi.cu next to the buffer it writes
 int set_last_error(int status, const char *message);
+// adds to what msda_b200_launches() reports; defined there too
+void count_launches(int kernels, int memsets);
 
 }  // namespace msda_b200

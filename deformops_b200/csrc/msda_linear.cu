@@ -141,6 +141,7 @@ int msda_b200_column_sums(const void *x, void *out, void *scratch, int64_t rows,
         default: return set_last_error(MSDA_B200_INVALID_ARGUMENT, "column_sums: dtype is not f32, f16 or bf16");
     }
     if (e != cudaSuccess) return set_last_error(MSDA_B200_CUDA_ERROR, cudaGetErrorString(e));
+    count_launches(2, 0);
     return MSDA_B200_OK;
 }
 

@@ -55,8 +55,6 @@ struct Abi {
     decltype(&msda_b200_column_sums_scratch_bytes) column_sums_scratch_bytes = nullptr;
 } abi;
 
-std::atomic<int64_t> g_kernels{0}, g_memsets{0};
-
 // One call: the operands as the kernels take them.  `ref` is undefined when `points` holds
 // locations, else `points` holds predicted offsets.
 struct Call {
@@ -124,7 +122,6 @@ Tensor run_forward(const Call &c) {
                          device.index(), stream);
     }
     check_status(st, c.ref.defined() ? "msda_b200_forward_offsets" : "msda_b200_forward");
-    g_kernels.fetch_add(1, std::memory_order_relaxed);
     return out;
 }
 
@@ -168,8 +165,6 @@ variable_list run_backward(const Call &c, const Tensor &grad_in) {
                           c.L, c.K, dtype, c.softmax, 1, device.index(), stream);
     }
     check_status(st, c.ref.defined() ? "msda_b200_backward_offsets" : "msda_b200_backward");
-    g_kernels.fetch_add(nbytes > 0 ? 3 : 1, std::memory_order_relaxed);
-    g_memsets.fetch_add(1, std::memory_order_relaxed);
     return {grad_value, grad_points, grad_attn};
 }
 
@@ -215,7 +210,6 @@ Tensor column_sums(const Tensor &x) {
                                  x.size(0), x.size(1), dtype_code(x.scalar_type()),
                                  c10::cuda::getCurrentCUDAStream(device.index()).stream()),
                  "msda_b200_column_sums");
-    g_kernels.fetch_add(2, std::memory_order_relaxed);
     return out;
 }
 
@@ -461,10 +455,6 @@ PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
-PyObject *py_launches(PyObject *, PyObject *) {
-    return Py_BuildValue("LL", (long long)g_kernels.load(), (long long)g_memsets.load());
-}
-
 template <typename F>
 PyCFunction as_method(F f) {
     return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f));
@@ -476,7 +466,6 @@ PyMethodDef methods[] = {
     {"linear", as_method(py_linear<1>), METH_FASTCALL, nullptr},
     {"linear_pair", as_method(py_linear<2>), METH_FASTCALL, nullptr},
     {"bind", as_method(py_bind), METH_FASTCALL, nullptr},
-    {"launches", py_launches, METH_NOARGS, "kernels and memsets issued through this module"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "msda_b200_host", nullptr, -1, methods,

@@ -69,35 +69,28 @@ _FORWARD_INPUTS = 9
 
 
 class _LaunchCounter:
-    """Counts launches issued by the package's calls: forward 1 kernel; backward with the scaled
-    float16 scratch 3 kernels (prepare, backward, finalize) and a 256-byte memset of the scratch
-    header, else 1 kernel and 1 memset of grad_value.  Calls that took the native path are
-    counted there and added here."""
+    """Kernels and memsets enqueued by the kernel library since :meth:`reset` (or its loading), as
+    the library counts them, whichever way its calls were made: a forward is one kernel, a backward
+    a memset and one kernel (float32, small 16-bit calls), three (16-bit with scratch) or four
+    for each turn over the samples (sorted points); a bias gradient two kernels."""
 
     def __init__(self) -> None:
-        self._counts = [0, 0]
-        self._native_base = (0, 0)
+        self._base = (0, 0)
 
     @staticmethod
-    def _native() -> tuple[int, int]:
-        host = _loader._host
-        return host.launches() if host is not None else (0, 0)
+    def _total() -> tuple[int, int]:
+        return _loader._shim.launches() if _loader.loaded() else (0, 0)
 
     def reset(self) -> None:
-        self._counts = [0, 0]
-        self._native_base = self._native()
-
-    def add(self, kernels: int, memsets: int = 0) -> None:
-        self._counts[0] += kernels
-        self._counts[1] += memsets
+        self._base = self._total()
 
     @property
     def kernels(self) -> int:
-        return self._counts[0] + self._native()[0] - self._native_base[0]
+        return self._total()[0] - self._base[0]
 
     @property
     def memsets(self) -> int:
-        return self._counts[1] + self._native()[1] - self._native_base[1]
+        return self._total()[1] - self._base[1]
 
 
 launch_counter = _LaunchCounter()
@@ -162,7 +155,6 @@ def _make_forward(softmax: bool) -> Callable[..., Tensor]:
                           int(softmax), value.device.index, ctypes.c_void_p(stream))
         if st != 0:
             _raise(shim, st, "msda_b200_forward")
-        launch_counter.add(1)
         return out
 
     return forward_cuda
@@ -195,7 +187,6 @@ def _make_backward(softmax: bool) -> Callable[..., tuple[Tensor, Tensor, Tensor]
                            int(softmax), 1, value.device.index, ctypes.c_void_p(stream))
         if st != 0:
             _raise(shim, st, "msda_b200_backward")
-        launch_counter.add((3 if nbytes else 1) if Q > 0 else 0, 1)
         return grad_value, grad_loc, grad_attn
 
     return backward_cuda
@@ -323,7 +314,6 @@ def _offsets_forward_cuda(value, spatial_shapes, level_start_index, reference_po
                               ctypes.c_void_p(stream))
     if st != 0:
         _raise(shim, st, "msda_b200_forward_offsets")
-    launch_counter.add(1)
     return out
 
 
@@ -354,7 +344,6 @@ def _offsets_backward_cuda(value, spatial_shapes, level_start_index, reference_p
         DTYPE_CODES[value.dtype], int(softmax), 1, value.device.index, ctypes.c_void_p(stream))
     if st != 0:
         _raise(shim, st, "msda_b200_backward_offsets")
-    launch_counter.add((3 if nbytes else 1) if Q > 0 else 0, 1)
     return grad_value, grad_offsets, grad_attn
 
 

@@ -24,8 +24,8 @@
  *   - Return value: MSDA_B200_OK or a negative status; the message of the last failure
  *     on the calling thread is available from msda_b200_last_error().  No exception or
  *     longjmp ever crosses the boundary.
- *   - Thread safety: no mutable global state; concurrent calls from several host
- *     threads (for example the autograd thread) are allowed.
+ *   - Thread safety: no mutable global state but the two counters of msda_b200_launches;
+ *     concurrent calls from several host threads (for example the autograd thread) are allowed.
  *   - Supported: dtype f32 / f16 / bf16 (and f64, see the enum); D a multiple of 4 (f32) or
  *     8 (f16, bf16);
  *     1 <= L <= 16; any K >= 1; S*G*D < 2^31 per sample.  B == 0 or Q == 0 is a
@@ -59,6 +59,9 @@ enum msda_b200_status {
 
 /* Version of this ABI; bumped on any signature change. */
 int msda_b200_abi_version(void);
+
+/* Kernels and memsets that calls of this library have enqueued since it was loaded, by all threads. */
+void msda_b200_launches(int64_t *kernels, int64_t *memsets);
 
 /* Message of the last failing call on this thread ("" if none). Never NULL. */
 const char *msda_b200_last_error(void);
@@ -94,7 +97,9 @@ int msda_b200_forward(const void *value, const int64_t *spatial_shapes,
  * in float16 (11 significant bits, packed 16-byte reductions) into an image of grad_value
  * held in the scratch (a level that receives more than 256 additions per element is given
  * several accumulators there), and a last pass unscales the sums into grad_value in `dtype`.  Such
- * a call enqueues a 256-byte memset and three kernels; for large shapes the second and third are
+ * a call enqueues a 256-byte memset and three kernels; with msda_b200_backward_workspace_bytes(...)
+ * of scratch a small one is a memset and one kernel, a densely sampled one a memset and four kernels
+ * for as many samples as the scratch holds at a time.  For large shapes all but the first are
  * launched as programmatic dependents of the one before (they become resident while it drains
  * and wait for its completion on the device), which CUDA-graph capture records as well.  With
  * scratch == NULL every contribution is added straight into grad_value in `dtype` (least

@@ -170,6 +170,25 @@ def test_empty_calls_return_zeros_without_launch():
     assert out.numel() == 0 and launch_counter.kernels == 0
 
 
+@pytest.mark.parametrize("dtype,Q,kernels", [
+    (torch.float32, 4000, 1), (torch.float16, 4000, 1),        # 128 000 points: one launch
+    (torch.float16, 16000, 3), (torch.bfloat16, 40000, 4),     # direct with scratch; sorted
+])
+def test_launch_counter_counts_what_is_launched(dtype, Q, kernels):
+    from deformops_b200.ops import launch_counter
+    from deformops_b200.registry import msda
+
+    shapes = torch.tensor([[20, 20], [10, 10]], device="cuda")
+    value = torch.randn(1, 500, 8, 32, device="cuda", dtype=dtype, requires_grad=True)
+    loc = torch.rand(1, Q, 8, 2, 2, 2, device="cuda")
+    attn = torch.rand(1, Q, 8, 4, device="cuda").to(dtype)
+    launch_counter.reset()
+    out = msda(value, shapes, torch.tensor([0, 400], device="cuda"), loc, attn)
+    assert (launch_counter.kernels, launch_counter.memsets) == (1, 0)
+    out.backward(torch.ones_like(out))
+    assert (launch_counter.kernels, launch_counter.memsets) == (1 + kernels, 1)
+
+
 def test_autocast_keeps_float32_locations():
     from deformops_b200.registry import msda
 

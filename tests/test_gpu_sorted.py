@@ -85,6 +85,7 @@ def test_samples_take_turns_when_the_scratch_holds_only_some():
     """Three samples of 4.1 M points, scratch for one and for two: the same gradients, from
     sample bases that are not 16-byte aligned in the weights (Q * G * P odd multiples of 2)."""
     from deformops_b200._loader import load_library
+    from deformops_b200.ops import launch_counter
 
     B, Q, G, D, K, levels = 3, 45763, 5, 16, 6, [(24, 20), (7, 5), (4, 3)]
     value, shapes, starts, loc, logits, grad_out = _inputs(3, B, Q, G, D, K, levels)
@@ -92,8 +93,10 @@ def test_samples_take_turns_when_the_scratch_holds_only_some():
     v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
     l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
     full = load_library().workspace_bytes(B, v.shape[1], G, D, Q, len(levels), K, 2, 0)
-    for nbytes in (full * 45 // 100, full * 9 // 10):
+    for nbytes, turns in ((full * 45 // 100, 3), (full * 9 // 10, 2)):
+        launch_counter.reset()
         got = _workspace_backward(v, sh, st, l, a, go, False, nbytes)
+        assert (launch_counter.kernels, launch_counter.memsets) == (4 * turns, turns)
         _check(got, (v, sh, st, l, a), go, False, shapes, l)
 
 
