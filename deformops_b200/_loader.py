@@ -46,7 +46,8 @@ class Shim:
     #: every symbol ``include/msda_b200.h`` declares
     SYMBOLS = ("msda_b200_abi_version", "msda_b200_last_error", "msda_b200_launches", "msda_b200_forward",
                "msda_b200_backward", "msda_b200_backward_scratch_bytes",
-               "msda_b200_backward_workspace_bytes", "msda_b200_column_sums",
+               "msda_b200_backward_workspace_bytes", "msda_b200_backward_offsets_workspace_bytes",
+               "msda_b200_column_sums",
                "msda_b200_column_sums_scratch_bytes",
                "msda_b200_forward_offsets", "msda_b200_backward_offsets",
                "msda_b200_backward_static_scratch", "msda_b200_launch_geometry")
@@ -76,6 +77,9 @@ class Shim:
         self.workspace_bytes = self.lib.msda_b200_backward_workspace_bytes
         self.workspace_bytes.restype = _i64
         self.workspace_bytes.argtypes = [_i64] * 7 + [_int, _int]
+        self.offsets_workspace_bytes = self.lib.msda_b200_backward_offsets_workspace_bytes
+        self.offsets_workspace_bytes.restype = _i64
+        self.offsets_workspace_bytes.argtypes = [_i64] * 7 + [_int, _int]
         self.column_sums = self.lib.msda_b200_column_sums
         self.column_sums.restype = _int
         self.column_sums.argtypes = [_vp, _vp, _vp, _i64, _i64, _int, _vp]
@@ -179,7 +183,8 @@ def host_module():
             functions = (shim.forward, shim.backward, shim.forward_offsets, shim.backward_offsets,
                          shim.workspace_bytes, shim.lib.msda_b200_last_error,
                          shim.lib.msda_b200_column_sums,
-                         shim.lib.msda_b200_column_sums_scratch_bytes)
+                         shim.lib.msda_b200_column_sums_scratch_bytes,
+                         shim.offsets_workspace_bytes)
             module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in functions))
             _host = module
         except Exception as exc:  # noqa: BLE001 - the Python operators remain

@@ -155,6 +155,24 @@ int check_points(const Points &pts, int offsets_dtype, int dtype, const char *wh
     return MSDA_B200_OK;
 }
 
+// Scratch with which a backward from locations or from offsets is fastest.
+int64_t workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q, int64_t L, int64_t K,
+                        int dtype, int apply_softmax, bool offsets) {
+    const int64_t scratch = msda_b200_backward_scratch_bytes(B, S, G, D, Q, L, K, dtype);
+    if (scratch == 0) return 0;
+    msda_b200::Params p{};
+    p.B = B, p.S = S, p.Q = Q;
+    p.G = (int)G, p.D = (int)D, p.L = (int)L, p.K = (int)K;
+    if (!msda_b200::sorting_pays(p, dtype, offsets))
+        return msda_b200::fused_backward_pays(p) ? (scratch + 15) / 16 * 16 + msda_b200::kFusedBytes : scratch;
+    // all samples at once, or as many as the target holds (at least one)
+    int64_t samples = B;
+    while (samples > 1 && msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples) > kWorkspaceTarget)
+        samples = samples > 8 ? samples - samples / 8 : samples - 1;
+    const int64_t sorted = msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples);
+    return sorted > scratch ? sorted : scratch;
+}
+
 int forward_impl(const void *value, const int64_t *spatial_shapes, const int64_t *level_start_index,
                  const Points &pts, const void *attn, void *out, int64_t B, int64_t S, int64_t G,
                  int64_t D, int64_t Q, int64_t L, int64_t K, int dtype, int apply_softmax,
@@ -198,19 +216,13 @@ int64_t msda_b200_backward_scratch_bytes(int64_t B, int64_t S, int64_t G, int64_
 
 int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q,
                                            int64_t L, int64_t K, int dtype, int apply_softmax) {
-    const int64_t scratch = msda_b200_backward_scratch_bytes(B, S, G, D, Q, L, K, dtype);
-    if (scratch == 0) return 0;
-    msda_b200::Params p{};
-    p.B = B, p.S = S, p.Q = Q;
-    p.G = (int)G, p.D = (int)D, p.L = (int)L, p.K = (int)K;
-    if (!msda_b200::sorting_pays(p, dtype))
-        return msda_b200::fused_backward_pays(p) ? (scratch + 15) / 16 * 16 + msda_b200::kFusedBytes : scratch;
-    // all samples at once, or as many as the target holds (at least one)
-    int64_t samples = B;
-    while (samples > 1 && msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples) > kWorkspaceTarget)
-        samples = samples > 8 ? samples - samples / 8 : samples - 1;
-    const int64_t sorted = msda_b200::sorted_workspace_bytes(p, apply_softmax != 0, samples);
-    return sorted > scratch ? sorted : scratch;
+    return workspace_bytes(B, S, G, D, Q, L, K, dtype, apply_softmax, false);
+}
+
+int64_t msda_b200_backward_offsets_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D,
+                                                   int64_t Q, int64_t L, int64_t K, int dtype,
+                                                   int apply_softmax) {
+    return workspace_bytes(B, S, G, D, Q, L, K, dtype, apply_softmax, true);
 }
 
 int msda_b200_launch_geometry(int64_t B, int64_t G, int64_t D, int64_t Q, int64_t L, int64_t K,
@@ -414,7 +426,7 @@ int backward_impl(const void *value, const int64_t *spatial_shapes,
     DeviceGuard guard(device);
     if (guard.err != cudaSuccess) return cuda_fail(guard.err, "backward: selecting the device");
     cudaError_t e;
-    if (use_scratch && msda_b200::sorting_pays(p, dtype)) {
+    if (use_scratch && msda_b200::sorting_pays(p, dtype, p.ref != nullptr)) {
         const bool softmax = apply_softmax != 0;
         const int64_t samples = msda_b200::sorted_samples_per_turn(p, softmax, scratch_bytes);
         if (samples > 0) {

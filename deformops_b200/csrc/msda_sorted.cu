@@ -1243,7 +1243,7 @@ int64_t round_up(int64_t n, int64_t to) { return (n + to - 1) / to * to; }
 //                               points on four levels: 490 -> 618, 600 -> 665, 509 -> 455; 40 on five,
 //                               where the few cells of the last one are counted by all: 1117 -> 1693,
 //                               1558 -> 1760, 1177 -> 1427
-bool sorting_pays(const Params &p, int dtype) {
+bool sorting_pays(const Params &p, int dtype, bool offsets) {
     const int64_t P = (int64_t)p.L * p.K, points = p.B * p.G * p.Q * P;
     if (dtype != 1 && dtype != 2) return false;
     if (p.D != 16 && p.D != 32 && p.D != 64) return false;
@@ -1253,9 +1253,9 @@ bool sorting_pays(const Params &p, int dtype) {
         return false;
     if (p.Q * P < 8 * p.S) return false;
     if (p.S > 55000 &&
-        (p.ref != nullptr || p.L > 4 || p.D == 16 || (p.D == 32 && p.Q * P < 24 * p.S)))
+        (offsets || p.L > 4 || p.D == 16 || (p.D == 32 && p.Q * P < 24 * p.S)))
         return false;
-    if (p.ref != nullptr && p.D < 64) return p.D == 32 && points >= 3000000;
+    if (offsets && p.D < 64) return p.D == 32 && points >= 3000000;
     return points >= 1000000;
 }
 

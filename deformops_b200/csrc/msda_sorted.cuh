@@ -31,7 +31,8 @@ struct SortPlan {
 };
 
 // Whether a call is dense enough for the sort to pay (and within the record's field widths).
-bool sorting_pays(const Params &p, int dtype);
+// `offsets`: the call takes reference points and offsets.
+bool sorting_pays(const Params &p, int dtype, bool offsets);
 // Fills the plan for `samples` samples over `workspace`; returns the bytes it takes.
 int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples, void *workspace);
 // The call restricted to samples b .. b + n - 1.

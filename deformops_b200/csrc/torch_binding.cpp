@@ -184,7 +184,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> offsets_backward(
     at::Tensor grad_attn = at::empty_like(attn);
     if (d.B == 0) return {grad_value, grad_offsets, grad_attn};
     const int code = dtype_code(value.scalar_type());
-    const int64_t nbytes = d.Q > 0 ? msda_b200_backward_workspace_bytes(d.B, d.S, d.G, d.D, d.Q, d.L, d.K, code, softmax) : 0;
+    const int64_t nbytes = d.Q > 0 ? msda_b200_backward_offsets_workspace_bytes(d.B, d.S, d.G, d.D, d.Q, d.L, d.K, code, softmax) : 0;
     at::Tensor scratch;
     if (nbytes > 0) scratch = at::empty({nbytes}, value.options().dtype(at::kByte));
     const int st = msda_b200_backward_offsets(

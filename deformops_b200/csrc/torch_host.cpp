@@ -53,6 +53,7 @@ struct Abi {
     decltype(&msda_b200_last_error) last_error = nullptr;
     decltype(&msda_b200_column_sums) column_sums = nullptr;
     decltype(&msda_b200_column_sums_scratch_bytes) column_sums_scratch_bytes = nullptr;
+    decltype(&msda_b200_backward_offsets_workspace_bytes) offsets_workspace_bytes = nullptr;
 } abi;
 
 // One call: the operands as the kernels take them.  `ref` is undefined when `points` holds
@@ -139,7 +140,8 @@ variable_list run_backward(const Call &c, const Tensor &grad_in) {
     Tensor grad_value = empty(c.value.sizes(), c.value.scalar_type(), device);
     Tensor grad_points = empty(c.points.sizes(), c.points.scalar_type(), device);
     Tensor grad_attn = empty(c.attn.sizes(), c.attn.scalar_type(), device);
-    const int64_t nbytes = abi.workspace_bytes(c.B, c.S, c.G, c.D, c.Q, c.L, c.K, dtype, c.softmax);
+    const int64_t nbytes = (c.ref.defined() ? abi.offsets_workspace_bytes : abi.workspace_bytes)(
+        c.B, c.S, c.G, c.D, c.Q, c.L, c.K, dtype, c.softmax);
     Tensor scratch;
     if (nbytes > 0) scratch = empty({nbytes}, at::kByte, device);
     void *scratch_ptr = nbytes > 0 ? scratch.mutable_data_ptr() : nullptr;
@@ -434,9 +436,9 @@ PyObject *py_linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // bind(addresses of the ABI functions in the order of struct Abi)
 PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
-    TORCH_CHECK(nargs == 8, "bind takes eight addresses");
-    void *p[8];
-    for (int i = 0; i < 8; ++i) {
+    TORCH_CHECK(nargs == 9, "bind takes nine addresses");
+    void *p[9];
+    for (int i = 0; i < 9; ++i) {
         p[i] = PyLong_AsVoidPtr(args[i]);
         if (p[i] == nullptr) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
@@ -450,6 +452,7 @@ PyObject *py_bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     abi.last_error = reinterpret_cast<decltype(abi.last_error)>(p[5]);
     abi.column_sums = reinterpret_cast<decltype(abi.column_sums)>(p[6]);
     abi.column_sums_scratch_bytes = reinterpret_cast<decltype(abi.column_sums_scratch_bytes)>(p[7]);
+    abi.offsets_workspace_bytes = reinterpret_cast<decltype(abi.offsets_workspace_bytes)>(p[8]);
     abi.forward = reinterpret_cast<decltype(abi.forward)>(p[0]);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS

@@ -332,8 +332,8 @@ def _offsets_backward_cuda(value, spatial_shapes, level_start_index, reference_p
     value, reference_points, offsets, attn, grad_output = map(
         _aligned, (value, reference_points, offsets, attn, grad_output))
     stream = torch.cuda.current_stream(value.device).cuda_stream
-    nbytes = (shim.workspace_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype], int(softmax))
-              if Q > 0 else 0)
+    nbytes = (shim.offsets_workspace_bytes(B, S, G, D, Q, L, K, DTYPE_CODES[value.dtype],
+                                           int(softmax)) if Q > 0 else 0)
     scratch = (torch.empty(nbytes, dtype=torch.uint8, device=value.device)
                if nbytes else None)
     st = shim.backward_offsets(

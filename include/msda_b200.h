@@ -141,6 +141,10 @@ int64_t msda_b200_backward_scratch_bytes(int64_t B, int64_t S, int64_t G, int64_
  */
 int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q,
                                            int64_t L, int64_t K, int dtype, int apply_softmax);
+/* The same for msda_b200_backward_offsets, which sorts fewer calls. */
+int64_t msda_b200_backward_offsets_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D,
+                                                   int64_t Q, int64_t L, int64_t K, int dtype,
+                                                   int apply_softmax);
 
 /*
  * out[c] = sum over r of x[r][c], for a contiguous (rows, cols) matrix: the bias gradient of a

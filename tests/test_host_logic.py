@@ -280,6 +280,18 @@ def test_large_pyramids_are_sorted_only_where_that_is_faster(S, L, K, G, D, sort
 
 
 
+@pytest.mark.parametrize("B, D, K, sorts", [
+    (4, 32, 4, True), (1, 32, 4, False), (16, 16, 4, False), (1, 64, 4, True),   # 8.3, 2.1, 33, 2.1 M points
+])
+def test_offsets_reserve_room_to_sort_only_where_they_sort(B, D, K, sorts):
+    from deformops_b200._loader import load_library
+
+    shim = load_library()
+    shape = (B, 21504, 8, D, 21504, 3, K, 2)
+    assert (shim.offsets_workspace_bytes(*shape, 1) > shim.scratch_bytes(*shape)) == sorts
+    assert shim.workspace_bytes(*shape, 1) > shim.scratch_bytes(*shape)
+
+
 def test_error_message_is_thread_local():
     import threading
 
