@@ -1170,12 +1170,12 @@ __global__ void __launch_bounds__(256, 4) sorted_finish_kernel(const __grid_cons
 template <typename T, int D, bool REF>
 cudaError_t launch_walk(const Params &p, const SortPlan &sp, bool softmax, cudaStream_t stream) {
     constexpr size_t smem = (size_t)kWalkWarps * walk_warp_bytes(D);
+    static_assert(smem <= kPlainSmem, "would have to be asked for on every device");
     auto walk = sorted_walk_kernel<T, D, REF>;
-    // as many CTAs as the GPU holds at once; the warps fetch their runs (asked once: every GPU
-    // this is built for has the same limits)
+    // as many CTAs as the GPU holds at once; the warps fetch their runs, so that any number
+    // serves (asked once: every GPU this is built for has the same limits)
     static const int resident = [walk] {
         int device = 0, sms = 0, per_sm = 0;
-        cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (cudaGetDevice(&device) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk, kWalkWarps * 32, smem) != cudaSuccess)
