@@ -440,6 +440,9 @@ def floors_leg(w, device, stream):
         return statistics.median(timed_steps(lambda i: fn(), 1, stream, torch.cuda.synchronize, reps))
 
     red_ms = median_ms(lambda: lib.floors_red_rows(vp(dst.data_ptr()), vp(rows.data_ptr()), n, 1, sp))
+    dst32 = torch.zeros(B * S * G * D, dtype=torch.float32, device=device)
+    red32_ms = median_ms(lambda: lib.floors_red_rows(vp(dst32.data_ptr()), vp(rows.data_ptr()), n, 2, sp))
+    del dst32
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     red_by_sms = {str(k): n / (median_ms(lambda k=k: lib.floors_red_rows_on(
         vp(dst.data_ptr()), vp(rows.data_ptr()), n, k, sp)) * 1e-3) for k in (sms, sms // 2, sms // 4)}
@@ -477,6 +480,7 @@ def floors_leg(w, device, stream):
         "corner_rows": n,
         "gather_rows_ms": gat_ms, "gather_rows_per_s": n / (gat_ms * 1e-3),
         "red_f16x2_rows_ms": red_ms, "red_f16x2_rows_per_s": n / (red_ms * 1e-3),
+        "red_f32_128_byte_rows_ms": red32_ms,
         "gather_red_rows_ms": both_ms, "gather_red_idle_smem_bytes_per_cta": bwd_smem,
         "red_f16x2_rows_per_s_by_issuing_sms": red_by_sms,
         "bulk_reduce_f16_rows_per_s_by_piece_bytes": bulk_by_piece,

@@ -6,7 +6,8 @@
 // per bilinear corner), so the access pattern is the operator's, minus every other instruction:
 //
 //   floors_red_rows     one packed 16-byte reduction per lane into `dst`; four lanes cover a row
-//                       (what the backward's grad_value scatter costs on its way to L2)
+//                       (what the backward's grad_value scatter costs on its way to L2); float32
+//                       rows are 128 bytes, eight lanes
 //   floors_red_rows_on  the same from a given number of SMs only (one CTA of 32 warps each):
 //                       shows whether the limit sits in the SMs or behind them
 //   floors_bulk_red_rows  the same additions sent by the copy engine instead of the load/store
@@ -33,16 +34,19 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// mode: 0 bf16x2, 1 f16x2
+// mode: 0 bf16x2, 1 f16x2, 2 f32
 template <int MODE, int THREADS>
 __global__ void __launch_bounds__(THREADS) red_rows_kernel(uint16_t *dst, const uint32_t *row_off,
                                                          int64_t rows) {
-    const int sub = threadIdx.x & 3;
-    const int64_t stride = (int64_t)gridDim.x * (THREADS / 4);
+    constexpr int LANES = MODE == 2 ? 8 : 4;
+    const int sub = threadIdx.x % LANES;
+    const int64_t stride = (int64_t)gridDim.x * (THREADS / LANES);
     const uint32_t one = MODE == 0 ? 0x3c003c00u : 0x14001400u;   // small finite addends
-    for (int64_t r = (int64_t)blockIdx.x * (THREADS / 4) + (threadIdx.x >> 2); r < rows; r += stride) {
-        uint16_t *a = dst + row_off[r] + sub * 8;
-        if (MODE == 0)
+    for (int64_t r = (int64_t)blockIdx.x * (THREADS / LANES) + threadIdx.x / LANES; r < rows; r += stride) {
+        uint16_t *a = dst + (MODE == 2 ? 2 * (size_t)row_off[r] : row_off[r]) + sub * 8;
+        if (MODE == 2)
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %1, %1, %1};" ::"l"(a), "f"(1e-3f));
+        else if (MODE == 0)
             asm volatile("red.relaxed.gpu.global.add.noftz.v4.bf16x2 [%0], {%1, %1, %1, %1};" ::"l"(a),
                          "r"(one));
         else
@@ -204,10 +208,13 @@ int grid_for(int ctas_per_sm) {
 
 extern "C" {
 
-// rows: number of 64-byte rows; row_off[i]: offset of row i in 16-bit elements from dst/src
-int floors_red_rows(void *dst, const uint32_t *row_off, int64_t rows, int f16, void *stream) {
+// rows: number of 64-byte rows; row_off[i]: offset of row i in elements from dst/src; type: 0
+// bf16, 1 f16, 2 f32 (whose dst is twice as large)
+int floors_red_rows(void *dst, const uint32_t *row_off, int64_t rows, int type, void *stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (f16)
+    if (type == 2)
+        red_rows_kernel<2, kThreads><<<grid_for(8), kThreads, 0, s>>>(static_cast<uint16_t *>(dst), row_off, rows);
+    else if (type == 1)
         red_rows_kernel<1, kThreads><<<grid_for(8), kThreads, 0, s>>>(static_cast<uint16_t *>(dst), row_off, rows);
     else
         red_rows_kernel<0, kThreads><<<grid_for(8), kThreads, 0, s>>>(static_cast<uint16_t *>(dst), row_off, rows);
