@@ -624,8 +624,11 @@ def main():
     for i in range(max(args.warmup, 3)):
         abi.step(sets[i % NUM_SETS])
     with ClockSampler(local_rank) as clocks:
+        before = shim.launches()
         repeats_ms = timed_steps(lambda i: abi.step(sets[i % NUM_SETS]), args.steps, stream, barrier,
                                  max(1, args.repeats))
+        # of one repeat, as the library counts them
+        kernels, memsets = ((n - m) // max(1, args.repeats) for n, m in zip(shim.launches(), before))
         # ---- roofline: per-kernel durations, events around each call, same rotation ------------
         evs = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(args.steps)]
         barrier()
@@ -819,9 +822,10 @@ def main():
             "repeats": {"count": len(repeats_ms), "ms_per_step_median": ms_per_step,
                         "ms_per_step_min": rep_min / args.steps, "ms_per_step_max": rep_max / args.steps},
             "clocks": clock_summary,
-            "gpu_launches": 5 * args.steps,
+            "gpu_launches": kernels,
             "kernels_ms": {"forward": fwd_ms, "backward_call": bwd_ms, **spread,
-                           "backward_call_launches": "memset + sort_count, sort_scatter, sorted_walk and sorted_finish kernels"},
+                           "backward_call_launches": f"{memsets // args.steps} memset and "
+                                                     f"{kernels // args.steps - 1} kernels"},
             "roofline": {"bound": "hbm", "kernel": "msda backward (whole call, grad_value clear included)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": peak_kind, "traffic": traffic,
