@@ -573,14 +573,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
     const int64_t base = pair0 * P + c.pt;
     const int nq = c.active ? c.nq : 0;
-    if (unsorted_call<T>(sp.header)) {
-        uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
-        const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
-        for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs;
-             i += (int64_t)gridDim.x * kSortThreads)
-            extras[i] = make_uint4(0u, 0u, 0u, 0u);
-        return;
-    }
+    // (asked here, needed only when records leave: the points' loads do not wait for the answer)
+    const bool unsorted = unsorted_call<T>(sp.header);
     __syncthreads();
     unsigned at[kSortPoints];     // cell << 16 | rank among the CTA's points of the cell; ~0: skipped
 #pragma unroll
@@ -592,6 +586,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
             const int q = c.ql + (r0 + r) * c.step;
             if (q < nq) {
                 xy[r] = point_xy<T, REF>(p, c, base, q);
+            }
+        }
+        // (behind all the locations, not beside each: with reference points and softmax 40.5 us
+        // against 45.5 of the ragged pyramid, 74 against 85 of the 512-pixel one)
+#pragma unroll
+        for (int r = 0; r < kSortBatch; ++r) {
+            const int q = c.ql + (r0 + r) * c.step;
+            if (q < nq) {
                 if constexpr (SOFTMAX) stats[r] = sp.stats[pair0 + (int64_t)(q * p.G)];
                 weight[r] = attn[base + (int64_t)(q * (p.G * P))];
             }
@@ -616,10 +618,18 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
                     at[r0 + r] = ((unsigned)pc.cell << 16) | atomicAdd(shift + pc.cell, 1u);
                 } else {
                     const unsigned place = atomicAdd(cursor + pc.cell, 1u);
-                    if (place < (unsigned)sp.plane_points) records[place] = record;
+                    if (place < (unsigned)sp.plane_points && !unsorted) records[place] = record;
                 }
             }
         }
+    }
+    if (unsorted) {
+        uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
+        const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
+        for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs;
+             i += (int64_t)gridDim.x * kSortThreads)
+            extras[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
     }
     if (in_shared) {
         __syncthreads();
