@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(256, MSDA_FIN_MIN_CTAS) finalize_kernel(const 
 // not when other CTAs arrive: a piece that was handed out is in the hands of a CTA that
 // runs and does not wait before it is done.  So however few CTAs the GPU has room for beside other
 // streams' kernels, they finish the call, and those that come late find nothing left.  (A
-// cooperative launch with grid barriers was as quick, 72.6 us of a decoder layer's forward + backward
-// against 72.9, but waited for room for all its CTAs: beside a one-thread kernel of 1 ms on another
+// cooperative launch with grid barriers needs no memset, 72.5 us of a decoder layer's forward + backward
+// against 73.7, but waited for room for all its CTAs: beside a one-thread kernel of 1 ms on another
 // stream a backward of 64 us took 1050; this one takes 69.)
 
 // The next piece of what `cell` counts, for the whole CTA; `slot` is shared.

@@ -687,7 +687,7 @@ cudaError_t launch_forward(const Params &p, int dtype, bool softmax, cudaStream_
 cudaError_t launch_backward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 // The scaled backward in one launch, for calls that are bound by the host: what its scratch needs
 // beyond the usual is a header of its own.  (Forward + backward of a decoder layer, host bound, B200:
-// 79.7 us with the three launches, 72.9 so.  On the GPU 51.2 us against 53.2 with 154 000 points, 77.9
+// 79.7 us with the three launches, 73.7 so.  On the GPU 51.2 us against 53.2 with 154 000 points, 77.9
 // against 75.8 with 262 000.)
 enum FusedCell : unsigned {                // a line of memory each
     kFusedGradOut = 0, kFusedAttn = 32,    // largest magnitudes

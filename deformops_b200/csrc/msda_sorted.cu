@@ -21,8 +21,8 @@
 // eight channels, instead of once per corner and point (at 21 504 queries and 12 points per query
 // 33 million rows of reductions become about 1 million).
 //
-// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 435 us
-// against 512 us, of which counting 51, writing records 105, the walk 247, the last pass 22;
+// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 429 us
+// against 512 us, of which counting 51, writing records 104, the walk 247, the last pass 22;
 // grad_value 1.7e-3 off the float32 result against 2.2e-3.
 //
 // Accumulation is float32 inside a warp's run of points; the few sums that meet in memory (two

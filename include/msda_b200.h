@@ -137,7 +137,8 @@ int64_t msda_b200_backward_scratch_bytes(int64_t B, int64_t S, int64_t G, int64_
  * msda_b200_backward_scratch_bytes(...).  A call that samples densely (several points per value
  * position) sorts its points by where they fall before it accumulates, 16 bytes a point plus the
  * tables, as many samples at a time as the scratch it is given holds: this is what all samples
- * take, or about 256 MiB if that is less.  With the smaller size it makes more passes.
+ * take, or about 256 MiB if that is less.  With less it takes more turns over the samples, or, where
+ * those would be too short, adds without sorting.
  */
 int64_t msda_b200_backward_workspace_bytes(int64_t B, int64_t S, int64_t G, int64_t D, int64_t Q,
                                            int64_t L, int64_t K, int dtype, int apply_softmax);
