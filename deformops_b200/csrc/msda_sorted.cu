@@ -418,6 +418,14 @@ __device__ __forceinline__ __half *unsorted_extras(const SortPlan &sp) {
     return reinterpret_cast<__half *>(sp.records);
 }
 
+// Clears them, the share of one CTA of a sort kernel.
+__device__ inline void clear_unsorted_extras(const Params &p, const SortPlan &sp) {
+    uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
+    const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
+    for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs; i += (int64_t)gridDim.x * kSortThreads)
+        extras[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // The points of a call without the sort.  A warp takes 32 adjacent points, each lane locates one;
 // then the D / 8 lanes of a slot gather and add a point's corners at a time, as in the direct
 // backward, the point's numbers coming and its gradients going by shuffles.  Such a call takes
@@ -573,6 +581,10 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
     const int64_t base = pair0 * P + c.pt;
     const int nq = c.active ? c.nq : 0;
+    if (!ct.fits) {      // (its points have no cells to be counted in)
+        clear_unsorted_extras(p, sp);
+        return;
+    }
     // (asked here, needed only when records leave: the points' loads do not wait for the answer)
     const bool unsorted = unsorted_call<T>(sp.header);
     __syncthreads();
@@ -624,11 +636,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
         }
     }
     if (unsorted) {
-        uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
-        const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
-        for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs;
-             i += (int64_t)gridDim.x * kSortThreads)
-            extras[i] = make_uint4(0u, 0u, 0u, 0u);
+        clear_unsorted_extras(p, sp);
         return;
     }
     if (in_shared) {
