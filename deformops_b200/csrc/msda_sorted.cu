@@ -38,6 +38,7 @@ constexpr int kSortThreads = 512;
 constexpr int kSortPoints = 8;         // points per thread of the sort kernels,
 constexpr int kSortBatch = 4;          // loaded this many at a time
 constexpr int kSharedCells = 8192;     // most cells of a plane that are counted in shared memory
+static_assert(kSharedCells % 8 == 0, "scan_cells");
 constexpr int kSortCtaPoints = kSortThreads * kSortPoints;
 constexpr int kWalkWarps = 4;          // warps per CTA of the walk, each on its own run
 
@@ -1323,8 +1324,9 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // ceil((W + 1) / 7) <= W leave at most two cells per pixel
     sp.prepare_ctas = (int)std::min<int64_t>(148 * 2, 1 + samples * (p.S + p.Q) * p.G * p.D / (8 * kSortThreads * 4));
     sp.cell_bound = (int)(2 * p.S + 2 * p.L);
-    // a pyramid of ordinary proportions has a cell per five to six pixels
-    sp.shared_cells = (int)std::min<int64_t>(kSharedCells, std::min<int64_t>(sp.cell_bound, round_up(p.S / 5 + 256, 8)));
+    // a pyramid of ordinary proportions has a cell per five to six pixels (whole eights: the scatter
+    // takes cells by eights, in 16-byte accesses to arrays that follow one another)
+    sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
     // Runs of a few hundred points (128 / 256 / 512: 290 / 254 / 276 us of walk at the headline
     // shape: shorter ones flush too often, longer ones end too unevenly), shorter where that would

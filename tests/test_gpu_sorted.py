@@ -69,6 +69,9 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     (torch.float16, False, 64, 8, [(16, 14)], 1, 32769, 4),
     (torch.bfloat16, False, 16, 1, [(20, 20), (10, 10), (5, 5), (3, 3), (2, 2)], 3, 8333, 9),
     (torch.float16, True, 16, 64, [(12, 33), (6, 17)], 1, 2051, 4),
+    # few positions: room for cells that is no multiple of eight
+    (torch.bfloat16, False, 32, 4, [(8, 8)], 1, 32771, 8),
+    (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
     # more cells than a CTA counts in shared memory: narrow levels
     (torch.bfloat16, False, 32, 4, [(3000, 2)], 1, 13000, 20),
 ])
