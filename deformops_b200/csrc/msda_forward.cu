@@ -164,6 +164,169 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
     }
 }
 
+// ---- dense calls of 16-bit values: 32 bytes per lane --------------------------------------------
+// The same sum with 32-byte loads: a slot is LPH = D / 16 lanes, a warp covers twice the pairs per
+// instruction, and a point's numbers go from the lane that placed it to its slot by shuffles, so that
+// all of the SM's memory that is not the level table stays L1.  What bounds it is what bounds
+// forward_kernel, one wavefront of the L1 data pipe per 64-byte corner row (79 % busy at the headline
+// shape, 4 x 21 504 queries of 12 points, 8 x 32 channels); of the rest a third of the wavefronts and a
+// seventh of the instructions are gone, and L1 hits 40 % of the sectors instead of 29 %.
+// Forward, B200, us, forward_kernel -> this: headline shape 164 -> 158, its 512-pixel pyramid 8 samples
+// 86 -> 82.5, four odd levels in float16 186 -> 174.5, softmax and offsets 109 -> 96; 6 x 64 channels,
+// 9 points, softmax and offsets 98 -> 80; 8 x 16 channels 129 -> 110; 2 x 128 149 -> 138.
+// Three CTAs of 80 registers: four of 64 spill (175), seven of four warps at 72 164; two points in
+// flight instead of one 160; one CTA per eight or sixteen groups instead of persistent ones 165, 168;
+// the next points' locations loaded a turn early 158.
+constexpr int kWideWarps = 8;
+
+template <typename T>
+__device__ __forceinline__ void gather32(float2 (&acc)[8], const char *at, float w) {
+    uint4 lo, hi;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
+        : "l"(at));
+    float2 f[4], g[4];
+    VecTraits<T>::unpack(lo, f);
+    VecTraits<T>::unpack(hi, g);
+    const float2 w2 = make_float2(w, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        ffma2(acc[i], f[i], w2);
+        ffma2(acc[4 + i], g[i], w2);
+    }
+}
+
+// The offsets or locations and the weights of PTS adjacent points (two: an even one first), in one
+// load each.
+template <typename T, bool REF, int PTS>
+__device__ __forceinline__ void load_points(const Params &p, int64_t e, float2 (&spot)[PTS], float (&weight)[PTS]) {
+    using VT = VecTraits<T>;
+    const T *attn = reinterpret_cast<const T *>(p.attn) + e;
+    if constexpr (PTS == 1) {
+        spot[0] = REF ? load_offset<T>(p, e) : ld_stream_f2(reinterpret_cast<const float2 *>(p.loc) + e);
+        weight[0] = VT::to_float(*attn);
+    } else {
+        if (REF && p.offsets16) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint32_t *>(p.loc) + e));
+            spot[0] = VT::unpack2(v.x), spot[1] = VT::unpack2(v.y);
+        } else {
+            const uint4 v = ld_stream16(reinterpret_cast<const float2 *>(p.loc) + e);
+            spot[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y));
+            spot[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w));
+        }
+        const float2 w = VT::unpack2(__ldg(reinterpret_cast<const uint32_t *>(attn)));
+        weight[0] = w.x, weight[1] = w.y;
+    }
+}
+
+template <typename T, bool SOFTMAX, bool REF, int LPH, int PTS>
+__global__ void __launch_bounds__(kWideWarps * 32, 3) forward_wide_kernel(const __grid_constant__ Params p) {
+    using VT = VecTraits<T>;
+    constexpr int kPairs = 32 / LPH;
+    __shared__ LevelTable lt;
+    load_level_table(lt, p);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = lane / LPH, sub = lane % LPH;
+    const int G = p.G, P = p.L * p.K;
+    const unsigned row_bytes = (unsigned)G * (LPH * 32u);
+    const float inv_K = 1.f / (float)p.K;
+    const int64_t total_pairs = p.B * p.Q * G;
+    const T *attn = reinterpret_cast<const T *>(p.attn);
+
+    for (int64_t group = (int64_t)blockIdx.x * kWideWarps + warp; group < p.num_groups;
+         group += (int64_t)gridDim.x * kWideWarps) {
+        const int64_t pair0 = group * kPairs;
+        const bool live = pair0 + slot < total_pairs;
+        const int64_t pair = live ? pair0 + slot : total_pairs - 1;
+        const unsigned bq = (unsigned)pair / (unsigned)G;
+        const int g = (int)((unsigned)pair - bq * (unsigned)G);
+        const int64_t b = bq / (unsigned)p.Q;
+        const char *vb = reinterpret_cast<const char *>(p.value) + (b * p.S * (int64_t)row_bytes + g * (LPH * 32) + sub * 32);
+        const int64_t e0 = pair * P;
+        float2 stats = make_float2(0.f, 0.f);
+        if constexpr (SOFTMAX) stats = slot_softmax_stats(attn + e0, P, LPH, sub, true);
+        float2 acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int r = 0; r < P; r += LPH * PTS) {
+            // ---- each lane of the slot takes PTS adjacent points
+            const int mine = r + sub * PTS;
+            float2 spot[PTS];
+            float weight[PTS];
+            if (mine < P) load_points<T, REF, PTS>(p, e0 + mine, spot, weight);
+#pragma unroll
+            for (int i = 0; i < PTS; ++i) {
+                const int pt = mine + i;
+                int place = 0, down = 0;
+                float w00 = 0.f, w01 = 0.f, w10 = 0.f, w11 = 0.f;
+                if (pt < P) {
+                    const int l = (int)(((float)pt + 0.5f) * inv_K);  // pt / K
+                    const int H = lt.H[l], W = lt.W[l];
+                    float2 xy = spot[i];
+                    if constexpr (REF) xy = location_from_offset(p, xy, (int64_t)bq, l, (float)W, (float)H);
+                    float a = weight[i];
+                    if constexpr (SOFTMAX) a = expf(a - stats.x) * stats.y;
+                    const PointGeom geo = locate(xy.x, xy.y, H, W, 0, 0);
+                    const int ra = max(geo.r0, 0), rb = max(min(geo.r0 + 1, H - 1), 0);
+                    const int ca = max(geo.c0, 0), cb = max(min(geo.c0 + 1, W - 1), 0);
+                    // (a sample has fewer than 2^31 / 16 positions: one word holds the step right too)
+                    place = (lt.start[l] + ra * W + ca) * 2 + (cb - ca);
+                    down = (rb - ra) * W;
+                    const float wr0 = 1.f - geo.fr, wc0 = 1.f - geo.fc;
+                    const unsigned f = geo.flags;
+                    w00 = f & kCorner00 ? a * (wr0 * wc0) : 0.f;
+                    w01 = f & kCorner01 ? a * (wr0 * geo.fc) : 0.f;
+                    w10 = f & kCorner10 ? a * (geo.fr * wc0) : 0.f;
+                    w11 = f & kCorner11 ? a * (geo.fr * geo.fc) : 0.f;
+                }
+#pragma unroll 1
+                for (int j = 0; j < LPH; ++j) {
+                    if (r + j * PTS + i >= P) break;
+                    const int from = LPH == 1 ? 0 : (lane & ~(LPH - 1)) + j;
+                    auto get = [&](auto v) { return LPH == 1 ? v : __shfl_sync(0xffffffffu, v, from); };
+                    const int pl = get(place), dy = get(down);
+                    const float a0 = get(w00), a1 = get(w01), a2 = get(w10), a3 = get(w11);
+                    const char *top = vb + (uint64_t)((unsigned)(pl >> 1) * row_bytes);
+                    const char *bot = top + (uint64_t)((unsigned)dy * row_bytes);
+                    const unsigned right = pl & 1 ? row_bytes : 0u;
+                    gather32<T>(acc, top, a0);
+                    gather32<T>(acc, top + right, a1);
+                    gather32<T>(acc, bot, a2);
+                    gather32<T>(acc, bot + right, a3);
+                }
+            }
+        }
+        if (live) {
+            char *o = reinterpret_cast<char *>(p.out) + pair * (LPH * 32) + sub * 32;
+            st_stream16(o, VT::pack(reinterpret_cast<const float2(&)[4]>(acc[0])));
+            st_stream16(o + 16, VT::pack(reinterpret_cast<const float2(&)[4]>(acc[4])));
+        }
+    }
+}
+
+template <typename T, bool SOFTMAX, bool REF, int LPH, int PTS>
+cudaError_t launch_wide_as(const Params &p, cudaStream_t stream) {
+    auto kernel = forward_wide_kernel<T, SOFTMAX, REF, LPH, PTS>;
+    static Residency residency;
+    Params q = p;
+    q.num_groups = (p.B * p.Q * p.G + 32 / LPH - 1) / (32 / LPH);
+    q.grid = (unsigned)((q.num_groups + kWideWarps - 1) / kWideWarps);
+    const unsigned resident = residency.ctas(kernel, kWideWarps * 32, 0);
+    if (resident > 0 && q.grid > resident) q.grid = resident;
+    kernel<<<q.grid, kWideWarps * 32, 0, stream>>>(q);
+    return cudaGetLastError();
+}
+template <typename T, bool SOFTMAX, bool REF, int LPH>
+cudaError_t launch_wide(const Params &p, cudaStream_t stream) {
+    // (two points a lane in slots of four lanes and more leave lanes idle in the last turn: 12 points
+    // of 64 channels 35 us against 33)
+    if constexpr (LPH < 4)
+        if (p.L * p.K % 2 == 0) return launch_wide_as<T, SOFTMAX, REF, LPH, 2>(p, stream);
+    return launch_wide_as<T, SOFTMAX, REF, LPH, 1>(p, stream);
+}
+
 template <typename T, bool SOFTMAX, bool REF, bool SMALL, typename Index>
 cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     const size_t smem = forward_smem_bytes(p, SOFTMAX);
@@ -188,6 +351,18 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+// 32-byte loads halve the warps of a call.  Where neighbouring queries sample neighbouring pixels, or
+// all pixels are sampled often, L1 makes up for it; few queries far apart wait for L2 instead (us,
+// forward_kernel -> forward_wide_kernel: 900 queries on 17 821 positions, 8 samples 32 -> 39; 1 800, 16
+// samples 84 -> 87; 7 000 on 21 504, 8 samples 111 -> 109, 10 752 166 -> 158).  Below six million output
+// elements the two lie within 3 % of one another (5.5 M: 46.2 -> 47.4), but for 16 channels (1.4 M:
+// 22.7 -> 18.6).  float32 gains nothing (262 -> 273): its rows are whole lines of L1 either way.
+bool wide_pays(const Params &p) {
+    const int64_t pairs = p.B * p.Q * p.G;
+    return (reinterpret_cast<uintptr_t>(p.value) & 31u) == 0 && 2 * p.Q >= p.S && pairs < (int64_t)1 << 31 &&
+           (p.D == 16 || pairs * p.D >= 6000000);
+}
+
 template <typename T, bool SOFTMAX, bool REF>
 cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
     // Up to four groups per SM the call lasts as long as one warp's chain of loads: more points in
@@ -195,6 +370,16 @@ cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
     // decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in flight 6.1, 6 6.6;
     // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
     constexpr int kSms = 148;
+    if constexpr (sizeof(T) == 2) {
+        if (p.num_groups > 4 * kSms && wide_pays(p)) {
+            switch (p.D) {
+                case 16: return launch_wide<T, SOFTMAX, REF, 1>(p, stream);
+                case 32: return launch_wide<T, SOFTMAX, REF, 2>(p, stream);
+                case 64: return launch_wide<T, SOFTMAX, REF, 4>(p, stream);
+                case 128: return launch_wide<T, SOFTMAX, REF, 8>(p, stream);
+            }
+        }
+    }
     if (p.num_groups > 4 * kSms)
         return p.B * p.Q * p.G < (int64_t)1 << 31 ? launch_as<T, SOFTMAX, REF, false, unsigned>(p, stream)
                                                   : launch_as<T, SOFTMAX, REF, false, int64_t>(p, stream);
