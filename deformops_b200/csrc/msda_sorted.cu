@@ -276,7 +276,7 @@ __device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &s
 
 // Exclusive prefix sum of a plane's cell counts by one CTA, in chunks of its size: `counts`
 // becomes the cursor the scatter kernel hands places out from, `offsets` the cells' first places
-// (offsets[cells]: the plane's points), `item_cell` the cell in which each run of
+// (offsets[cells]: the plane's points), `item_cell` the cell in which each unit of
 // sp.item_points places begins.
 __device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item_cell, int cells,
                                   int item_points) {
@@ -855,24 +855,27 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
 
     // ---- runs of places, handed out as the warps come for them
     for (;;) {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(sp.header + kNextItem, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= (unsigned)(p.B * p.G) * (unsigned)sp.items) break;
-        const int plane = (int)(item / (unsigned)sp.items);
-        const int run = (int)(item - (unsigned)plane * (unsigned)sp.items);
-        const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
-        const int total = (int)offsets[cells];
-        int cell = sp.item_cell[(int64_t)plane * sp.items + run];
-        int pos = run * sp.item_points;
-        const int stop = min(pos + sp.item_points, total);
+        unsigned run = 0;
+        if (lane == 0) run = atomicAdd(sp.header + kNextItem, 1u);
+        run = __shfl_sync(0xffffffffu, run, 0);
+        if (run >= sp.all_runs) break;
+        const int size = run < sp.runs[0] ? 3 : run < sp.runs[1] ? 2 : run < sp.runs[2] ? 1 : 0;   // 2^size units
+        const unsigned first = (run << size) + (size == 3 ? 0u : sp.unit0[2 - size]);
+        const int plane = (int)(first / (unsigned)sp.items);
+        int pos = (int)(first - (unsigned)plane * (unsigned)sp.items) * sp.item_points;
+        const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
+        // (places beyond the plane's points hold no record: what is read there is not kept)
+        uint4 rec = __ldcg(records + min((int64_t)(pos + lane), sp.plane_points - 1));
+        int cell = sp.item_cell[first];
+        const int total = (int)sp.offsets[(int64_t)plane * sp.cell_stride + cells];
+        const int stop = min(pos + (sp.item_points << size), total);
         if (pos >= stop) continue;
-
+        if (pos + lane >= total) rec = make_uint4(0u, 0u, 0u, 0u);
+        const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
         const int b = plane / p.G, g = plane - b * p.G;
         const T *value = reinterpret_cast<const T *>(p.value) + ((int64_t)b * p.S * p.G + g) * D;
         const T *grad_out = reinterpret_cast<const T *>(p.grad_out) + ((int64_t)b * p.Q * p.G + g) * D;
         __half *image = reinterpret_cast<__half *>(p.grad_value) + ((int64_t)b * p.S * p.G + g) * D;
-        const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
         // element of the per-point outputs that point 0 of query 0 of this plane has
         const int64_t plane_point = ((int64_t)b * p.Q * p.G + g) * (p.L * p.K);
 
@@ -936,7 +939,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
         int cell_end;
         cell_at(pos, cell_end);
         int n = min(min(kStep, cell_end - pos), stop - pos);
-        uint4 rec = fetch_record(pos), rec_next = fetch_record(pos + n);
+        uint4 rec_next = fetch_record(pos + n);
         uint32_t buffer = s_rows;
         fetch_rows(rec, n, buffer);
 
@@ -1202,7 +1205,7 @@ cudaError_t launch_walk(const Params &p, const SortPlan &sp, bool softmax, cudaS
         return sms * per_sm;
     }();
     if (resident <= 0) return cudaErrorInvalidConfiguration;
-    const int64_t ctas = (p.B * p.G * (int64_t)sp.items + kWalkWarps - 1) / kWalkWarps;
+    const int64_t ctas = ((int64_t)sp.all_runs + kWalkWarps - 1) / kWalkWarps;
     return launch_after_predecessor(walk, (unsigned)std::min<int64_t>(ctas, resident), kWalkWarps * 32, smem, stream,
                                     p, sp, softmax);
 }
@@ -1328,15 +1331,27 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // takes cells by eights, in 16-byte accesses to arrays that follow one another)
     sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
-    // Runs of a few hundred points (128 / 256 / 512: 290 / 254 / 276 us of walk at the headline
-    // shape: shorter ones flush too often, longer ones end too unevenly), shorter where that would
-    // leave the GPU's warps without one, longer where a pixel collects thousands of points: every
-    // run adds to it once, in float16
-    const int64_t even = planes * sp.plane_points / (148 * 16 * 4);
+    // Runs of the walk: a long one is flushed and started less often, but the last ones to end leave
+    // the others' SMs idle.  So they begin at eight units of 64 points and get shorter towards the
+    // end: eight and four while two of them are left for every warp, two while one is, then one
+    // (backward, us, all runs of 256 points -> this: headline shape 425 -> 415, 512-pixel pyramid 224
+    // -> 213, four odd levels in float16 440 -> 424, ragged pyramid of 64 channels 205 -> 195; with one
+    // of every length left 426, 217, 434, 212; three 423, 222, 423, 192).  Units are longer where a pixel
+    // collects thousands of points: every run adds to it once, in float16
     const int64_t density = sp.plane_points / std::max<int64_t>(p.S, 1);
-    sp.item_points = (int)(std::min<int64_t>(256, std::max<int64_t>(128, even / 32 * 32)) *
-                           std::min<int64_t>(16, 1 + density / 128));
-    sp.items = (int)((sp.plane_points + sp.item_points - 1) / sp.item_points);
+    sp.item_points = (int)(64 * std::min<int64_t>(16, 1 + density / 128));
+    sp.items = (int)round_up((sp.plane_points + sp.item_points - 1) / sp.item_points, 8);   // (no run in two planes)
+    const int64_t warps = 148 * kWalkWarps * walk_ctas(p.D);
+    int64_t units = planes * sp.items, runs = 0;
+    for (int i = 0; i < 3; ++i) {
+        const int64_t spare = (i < 2 ? 2 : 1) * warps, size = 8 >> i;
+        const int64_t n = std::max<int64_t>(0, units / size - spare);
+        runs += n;
+        units -= n * size;
+        sp.runs[i] = (unsigned)runs;
+        sp.unit0[i] = (unsigned)(planes * sp.items - units - (runs * (size / 2)));
+    }
+    sp.all_runs = (unsigned)(runs + units);
     char *at = static_cast<char *>(workspace);
     int64_t used = 0;
     auto take = [&](int64_t bytes) {

@@ -16,7 +16,7 @@ struct SortPlan {
     unsigned *tickets;       // per plane: CTAs of the counting kernel that have finished
     unsigned *counts;        // per plane and cell: points, later the next free place
     unsigned *offsets;       // per plane and cell: first place
-    int *item_cell;          // per plane and run of item_points places: the cell it begins in
+    int *item_cell;          // per plane and unit of item_points places: the cell it begins in
     uint4 *records;          // per plane: the points in order of their cells
     float *grad_prob;        // gradient of every weight (softmax: of the probability), float32
     float2 *stats;           // softmax only: (max, 1 / sum) of every pair's logits
@@ -27,7 +27,10 @@ struct SortPlan {
     int shared_cells;        // cells a sort CTA has room for in shared memory
     int chunk_queries, chunks;
     int prepare_ctas;        // CTAs of the counting kernel that prepare instead
-    int item_points, items;
+    int item_points, items;  // places of a unit, units of a plane
+    // the walk's runs: below runs[0] of eight units, below runs[1] of four, below runs[2] of two, then of
+    // one.  The first unit of run r is r * its length + unit0[i] (nothing before runs[0])
+    unsigned runs[3], unit0[3], all_runs;
 };
 
 // Whether a call is dense enough for the sort to pay (and within the record's field widths).

@@ -72,6 +72,8 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     # few positions: room for cells that is no multiple of eight
     (torch.bfloat16, False, 32, 4, [(8, 8)], 1, 32771, 8),
     (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
+    # enough points for runs of all four lengths (the ones above have short runs only)
+    (torch.bfloat16, False, 16, 4, [(60, 60), (30, 30)], 2, 27011, 8),
     # more cells than a CTA counts in shared memory: narrow levels
     (torch.bfloat16, False, 32, 4, [(3000, 2)], 1, 13000, 20),
 ])
