@@ -85,26 +85,27 @@ struct SortLane {
     int64_t q0;             // first query of the chunk
     bool active;
 };
-__device__ __forceinline__ SortLane sort_lane(const Params &p, const SortPlan &sp, const LevelTable &lt,
-                                              const CellTable &ct, unsigned cta) {
+// `points` of every query from `point0` on are the CTA's.
+template <int THREADS>
+__device__ __forceinline__ SortLane sort_lane(const Params &p, const LevelTable &lt, const CellTable &ct, unsigned cta,
+                                              int chunks, int chunk_queries, int points, int point0) {
     SortLane s;
-    const unsigned per_sample = (unsigned)sp.chunks * (unsigned)p.G;
+    const unsigned per_sample = (unsigned)chunks * (unsigned)p.G;
     s.b = (int)(cta / per_sample);
     const int chunk = (int)((cta - (unsigned)s.b * per_sample) / (unsigned)p.G);
     s.g = (int)(cta - (unsigned)s.b * per_sample) - chunk * p.G;
     s.plane = s.b * p.G + s.g;
-    const int P = p.L * p.K;
-    s.step = kSortThreads / P;
-    s.ql = (int)threadIdx.x / P;
-    s.pt = (int)threadIdx.x - s.ql * P;
+    s.step = THREADS / points;
+    s.ql = (int)threadIdx.x / points;
+    s.pt = point0 + (int)threadIdx.x - s.ql * points;
     s.l = s.pt / p.K;
     s.active = s.ql < s.step;
     s.H = lt.H[s.l];
     s.W = lt.W[s.l];
     s.cell0 = ct.first[s.l];
     s.rows = ct.rows[s.l];
-    s.q0 = (int64_t)chunk * sp.chunk_queries;
-    s.nq = (int)min((int64_t)sp.chunk_queries, p.Q - s.q0);
+    s.q0 = (int64_t)chunk * chunk_queries;
+    s.nq = (int)min((int64_t)chunk_queries, p.Q - s.q0);
     return s;
 }
 
@@ -143,7 +144,7 @@ __device__ __forceinline__ float2 point_xy(const Params &p, const SortLane &s, i
 
 // Adds the counts the CTA made in shared memory to the plane's.
 __device__ __forceinline__ void merge_counts(const unsigned *hist, unsigned *plane, int cells) {
-    for (int c = threadIdx.x; c < cells; c += kSortThreads)
+    for (int c = threadIdx.x; c < cells; c += blockDim.x)
         if (hist[c] != 0) atomicAdd(plane + c, hist[c]);
 }
 
@@ -278,12 +279,13 @@ __device__ __forceinline__ void prepare_share(const Params &p, const SortPlan &s
 // becomes the cursor the scatter kernel hands places out from, `offsets` the cells' first places
 // (offsets[cells]: the plane's points), `item_cell` the cell in which each unit of
 // sp.item_points places begins.
-__device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item_cell, int cells,
+template <int THREADS>
+__device__ __forceinline__ void scan_plane(unsigned *counts, unsigned *offsets, int *item_cell, int cells,
                                   int item_points) {
-    __shared__ unsigned warp_sums[kSortThreads / 32];
+    __shared__ unsigned warp_sums[THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned base = 0;
-    for (int c0 = 0; c0 < cells; c0 += kSortThreads * 4) {
+    for (int c0 = 0; c0 < cells; c0 += THREADS * 4) {
         const int at = c0 + threadIdx.x * 4;
         unsigned n[4], sum = 0;
 #pragma unroll
@@ -301,7 +303,7 @@ __device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item
         __syncthreads();
         unsigned before = 0, total = 0;
 #pragma unroll
-        for (int w = 0; w < kSortThreads / 32; ++w) {
+        for (int w = 0; w < THREADS / 32; ++w) {
             const unsigned s = warp_sums[w];
             before += w < warp ? s : 0u;
             total += s;
@@ -325,12 +327,20 @@ __device__ inline void scan_plane(unsigned *counts, unsigned *offsets, int *item
 }
 
 // ---- pass 1: count the points of every cell -------------------------------------------------------
-// Bound by latency: a CTA's life is a dozen round trips to memory, so more CTAs per SM count for
-// more than registers (2 / 3 / 4 per SM: 64 / 55 / 50 us at the headline shape; reading its
-// operands alone takes 28 us).
-template <typename T, bool SOFTMAX, bool REF>
-__global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __grid_constant__ Params p,
-                                                                     const __grid_constant__ SortPlan sp) {
+// Bound by latency: a CTA's life is a dozen round trips to memory, so more warps per SM count for
+// more than registers (2 / 3 / 4 CTAs of 512 threads per SM: 64 / 55 / 50 us at the headline shape;
+// reading its operands alone takes 28 us).
+//
+// BY_LEVEL: a CTA takes the points that a stretch of queries has on one level (levels vary after heads):
+// its cells are a level's only, so that a stretch can be longer and the counts of a cell are merged less
+// often (headline shape 53 -> 46 us, 512-pixel pyramid 26.5 -> 24, four odd levels 52 -> 48).  Offsets,
+// half as long and evaluated at more expense, are better off with all levels of a query side by side
+// (ragged pyramid 29 us against 38).
+__host__ __device__ constexpr int count_threads(bool by_level) { return by_level ? 256 : kSortThreads; }
+template <typename T, bool SOFTMAX, bool REF, bool BY_LEVEL>
+__global__ void __launch_bounds__(count_threads(BY_LEVEL), 2048 / count_threads(BY_LEVEL))
+    sort_count_kernel(const __grid_constant__ Params p, const __grid_constant__ SortPlan sp) {
+    constexpr int kThreads = count_threads(BY_LEVEL);
     grid_launch_dependents();
     // the first CTAs look for the magnitudes and clear grad_value, beside those that count
     if (blockIdx.x < (unsigned)sp.prepare_ctas) {
@@ -349,21 +359,32 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __gri
         if (threadIdx.x == 0) sp.header[kNoCells] = 1u;   // (every CTA says the same)
         return;
     }
-    const int cells = ct.first[p.L];
-    const bool in_shared = cells <= sp.shared_cells;
+    SortLane c;
+    unsigned cta = blockIdx.x - (unsigned)sp.prepare_ctas;
+    int cell0 = 0, cells = ct.first[p.L];
+    if constexpr (BY_LEVEL) {
+        const unsigned heads = cta / (unsigned)p.G, stretch = heads / (unsigned)p.L;
+        const int level = (int)(heads - stretch * (unsigned)p.L);
+        c = sort_lane<kThreads>(p, lt, ct, stretch * (unsigned)p.G + (cta - heads * (unsigned)p.G), sp.count_stretches,
+                                sp.count_queries, p.K, level * p.K);
+        cell0 = ct.first[level];
+        cells = ct.first[level + 1] - cell0;
+    } else {
+        c = sort_lane<kThreads>(p, lt, ct, cta, sp.count_stretches, sp.count_queries, p.L * p.K, 0);
+    }
+    c.cell0 -= cell0;
+    const bool in_shared = cells <= sp.count_cells;
     if (in_shared)
-        for (int i = threadIdx.x; i < cells; i += kSortThreads) hist[i] = 0u;
-    const SortLane c = sort_lane(p, sp, lt, ct, blockIdx.x - sp.prepare_ctas);
+        for (int i = threadIdx.x; i < cells; i += kThreads) hist[i] = 0u;
     unsigned *counts = sp.counts + (int64_t)c.plane * sp.cell_stride;
-    const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the chunk's first query
     __syncthreads();
     if (c.active) {
-        const int64_t base = pair0 * (p.L * p.K) + c.pt;
-        for (int r0 = 0; r0 < kSortPoints; r0 += kSortBatch) {
+        const int64_t base = (((int64_t)c.b * p.Q + c.q0) * p.G + c.g) * (p.L * p.K) + c.pt;
+        for (int q0 = c.ql; q0 < c.nq; q0 += kSortBatch * c.step) {
             float2 xy[kSortBatch];
 #pragma unroll
             for (int r = 0; r < kSortBatch; ++r) {
-                const int q = c.ql + (r0 + r) * c.step;
+                const int q = q0 + r * c.step;
                 xy[r] = q < c.nq ? point_xy<T, REF>(p, c, base, q) : make_float2(-1e9f, -1e9f);
             }
             PointCell at;
@@ -373,21 +394,21 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_count_kernel(const __gri
                 if (in_shared)
                     atomicAdd(hist + at.cell, 1u);
                 else
-                    atomicAdd(counts + at.cell, 1u);
+                    atomicAdd(counts + cell0 + at.cell, 1u);
             }
         }
     }
     __syncthreads();
-    if (in_shared) merge_counts(hist, counts, cells);
+    if (in_shared) merge_counts(hist, counts + cell0, cells);
     // the plane's last CTA turns its counts into places
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(sp.tickets + c.plane, 1u) == (unsigned)(sp.chunks - 1);
+    if (threadIdx.x == 0) last = atomicAdd(sp.tickets + c.plane, 1u) == (unsigned)(sp.count_ctas - 1);
     __syncthreads();
     if (last) {
         __threadfence();
-        scan_plane(counts, sp.offsets + (int64_t)c.plane * sp.cell_stride,
-                   sp.item_cell + (int64_t)c.plane * sp.items, cells, sp.item_points);
+        scan_plane<kThreads>(counts, sp.offsets + (int64_t)c.plane * sp.cell_stride,
+                             sp.item_cell + (int64_t)c.plane * sp.items, ct.first[p.L], sp.item_points);
     }
 }
 
@@ -572,7 +593,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     const bool in_shared = cells <= sp.shared_cells;
     if (in_shared)
         for (int i = threadIdx.x; i < cells; i += kSortThreads) shift[i] = 0u;
-    const SortLane c = sort_lane(p, sp, lt, ct, blockIdx.x);
+    const SortLane c = sort_lane<kSortThreads>(p, lt, ct, blockIdx.x, sp.chunks, sp.chunk_queries, p.L * p.K, 0);
     grid_launch_dependents();
     grid_dependency_wait();     // everything above reads the caller's tables only
     unsigned *cursor = sp.counts + (int64_t)c.plane * sp.cell_stride;
@@ -1213,13 +1234,15 @@ cudaError_t launch_walk(const Params &p, const SortPlan &sp, bool softmax, cudaS
 template <typename T, int D, bool SOFTMAX>
 cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_t stream) {
     const unsigned planes = (unsigned)(p.B * p.G);
-    const size_t hist = (size_t)sp.shared_cells * sizeof(unsigned);
+    const size_t hist = (size_t)sp.count_cells * sizeof(unsigned);
     const size_t scatter_smem = (size_t)kSortCtaPoints * 20 + (size_t)sp.shared_cells * 6;
     cudaError_t e = cudaMemsetAsync(sp.header, 0, sp.cleared_bytes, stream);
     if (e != cudaSuccess) return e;
-    auto count = p.ref != nullptr ? sort_count_kernel<T, SOFTMAX, true> : sort_count_kernel<T, SOFTMAX, false>;
+    auto count = p.ref != nullptr     ? sort_count_kernel<T, SOFTMAX, true, false>
+                 : sp.count_by_level ? sort_count_kernel<T, SOFTMAX, false, true>
+                                     : sort_count_kernel<T, SOFTMAX, false, false>;
     auto scatter = p.ref != nullptr ? sort_scatter_kernel<T, SOFTMAX, true> : sort_scatter_kernel<T, SOFTMAX, false>;
-    count<<<planes * (unsigned)sp.chunks + sp.prepare_ctas, kSortThreads, hist, stream>>>(p, sp);
+    count<<<planes * (unsigned)sp.count_ctas + sp.prepare_ctas, count_threads(sp.count_by_level), hist, stream>>>(p, sp);
     e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
     if (e != cudaSuccess) return e;
     e = launch_after_predecessor(scatter, planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream, p, sp);
@@ -1323,6 +1346,15 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     sp.plane_points = p.Q * P;
     sp.chunk_queries = (int)(kSortThreads / P * kSortPoints);
     sp.chunks = (int)((p.Q + sp.chunk_queries - 1) / sp.chunk_queries);
+    // (by level: stretches that leave four CTAs per SM, but no counts of few points to merge)
+    sp.count_by_level = p.ref == nullptr && p.K <= count_threads(true);
+    sp.count_queries = sp.chunk_queries;
+    if (sp.count_by_level) {
+        const int64_t share = std::min<int64_t>(std::max<int64_t>(planes * sp.plane_points / (148 * 4), 2048), 16384);
+        sp.count_queries = (int)round_up(share / p.K, count_threads(true) / p.K * kSortBatch);
+    }
+    sp.count_stretches = (int)((p.Q + sp.count_queries - 1) / sp.count_queries);
+    sp.count_ctas = sp.count_stretches * (sp.count_by_level ? p.L : 1);
     // a strip is at most 7 pixels short of its width and a level one row high: H + 1 <= 2 H and
     // ceil((W + 1) / 7) <= W leave at most two cells per pixel
     sp.prepare_ctas = (int)std::min<int64_t>(148 * 2, 1 + samples * (p.S + p.Q) * p.G * p.D / (8 * kSortThreads * 4));
@@ -1330,6 +1362,8 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // a pyramid of ordinary proportions has a cell per five to six pixels (whole eights: the scatter
     // takes cells by eights, in 16-byte accesses to arrays that follow one another)
     sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
+    // (the finest of several levels has four fifths of the positions; eight CTAs per SM need the room)
+    sp.count_cells = sp.count_by_level && p.L > 1 ? (int)std::min<int64_t>(sp.shared_cells, p.S / 8 + 256) : sp.shared_cells;
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
     // Runs of the walk: a long one is flushed and started less often, but the last ones to end leave
     // the others' SMs idle.  So they begin at eight units of 64 points and get shorter towards the

@@ -24,8 +24,12 @@ struct SortPlan {
     int64_t cell_stride;     // elements between planes in counts / offsets
     size_t cleared_bytes;    // header, tickets and counts, to be zero at the start
     int cell_bound;          // cells a plane has room for
-    int shared_cells;        // cells a sort CTA has room for in shared memory
-    int chunk_queries, chunks;
+    int shared_cells;        // cells a scatter CTA has room for in shared memory
+    int count_cells;         // the same of the counting kernel
+    int chunk_queries, chunks;             // queries of a scatter CTA, such stretches of a sample
+    bool count_by_level;                   // CTAs of the counting kernel take one level
+    int count_queries, count_stretches;    // the same of the counting kernel
+    int count_ctas;                        // its CTAs per plane
     int prepare_ctas;        // CTAs of the counting kernel that prepare instead
     int item_points, items;  // places of a unit, units of a plane
     // the walk's runs: below runs[0] of eight units, below runs[1] of four, below runs[2] of two, then of
