@@ -151,12 +151,13 @@ __device__ __forceinline__ void merge_counts(const unsigned *hist, unsigned *pla
 // Takes the CTA's counts per cell to `begin`, where the cell's points begin in the CTA's order,
 // and leaves in their place the difference to where they begin in the plane's.  Returns how
 // many points there are.
+template <int THREADS>
 __device__ __forceinline__ unsigned scan_cells(unsigned *counts, unsigned short *begin, unsigned *cursor,
                                                unsigned *warp_sums, int cells) {
     constexpr int kEach = 8;      // adjacent cells a thread takes (the arrays are padded to this)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned base = 0;
-    for (int c0 = 0; c0 < cells; c0 += kSortThreads * kEach) {
+    for (int c0 = 0; c0 < cells; c0 += THREADS * kEach) {
         const int at = c0 + threadIdx.x * kEach;
         unsigned n[kEach], place[kEach], sum = 0;
 #pragma unroll
@@ -181,7 +182,7 @@ __device__ __forceinline__ unsigned scan_cells(unsigned *counts, unsigned short 
         __syncthreads();
         unsigned before = 0, total = 0;
 #pragma unroll
-        for (int w = 0; w < kSortThreads / 32; ++w) {
+        for (int w = 0; w < THREADS / 32; ++w) {
             const unsigned s = warp_sums[w];
             before += w < warp ? s : 0u;
             total += s;
@@ -444,7 +445,7 @@ __device__ __forceinline__ __half *unsorted_extras(const SortPlan &sp) {
 __device__ inline void clear_unsorted_extras(const Params &p, const SortPlan &sp) {
     uint4 *extras = reinterpret_cast<uint4 *>(unsorted_extras(sp));
     const int64_t vecs = p.B * (extra_elems_per_sample(p.Q, p.G, p.D, p.L, p.K) / 8);
-    for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < vecs; i += (int64_t)gridDim.x * kSortThreads)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (int64_t)gridDim.x * blockDim.x)
         extras[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     }
     if (in_shared) {
         __syncthreads();
-        const unsigned points = scan_cells(shift, begin, cursor, warp_sums, cells);
+        const unsigned points = scan_cells<kSortThreads>(shift, begin, cursor, warp_sums, cells);
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kSortPoints; ++r) {
@@ -680,6 +681,138 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
             if (place < (unsigned)sp.plane_points) records[place] = local[order[i]];
         }
     }
+}
+
+// The same a level at a time, for locations of larger planes: a level has a third of the cells to look
+// through and merge per turn, and a cell's records leave in longer runs; the price is that a load
+// touches a line of memory for every query (why short offsets and small planes keep the other).  The
+// fractions and weights stay in registers until their place in the turn's order is known: few threads
+// with many registers, and persistent CTAs.  Bound by the latency of its phases (load/store pipe 62 %
+// busy, issue slots 43 %, DRAM 40 %).
+// Backward, B200, us, all levels -> this: headline shape 410 -> 394, random locations 433 -> 415, four
+// odd levels in float16 423 -> 414, 27 776 positions 447 -> 404, 42 500 301 -> 280, 58 968 of 64 channels
+// 503 -> 416.  (320 threads of 96 registers; 256 x 3 of 80: 428 for 394; 384 of 80 and six points 400;
+// 512 of 64, which spill, 412; without registers, as above, 256 x 3 407.)
+constexpr int kLevelThreads = 320;
+constexpr int kLevelPoints = 8;        // points per thread and turn,
+constexpr int kLevelBatch = 4;         // loaded this many at a time
+constexpr int kLevelTurn = kLevelThreads * kLevelPoints;
+constexpr int kLevelCells = 10752;     // most cells of a level, so that two CTAs fit an SM
+static_assert(3 * kLevelPoints <= 32, "the columns of a thread's points share a word");
+template <typename T, bool SOFTMAX>
+__global__ void __launch_bounds__(kLevelThreads, 2) sort_scatter_level_kernel(const __grid_constant__ Params p,
+                                                                             const __grid_constant__ SortPlan sp) {
+    using VT = VecTraits<T>;
+    extern __shared__ uint4 smem[];
+    __shared__ LevelTable lt;
+    __shared__ CellTable ct;
+    __shared__ unsigned warp_sums[kLevelThreads / 32];
+    // the turn's records in order of their cells, the cell of each; per cell: its count, then what takes
+    // a place in the turn's order to one in the plane's, and its first place in the turn's
+    uint4 *local = smem;
+    unsigned *shift = reinterpret_cast<unsigned *>(local + kLevelTurn);
+    unsigned short *cell_of = reinterpret_cast<unsigned short *>(shift + sp.level_cells);
+    unsigned short *begin = cell_of + kLevelTurn;
+    load_level_table(lt, p);
+    for (int i = threadIdx.x; i < sp.level_cells; i += kLevelThreads) shift[i] = 0u;
+    __syncthreads();
+    if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
+    __syncthreads();
+    grid_launch_dependents();
+    grid_dependency_wait();     // everything above reads the caller's tables only
+    if (!ct.fits) {      // (its points have no cells to be counted in)
+        clear_unsorted_extras(p, sp);
+        return;
+    }
+    const T *attn = reinterpret_cast<const T *>(p.attn);
+    const int P = p.L * p.K;
+    // (asked here, needed only when records leave: the points' loads do not wait for the answer)
+    const bool unsorted = unsorted_call<T>(sp.header);
+    for (unsigned turn = blockIdx.x; turn < sp.level_turns; turn += gridDim.x) {
+        const unsigned heads = turn / (unsigned)p.G, stretch = heads / (unsigned)p.L;
+        const int level = (int)(heads - stretch * (unsigned)p.L);
+        SortLane c = sort_lane<kLevelThreads>(p, lt, ct, stretch * (unsigned)p.G + (turn - heads * (unsigned)p.G),
+                                              sp.level_stretches, sp.level_queries, p.K, level * p.K);
+        const int cell0 = ct.first[level], cells = ct.first[level + 1] - cell0;
+        c.cell0 -= cell0;
+        const bool in_shared = cells <= sp.level_cells;
+        unsigned *cursor = sp.counts + (int64_t)c.plane * sp.cell_stride + cell0;
+        uint4 *records = sp.records + (int64_t)c.plane * sp.plane_points;
+        const int64_t pair0 = ((int64_t)c.b * p.Q + c.q0) * p.G + c.g;   // of the stretch's first query
+        const int64_t base = pair0 * P + c.pt;
+        const int nq = c.active ? c.nq : 0;
+        auto record_of = [&](int q, float fc, float fr, float a, unsigned col) {
+            return make_uint4(__float_as_uint(fc), __float_as_uint(fr), __float_as_uint(a),
+                              ((unsigned)(c.q0 + q) << 12) | ((unsigned)c.pt << 3) | col);
+        };
+        unsigned at[kLevelPoints];     // cell << 16 | rank among the turn's points of the cell; ~0: skipped
+        float3 kept[kLevelPoints];     // fractions and weight
+        unsigned cols = 0;             // columns in their cells, three bits each
+#pragma unroll
+        for (int r0 = 0; r0 < kLevelPoints; r0 += kLevelBatch) {
+            float2 xy[kLevelBatch], stats[SOFTMAX ? kLevelBatch : 1];
+            T weight[kLevelBatch];
+#pragma unroll
+            for (int r = 0; r < kLevelBatch; ++r) {
+                const int q = c.ql + (r0 + r) * c.step;
+                if (q < nq) xy[r] = point_xy<T, false>(p, c, base, q);
+            }
+#pragma unroll
+            for (int r = 0; r < kLevelBatch; ++r) {
+                const int q = c.ql + (r0 + r) * c.step;
+                if (q < nq) {
+                    if constexpr (SOFTMAX) stats[r] = sp.stats[pair0 + (int64_t)(q * p.G)];
+                    weight[r] = attn[base + (int64_t)(q * (p.G * P))];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kLevelBatch; ++r) {
+                at[r0 + r] = ~0u;
+                const int q = c.ql + (r0 + r) * c.step;
+                if (q >= nq) continue;
+                PointCell pc;
+                if (!find_cell(c, xy[r], pc)) {
+                    // a skipped point: exact zeros
+                    store_point_gradients<T>(p, sp, base + (int64_t)(q * (p.G * P)), make_float2(0.f, 0.f), 0.f);
+                } else {
+                    float a = VT::to_float(weight[r]);
+                    if constexpr (SOFTMAX) a = expf(a - stats[r].x) * stats[r].y;
+                    if (in_shared) {
+                        kept[r0 + r] = make_float3(pc.fc, pc.fr, a);
+                        cols |= (unsigned)pc.col << (3 * (r0 + r));
+                        at[r0 + r] = ((unsigned)pc.cell << 16) | atomicAdd(shift + pc.cell, 1u);
+                    } else {
+                        const unsigned place = atomicAdd(cursor + pc.cell, 1u);
+                        if (place < (unsigned)sp.plane_points && !unsorted)
+                            records[place] = record_of(q, pc.fc, pc.fr, a, (unsigned)pc.col);
+                    }
+                }
+            }
+        }
+        if (unsorted) break;      // (every point's gradients are the walk's then)
+        if (!in_shared) continue;
+        __syncthreads();
+        const unsigned points = scan_cells<kLevelThreads>(shift, begin, cursor, warp_sums, cells);
+#pragma unroll
+        for (int r = 0; r < kLevelPoints; ++r) {
+            if (at[r] == ~0u) continue;
+            const unsigned i = begin[at[r] >> 16] + (at[r] & 0xffffu);
+            local[i] = record_of(c.ql + r * c.step, kept[r].x, kept[r].y, kept[r].z, (cols >> (3 * r)) & 7u);
+            cell_of[i] = (unsigned short)(at[r] >> 16);
+        }
+        __syncthreads();
+        // neighbours in the turn's order are neighbours in the plane's for as long as a cell lasts
+#pragma unroll 4
+        for (unsigned i = threadIdx.x; i < points; i += kLevelThreads) {
+            const unsigned place = i + shift[cell_of[i]];
+            if (place < (unsigned)sp.plane_points) records[place] = local[i];
+        }
+        __syncthreads();
+        // (scan_cells wrote cells of whole eights)
+        for (int i = threadIdx.x; i < ((cells + 7) & ~7); i += kLevelThreads) shift[i] = 0u;
+        __syncthreads();
+    }
+    if (unsorted) clear_unsorted_extras(p, sp);
 }
 
 // ---- the walk over sorted points ------------------------------------------------------------------
@@ -1243,9 +1376,20 @@ cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_
                                      : sort_count_kernel<T, SOFTMAX, false, false>;
     auto scatter = p.ref != nullptr ? sort_scatter_kernel<T, SOFTMAX, true> : sort_scatter_kernel<T, SOFTMAX, false>;
     count<<<planes * (unsigned)sp.count_ctas + sp.prepare_ctas, count_threads(sp.count_by_level), hist, stream>>>(p, sp);
-    e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
-    if (e != cudaSuccess) return e;
-    e = launch_after_predecessor(scatter, planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream, p, sp);
+    if (sp.scatter_by_level) {
+        auto by_level = sort_scatter_level_kernel<T, SOFTMAX>;
+        const size_t smem = (size_t)kLevelTurn * 18 + (size_t)sp.level_cells * 6;
+        e = cudaFuncSetAttribute(by_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        static Residency residency;
+        const unsigned resident = residency.ctas(by_level, kLevelThreads, smem);
+        e = launch_after_predecessor(by_level, resident == 0 ? sp.level_turns : std::min(resident, sp.level_turns),
+                                     kLevelThreads, smem, stream, p, sp);
+    } else {
+        e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
+        if (e != cudaSuccess) return e;
+        e = launch_after_predecessor(scatter, planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream, p, sp);
+    }
     if (e != cudaSuccess) return e;
     e = p.ref != nullptr ? launch_walk<T, D, true>(p, sp, SOFTMAX, stream)
                          : launch_walk<T, D, false>(p, sp, SOFTMAX, stream);
@@ -1279,15 +1423,14 @@ int64_t round_up(int64_t n, int64_t to) { return (n + to - 1) / to * to; }
 //   offsets instead of          the arithmetic of the locations is done once more: 16 channels
 //   locations                   228 -> 251, 32: 157 -> 159 at 2 M points, 285 -> 275 at 4 M, 551
 //                               -> 503 at 8 M; 64 (1.8 M points): 241 -> 202
-//   positions                   the scatter kernel has two CTAs per SM up to 26 000, then one: at 42 000
-//                               510 -> 454, at 51 450 329 -> 298.  From about 55 000 a plane has more
-//                               than kSharedCells cells (one per 6.8 positions) and its records leave
-//                               unordered: 12 points per position, 58 968 positions, 16 channels 327 ->
-//                               345, 32: 370 -> 376, 64: 331 -> 251; 73 500: 747 -> 962, 880 -> 1027,
-//                               796 -> 665; 24 points, 73 500: 816 -> 769, 923 -> 814, 712 -> 529; 16
-//                               points on four levels: 490 -> 618, 600 -> 665, 509 -> 455; 40 on five,
-//                               where the few cells of the last one are counted by all: 1117 -> 1693,
-//                               1558 -> 1760, 1177 -> 1427
+//   positions                   12 points per position, 58 968 positions: 16 channels 591 -> 577, 32: 697
+//                               -> 640; 73 500: 740 -> 766, 880 -> 857; 16 points on four levels 1149 ->
+//                               1040.  From about 85 000 the finest level has more than kLevelCells
+//                               cells and its records leave unordered: 100 000 553 -> 677, 621 -> 765,
+//                               134 400 719 -> 850, 806 -> 905.  The line lies below, at 55 000, where what is
+//                               left to gain, 3 to 8 %, is not worth three times the scratch, but for
+//                               64 channels (331 -> 251 at 58 968) and 24 points of 32 (923 -> 686 at 73 500).
+//                               Offsets: more than kSharedCells cells from there on
 bool sorting_pays(const Params &p, int dtype, bool offsets) {
     const int64_t P = (int64_t)p.L * p.K, points = p.B * p.G * p.Q * P;
     if (dtype != 1 && dtype != 2) return false;
@@ -1362,8 +1505,17 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // a pyramid of ordinary proportions has a cell per five to six pixels (whole eights: the scatter
     // takes cells by eights, in 16-byte accesses to arrays that follow one another)
     sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
-    // (the finest of several levels has four fifths of the positions; eight CTAs per SM need the room)
-    sp.count_cells = sp.count_by_level && p.L > 1 ? (int)std::min<int64_t>(sp.shared_cells, p.S / 8 + 256) : sp.shared_cells;
+    // (backward, us, all levels -> by level: 5 376 positions 210.6 -> 213.7, 8 400 300 -> 304, 11 192 223.3 ->
+    // 224, 14 196 280 -> 273, 18 900 of 16 channels 317 -> 309)
+    sp.scatter_by_level = p.ref == nullptr && p.K <= kLevelThreads && p.S >= 12000;
+    sp.level_queries = (int)(kLevelThreads / p.K * kLevelPoints);
+    sp.level_stretches = sp.scatter_by_level ? (int)((p.Q + sp.level_queries - 1) / sp.level_queries) : 0;
+    sp.level_turns = (unsigned)(planes * p.L * sp.level_stretches);
+    // (the finest of several levels has four fifths of the positions; the counting kernel's CTAs per
+    // SM need the room)
+    sp.level_cells = (int)std::min<int64_t>(
+        kLevelCells, round_up(std::min<int64_t>(sp.cell_bound, p.L > 1 ? p.S / 8 + 256 : p.S / 5 + 256), 8));
+    sp.count_cells = sp.count_by_level ? sp.level_cells : sp.shared_cells;
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
     // Runs of the walk: a long one is flushed and started less often, but the last ones to end leave
     // the others' SMs idle.  So they begin at eight units of 64 points and get shorter towards the

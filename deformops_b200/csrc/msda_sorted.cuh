@@ -27,6 +27,10 @@ struct SortPlan {
     int shared_cells;        // cells a scatter CTA has room for in shared memory
     int count_cells;         // the same of the counting kernel
     int chunk_queries, chunks;             // queries of a scatter CTA, such stretches of a sample
+    bool scatter_by_level;                 // a turn of the scatter takes one level:
+    int level_queries, level_stretches;    // its queries, such stretches of a sample,
+    unsigned level_turns;                  // its turns,
+    int level_cells;                       // cells it has room for
     bool count_by_level;                   // CTAs of the counting kernel take one level
     int count_queries, count_stretches;    // the same of the counting kernel
     int count_ctas;                        // its CTAs per plane

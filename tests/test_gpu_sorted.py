@@ -74,6 +74,11 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
     # enough points for runs of all four lengths (the ones above have short runs only)
     (torch.bfloat16, False, 16, 4, [(60, 60), (30, 30)], 2, 27011, 8),
+    # 12 000 positions and more are sorted a level at a time: point counts that leave threads idle, tiny
+    # levels, one level, and one with more cells than a turn has room for
+    (torch.bfloat16, False, 32, 3, [(110, 113), (3, 5), (1, 1)], 1, 12001, 10),
+    (torch.float16, True, 16, 5, [(125, 100)], 3, 20011, 4),
+    (torch.bfloat16, True, 64, 8, [(6500, 2), (10, 10)], 1, 7001, 10),
     # more cells than a CTA counts in shared memory: narrow levels
     (torch.bfloat16, False, 32, 4, [(3000, 2)], 1, 13000, 20),
 ])
@@ -211,3 +216,26 @@ def test_non_finite_weights_stay_in_their_corners(dtype, softmax, bad):
         assert rel_err(to_np(x[fine]), to_np(y[fine])) <= bar
     spoilt = int((~torch.isfinite(got[0])).sum())
     assert spoilt == 0 if bad == float("-inf") else 0 < spoilt <= len(levels) * K * 4 * D
+
+
+@pytest.mark.parametrize("levels,overlap", [([(125, 100)], False), ([(13000, 1)] * 3, True)])
+def test_unsorted_points_of_large_planes(levels, overlap):
+    """What cannot be sorted, at a size that is sorted a level at a time: a NaN weight; levels on the same
+    rows with more cells than a plane has room for."""
+    B, Q, G, D, K = 1, 40009 // len(levels), 8, 32, 4
+    value, shapes, starts, loc, logits, grad_out = _inputs(11, B, Q, G, D, K, levels)
+    attn = logits.softmax(-1)
+    if overlap:
+        value, starts = value[:, :13000].contiguous(), torch.zeros_like(starts)
+    else:
+        loc[0, 11, 3, 0, 1] = torch.tensor([50.3 / 100, 60.1 / 125])
+        attn[0, 11, 3, 1] = float("nan")
+    dtype = torch.bfloat16
+    v, a, go = dev(value, dtype), dev(attn, dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = _workspace_backward(v, sh, st, l, a, go, False)
+    direct = abi_backward(v, sh, st, l, a, go)
+    for x, y, bar in zip(got, direct, (2e-2, 1e-4, 2e-2)):
+        fine = torch.isfinite(y)
+        assert torch.equal(torch.isfinite(x), fine)
+        assert rel_err(to_np(x[fine]), to_np(y[fine])) <= bar
