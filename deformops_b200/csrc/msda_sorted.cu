@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     }
 }
 
-// The same a level at a time, for locations of larger planes: a level has a third of the cells to look
+// The same a level at a time, for larger planes: a level has a third of the cells to look
 // through and merge per turn, and a cell's records leave in longer runs; the price is that a load
 // touches a line of memory for every query (why short offsets and small planes keep the other).  The
 // fractions and weights stay in registers until their place in the turn's order is known: few threads
@@ -699,7 +699,7 @@ constexpr int kLevelBatch = 4;         // loaded this many at a time
 constexpr int kLevelTurn = kLevelThreads * kLevelPoints;
 constexpr int kLevelCells = 10752;     // most cells of a level, so that two CTAs fit an SM
 static_assert(3 * kLevelPoints <= 32, "the columns of a thread's points share a word");
-template <typename T, bool SOFTMAX>
+template <typename T, bool SOFTMAX, bool REF>
 __global__ void __launch_bounds__(kLevelThreads, 2) sort_scatter_level_kernel(const __grid_constant__ Params p,
                                                                              const __grid_constant__ SortPlan sp) {
     using VT = VecTraits<T>;
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) sort_scatter_level_kernel(co
 #pragma unroll
             for (int r = 0; r < kLevelBatch; ++r) {
                 const int q = c.ql + (r0 + r) * c.step;
-                if (q < nq) xy[r] = point_xy<T, false>(p, c, base, q);
+                if (q < nq) xy[r] = point_xy<T, REF>(p, c, base, q);
             }
 #pragma unroll
             for (int r = 0; r < kLevelBatch; ++r) {
@@ -1377,12 +1377,13 @@ cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_
     auto scatter = p.ref != nullptr ? sort_scatter_kernel<T, SOFTMAX, true> : sort_scatter_kernel<T, SOFTMAX, false>;
     count<<<planes * (unsigned)sp.count_ctas + sp.prepare_ctas, count_threads(sp.count_by_level), hist, stream>>>(p, sp);
     if (sp.scatter_by_level) {
-        auto by_level = sort_scatter_level_kernel<T, SOFTMAX>;
+        auto by_level = p.ref != nullptr ? sort_scatter_level_kernel<T, SOFTMAX, true>
+                                         : sort_scatter_level_kernel<T, SOFTMAX, false>;
         const size_t smem = (size_t)kLevelTurn * 18 + (size_t)sp.level_cells * 6;
         e = cudaFuncSetAttribute(by_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        static Residency residency;
-        const unsigned resident = residency.ctas(by_level, kLevelThreads, smem);
+        static Residency residency[2];
+        const unsigned resident = residency[p.ref != nullptr].ctas(by_level, kLevelThreads, smem);
         e = launch_after_predecessor(by_level, resident == 0 ? sp.level_turns : std::min(resident, sp.level_turns),
                                      kLevelThreads, smem, stream, p, sp);
     } else {
@@ -1506,8 +1507,9 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // takes cells by eights, in 16-byte accesses to arrays that follow one another)
     sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
     // (backward, us, all levels -> by level: 5 376 positions 210.6 -> 213.7, 8 400 300 -> 304, 11 192 223.3 ->
-    // 224, 14 196 280 -> 273, 18 900 of 16 channels 317 -> 309)
-    sp.scatter_by_level = p.ref == nullptr && p.K <= kLevelThreads && p.S >= 12000;
+    // 224, 14 196 280 -> 273, 18 900 of 16 channels 317 -> 309; offsets: 14 196 211 -> 218, 21 504 497 -> 502,
+    // 27 900, where the other kernel has one CTA per SM only, 599 -> 534, 42 500 382 -> 345)
+    sp.scatter_by_level = p.K <= kLevelThreads && p.S >= (p.ref != nullptr ? 26000 : 12000);
     sp.level_queries = (int)(kLevelThreads / p.K * kLevelPoints);
     sp.level_stretches = sp.scatter_by_level ? (int)((p.Q + sp.level_queries - 1) / sp.level_queries) : 0;
     sp.level_turns = (unsigned)(planes * p.L * sp.level_stretches);

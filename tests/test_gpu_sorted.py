@@ -110,12 +110,16 @@ def test_samples_take_turns_when_the_scratch_holds_only_some():
         _check(got, (v, sh, st, l, a), go, False, shapes, l)
 
 
-@pytest.mark.parametrize("coords,offset_dtype", [(2, torch.bfloat16), (4, torch.float32)])
-def test_sorted_backward_from_offsets(coords, offset_dtype):
-    """Reference points and offsets in place of locations (three million points)."""
+@pytest.mark.parametrize("coords,offset_dtype,shape", [
+    (2, torch.bfloat16, (1, 24000, 8, 32, 8, [(15, 22), (8, 11)])),        # three million points
+    (4, torch.float32, (1, 24000, 8, 32, 8, [(15, 22), (8, 11)])),
+    (2, torch.bfloat16, (1, 23201, 5, 64, 5, [(170, 150), (20, 30)])),     # sorted a level at a time
+])
+def test_sorted_backward_from_offsets(coords, offset_dtype, shape):
+    """Reference points and offsets in place of locations."""
     from deformops_b200.registry import locations_from_offsets, msda, msda_from_offsets
 
-    B, Q, G, D, K, levels = 1, 24000, 8, 32, 8, [(15, 22), (8, 11)]
+    B, Q, G, D, K, levels = shape
     value, shapes, starts, loc, logits, grad_out = _inputs(5, B, Q, G, D, K, levels)
     dtype = torch.bfloat16
     g = torch.Generator().manual_seed(6)
