@@ -167,16 +167,18 @@ __global__ void __launch_bounds__(256, SMALL ? 2 : MSDA_FWD_MIN_CTAS) forward_ke
 // ---- dense calls of 16-bit values: 32 bytes per lane --------------------------------------------
 // The same sum with 32-byte loads: a slot is LPH = D / 16 lanes, a warp covers twice the pairs per
 // instruction, and a point's numbers go from the lane that placed it to its slot by shuffles, so that
-// all of the SM's memory that is not the level table stays L1.  What bounds it is what bounds
+// all of the SM's memory that is not the level table stays L1.  It adds the same products in the same
+// order: which of the two kernels a call takes does not show in its results.  What bounds it is what bounds
 // forward_kernel, one wavefront of the L1 data pipe per 64-byte corner row (79 % busy at the headline
 // shape, 4 x 21 504 queries of 12 points, 8 x 32 channels); of the rest a third of the wavefronts and a
 // seventh of the instructions are gone, and L1 hits 40 % of the sectors instead of 29 %.
-// Forward, B200, us, forward_kernel -> this: headline shape 164 -> 158, its 512-pixel pyramid 8 samples
-// 86 -> 82.5, four odd levels in float16 186 -> 174.5, softmax and offsets 109 -> 96; 6 x 64 channels,
-// 9 points, softmax and offsets 98 -> 80; 8 x 16 channels 129 -> 110; 2 x 128 149 -> 138.
+// Forward, B200, us, forward_kernel -> this: headline shape 164 -> 160, its 512-pixel pyramid 8 samples
+// 86 -> 82, four odd levels in float16 185.5 -> 182, softmax and offsets 109 -> 96; 6 x 64 channels,
+// 9 points, softmax and offsets 98 -> 82; 8 x 16 channels 129 -> 111; 2 x 128 149 -> 138.
 // Three CTAs of 80 registers: four of 64 spill (175), seven of four warps at 72 164; two points in
 // flight instead of one 160; one CTA per eight or sixteen groups instead of persistent ones 165, 168;
-// the next points' locations loaded a turn early 158.
+// the next points' locations loaded a turn early, no difference.  With adjacent points in one load,
+// added in another order than forward_kernel's, 158 (float16 174.5).
 constexpr int kWideWarps = 8;
 
 template <typename T>
@@ -196,8 +198,7 @@ __device__ __forceinline__ void gather32(float2 (&acc)[8], const char *at, float
     }
 }
 
-// The offsets or locations and the weights of PTS adjacent points (two: an even one first), in one
-// load each.
+// The offsets or locations and the weights of PTS adjacent points (two: an even one first), in one load each.
 template <typename T, bool REF, int PTS>
 __device__ __forceinline__ void load_points(const Params &p, int64_t e, float2 (&spot)[PTS], float (&weight)[PTS]) {
     using VT = VecTraits<T>;
@@ -217,6 +218,23 @@ __device__ __forceinline__ void load_points(const Params &p, int64_t e, float2 (
         const float2 w = VT::unpack2(__ldg(reinterpret_cast<const uint32_t *>(attn)));
         weight[0] = w.x, weight[1] = w.y;
     }
+}
+
+// slot_softmax_stats() of a slot of twice as many lanes, a lane doing the work of two: the same additions in
+// the same order.
+template <int LPH, typename T>
+__device__ __forceinline__ float2 wide_softmax_stats(const T *logits, int P, int sub) {
+    float m = -INFINITY;
+    for (int i = sub; i < P; i += LPH) m = fmaxf(m, VecTraits<T>::to_float(logits[i]));
+#pragma unroll
+    for (int o = LPH >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float sum = 0.f, other = 0.f;
+    for (int i = sub; i < P; i += 2 * LPH) sum += expf(VecTraits<T>::to_float(logits[i]) - m);
+    for (int i = sub + LPH; i < P; i += 2 * LPH) other += expf(VecTraits<T>::to_float(logits[i]) - m);
+    sum += other;
+#pragma unroll
+    for (int o = LPH >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return make_float2(m, 1.f / sum);
 }
 
 template <typename T, bool SOFTMAX, bool REF, int LPH, int PTS>
@@ -245,20 +263,31 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) forward_wide_kernel(const 
         const char *vb = reinterpret_cast<const char *>(p.value) + (b * p.S * (int64_t)row_bytes + g * (LPH * 32) + sub * 32);
         const int64_t e0 = pair * P;
         float2 stats = make_float2(0.f, 0.f);
-        if constexpr (SOFTMAX) stats = slot_softmax_stats(attn + e0, P, LPH, sub, true);
+        if constexpr (SOFTMAX) stats = wide_softmax_stats<LPH>(attn + e0, P, sub);
         float2 acc[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = make_float2(0.f, 0.f);
 #pragma unroll 1
         for (int r = 0; r < P; r += LPH * PTS) {
-            // ---- each lane of the slot takes PTS adjacent points
-            const int mine = r + sub * PTS;
+            // ---- each lane of the slot takes PTS points: adjacent ones where the slot is one lane, else
+            // one of every LPH
+            const int mine = r + sub * (LPH == 1 ? PTS : 1);
             float2 spot[PTS];
             float weight[PTS];
-            if (mine < P) load_points<T, REF, PTS>(p, e0 + mine, spot, weight);
+            if constexpr (LPH == 1) {
+                if (mine < P) load_points<T, REF, PTS>(p, e0 + mine, spot, weight);
+            } else {
+#pragma unroll
+                for (int i = 0; i < PTS; ++i) {
+                    float2 one_spot[1];
+                    float one_weight[1];
+                    if (mine + i * LPH < P) load_points<T, REF, 1>(p, e0 + mine + i * LPH, one_spot, one_weight);
+                    spot[i] = one_spot[0], weight[i] = one_weight[0];
+                }
+            }
 #pragma unroll
             for (int i = 0; i < PTS; ++i) {
-                const int pt = mine + i;
+                const int pt = mine + i * (LPH == 1 ? 1 : LPH);
                 int place = 0, down = 0;
                 float w00 = 0.f, w01 = 0.f, w10 = 0.f, w11 = 0.f;
                 if (pt < P) {
@@ -281,9 +310,10 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) forward_wide_kernel(const 
                     w10 = f & kCorner10 ? a * (geo.fr * wc0) : 0.f;
                     w11 = f & kCorner11 ? a * (geo.fr * geo.fc) : 0.f;
                 }
+                // ---- and the slot gathers them, in the order of the points
 #pragma unroll 1
                 for (int j = 0; j < LPH; ++j) {
-                    if (r + j * PTS + i >= P) break;
+                    if (r + i * LPH + j >= P) break;
                     const int from = LPH == 1 ? 0 : (lane & ~(LPH - 1)) + j;
                     auto get = [&](auto v) { return LPH == 1 ? v : __shfl_sync(0xffffffffu, v, from); };
                     const int pl = get(place), dy = get(down);
@@ -320,10 +350,10 @@ cudaError_t launch_wide_as(const Params &p, cudaStream_t stream) {
 }
 template <typename T, bool SOFTMAX, bool REF, int LPH>
 cudaError_t launch_wide(const Params &p, cudaStream_t stream) {
-    // (two points a lane in slots of four lanes and more leave lanes idle in the last turn: 12 points
-    // of 64 channels 35 us against 33)
+    // (two points a lane: their loads go out together.  Slots of four lanes are better off without, 84
+    // us against 82 of the ragged pyramid)
     if constexpr (LPH < 4)
-        if (p.L * p.K % 2 == 0) return launch_wide_as<T, SOFTMAX, REF, LPH, 2>(p, stream);
+        if (LPH > 1 || p.L * p.K % 2 == 0) return launch_wide_as<T, SOFTMAX, REF, LPH, 2>(p, stream);
     return launch_wide_as<T, SOFTMAX, REF, LPH, 1>(p, stream);
 }
 
