@@ -21,8 +21,8 @@
 // eight channels, instead of once per corner and point (at 21 504 queries and 12 points per query
 // 33 million rows of reductions become about 1 million).
 //
-// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 429 us
-// against 512 us, of which counting 51, writing records 104, the walk 247, the last pass 22;
+// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 394 us
+// against 512 us, of which counting 44, writing records 92, the walk 237, the last pass 22;
 // grad_value 1.7e-3 off the float32 result against 2.2e-3.
 //
 // Accumulation is float32 inside a warp's run of points; the few sums that meet in memory (two
@@ -938,7 +938,7 @@ __device__ __forceinline__ void flush_row(float (&acc)[D / 8][4], int half, floa
 
 // What bounds the walk is the SM's load/store pipe, about five of its cycles a point (ncu, the
 // headline shape: 64 % busy while the SM works, issue slots 50 %, tensor cores 24 %): the two
-// stores per point to addresses of their own take 45 us of 247, the grad_out rows 27, the rest
+// stores per point to addresses of their own take 45 us of 237, the grad_out rows 27, the rest
 // goes through shared memory.  Hence the weights' way over the tensor cores below.  More warps do
 // not help - 12, 16, 20, 24 per SM: 252, 246, 261, 312 us - nor does having grad_out rows in
 // registers instead of shared memory (300 us), or the next cell's value row early (257 us).
