@@ -400,6 +400,7 @@ struct LevelTable {
     int W[kMaxLevels];
     int start[kMaxLevels];          // first position of the level on the S axis
     int rowstride[kMaxLevels];      // elements between image rows: W * G * D
+    float rcp_w[kMaxLevels], rcp_h[kMaxLevels];   // 1 / W, 1 / H, for location_from_offset()
     // scaled float16 backward: accumulators per element of the level (1 = the image only) and
     // where the level's additional replicas start in a sample's block of extras
     int rep[kMaxLevels];
@@ -439,6 +440,8 @@ __device__ __forceinline__ void load_level_table(LevelTable &t, const Params &p)
         t.W[threadIdx.x] = W;
         t.start[threadIdx.x] = fits ? (int)first : 0;
         t.rowstride[threadIdx.x] = W * p.G * p.D;
+        t.rcp_w[threadIdx.x] = 1.f / (float)W;
+        t.rcp_h[threadIdx.x] = 1.f / (float)H;
         t.level_elems[threadIdx.x] = (unsigned)H * (unsigned)W * (unsigned)(p.G * p.D);
     }
 }
@@ -502,6 +505,25 @@ __device__ __forceinline__ float2 location_from_offset(const Params &p, float2 o
     const float4 r = __ldg(reinterpret_cast<const float4 *>(p.ref) + bq * p.L + l);
     const float Kf = (float)p.K;
     return make_float2(r.x + off.x / Kf * r.z * 0.5f, r.y + off.y / Kf * r.w * 0.5f);
+}
+// x / n for a whole number n below 2^20 and rcp = 1 / n, in three instructions: Markstein's correction of
+// an approximate quotient by its exact remainder ("Computation of elementary functions on the IBM RISC
+// System/6000", 1990).  q is at most two units in its last place off and the remainder, a multiple of that
+// unit below 2^22 of them, exact; a quotient by such an n lies at least 2^-21 units from a rounding
+// boundary, what the correction loses is 2^-23.  So the result is the quotient rounded to nearest, as
+// the division gives it; where q leaves the normal range, or x is no number, a location so far off or so
+// near its reference point that the pixel coordinate is the same.
+__device__ __forceinline__ float quotient(float x, float n, float rcp) {
+    const float q = x * rcp;
+    return fmaf(fmaf(-q, n, x), rcp, q);
+}
+// The same location without divisions (offsets at the headline shape, us: forward 186.1 -> 183.9,
+// backward, whose sort kernels use it, 492.5 -> 487.2; ragged pyramid 194.8 -> 192.4).
+__device__ __forceinline__ float2 location_from_offset(const Params &p, float2 off, int64_t bq, int l,
+                                                       float Wf, float Hf, float rcp_w, float rcp_h) {
+    if (p.ref_coords != 2) return location_from_offset(p, off, bq, l, Wf, Hf);
+    const float2 r = __ldg(reinterpret_cast<const float2 *>(p.ref) + bq * p.L + l);
+    return make_float2(r.x + quotient(off.x, Wf, rcp_w), r.y + quotient(off.y, Hf, rcp_h));
 }
 // Derivative of the pixel coordinate with respect to that offset.
 __device__ __forceinline__ float2 offset_derivative(const Params &p, int64_t bq, int l, float Wf, float Hf) {

@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) forward_wide_kernel(const 
                     const int l = (int)(((float)pt + 0.5f) * inv_K);  // pt / K
                     const int H = lt.H[l], W = lt.W[l];
                     float2 xy = spot[i];
-                    if constexpr (REF) xy = location_from_offset(p, xy, (int64_t)bq, l, (float)W, (float)H);
+                    if constexpr (REF)
+                        xy = location_from_offset(p, xy, (int64_t)bq, l, (float)W, (float)H, lt.rcp_w[l], lt.rcp_h[l]);
                     float a = weight[i];
                     if constexpr (SOFTMAX) a = expf(a - stats.x) * stats.y;
                     const PointGeom geo = locate(xy.x, xy.y, H, W, 0, 0);

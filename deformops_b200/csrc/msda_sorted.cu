@@ -81,6 +81,7 @@ struct SortLane {
     int plane, b, g;
     int pt, l;              // point of the query and its level
     int H, W, cell0, rows;  // of the level
+    float rcp_w, rcp_h;     // 1 / W, 1 / H
     int ql, nq, step;       // first query of the thread (chunk-relative), queries of the chunk, stride
     int64_t q0;             // first query of the chunk
     bool active;
@@ -102,6 +103,7 @@ __device__ __forceinline__ SortLane sort_lane(const Params &p, const LevelTable 
     s.active = s.ql < s.step;
     s.H = lt.H[s.l];
     s.W = lt.W[s.l];
+    s.rcp_w = lt.rcp_w[s.l], s.rcp_h = lt.rcp_h[s.l];
     s.cell0 = ct.first[s.l];
     s.rows = ct.rows[s.l];
     s.q0 = (int64_t)chunk * chunk_queries;
@@ -136,7 +138,7 @@ __device__ __forceinline__ float2 point_xy(const Params &p, const SortLane &s, i
     if constexpr (REF) {
         const float2 off = p.offsets16 ? VecTraits<T>::unpack2(__ldg(reinterpret_cast<const uint32_t *>(p.loc) + e))
                                        : __ldg(reinterpret_cast<const float2 *>(p.loc) + e);
-        return location_from_offset(p, off, (int64_t)s.b * p.Q + s.q0 + q, s.l, (float)s.W, (float)s.H);
+        return location_from_offset(p, off, (int64_t)s.b * p.Q + s.q0 + q, s.l, (float)s.W, (float)s.H, s.rcp_w, s.rcp_h);
     } else {
         return __ldg(reinterpret_cast<const float2 *>(p.loc) + e);
     }

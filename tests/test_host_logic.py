@@ -348,3 +348,30 @@ def test_reference_op_names_can_be_offered_without_the_reference():
         "print('ok')\n")
     res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
     assert res.returncode == 0 and "ok" in res.stdout, res.stderr[-2000:]
+
+
+def test_quotients_by_level_sizes_round_as_a_division():
+    """``quotient()`` of csrc/msda_common.cuh, step by step in exact arithmetic, against the float32 division:
+    the locations that the fused kernels form have to be those of the expressions they replace."""
+    from fractions import Fraction
+
+    import numpy as np
+
+    rng = np.random.default_rng(3)
+    f32 = np.float32
+
+    def rounded(v):                       # nearest float32 of an exact value in the normal range
+        near = f32(float(v))
+        around = [near, np.nextafter(near, f32(np.inf)), np.nextafter(near, f32(-np.inf))]
+        best = min(abs(Fraction(float(c)) - v) for c in around)
+        ties = [c for c in around if abs(Fraction(float(c)) - v) == best]
+        return ties[0] if len(ties) == 1 else next(c for c in ties if int(c.view(np.uint32)) % 2 == 0)
+
+    for _ in range(4000):
+        n = f32(int(np.exp(rng.uniform(0, np.log(2.0 ** 20)))))
+        x = f32(rng.standard_normal() * 10.0 ** rng.uniform(-6, 4))
+        rcp = f32(1) / n
+        q = x * rcp
+        remainder = rounded(Fraction(float(x)) - Fraction(float(q)) * int(n))
+        got = rounded(Fraction(float(remainder)) * Fraction(float(rcp)) + Fraction(float(q)))
+        assert got == x / n, (x, n)
