@@ -385,13 +385,21 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
 // 32-byte loads halve the warps of a call.  Where neighbouring queries sample neighbouring pixels, or
 // all pixels are sampled often, L1 makes up for it; few queries far apart wait for L2 instead (us,
 // forward_kernel -> forward_wide_kernel: 900 queries on 17 821 positions, 8 samples 32 -> 39; 1 800, 16
-// samples 84 -> 87; 7 000 on 21 504, 8 samples 111 -> 109, 10 752 166 -> 158).  Below six million output
-// elements the two lie within 3 % of one another (5.5 M: 46.2 -> 47.4), but for 16 channels (1.4 M:
-// 22.7 -> 18.6).  float32 gains nothing (262 -> 273): its rows are whole lines of L1 either way.
-bool wide_pays(const Params &p) {
+// samples 84 -> 87; 7 000 on 21 504, 8 samples 111 -> 109, 10 752 166 -> 158).  Of the dense calls the last
+// round of the persistent warps decides, 24 per SM here and 32 there: a round of this kernel takes
+// 1.38 times one of the other (12.2 against 8.8 us, 12 points of 32 channels), with offsets or a
+// softmax 1.25 times.  Rounds of either, us: 2 and 3, 26.8 -> 24.7; 3 and 4, 37 -> 37, offsets
+// of 64 channels 32.9 -> 30.9; 4 and 5, 46.2 -> 47.4, offsets 55.4 -> 53.9; 4 and 6, 57.9 -> 53.5.  Of many
+// rounds the last counts for little: 7 and 10, 86 -> 82; 8 and 11 (64 channels) 75.7 -> 69.8; 13 and 19, 164 -> 160.  16 channels gain throughout (22.7 -> 18.6 .. 129 -> 111).  float32 gains nothing (262
+// -> 273): its rows are whole lines of L1 either way.
+bool wide_pays(const Params &p, bool softmax_or_offsets) {
     const int64_t pairs = p.B * p.Q * p.G;
-    return (reinterpret_cast<uintptr_t>(p.value) & 31u) == 0 && 2 * p.Q >= p.S && pairs < (int64_t)1 << 31 &&
-           (p.D == 16 || pairs * p.D >= 6000000);
+    if ((reinterpret_cast<uintptr_t>(p.value) & 31u) != 0 || 2 * p.Q < p.S || pairs >= (int64_t)1 << 31) return false;
+    if (p.D == 16) return true;
+    const int64_t wide = 148 * 24 * (512 / p.D), other = 148 * 32 * (256 / p.D);     // pairs of a round
+    const int64_t rounds = (pairs + wide - 1) / wide, other_rounds = (pairs + other - 1) / other;
+    if (rounds > 6) return true;
+    return softmax_or_offsets ? 5 * rounds <= 4 * other_rounds : 18 * rounds <= 13 * other_rounds;
 }
 
 template <typename T, bool SOFTMAX, bool REF>
@@ -402,7 +410,7 @@ cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
     // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
     constexpr int kSms = 148;
     if constexpr (sizeof(T) == 2) {
-        if (p.num_groups > 4 * kSms && wide_pays(p)) {
+        if (p.num_groups > 4 * kSms && wide_pays(p, SOFTMAX || REF)) {
             switch (p.D) {
                 case 16: return launch_wide<T, SOFTMAX, REF, 1>(p, stream);
                 case 32: return launch_wide<T, SOFTMAX, REF, 2>(p, stream);

@@ -1,7 +1,7 @@
 """The forward with 32-byte loads per lane (dense calls of 16-bit values), against the float64 oracle.
 
 The sizes are those its rule sends there (two queries or more per four positions; 16 channels and some
-ten thousand pairs, or six million output elements), with point counts that leave the last turn of a slot
+ten thousand pairs, or enough rounds of its warps), with point counts that leave the last turn of a slot
 partly empty, pair counts that leave the last warp so, and a value tensor that is not 32-byte aligned,
 which takes the other kernel and has to give the same bits.
 """
@@ -22,9 +22,9 @@ pytestmark = pytest.mark.gpu
 CASES = [
     ([(19, 23), (5, 7), (1, 1)], 3, 1001, 4, 16, 1, torch.float16, False, 0),      # 3 points, 1 lane a slot
     ([(19, 23), (5, 7)], 3, 1001, 4, 16, 3, torch.bfloat16, True, 2),              # 6 points, two a lane
-    ([(31, 17)], 3, 12501, 5, 32, 2, torch.bfloat16, False, 0),                    # fewer points than a turn
-    ([(31, 17), (9, 4), (3, 2)], 3, 12501, 5, 32, 2, torch.float16, True, 4),      # 6: half a last turn
-    ([(31, 17), (9, 4), (3, 2)], 3, 12501, 5, 32, 3, torch.bfloat16, False, 0),    # 9: one point a lane
+    ([(31, 17)], 3, 6251, 5, 32, 2, torch.bfloat16, False, 0),                    # fewer points than a turn
+    ([(31, 17), (9, 4), (3, 2)], 3, 6251, 5, 32, 2, torch.float16, True, 4),      # 6: half a last turn
+    ([(31, 17), (9, 4), (3, 2)], 3, 6251, 5, 32, 3, torch.bfloat16, False, 0),    # 9: one point a lane
     ([(40, 30), (7, 1)], 1, 33337, 3, 64, 3, torch.float16, False, 0),             # 6 points, slots of four
     ([(40, 30), (7, 1)], 1, 33337, 3, 64, 4, torch.bfloat16, True, 2),
     ([(12, 50)], 2, 12345, 2, 128, 5, torch.bfloat16, False, 0),                   # 5 points, slots of eight
