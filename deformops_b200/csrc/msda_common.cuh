@@ -428,6 +428,8 @@ __device__ inline void plan_replicas(LevelTable &t, const Params &p) {
 // (non-positive size, negative start, or start + H*W beyond S) becomes an empty level at
 // position 0: every point on it is skipped, so a malformed table produces zeros for that level
 // instead of an access outside `value` / `grad_value`.
+// RECIPROCALS: rcp_w, rcp_h too (a small call lasts as long as one warp's chain, and feels two divisions).
+template <bool RECIPROCALS = false>
 __device__ __forceinline__ void load_level_table(LevelTable &t, const Params &p) {
     if (threadIdx.x < p.L) {
         const int64_t h = p.spatial_shapes[2 * threadIdx.x];
@@ -440,8 +442,10 @@ __device__ __forceinline__ void load_level_table(LevelTable &t, const Params &p)
         t.W[threadIdx.x] = W;
         t.start[threadIdx.x] = fits ? (int)first : 0;
         t.rowstride[threadIdx.x] = W * p.G * p.D;
-        t.rcp_w[threadIdx.x] = 1.f / (float)W;
-        t.rcp_h[threadIdx.x] = 1.f / (float)H;
+        if constexpr (RECIPROCALS) {
+            t.rcp_w[threadIdx.x] = 1.f / (float)W;
+            t.rcp_h[threadIdx.x] = 1.f / (float)H;
+        }
         t.level_elems[threadIdx.x] = (unsigned)H * (unsigned)W * (unsigned)(p.G * p.D);
     }
 }

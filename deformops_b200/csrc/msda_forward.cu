@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) forward_wide_kernel(const 
     using VT = VecTraits<T>;
     constexpr int kPairs = 32 / LPH;
     __shared__ LevelTable lt;
-    load_level_table(lt, p);
+    load_level_table<REF>(lt, p);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = lane / LPH, sub = lane % LPH;

@@ -103,7 +103,7 @@ __device__ __forceinline__ SortLane sort_lane(const Params &p, const LevelTable 
     s.active = s.ql < s.step;
     s.H = lt.H[s.l];
     s.W = lt.W[s.l];
-    s.rcp_w = lt.rcp_w[s.l], s.rcp_h = lt.rcp_h[s.l];
+    s.rcp_w = lt.rcp_w[s.l], s.rcp_h = lt.rcp_h[s.l];      // (set where there are offsets)
     s.cell0 = ct.first[s.l];
     s.rows = ct.rows[s.l];
     s.q0 = (int64_t)chunk * chunk_queries;
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(count_threads(BY_LEVEL), 2048 / count_threads(
     __shared__ LevelTable lt;
     __shared__ CellTable ct;
     __shared__ bool last;
-    load_level_table(lt, p);
+    load_level_table<REF>(lt, p);
     __syncthreads();
     if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
     __syncthreads();
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
     unsigned short *order = reinterpret_cast<unsigned short *>(shift + sp.shared_cells);
     unsigned short *cell_of = order + kSortCtaPoints;
     unsigned short *begin = cell_of + kSortCtaPoints;
-    load_level_table(lt, p);
+    load_level_table<REF>(lt, p);
     __syncthreads();
     if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
     __syncthreads();
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) sort_scatter_level_kernel(co
     unsigned *shift = reinterpret_cast<unsigned *>(local + kLevelTurn);
     unsigned short *cell_of = reinterpret_cast<unsigned short *>(shift + sp.level_cells);
     unsigned short *begin = cell_of + kLevelTurn;
-    load_level_table(lt, p);
+    load_level_table<REF>(lt, p);
     for (int i = threadIdx.x; i < sp.level_cells; i += kLevelThreads) shift[i] = 0u;
     __syncthreads();
     if (threadIdx.x == 0) plan_cells(ct, lt, p.L, sp.cell_bound);
