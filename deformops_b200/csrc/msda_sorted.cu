@@ -1009,22 +1009,26 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
     // the identity as the A operand of an m16n8k16 product (upper left and lower right corner)
     const uint32_t one = VT::pack2(make_float2(j == 2 * c ? 1.f : 0.f, j == 2 * c + 1 ? 1.f : 0.f));
 
+    const bool coarse_first = lt.H[p.L - 1] * lt.W[p.L - 1] > lt.H[0] * lt.W[0];
     // ---- runs of places, handed out as the warps come for them
     for (;;) {
         unsigned run = 0;
         if (lane == 0) run = atomicAdd(sp.header + kNextItem, 1u);
         run = __shfl_sync(0xffffffffu, run, 0);
         if (run >= sp.all_runs) break;
-        const int size = run < sp.runs[0] ? 3 : run < sp.runs[1] ? 2 : run < sp.runs[2] ? 1 : 0;   // 2^size units
-        const unsigned first = (run << size) + (size == 3 ? 0u : sp.unit0[2 - size]);
-        const int plane = (int)(first / (unsigned)sp.items);
-        int pos = (int)(first - (unsigned)plane * (unsigned)sp.items) * sp.item_points;
+        const WalkRuns &kind = sp.runs[run < sp.runs[1].run0 ? 0 : run < sp.runs[2].run0 ? 1 : 2];
+        const unsigned nth = (run - kind.run0) / kind.each;
+        const int plane = (int)(kind.plane0 + nth);
+        unsigned unit = kind.unit0 + ((run - kind.run0 - nth * kind.each) << kind.log2_size);
+        // (short runs belong on the finest level)
+        if (coarse_first) unit = (unsigned)sp.items - unit - (1u << kind.log2_size);
+        int pos = (int)unit * sp.item_points;
         const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
         // (places beyond the plane's points hold no record: what is read there is not kept)
         uint4 rec = __ldcg(records + min((int64_t)(pos + lane), sp.plane_points - 1));
-        int cell = sp.item_cell[first];
+        int cell = sp.item_cell[(unsigned)plane * (unsigned)sp.items + unit];
         const int total = (int)sp.offsets[(int64_t)plane * sp.cell_stride + cells];
-        const int stop = min(pos + (sp.item_points << size), total);
+        const int stop = min(pos + (sp.item_points << kind.log2_size), total);
         if (pos >= stop) continue;
         if (pos + lane >= total) rec = make_uint4(0u, 0u, 0u, 0u);
         const unsigned *offsets = sp.offsets + (int64_t)plane * sp.cell_stride;
@@ -1486,6 +1490,55 @@ int64_t sorted_workspace_bytes(const Params &p, bool softmax, int64_t samples) {
     return plan_sorted(sp, p, softmax, samples, nullptr);
 }
 
+// Runs of the walk.  Where a run ends, the sums of two pixel rows leave it unfinished and meet in float16
+// once more.  So no plane is in more runs than if all had `length` points: 128 to 256, by what a warp's
+// share leaves room for, and more where a pixel collects thousands of points.  Within that, a long run is
+// flushed and started less often, but the last ones to end leave the other warps idle:
+//   six runs of `length` and more a warp   twice the length, until two of `length` are left for every
+//                                 warp (planes in order: what a plane's levels share stays in L2)
+//   two to six, or 64 channels    every plane has some of twice, of once and of half the length: the long
+//                                 ones are handed out first, the short ones lie on its finest level, where
+//                                 the fewest points share a pixel.  That costs L2 hits (1024 pixels, 2 samples,
+//                                 6.8 runs a warp: 232 us against 222), but less than a nearly empty last
+//                                 round of whole runs
+//   fewer                         all of `length`
+// Backward, B200, us, all of `length` -> this: headline shape 408 -> 401, 16 samples 1616 -> 1578, four odd
+// levels in float16 431 -> 419, 512-pixel pyramid 8 samples 223 -> 220, 4 samples 134 -> 127; 64 channels:
+// ragged pyramid with offsets 207 -> 193, 512 pixels 16 samples 295 -> 269.  Runs of 512 points getting
+// shorter to 64 in the order of the planes: 399, 1575, 412, 217, 124, 196, 274, but the last plane's
+// float16 grad_value was 5.6e-4 off and the first's 3.6e-4 where all are 3.6e-4 to 4.0e-4 now (four odd
+// levels 8.1e-4 and 4.2e-4; now 4.2e-4 to 5.0e-4)
+void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
+    const int64_t warps = 148 * kWalkWarps * walk_ctas(p.D);
+    const int64_t share = planes * sp.plane_points / (148 * 16 * 4), density = sp.plane_points / std::max<int64_t>(p.S, 1);
+    const int64_t length = std::min<int64_t>(256, std::max<int64_t>(128, share / 32 * 32)) *
+                           std::min<int64_t>(16, 1 + density / 128);
+    sp.item_points = (int)(length / 2);
+    sp.items = (int)round_up((sp.plane_points + sp.item_points - 1) / sp.item_points, 4);   // (no run in two planes)
+    const int64_t units = planes * sp.items;
+    int64_t whole = 0;             // planes of long runs only
+    int64_t spread = 0;            // runs of `length` of every plane beside its long and short ones
+    if (units >= 12 * warps && p.D < 64)
+        whole = std::max<int64_t>(0, planes - (4 * warps + sp.items - 1) / sp.items);
+    else if (units >= 4 * warps)
+        spread = std::min((warps + planes - 1) / planes, (int64_t)(sp.items - 4) / 8);   // (items / 2 - 1 runs at most)
+    unsigned runs = 0;
+    auto add = [&](int kind, int64_t plane, int64_t of_planes, int64_t unit, int64_t each, int log2_size) {
+        sp.runs[kind] = {runs, (unsigned)plane, (unsigned)std::max<int64_t>(each, 1), (unsigned)unit, log2_size};
+        runs += (unsigned)(of_planes * each);
+    };
+    if (spread > 0) {              // 2 * spread units in short runs, as many in runs of `length`
+        add(0, 0, planes, 4 * spread, sp.items / 4 - spread, 2);
+        add(1, 0, planes, 2 * spread, spread, 1);
+        add(2, 0, planes, 0, 2 * spread, 0);
+    } else {
+        add(0, 0, whole, 0, sp.items / 4, 2);
+        add(1, whole, planes - whole, 0, sp.items / 2, 1);
+        add(2, planes, 0, 0, 0, 0);
+    }
+    sp.all_runs = runs;
+}
+
 int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples, void *workspace) {
     const int64_t P = (int64_t)p.L * p.K;
     const int64_t planes = samples * p.G;
@@ -1521,27 +1574,7 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
         kLevelCells, round_up(std::min<int64_t>(sp.cell_bound, p.L > 1 ? p.S / 8 + 256 : p.S / 5 + 256), 8));
     sp.count_cells = sp.count_by_level ? sp.level_cells : sp.shared_cells;
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
-    // Runs of the walk: a long one is flushed and started less often, but the last ones to end leave
-    // the others' SMs idle.  So they begin at eight units of 64 points and get shorter towards the
-    // end: eight and four while two of them are left for every warp, two while one is, then one
-    // (backward, us, all runs of 256 points -> this: headline shape 425 -> 415, 512-pixel pyramid 224
-    // -> 213, four odd levels in float16 440 -> 424, ragged pyramid of 64 channels 205 -> 195; with one
-    // of every length left 426, 217, 434, 212; three 423, 222, 423, 192).  Units are longer where a pixel
-    // collects thousands of points: every run adds to it once, in float16
-    const int64_t density = sp.plane_points / std::max<int64_t>(p.S, 1);
-    sp.item_points = (int)(64 * std::min<int64_t>(16, 1 + density / 128));
-    sp.items = (int)round_up((sp.plane_points + sp.item_points - 1) / sp.item_points, 8);   // (no run in two planes)
-    const int64_t warps = 148 * kWalkWarps * walk_ctas(p.D);
-    int64_t units = planes * sp.items, runs = 0;
-    for (int i = 0; i < 3; ++i) {
-        const int64_t spare = (i < 2 ? 2 : 1) * warps, size = 8 >> i;
-        const int64_t n = std::max<int64_t>(0, units / size - spare);
-        runs += n;
-        units -= n * size;
-        sp.runs[i] = (unsigned)runs;
-        sp.unit0[i] = (unsigned)(planes * sp.items - units - (runs * (size / 2)));
-    }
-    sp.all_runs = (unsigned)(runs + units);
+    plan_runs(sp, p, planes);
     char *at = static_cast<char *>(workspace);
     int64_t used = 0;
     auto take = [&](int64_t bytes) {

@@ -10,6 +10,12 @@ namespace msda_b200 {
 
 constexpr int kCols = 7;   // pixel columns (of the top left corner) of a cell
 
+// Runs of one length: `each` in every plane from plane0 on, of 2^log2_size units, the first at unit0.
+struct WalkRuns {
+    unsigned run0, plane0, each, unit0;
+    int log2_size;
+};
+
 // Layout of the workspace and shape of the launches for the samples of one pass.
 struct SortPlan {
     unsigned *header;        // magnitude cells (as in the scaled float16 scratch)
@@ -36,9 +42,8 @@ struct SortPlan {
     int count_ctas;                        // its CTAs per plane
     int prepare_ctas;        // CTAs of the counting kernel that prepare instead
     int item_points, items;  // places of a unit, units of a plane
-    // the walk's runs: below runs[0] of eight units, below runs[1] of four, below runs[2] of two, then of
-    // one.  The first unit of run r is r * its length + unit0[i] (nothing before runs[0])
-    unsigned runs[3], unit0[3], all_runs;
+    WalkRuns runs[3];        // by the order they are handed out in
+    unsigned all_runs;
 };
 
 // Whether a call is dense enough for the sort to pay (and within the record's field widths).

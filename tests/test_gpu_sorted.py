@@ -72,7 +72,7 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     # few positions: room for cells that is no multiple of eight
     (torch.bfloat16, False, 32, 4, [(8, 8)], 1, 32771, 8),
     (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
-    # enough points for runs of all four lengths (the ones above have short runs only)
+    # enough points for runs of all three lengths (the ones above have runs of one length only)
     (torch.bfloat16, False, 16, 4, [(60, 60), (30, 30)], 2, 27011, 8),
     # 12 000 positions and more are sorted a level at a time: point counts that leave threads idle, tiny
     # levels, one level, and one with more cells than a turn has room for
@@ -243,3 +243,23 @@ def test_unsorted_points_of_large_planes(levels, overlap):
         fine = torch.isfinite(y)
         assert torch.equal(torch.isfinite(x), fine)
         assert rel_err(to_np(x[fine]), to_np(y[fine])) <= bar
+
+
+@pytest.mark.parametrize("levels,B,Q,K", [
+    ([(40, 54), (20, 27), (10, 14), (5, 7)], 12, 2870, 4),       # runs of two lengths, plane after plane
+    ([(5, 7), (10, 14), (20, 27), (40, 54)], 5, 2870, 4),        # of three in every plane, the finest level last
+    ([(32, 32), (16, 16), (8, 8)], 2, 8192, 8),                  # the same, hundreds of points a pixel
+])
+def test_every_plane_is_as_accurate(levels, B, Q, K):
+    """The error of grad_value must not depend on where in the batch a sample stands.  What the planes
+    differ in is how many sums meet in float16: no plane is cut into more than twice the runs of
+    another, and rounding errors add in squares, so theirs differ by sqrt(2) at most."""
+    G, D = 8, 32
+    value, shapes, starts, loc, logits, grad_out = _inputs(12, B, Q, G, D, K, levels, spread=0.1)
+    dtype = torch.float16
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(grad_out, dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = to_np(_workspace_backward(v, sh, st, l, a, go, False)[0])
+    truth = orc.backward(*[t.cpu() for t in (v, sh, st, l, a)], go.cpu(), softmax=False)[0]
+    error = (((got - truth) ** 2).sum((1, 3)) / (truth ** 2).sum((1, 3))) ** 0.5
+    assert error.max() <= 2 ** 0.5 * error.min(), error
