@@ -1539,6 +1539,21 @@ void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
     sp.all_runs = runs;
 }
 
+// Room for the cells of one level.  A level has one per five to seven positions; the finest of several that
+// halve has three quarters to four fifths of the plane's, which S / 8 holds, but one of nine tenths or
+// more needs S / 5.  It is given that up to `most`, as long as it takes no L1 from the loads (us, backward,
+// B200, S / 8 -> this: 128x128 + 32x32 267.9 -> 263.6, of 16 points a position 219.6 -> 211.5, 150x150 + 38x38
+// 342 -> 332; with S / 5 always, 398 -> 401 at the headline shape, whose levels fit either way, and 271 -> 307 of
+// four levels of 42 500 positions).  The scatter of a level beyond its room, which leaves unordered, is no
+// slower than one with that much less L1: 332 and 338 of 150x150 + 38x38, 301 and 308 of 192x192 + 48x48.
+constexpr int kLevelRoom = 3280;       // two scatter CTAs take 132 KB, a step of what the SM can set aside
+constexpr int kCountRoom = 3760;       // eight counting CTAs take as much
+int level_room(const Params &p, int cell_bound, int most) {
+    const int64_t several = p.S / 8 + 256, one = p.S / 5 + 256;
+    const int64_t cells = p.L == 1 ? one : std::max(several, std::min<int64_t>(one, most));
+    return (int)std::min<int64_t>(kLevelCells, round_up(std::min<int64_t>(cell_bound, cells), 8));
+}
+
 int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples, void *workspace) {
     const int64_t P = (int64_t)p.L * p.K;
     const int64_t planes = samples * p.G;
@@ -1568,11 +1583,8 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     sp.level_queries = (int)(kLevelThreads / p.K * kLevelPoints);
     sp.level_stretches = sp.scatter_by_level ? (int)((p.Q + sp.level_queries - 1) / sp.level_queries) : 0;
     sp.level_turns = (unsigned)(planes * p.L * sp.level_stretches);
-    // (the finest of several levels has four fifths of the positions; the counting kernel's CTAs per
-    // SM need the room)
-    sp.level_cells = (int)std::min<int64_t>(
-        kLevelCells, round_up(std::min<int64_t>(sp.cell_bound, p.L > 1 ? p.S / 8 + 256 : p.S / 5 + 256), 8));
-    sp.count_cells = sp.count_by_level ? sp.level_cells : sp.shared_cells;
+    sp.level_cells = level_room(p, sp.cell_bound, kLevelRoom);
+    sp.count_cells = sp.count_by_level ? level_room(p, sp.cell_bound, kCountRoom) : sp.shared_cells;
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
     plan_runs(sp, p, planes);
     char *at = static_cast<char *>(workspace);
