@@ -98,7 +98,7 @@ int plan(msda_b200::Params &p, int64_t B, int64_t S, int64_t G, int64_t D, int64
     while (p.threads > 32 && (msda_b200::backward_smem_bytes(p, softmax) > kSmemBudget ||
                               msda_b200::forward_smem_bytes(p, softmax) > kSmemBudget))
         p.threads >>= 1;
-    if (msda_b200::backward_smem_bytes(p, softmax) > 200 * 1024)
+    if (msda_b200::backward_smem_bytes(p, softmax) > msda_b200::kMostSmem)
         return fail(MSDA_B200_UNSUPPORTED, "L*K = %d is too large for the shared-memory staging", P);
     const int nwarps = p.threads / 32;
     p.num_groups = (B * Q * G + ppw - 1) / ppw;

@@ -476,8 +476,7 @@ cudaError_t launch_kernel(const Params &p, cudaStream_t stream) {
     const size_t smem = backward_smem_bytes(p, SOFTMAX);
     auto kernel = backward_kernel<T, SOFTMAX, SCALED, false>;
     if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
-        cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_most_smem(kernel);
         if (e != cudaSuccess) return e;
     }
     // Two adjacent passes per CTA once that still leaves every SM several waves of CTAs
@@ -501,8 +500,7 @@ cudaError_t launch_fused(const Params &p, cudaStream_t stream) {
     const size_t smem = backward_smem_bytes(p, SOFTMAX);
     auto kernel = backward_kernel<T, SOFTMAX, true, true>;
     if (smem > kPlainSmem) {
-        cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_most_smem(kernel);
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaMemsetAsync(p.fused_header, 0, kFusedBytes, stream);

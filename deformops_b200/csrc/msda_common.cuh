@@ -277,6 +277,14 @@ inline cudaError_t launch_after_predecessor(Kernel kernel, unsigned grid, unsign
 // Shared memory a kernel may ask for without opting in, beside the level table and the like that
 // these kernels hold statically.
 constexpr size_t kPlainSmem = 46 * 1024;
+// The most any call asks for (more than this is refused).  A kernel that may need more than kPlainSmem is
+// always allowed all of it: with the size of the call at hand, two host threads whose calls differ
+// would lower each other's limit between setting it and launching, and the launch would be refused.
+constexpr size_t kMostSmem = 200 * 1024;
+template <typename Kernel>
+inline cudaError_t allow_most_smem(Kernel kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem);
+}
 
 // CTAs of a kernel the GPU holds at once for a block size and a shared memory size.  The runtime is
 // asked once per combination (a query costs the host about as much as a launch).  Every GPU this

@@ -363,8 +363,7 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     const size_t smem = forward_smem_bytes(p, SOFTMAX);
     auto kernel = forward_kernel<T, SOFTMAX, REF, SMALL, Index>;
     if (smem > kPlainSmem) {  // opt in to large dynamic shared memory only when needed
-        cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_most_smem(kernel);
         if (e != cudaSuccess) return e;
     }
     // Persistent CTAs: launch no more CTAs than the GPU holds at once and let each walk the

@@ -1386,14 +1386,14 @@ cudaError_t launch_sorted_typed(const Params &p, const SortPlan &sp, cudaStream_
         auto by_level = p.ref != nullptr ? sort_scatter_level_kernel<T, SOFTMAX, true>
                                          : sort_scatter_level_kernel<T, SOFTMAX, false>;
         const size_t smem = (size_t)kLevelTurn * 18 + (size_t)sp.level_cells * 6;
-        e = cudaFuncSetAttribute(by_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_most_smem(by_level);
         if (e != cudaSuccess) return e;
         static Residency residency[2];
         const unsigned resident = residency[p.ref != nullptr].ctas(by_level, kLevelThreads, smem);
         e = launch_after_predecessor(by_level, resident == 0 ? sp.level_turns : std::min(resident, sp.level_turns),
                                      kLevelThreads, smem, stream, p, sp);
     } else {
-        e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem);
+        e = allow_most_smem(scatter);
         if (e != cudaSuccess) return e;
         e = launch_after_predecessor(scatter, planes * (unsigned)sp.chunks, kSortThreads, scatter_smem, stream, p, sp);
     }

@@ -263,3 +263,46 @@ def test_every_plane_is_as_accurate(levels, B, Q, K):
     truth = orc.backward(*[t.cpu() for t in (v, sh, st, l, a)], go.cpu(), softmax=False)[0]
     error = (((got - truth) ** 2).sum((1, 3)) / (truth ** 2).sum((1, 3))) ** 0.5
     assert error.max() <= 2 ** 0.5 * error.min(), error
+
+
+def test_threads_with_different_planes_do_not_limit_each_other():
+    """Calls of two pyramids from two host threads: the kernels' allowance for shared memory, which belongs
+    to the device's context, must do for both whenever either is launched."""
+    import threading
+
+    from deformops_b200._loader import load_library
+
+    shim = load_library()
+    B, G, D, K = 1, 8, 16, 4
+    failed = []
+
+    def worker(levels, Q, seed):
+        torch.cuda.set_device(0)
+        value, shapes, starts, loc, logits, grad_out = _inputs(seed, B, Q, G, D, K, levels)
+        L, S = len(levels), value.shape[1]
+        v, a, go = (dev(t, torch.bfloat16) for t in (value, logits.softmax(-1), grad_out))
+        l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+        grads = [torch.empty_like(t) for t in (v, l, a)]
+        nbytes = shim.workspace_bytes(B, S, G, D, Q, L, K, 2, 0)
+        if nbytes <= shim.scratch_bytes(B, S, G, D, Q, L, K, 2):
+            failed.append("the scratch is the plain one")
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        args = (_p(v), _p(sh), _p(st), _p(l), _p(a), _p(go), *[_p(t) for t in grads], _p(scratch), nbytes,
+                0, B, S, G, D, Q, L, K, 2, 0, 1, 0, ctypes.c_void_p(stream.cuda_stream))
+        for _ in range(60):
+            barrier.wait()          # both threads enqueue at the same time, and neither waits for the GPU
+            for _ in range(50):
+                if shim.backward(*args):
+                    failed.append(shim.last_error())
+            stream.synchronize()
+
+    # with and without a level at a time, two sizes of each
+    for small, large in (([(60, 60)], [(75, 100)]), ([(110, 110)], [(125, 125)])):
+        barrier = threading.Barrier(2, timeout=60)
+        threads = [threading.Thread(target=worker, args=(levels, 33000, i)) for i, levels in enumerate((small, large))]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+    assert not failed, (len(failed), failed[0])
