@@ -700,6 +700,7 @@ constexpr int kLevelPoints = 8;        // points per thread and turn,
 constexpr int kLevelBatch = 4;         // loaded this many at a time
 constexpr int kLevelTurn = kLevelThreads * kLevelPoints;
 constexpr int kLevelCells = 10752;     // most cells of a level, so that two CTAs fit an SM
+constexpr int kCountRoom = 3760;       // cells that any level may have in the counting kernel (plan_sorted)
 static_assert(3 * kLevelPoints <= 32, "the columns of a thread's points share a word");
 template <typename T, bool SOFTMAX, bool REF>
 __global__ void __launch_bounds__(kLevelThreads, 2) sort_scatter_level_kernel(const __grid_constant__ Params p,
@@ -1492,22 +1493,26 @@ int64_t sorted_workspace_bytes(const Params &p, bool softmax, int64_t samples) {
 
 // Runs of the walk.  Where a run ends, the sums of two pixel rows leave it unfinished and meet in float16
 // once more.  So no plane is in more runs than if all had `length` points: 128 to 256, by what a warp's
-// share leaves room for, and more where a pixel collects thousands of points.  Within that, a long run is
+// share leaves room for, and more where a pixel collects hundreds of points.  Within that, a long run is
 // flushed and started less often, but the last ones to end leave the other warps idle:
-//   six runs of `length` and more a warp   twice the length, until two of `length` are left for every
+//   six runs of `length` and more a warp   twice the length, until four of `length` are left for every
 //                                 warp (planes in order: what a plane's levels share stays in L2)
 //   two to six, or 64 channels    every plane has some of twice, of once and of half the length: the long
 //                                 ones are handed out first, the short ones lie on its finest level, where
 //                                 the fewest points share a pixel.  That costs L2 hits (1024 pixels, 2 samples,
 //                                 6.8 runs a warp: 232 us against 222), but less than a nearly empty last
 //                                 round of whole runs
-//   fewer                         all of `length`
-// Backward, B200, us, all of `length` -> this: headline shape 408 -> 401, 16 samples 1616 -> 1578, four odd
-// levels in float16 431 -> 419, 512-pixel pyramid 8 samples 223 -> 220, 4 samples 134 -> 127; 64 channels:
-// ragged pyramid with offsets 207 -> 193, 512 pixels 16 samples 295 -> 269.  Runs of 512 points getting
-// shorter to 64 in the order of the planes: 399, 1575, 412, 217, 124, 196, 274, but the last plane's
-// float16 grad_value was 5.6e-4 off and the first's 3.6e-4 where all are 3.6e-4 to 4.0e-4 now (four odd
-// levels 8.1e-4 and 4.2e-4; now 4.2e-4 to 5.0e-4)
+//   fewer, or hundreds of points a pixel   all of `length`
+// Backward, B200, us, all of `length` -> this: headline shape 403 -> 398, 16 samples 1598 -> 1572, four odd
+// levels in float16 429 -> 421, 27 750 positions 401 -> 392, 512-pixel pyramid 8 samples 221 -> 221, 4 samples
+// 134 -> 126; 64 channels: ragged pyramid with offsets 206 -> 192, 512 pixels 16 samples 295 -> 268.  (Two runs
+// of `length` left instead of four: 398, 1571, 420, 389, 220, but 277 instead of 252 at 120x120 + 30x30,
+// whose strips are seven runs of 512 points, and 310 instead of 296 with 60x60 between them.)
+// Runs of 512 points getting shorter to 64 in the order of the planes: 393, 1563, 413, 399, 212, 122, 195,
+// 274, but the float16 grad_value of the last plane was 5.6e-4 off and of the first 3.6e-4, where they are
+// 4.0e-4 and 3.6e-4 now and 4.0e-4 with one length (four odd levels 8.1e-4 and 4.2e-4; now 5.1e-4 and
+// 4.2e-4; 5.0e-4).  With short runs in every plane it is nine tenths of that with one length, a twentieth
+// more on the finest level alone.
 void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
     const int64_t warps = 148 * kWalkWarps * walk_ctas(p.D);
     const int64_t share = planes * sp.plane_points / (148 * 16 * 4), density = sp.plane_points / std::max<int64_t>(p.S, 1);
@@ -1519,8 +1524,8 @@ void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
     int64_t whole = 0;             // planes of long runs only
     int64_t spread = 0;            // runs of `length` of every plane beside its long and short ones
     if (units >= 12 * warps && p.D < 64)
-        whole = std::max<int64_t>(0, planes - (4 * warps + sp.items - 1) / sp.items);
-    else if (units >= 4 * warps)
+        whole = std::max<int64_t>(0, planes - (8 * warps + sp.items - 1) / sp.items);
+    else if (units >= 4 * warps && density < 128)
         spread = std::min((warps + planes - 1) / planes, (int64_t)(sp.items - 4) / 8);   // (items / 2 - 1 runs at most)
     unsigned runs = 0;
     auto add = [&](int kind, int64_t plane, int64_t of_planes, int64_t unit, int64_t each, int log2_size) {
@@ -1537,21 +1542,6 @@ void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
         add(2, planes, 0, 0, 0, 0);
     }
     sp.all_runs = runs;
-}
-
-// Room for the cells of one level.  A level has one per five to seven positions; the finest of several that
-// halve has three quarters to four fifths of the plane's, which S / 8 holds, but one of nine tenths or
-// more needs S / 5.  It is given that up to `most`, as long as it takes no L1 from the loads (us, backward,
-// B200, S / 8 -> this: 128x128 + 32x32 267.9 -> 263.6, of 16 points a position 219.6 -> 211.5, 150x150 + 38x38
-// 342 -> 332; with S / 5 always, 398 -> 401 at the headline shape, whose levels fit either way, and 271 -> 307 of
-// four levels of 42 500 positions).  The scatter of a level beyond its room, which leaves unordered, is no
-// slower than one with that much less L1: 332 and 338 of 150x150 + 38x38, 301 and 308 of 192x192 + 48x48.
-constexpr int kLevelRoom = 3280;       // two scatter CTAs take 132 KB, a step of what the SM can set aside
-constexpr int kCountRoom = 3760;       // eight counting CTAs take as much
-int level_room(const Params &p, int cell_bound, int most) {
-    const int64_t several = p.S / 8 + 256, one = p.S / 5 + 256;
-    const int64_t cells = p.L == 1 ? one : std::max(several, std::min<int64_t>(one, most));
-    return (int)std::min<int64_t>(kLevelCells, round_up(std::min<int64_t>(cell_bound, cells), 8));
 }
 
 int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples, void *workspace) {
@@ -1583,8 +1573,19 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     sp.level_queries = (int)(kLevelThreads / p.K * kLevelPoints);
     sp.level_stretches = sp.scatter_by_level ? (int)((p.Q + sp.level_queries - 1) / sp.level_queries) : 0;
     sp.level_turns = (unsigned)(planes * p.L * sp.level_stretches);
-    sp.level_cells = level_room(p, sp.cell_bound, kLevelRoom);
-    sp.count_cells = sp.count_by_level ? level_room(p, sp.cell_bound, kCountRoom) : sp.shared_cells;
+    // A level has a cell per five to seven positions; the finest of several that halve has four fifths of the
+    // positions, the one of two may have nine tenths.  Room for more than the former takes L1 from the loads
+    // (S / 5 in both kernels: headline shape 398 -> 401, four levels of 42 500 positions 271 -> 307), but for
+    // kCountRoom in the counting kernel: eight CTAs take 132 KB then, a step of what an SM can set aside, as
+    // they do at the headline shape (128x128 + 32x32 of 16 points a position 220 -> 211, 150x150 + 38x38
+    // 342 -> 332).  The scatter is no faster for it: a level beyond its room leaves unordered, 128x128 + 32x32
+    // at 259 us, in order 260; 140x140 + 35x35 352, 357; 192x192 + 48x48 301, 308
+    auto room = [&](int64_t least) {
+        const int64_t cells = p.L > 1 ? std::max(p.S / 8 + 256, least) : p.S / 5 + 256;
+        return (int)std::min<int64_t>(kLevelCells, round_up(std::min<int64_t>(sp.cell_bound, cells), 8));
+    };
+    sp.level_cells = room(0);
+    sp.count_cells = sp.count_by_level ? room(std::min<int64_t>(kCountRoom, p.S / 5 + 256)) : sp.shared_cells;
     sp.cell_stride = round_up(sp.cell_bound + 1, 32);
     plan_runs(sp, p, planes);
     char *at = static_cast<char *>(workspace);
