@@ -72,13 +72,17 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     # few positions: room for cells that is no multiple of eight
     (torch.bfloat16, False, 32, 4, [(8, 8)], 1, 32771, 8),
     (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
-    # enough points for runs of all three lengths (the ones above have runs of one length only)
+    # runs of three lengths in every plane; of two, plane after plane (above: of three, or of one length)
     (torch.bfloat16, False, 16, 4, [(60, 60), (30, 30)], 2, 27011, 8),
+    (torch.bfloat16, True, 16, 4, [(60, 60), (30, 30)], 2, 35011, 8),
     # 12 000 positions and more are sorted a level at a time: point counts that leave threads idle, tiny
     # levels, one level, and one with more cells than a turn has room for
     (torch.bfloat16, False, 32, 3, [(110, 113), (3, 5), (1, 1)], 1, 12001, 10),
     (torch.float16, True, 16, 5, [(125, 100)], 3, 20011, 4),
     (torch.bfloat16, True, 64, 8, [(6500, 2), (10, 10)], 1, 7001, 10),
+    # the largest room for a level's cells (10 122 of 10 752), larger levels first and last
+    (torch.bfloat16, False, 64, 8, [(240, 290), (120, 145)], 1, 43501, 2),
+    (torch.float16, True, 64, 8, [(120, 145), (240, 290)], 1, 43501, 2),
     # more cells than a CTA counts in shared memory: narrow levels
     (torch.bfloat16, False, 32, 4, [(3000, 2)], 1, 13000, 20),
 ])
