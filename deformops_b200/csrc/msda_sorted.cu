@@ -21,9 +21,9 @@
 // eight channels, instead of once per corner and point (at 21 504 queries and 12 points per query
 // 33 million rows of reductions become about 1 million).
 //
-// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 394 us
-// against 512 us, of which counting 44, writing records 92, the walk 237, the last pass 22;
-// grad_value 1.7e-3 off the float32 result against 2.2e-3.
+// Measured at the headline shape (4 x 21 504 queries, 8.3 M points, bf16): backward call 398 us
+// against 512 us, of which counting 42, writing records 92, the walk 243, the last pass 22, each by itself;
+// grad_value 1.72e-3 off the float64 result, most of it bfloat16's own rounding (float16: 3.7e-4).
 //
 // Accumulation is float32 inside a warp's run of points; the few sums that meet in memory (two
 // strips share a column, two runs share a row) meet in float16, scaled as in the direct backward
@@ -336,9 +336,11 @@ __device__ __forceinline__ void scan_plane(unsigned *counts, unsigned *offsets, 
 //
 // BY_LEVEL: a CTA takes the points that a stretch of queries has on one level (levels vary after heads):
 // its cells are a level's only, so that a stretch can be longer and the counts of a cell are merged less
-// often (headline shape 53 -> 46 us, 512-pixel pyramid 26.5 -> 24, four odd levels 52 -> 48).  Offsets,
-// half as long and evaluated at more expense, are better off with all levels of a query side by side
-// (ragged pyramid 29 us against 38).
+// often.  Backward, B200, us, all levels -> this: headline shape 404 -> 398, 512 pixels 8 samples 224 -> 221,
+// four odd levels in float16 422 -> 418, 59 104 positions (2 samples, 4 x 64 channels) 487 -> 416; 1, 2 and 8
+// points a level of 14 196 positions 593 -> 591, 527 -> 522, 440 -> 428.  Offsets, half as long and evaluated
+// at more expense, are better off with all levels of a query side by side (ragged pyramid, this kernel 29
+// us against 38).
 __host__ __device__ constexpr int count_threads(bool by_level) { return by_level ? 256 : kSortThreads; }
 template <typename T, bool SOFTMAX, bool REF, bool BY_LEVEL>
 __global__ void __launch_bounds__(count_threads(BY_LEVEL), 2048 / count_threads(BY_LEVEL))
@@ -691,10 +693,13 @@ __global__ void __launch_bounds__(kSortThreads, 2) sort_scatter_kernel(const __g
 // fractions and weights stay in registers until their place in the turn's order is known: few threads
 // with many registers, and persistent CTAs.  Bound by the latency of its phases (load/store pipe 62 %
 // busy, issue slots 43 %, DRAM 40 %).
-// Backward, B200, us, all levels -> this: headline shape 410 -> 394, random locations 433 -> 415, four
-// odd levels in float16 423 -> 414, 27 776 positions 447 -> 404, 42 500 301 -> 280, 58 968 of 64 channels
-// 503 -> 416.  (320 threads of 96 registers; 256 x 3 of 80: 428 for 394; 384 of 80 and six points 400;
-// 512 of 64, which spill, 412; without registers, as above, 256 x 3 407.)
+// Backward, B200, us, all levels -> this (4 points a level of 8 x 32 channels unless said): headline shape
+// 414 -> 398, queries anywhere 437 -> 419, four odd levels in float16 427 -> 418, 2 samples of 27 750 positions
+// on five levels 440 -> 396, one of 42 500 on four 296 -> 274, 2 of 59 104 with 4 x 64 channels 496 -> 416;
+// 14 196 positions with 1, 2 and 8 points a level 618 -> 590, 545 -> 522, 442 -> 428: one line of memory per
+// query and load is no loss with few points either.  (320 threads of 96 registers; when it took 394 us: 256 x 3
+// of 80: 428; 384 of 80 and six points 400; 512 of 64, which spill, 412; without registers, as above, 256 x 3
+// 407.)
 constexpr int kLevelThreads = 320;
 constexpr int kLevelPoints = 8;        // points per thread and turn,
 constexpr int kLevelBatch = 4;         // loaded this many at a time
@@ -939,12 +944,12 @@ __device__ __forceinline__ void flush_row(float (&acc)[D / 8][4], int half, floa
     }
 }
 
-// What bounds the walk is the SM's load/store pipe, about five of its cycles a point (ncu, the
-// headline shape: 64 % busy while the SM works, issue slots 50 %, tensor cores 24 %): the two
-// stores per point to addresses of their own take 45 us of 237, the grad_out rows 27, the rest
-// goes through shared memory.  Hence the weights' way over the tensor cores below.  More warps do
-// not help - 12, 16, 20, 24 per SM: 252, 246, 261, 312 us - nor does having grad_out rows in
-// registers instead of shared memory (300 us), or the next cell's value row early (257 us).
+// What bounds the walk is the latency of a step's chain beside the SM's load/store pipe, about five of its
+// cycles a point (ncu, the headline shape: 67 % busy while the SM works, issue slots 49 %, tensor cores
+// 30 %): without the two stores per point to addresses of their own the call takes 364 us instead of 398,
+// the rest goes through shared memory.  Hence the weights' way over the tensor cores below.  More warps do
+// not help - 12, 16, 20, 24 per SM: 252, 246, 261, 312 us when this kernel took 246 - nor did having grad_out
+// rows in registers instead of shared memory (300 us), or the next cell's value row early (257 us).
 // (CTAs per SM the registers are held to: more than these spill)
 constexpr int walk_ctas(int D) { return D == 64 ? 3 : 4; }
 __host__ __device__ constexpr int walk_warp_bytes(int D) { return 2 * kStep * D * 2 + kStep * 16 + kStep / 8 * 512; }
@@ -1010,6 +1015,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
     // the identity as the A operand of an m16n8k16 product (upper left and lower right corner)
     const uint32_t one = VT::pack2(make_float2(j == 2 * c ? 1.f : 0.f, j == 2 * c + 1 ? 1.f : 0.f));
 
+    // (short runs belong on the finest level)
     const bool coarse_first = lt.H[p.L - 1] * lt.W[p.L - 1] > lt.H[0] * lt.W[0];
     // ---- runs of places, handed out as the warps come for them
     for (;;) {
@@ -1017,11 +1023,13 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_ctas(D))
         if (lane == 0) run = atomicAdd(sp.header + kNextItem, 1u);
         run = __shfl_sync(0xffffffffu, run, 0);
         if (run >= sp.all_runs) break;
-        const WalkRuns &kind = sp.runs[run < sp.runs[1].run0 ? 0 : run < sp.runs[2].run0 ? 1 : 2];
+        int k = 0;
+#pragma unroll
+        for (int i = 1; i < kRunKinds; ++i) k += run >= sp.runs[i].run0;
+        const WalkRuns &kind = sp.runs[k];
         const unsigned nth = (run - kind.run0) / kind.each;
         const int plane = (int)(kind.plane0 + nth);
         unsigned unit = kind.unit0 + ((run - kind.run0 - nth * kind.each) << kind.log2_size);
-        // (short runs belong on the finest level)
         if (coarse_first) unit = (unsigned)sp.items - unit - (1u << kind.log2_size);
         int pos = (int)unit * sp.item_points;
         const uint4 *records = sp.records + (int64_t)plane * sp.plane_points;
@@ -1431,13 +1439,14 @@ int64_t round_up(int64_t n, int64_t to) { return (n + to - 1) / to * to; }
 //   offsets instead of          the arithmetic of the locations is done once more: 16 channels
 //   locations                   228 -> 251, 32: 157 -> 159 at 2 M points, 285 -> 275 at 4 M, 551
 //                               -> 503 at 8 M; 64 (1.8 M points): 241 -> 202
-//   positions                   12 points per position, 58 968 positions: 16 channels 591 -> 577, 32: 697
-//                               -> 640; 73 500: 740 -> 766, 880 -> 857; 16 points on four levels 1149 ->
-//                               1040.  From about 85 000 the finest level has more than kLevelCells
-//                               cells and its records leave unordered: 100 000 553 -> 677, 621 -> 765,
-//                               134 400 719 -> 850, 806 -> 905.  The line lies below, at 55 000, where what is
-//                               left to gain, 3 to 8 %, is not worth three times the scratch, but for
-//                               64 channels (331 -> 251 at 58 968) and 24 points of 32 (923 -> 686 at 73 500).
+//   positions                   12 points per position, 2 samples, 59 104 positions: 16 channels 590 -> 574,
+//                               32: 696 -> 635; 73 549: 739 -> 775, 880 -> 866; 16 points on four levels
+//                               1148 -> 1033.  From about 85 000 the finest level has more than kLevelCells
+//                               cells and its records leave unordered, one sample: 102 900 552 -> 668, 620 ->
+//                               757, 134 400 720 -> 840, 805 -> 900.  The line lies below, at 55 000, where
+//                               what is left to gain, 2 to 10 %, is not worth three times the scratch, but for
+//                               64 channels (4 heads, 12 points, 59 104: one sample 308 -> 224, two 599 ->
+//                               416) and 24 points of 32 (73 549: one sample 912 -> 679, two 1805 -> 1359).
 //                               Offsets: more than kSharedCells cells from there on
 bool sorting_pays(const Params &p, int dtype, bool offsets) {
     const int64_t P = (int64_t)p.L * p.K, points = p.B * p.G * p.Q * P;
@@ -1493,53 +1502,47 @@ int64_t sorted_workspace_bytes(const Params &p, bool softmax, int64_t samples) {
 
 // Runs of the walk.  Where a run ends, the sums of two pixel rows leave it unfinished and meet in float16
 // once more.  So no plane is in more runs than if all had `length` points: 128 to 256, by what a warp's
-// share leaves room for, and more where a pixel collects hundreds of points.  Within that, a long run is
-// flushed and started less often, but the last ones to end leave the other warps idle:
-//   six runs of `length` and more a warp   twice the length, until four of `length` are left for every
-//                                 warp (planes in order: what a plane's levels share stays in L2)
-//   two to six, or 64 channels    every plane has some of twice, of once and of half the length: the long
-//                                 ones are handed out first, the short ones lie on its finest level, where
-//                                 the fewest points share a pixel.  That costs L2 hits (1024 pixels, 2 samples,
-//                                 6.8 runs a warp: 232 us against 222), but less than a nearly empty last
-//                                 round of whole runs
-//   fewer, or hundreds of points a pixel   all of `length`
-// Backward, B200, us, all of `length` -> this: headline shape 403 -> 398, 16 samples 1598 -> 1572, four odd
-// levels in float16 429 -> 421, 27 750 positions 401 -> 392, 512-pixel pyramid 8 samples 221 -> 221, 4 samples
-// 134 -> 126; 64 channels: ragged pyramid with offsets 206 -> 192, 512 pixels 16 samples 295 -> 268.  (Two runs
-// of `length` left instead of four: 398, 1571, 420, 389, 220, but 277 instead of 252 at 120x120 + 30x30,
-// whose strips are seven runs of 512 points, and 310 instead of 296 with 60x60 between them.)
-// Runs of 512 points getting shorter to 64 in the order of the planes: 393, 1563, 413, 399, 212, 122, 195,
-// 274, but the float16 grad_value of the last plane was 5.6e-4 off and of the first 3.6e-4, where they are
-// 4.0e-4 and 3.6e-4 now and 4.0e-4 with one length (four odd levels 8.1e-4 and 4.2e-4; now 5.1e-4 and
-// 4.2e-4; 5.0e-4).  With short runs in every plane it is nine tenths of that with one length, a twentieth
-// more on the finest level alone.
+// share leaves room for, and more where a pixel collects hundreds of points (all have it there, and where
+// there are fewer than two for every warp).  Within that, a long run is flushed and started less often, but
+// the last ones to end leave the other warps idle: runs have twice the length, and the last planes - all
+// planes of a small call - have some of once and of half of it too, together one and two for every warp.
+// Of these planes the long runs are handed out first; the short ones lie on their finest level, where the
+// fewest points share a pixel.
+// Backward, B200, us, all of `length` -> this: headline shape 408 -> 398, 16 samples 1618 -> 1571, four odd
+// levels in float16 430 -> 415, 512-pixel pyramid 8 samples 224 -> 215, with offsets 271 -> 258, 4 samples 135
+// -> 127; 64 channels: ragged pyramid with offsets 208 -> 194, 512 pixels 16 samples 298 -> 270.  Which planes:
+// eight runs' worth of them for every warp (sixteen: 415 at the headline shape, all 431: what a plane's levels
+// share is no longer in L2 when its short runs come), but sixteen at 64 channels (eight: 198, 277).  No short
+// runs, four of `length` left for every warp: 402, 1586, 423, 223, 271.
+// Runs of 512 points getting shorter to 64 in the order of the planes take 399, 1579, 413, 217, 258, 124,
+// 196, 276, but the float16 grad_value of the last plane is 5.6e-4 off then and of the first 3.6e-4 (four
+// odd levels 8.2e-4 and 4.2e-4), where they are 3.7e-4 and 3.6e-4 (4.3e-4, 4.2e-4) with these runs and 4.0e-4
+// (5.0e-4) with all of `length`.
 void plan_runs(SortPlan &sp, const Params &p, int64_t planes) {
     const int64_t warps = 148 * kWalkWarps * walk_ctas(p.D);
-    const int64_t share = planes * sp.plane_points / (148 * 16 * 4), density = sp.plane_points / std::max<int64_t>(p.S, 1);
+    const int64_t share = planes * sp.plane_points / (148 * 16 * 4);
+    const int64_t density = sp.plane_points / std::max<int64_t>(p.S, 1);
     const int64_t length = std::min<int64_t>(256, std::max<int64_t>(128, share / 32 * 32)) *
                            std::min<int64_t>(16, 1 + density / 128);
     sp.item_points = (int)(length / 2);
     sp.items = (int)round_up((sp.plane_points + sp.item_points - 1) / sp.item_points, 4);   // (no run in two planes)
-    const int64_t units = planes * sp.items;
-    int64_t whole = 0;             // planes of long runs only
-    int64_t spread = 0;            // runs of `length` of every plane beside its long and short ones
-    if (units >= 12 * warps && p.D < 64)
-        whole = std::max<int64_t>(0, planes - (8 * warps + sp.items - 1) / sp.items);
-    else if (units >= 4 * warps && density < 128)
-        spread = std::min((warps + planes - 1) / planes, (int64_t)(sp.items - 4) / 8);   // (items / 2 - 1 runs at most)
     unsigned runs = 0;
-    auto add = [&](int kind, int64_t plane, int64_t of_planes, int64_t unit, int64_t each, int log2_size) {
-        sp.runs[kind] = {runs, (unsigned)plane, (unsigned)std::max<int64_t>(each, 1), (unsigned)unit, log2_size};
+    int kind = 0;
+    auto add = [&](int64_t plane, int64_t of_planes, int64_t unit, int64_t each, int log2_size) {
+        sp.runs[kind++] = {runs, (unsigned)plane, (unsigned)std::max<int64_t>(each, 1), (unsigned)unit, log2_size};
         runs += (unsigned)(of_planes * each);
     };
-    if (spread > 0) {              // 2 * spread units in short runs, as many in runs of `length`
-        add(0, 0, planes, 4 * spread, sp.items / 4 - spread, 2);
-        add(1, 0, planes, 2 * spread, spread, 1);
-        add(2, 0, planes, 0, 2 * spread, 0);
+    if (planes * sp.items >= 4 * warps && density < 128) {
+        const int64_t mixed = std::min(planes, ((p.D == 64 ? 16 : 8) * warps + sp.items - 1) / sp.items);
+        // (in each n runs of `length`, 2 * n of half and items / 4 - n of twice that: items / 2 - 1 at most)
+        const int64_t n = std::min((warps + mixed - 1) / mixed, (int64_t)(sp.items - 4) / 8);
+        add(0, planes - mixed, 0, sp.items / 4, 2);
+        add(planes - mixed, mixed, 4 * n, sp.items / 4 - n, 2);
+        add(planes - mixed, mixed, 2 * n, n, 1);
+        add(planes - mixed, mixed, 0, 2 * n, 0);
     } else {
-        add(0, 0, whole, 0, sp.items / 4, 2);
-        add(1, whole, planes - whole, 0, sp.items / 2, 1);
-        add(2, planes, 0, 0, 0, 0);
+        add(0, planes, 0, sp.items / 2, 1);
+        while (kind < kRunKinds) add(planes, 0, 0, 0, 0);
     }
     sp.all_runs = runs;
 }
@@ -1566,9 +1569,9 @@ int64_t plan_sorted(SortPlan &sp, const Params &p, bool softmax, int64_t samples
     // a pyramid of ordinary proportions has a cell per five to six pixels (whole eights: the scatter
     // takes cells by eights, in 16-byte accesses to arrays that follow one another)
     sp.shared_cells = (int)std::min<int64_t>(kSharedCells, round_up(std::min<int64_t>(sp.cell_bound, p.S / 5 + 256), 8));
-    // (backward, us, all levels -> by level: 5 376 positions 210.6 -> 213.7, 8 400 300 -> 304, 11 192 223.3 ->
-    // 224, 14 196 280 -> 273, 18 900 of 16 channels 317 -> 309; offsets: 14 196 211 -> 218, 21 504 497 -> 502,
-    // 27 900, where the other kernel has one CTA per SM only, 599 -> 534, 42 500 382 -> 345)
+    // (backward, us, all levels -> by level: 5 376 positions, 8 samples 221 -> 224, 8 400, 4 samples 167 -> 170,
+    // 14 196 270 -> 264; offsets: 14 196 323 -> 335, 21 504 497 -> 499, 27 750, 2 samples, where the other
+    // kernel has one CTA per SM only, 584 -> 519, 42 500, one sample 369 -> 332)
     sp.scatter_by_level = p.K <= kLevelThreads && p.S >= (p.ref != nullptr ? 26000 : 12000);
     sp.level_queries = (int)(kLevelThreads / p.K * kLevelPoints);
     sp.level_stretches = sp.scatter_by_level ? (int)((p.Q + sp.level_queries - 1) / sp.level_queries) : 0;

@@ -10,6 +10,8 @@ namespace msda_b200 {
 
 constexpr int kCols = 7;   // pixel columns (of the top left corner) of a cell
 
+constexpr int kRunKinds = 4;
+
 // Runs of one length: `each` in every plane from plane0 on, of 2^log2_size units, the first at unit0.
 struct WalkRuns {
     unsigned run0, plane0, each, unit0;
@@ -42,7 +44,7 @@ struct SortPlan {
     int count_ctas;                        // its CTAs per plane
     int prepare_ctas;        // CTAs of the counting kernel that prepare instead
     int item_points, items;  // places of a unit, units of a plane
-    WalkRuns runs[3];        // by the order they are handed out in
+    WalkRuns runs[kRunKinds];   // by the order they are handed out in
     unsigned all_runs;
 };
 

@@ -72,7 +72,7 @@ def _check(got, ins, grad_out, softmax, shapes, loc):
     # few positions: room for cells that is no multiple of eight
     (torch.bfloat16, False, 32, 4, [(8, 8)], 1, 32771, 8),
     (torch.float16, True, 64, 4, [(5, 3), (2, 2), (1, 1)], 2, 11003, 4),
-    # runs of three lengths in every plane; of two, plane after plane (above: of three, or of one length)
+    # runs of three lengths in every plane; in the last planes only
     (torch.bfloat16, False, 16, 4, [(60, 60), (30, 30)], 2, 27011, 8),
     (torch.bfloat16, True, 16, 4, [(60, 60), (30, 30)], 2, 35011, 8),
     # 12 000 positions and more are sorted a level at a time: point counts that leave threads idle, tiny
@@ -250,9 +250,9 @@ def test_unsorted_points_of_large_planes(levels, overlap):
 
 
 @pytest.mark.parametrize("levels,B,Q,K", [
-    ([(40, 54), (20, 27), (10, 14), (5, 7)], 12, 2870, 4),       # runs of two lengths, plane after plane
-    ([(5, 7), (10, 14), (20, 27), (40, 54)], 5, 2870, 4),        # of three in every plane, the finest level last
-    ([(32, 32), (16, 16), (8, 8)], 2, 8192, 8),                  # the same, hundreds of points a pixel
+    ([(40, 54), (20, 27), (10, 14), (5, 7)], 12, 2870, 4),       # short runs in the last planes only
+    ([(5, 7), (10, 14), (20, 27), (40, 54)], 5, 2870, 4),        # in every plane, the finest level last
+    ([(32, 32), (16, 16), (8, 8)], 2, 8192, 8),                  # runs of one length: hundreds of points a pixel
 ])
 def test_every_plane_is_as_accurate(levels, B, Q, K):
     """The error of grad_value must not depend on where in the batch a sample stands.  What the planes

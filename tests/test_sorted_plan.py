@@ -29,7 +29,7 @@ int main(int argc, char **argv) {
         plan_sorted(sp, p, n[8] != 0, p.B, nullptr);
         printf("{\"pays\": %d, \"unit\": %d, \"units\": %d, \"all_runs\": %u, \"runs\": [",
                (int)sorting_pays(p, 2, n[7] != 0), sp.item_points, sp.items, sp.all_runs);
-        for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < kRunKinds; ++k)
             printf("%s[%u, %u, %u, %u, %d]", k ? ", " : "", sp.runs[k].run0, sp.runs[k].plane0, sp.runs[k].each,
                    sp.runs[k].unit0, sp.runs[k].log2_size);
         printf("], \"by_level\": %d, \"count_by_level\": %d, \"level_cells\": %d, \"count_cells\": %d, "
@@ -68,19 +68,19 @@ def _runs(plan, planes):
     """Every run as (plane, first unit, units), as the walk kernel finds them."""
     kinds = plan["runs"]
     for run in range(plan["all_runs"]):
-        run0, plane0, each, unit0, log2 = kinds[0 if run < kinds[1][0] else 1 if run < kinds[2][0] else 2]
+        run0, plane0, each, unit0, log2 = kinds[sum(run >= kind[0] for kind in kinds[1:])]
         plane, nth = divmod(run - run0, each)
         yield plane0 + plane, unit0 + (nth << log2), 1 << log2
 
 
 # B, S, G, D, Q, L, K, offsets, softmax
 RUN_CALLS = [
-    (4, 21504, 8, 32, 21504, 3, 4, 0, 0),       # many runs per warp: long ones, the last planes' shorter
+    (4, 21504, 8, 32, 21504, 3, 4, 0, 0),       # many runs per warp: short ones in the last planes only
     (16, 21504, 8, 16, 21504, 3, 4, 0, 0),
     (2, 27750, 8, 32, 27750, 5, 4, 1, 1),
     (1, 20000, 1, 32, 250007, 2, 8, 0, 0),      # the same of one plane
     (8, 5376, 8, 32, 5376, 3, 4, 0, 0),
-    (3, 5376, 8, 32, 5376, 3, 4, 0, 0),         # few: long and short ones in every plane
+    (3, 5376, 8, 32, 5376, 3, 4, 0, 0),         # few: short ones in every plane
     (3, 11192, 6, 64, 11192, 3, 3, 1, 1),
     (16, 21504, 4, 64, 21504, 3, 4, 0, 0),      # 64 channels, many
     (2, 1344, 8, 32, 8192, 3, 8, 0, 0),         # hundreds of points per position
