@@ -16,6 +16,8 @@
 //      the nearest pixel inside, so no value is ever blended in from a clamped position)
 //      and accumulate in float32 with packed f32x2 FMAs;
 //   3. one 16-byte streaming store per lane: a warp writes a query's G*D row contiguously.
+// That is forward_kernel, which takes every call it is given.  Dense calls of 16-bit values take
+// forward_wide_kernel, 32 bytes per lane and shuffles instead of descriptors, where wide_pays() says so.
 #include "msda_common.cuh"
 
 // tuning knobs (compile-time): points whose corner loads are in flight together, and the
@@ -385,12 +387,16 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
 // all pixels are sampled often, L1 makes up for it; few queries far apart wait for L2 instead (us,
 // forward_kernel -> forward_wide_kernel: 900 queries on 17 821 positions, 8 samples 32 -> 39; 1 800, 16
 // samples 84 -> 87; 7 000 on 21 504, 8 samples 111 -> 109, 10 752 166 -> 158).  Of the dense calls the last
-// round of the persistent warps decides, 24 per SM here and 32 there: a round of this kernel takes
-// 1.38 times one of the other (12.2 against 8.8 us, 12 points of 32 channels), with offsets or a
-// softmax 1.25 times.  Rounds of either, us: 2 and 3, 26.8 -> 24.7; 3 and 4, 37 -> 37, offsets
-// of 64 channels 32.9 -> 30.9; 4 and 5, 46.2 -> 47.4, offsets 55.4 -> 53.9; 4 and 6, 57.9 -> 53.5.  Of many
-// rounds the last counts for little: 7 and 10, 86 -> 82; 8 and 11 (64 channels) 75.7 -> 69.8; 13 and 19, 164 -> 160.  16 channels gain throughout (22.7 -> 18.6 .. 129 -> 111).  float32 gains nothing (262
-// -> 273): its rows are whole lines of L1 either way.
+// round of the persistent warps decides, 24 per SM here and 32 there (what their launch bounds hold the
+// registers to): a round of this kernel takes 1.38 times one of the other (12.2 against 8.8 us, 12 points of
+// 32 channels), with offsets or a softmax 1.25 times.  Rounds of either, us: 2 and 3, 26.8 -> 24.7; 3 and 4,
+// 37 -> 37, offsets of 64 channels 32.9 -> 30.9; 4 and 5, 46.2 -> 47.4, offsets 55.4 -> 53.9; 4 and 6, 57.9 ->
+// 53.5.  Of many rounds the last counts for little: 7 and 10, 86 -> 82; 8 and 11 (64 channels) 75.7 -> 69.8; 13
+// and 19, 164 -> 160.  16 channels gain throughout (22.7 -> 18.6 .. 129 -> 111).  float32 gains nothing (262 ->
+// 273): its rows are whole lines of L1 either way.
+// Over 32, 64 and 128 channels, 3 to 24 points and 2 to 8 samples of 5 376 queries, what the rule picks is
+// never slower than forward_kernel by more than 2 % but once (128 channels, offsets, 3 and 4 rounds: 33.0 ->
+// 34.9); calls of 3 points that it keeps from this kernel would gain up to a quarter (18.5 -> 14.6).
 bool wide_pays(const Params &p, bool softmax_or_offsets) {
     const int64_t pairs = p.B * p.Q * p.G;
     if ((reinterpret_cast<uintptr_t>(p.value) & 31u) != 0 || 2 * p.Q < p.S || pairs >= (int64_t)1 << 31) return false;
