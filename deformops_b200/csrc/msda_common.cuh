@@ -718,6 +718,8 @@ __device__ __forceinline__ void finalize_image(const Params &p, const LevelTable
 
 // launchers implemented in msda_forward.cu / msda_backward.cu; dtype: 0 f32, 1 f16, 2 bf16
 cudaError_t launch_forward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
+// Whether a call of 16-bit values takes the forward kernel of 32-byte loads.
+bool forward_is_wide(const Params &p, bool softmax);
 cudaError_t launch_backward(const Params &p, int dtype, bool softmax, cudaStream_t stream);
 // The scaled backward in one launch, for calls that are bound by the host: what its scratch needs
 // beyond the usual is a header of its own.  (Forward + backward of a decoder layer, host bound, B200:

@@ -17,7 +17,7 @@
 //      and accumulate in float32 with packed f32x2 FMAs;
 //   3. one 16-byte streaming store per lane: a warp writes a query's G*D row contiguously.
 // That is forward_kernel, which takes every call it is given.  Dense calls of 16-bit values take
-// forward_wide_kernel, 32 bytes per lane and shuffles instead of descriptors, where wide_pays() says so.
+// forward_wide_kernel, 32 bytes per lane and shuffles instead of descriptors, where forward_is_wide() says so.
 #include "msda_common.cuh"
 
 // tuning knobs (compile-time): points whose corner loads are in flight together, and the
@@ -383,6 +383,12 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+// Up to four groups per SM a call lasts as long as one warp's chain of loads (launch_sized).
+constexpr int kSms = 148;
+bool small_call(const Params &p) { return p.num_groups <= 4 * kSms; }
+
+}  // namespace
+
 // 32-byte loads halve the warps of a call.  Where neighbouring queries sample neighbouring pixels, or
 // all pixels are sampled often, L1 makes up for it; few queries far apart wait for L2 instead (us,
 // forward_kernel -> forward_wide_kernel: 900 queries on 17 821 positions, 8 samples 32 -> 39; 1 800, 16
@@ -397,25 +403,26 @@ cudaError_t launch_as(const Params &p, cudaStream_t stream) {
 // Over 32, 64 and 128 channels, 3 to 24 points and 2 to 8 samples of 5 376 queries, what the rule picks is
 // never slower than forward_kernel by more than 2 % but once (128 channels, offsets, 3 and 4 rounds: 33.0 ->
 // 34.9); calls of 3 points that it keeps from this kernel would gain up to a quarter (18.5 -> 14.6).
-bool wide_pays(const Params &p, bool softmax_or_offsets) {
+bool forward_is_wide(const Params &p, bool softmax) {
+    if (small_call(p) || (p.D != 16 && p.D != 32 && p.D != 64 && p.D != 128)) return false;
     const int64_t pairs = p.B * p.Q * p.G;
     if ((reinterpret_cast<uintptr_t>(p.value) & 31u) != 0 || 2 * p.Q < p.S || pairs >= (int64_t)1 << 31) return false;
     if (p.D == 16) return true;
-    const int64_t wide = 148 * 24 * (512 / p.D), other = 148 * 32 * (256 / p.D);     // pairs of a round
+    const int64_t wide = kSms * 24 * (512 / p.D), other = kSms * 32 * (256 / p.D);     // pairs of a round
     const int64_t rounds = (pairs + wide - 1) / wide, other_rounds = (pairs + other - 1) / other;
     if (rounds > 6) return true;
-    return softmax_or_offsets ? 5 * rounds <= 4 * other_rounds : 18 * rounds <= 13 * other_rounds;
+    return softmax || p.ref != nullptr ? 5 * rounds <= 4 * other_rounds : 18 * rounds <= 13 * other_rounds;
 }
+
+namespace {
 
 template <typename T, bool SOFTMAX, bool REF>
 cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
-    // Up to four groups per SM the call lasts as long as one warp's chain of loads: more points in
-    // flight per warp, and as few warps per CTA as still reach every SM.  Measured on B200, a
-    // decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in flight 6.1, 6 6.6;
-    // of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
-    constexpr int kSms = 148;
+    // Small calls: more points in flight per warp, and as few warps per CTA as still reach every SM.
+    // Measured on B200, a decoder's 300 queries of 16 points, kernel: 8.1 us against 6.3 (8 points in
+    // flight 6.1, 6 6.6; of 12 points 6.9 against 6.0, 6.4, 5.9); nine groups per SM, 7.4 us, gain nothing.
     if constexpr (sizeof(T) == 2) {
-        if (p.num_groups > 4 * kSms && wide_pays(p, SOFTMAX || REF)) {
+        if (forward_is_wide(p, SOFTMAX)) {
             switch (p.D) {
                 case 16: return launch_wide<T, SOFTMAX, REF, 1>(p, stream);
                 case 32: return launch_wide<T, SOFTMAX, REF, 2>(p, stream);
@@ -424,7 +431,7 @@ cudaError_t launch_sized(const Params &p, cudaStream_t stream) {
             }
         }
     }
-    if (p.num_groups > 4 * kSms)
+    if (!small_call(p))
         return p.B * p.Q * p.G < (int64_t)1 << 31 ? launch_as<T, SOFTMAX, REF, false, unsigned>(p, stream)
                                                   : launch_as<T, SOFTMAX, REF, false, int64_t>(p, stream);
     Params q = p;

@@ -18,7 +18,7 @@ from tests._golden import rel_err
 
 pytestmark = pytest.mark.gpu
 
-# levels, B, Q, G, D, K, dtype, softmax, reference coordinates (0: locations)
+# levels, B, Q, G, D, K, dtype, softmax, reference coordinates (0: locations; below 0: offsets in float32)
 CASES = [
     ([(19, 23), (5, 7), (1, 1)], 3, 1001, 4, 16, 1, torch.float16, False, 0),      # 3 points, 1 lane a slot
     ([(19, 23), (5, 7)], 3, 1001, 4, 16, 3, torch.bfloat16, True, 2),              # 6 points, two a lane
@@ -31,6 +31,13 @@ CASES = [
     # offsets divided by sizes that have no exact reciprocal: the other kernel divides
     ([(49, 33), (1021, 3), (11, 107), (7, 1)], 3, 6251, 5, 32, 2, torch.float16, False, 2),
     ([(83, 41), (3, 347), (25, 13)], 2, 12501, 3, 64, 1, torch.float16, True, 2),
+    # two points a lane in one load: locations; float32 offsets
+    ([(19, 23), (5, 7)], 3, 1001, 4, 16, 2, torch.float16, False, 0),
+    ([(19, 23), (5, 7)], 3, 1001, 4, 16, 3, torch.bfloat16, True, 0),
+    ([(19, 23), (5, 7)], 3, 1001, 4, 16, 2, torch.float16, True, -2),
+    ([(31, 17), (9, 4), (3, 2)], 3, 6251, 5, 32, 2, torch.bfloat16, False, -4),
+    ([(12, 50), (6, 25)], 2, 12345, 3, 128, 5, torch.float16, True, 2),           # slots of eight, 10 points
+    ([(12, 50), (6, 25)], 2, 12345, 3, 128, 3, torch.bfloat16, True, -2),
 ]
 
 
@@ -47,8 +54,9 @@ def test_wide_forward_matches_the_oracle(levels, B, Q, G, D, K, dtype, softmax, 
     sh, st = dev(shapes), dev(starts)
     wh = torch.tensor(shapes[:, ::-1].copy(), dtype=torch.float32).view(1, 1, 1, L, 1, 2)
     if coords:
+        offsets = (2 * torch.randn(B, Q, G, L, K, 2, generator=gen)).to(dtype if coords > 0 else torch.float32)
+        coords = abs(coords)
         ref = torch.rand(B, Q, L, coords, generator=gen)
-        offsets = (2 * torch.randn(B, Q, G, L, K, 2, generator=gen)).to(dtype)
         r = ref.view(B, Q, 1, L, 1, coords)
         loc = (r + offsets.float() / wh if coords == 2
                else r[..., :2] + offsets.float() / K * r[..., 2:] * 0.5)

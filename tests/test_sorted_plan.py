@@ -3,14 +3,9 @@ from the call's shape alone: a small program linked to the library prints it."""
 
 from __future__ import annotations
 
-import json
-import pathlib
-import shutil
-import subprocess
-
 import pytest
 
-from deformops_b200._build import LIB_PATH, NVCC_FLAGS, CSRC, build_library
+from tests._host_program import host_program
 
 PROGRAM = r"""
 #include <cstdio>
@@ -44,24 +39,7 @@ int main(int argc, char **argv) {
 @pytest.fixture(scope="module")
 def plans(tmp_path_factory):
     """``plans(call, ...)``: a plan per ``(B, S, G, D, Q, L, K, offsets, softmax)``."""
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    if not pathlib.Path(nvcc).exists():
-        pytest.skip("nvcc not installed")
-    build_library()
-    where = tmp_path_factory.mktemp("plan")
-    source, program = where / "plan.cu", where / "plan"
-    source.write_text(PROGRAM)
-    done = subprocess.run([nvcc, *NVCC_FLAGS, f"-I{CSRC}", str(source), "-o", str(program), str(LIB_PATH),
-                           "-Xlinker", f"-rpath={LIB_PATH.parent}"], capture_output=True, text=True)
-    assert done.returncode == 0, done.stderr
-
-    def run(*calls):
-        done = subprocess.run([str(program), *[str(int(x)) for call in calls for x in call]],
-                              capture_output=True, text=True)
-        assert done.returncode == 0, done.stderr
-        return [json.loads(line) for line in done.stdout.splitlines()]
-
-    return run
+    return host_program(PROGRAM, tmp_path_factory.mktemp("plan"))
 
 
 def _runs(plan, planes):
