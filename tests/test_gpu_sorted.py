@@ -310,3 +310,18 @@ def test_threads_with_different_planes_do_not_limit_each_other():
         [t.start() for t in threads]
         [t.join() for t in threads]
     assert not failed, (len(failed), failed[0])
+
+
+def test_a_pixel_that_collects_tens_of_thousands_of_points():
+    """A level of one pixel beside a large one, gradients of one sign: no plane's sums may meet in float16 more often
+    than runs of 256 points make them.  A sum of n equal terms, rounded as it grows, is at most n / 2 times half a
+    unit off at its end."""
+    levels, B, Q, G, D, K = [(125, 100), (1, 1)], 3, 20011, 5, 16, 4
+    value, shapes, starts, loc, logits, grad_out = _inputs(13, B, Q, G, D, K, levels)
+    dtype = torch.float16
+    v, a, go = dev(value, dtype), dev(logits.softmax(-1), dtype), dev(torch.ones_like(grad_out), dtype)
+    l, sh, st = dev(loc, torch.float32), dev(shapes), dev(starts)
+    got = to_np(_workspace_backward(v, sh, st, l, a, go, False)[0])[:, -1]
+    truth = orc.backward(*[t.cpu() for t in (v, sh, st, l, a)], go.cpu(), softmax=False)[0][:, -1]
+    error = abs(got / truth - 1).max(-1)
+    assert error.max() <= Q * K / 256 / 2 * 2.0 ** -12, error
