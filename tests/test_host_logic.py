@@ -375,3 +375,43 @@ def test_quotients_by_level_sizes_round_as_a_division():
         remainder = rounded(Fraction(float(x)) - Fraction(float(q)) * int(n))
         got = rounded(Fraction(float(remainder)) * Fraction(float(rcp)) + Fraction(float(q)))
         assert got == x / n, (x, n)
+
+
+def test_quotients_next_to_rounding_boundaries():
+    """The same by larger odd n, up to 2^24, for the x that bring the quotient within 3 / (2 n) units of the middle
+    between two floats: x 2^k = m n + d for an odd m of 25 bits and a small d."""
+    from fractions import Fraction
+
+    import numpy as np
+
+    rng = np.random.default_rng(4)
+    f32 = np.float32
+
+    def rounded(v):                       # nearest float32 of an exact value in the normal range
+        near = f32(float(v))
+        around = [near, np.nextafter(near, f32(np.inf)), np.nextafter(near, f32(-np.inf))]
+        best = min(abs(Fraction(float(c)) - v) for c in around)
+        ties = [c for c in around if abs(Fraction(float(c)) - v) == best]
+        return ties[0] if len(ties) == 1 else next(c for c in ties if int(c.view(np.uint32)) % 2 == 0)
+
+    seen = 0
+    for bits in (20, 21, 22, 23):
+        # (where the reciprocal can be furthest off, and anywhere)
+        numbers = [2 ** (bits + 1) - 1 - 2 * i for i in range(100)]
+        numbers += [int(i) | 1 for i in rng.integers(2 ** bits, 2 ** (bits + 1), 100)]
+        for n in numbers:
+            for k in (bits + 1, bits + 2):
+                for d in (-3, -1, 1, 3):
+                    m = -d * pow(n, -1, 2 ** k) % 2 ** k
+                    while m < 2 ** 24:
+                        m += 2 ** k
+                    x = (m * n + d) >> k
+                    if m >= 2 ** 25 or not 2 ** 23 <= x < 2 ** 24:
+                        continue
+                    x, size = f32(x) * f32(2.0 ** -23), f32(n)
+                    rcp = f32(1) / size
+                    q = x * rcp
+                    remainder = rounded(Fraction(float(x)) - Fraction(float(q)) * n)
+                    assert rounded(Fraction(float(remainder)) * Fraction(float(rcp)) + Fraction(float(q))) == x / size
+                    seen += 1
+    assert seen > 500
