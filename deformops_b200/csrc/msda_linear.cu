@@ -67,7 +67,9 @@ __global__ void __launch_bounds__(kThreads) column_partials_kernel(const T *__re
 }
 
 // Bound by latency: every thread has all its parts in flight (at most 296 over 32 rows of threads; 4.5 us
-// -> 3.4 against 8 rows and five round trips), and the kernel is launched while the sums are formed.
+// -> 3.4 against 8 rows and five round trips), and the kernel is launched while the sums are formed.  Small
+// matrices too: that launch costs the host no more than another (both sums, us a call, called in a row: 300 x 256
+// 8.2 -> 5.6, 3 600 x 256 8.2 -> 6.1, 43 008 x 256 10.3 -> 8.2; host 6.5 .. 6.9 -> 5.5 .. 6.0).
 constexpr int kFinishRows = 32;
 template <typename T>
 __global__ void __launch_bounds__(kFinishRows * 32) column_finish_kernel(const float *__restrict__ partial,
