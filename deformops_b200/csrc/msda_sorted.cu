@@ -945,8 +945,8 @@ __device__ __forceinline__ void flush_row(float (&acc)[D / 8][4], int half, floa
 }
 
 // What bounds the walk is the latency of a step's chain beside the SM's load/store pipe, about five of its
-// cycles a point (ncu, the headline shape: 67 % busy while the SM works, issue slots 49 %, tensor cores
-// 30 %): without the two stores per point to addresses of their own the call takes 364 us instead of 398,
+// cycles a point (ncu, the headline shape: 63 % busy while the SM works, issue slots 47 %, tensor cores
+// 29 %): without the two stores per point to addresses of their own the call takes 364 us instead of 398,
 // the rest goes through shared memory.  Hence the weights' way over the tensor cores below.  More warps do
 // not help - 12, 16, 20, 24 per SM: 252, 246, 261, 312 us when this kernel took 246 - nor did having grad_out
 // rows in registers instead of shared memory (300 us), or the next cell's value row early (257 us).
